@@ -240,28 +240,53 @@ __global__ void __launch_bounds__(128) grouped_gemm_kernel(GroupGemmParams p) {
   }
 }
 
-// The tile list of rows sorted by group, every group's run padded to whole tiles: from the groups'
+// The tile list of rows sorted by group, every group's run padded to whole tiles of `tile_rows`: from the groups'
 // row counts.  start[g]: first row of group g's run; tiles[i] = (group, first row, rows), idle
-// entries (group -1) up to max_tiles.  One thread: a few hundred entries at most.
-__global__ void run_tiles_kernel(const int32_t* __restrict__ counts, int groups, int max_tiles,
-                                 int32_t* __restrict__ start, int32_t* __restrict__ tiles) {
+// entries (group -1) up to max_tiles.  One block: a thread a group, a scan over the groups' tile counts
+// instead of one thread walking over all of them.
+constexpr int TILES_THREADS = 256;
+
+__global__ void __launch_bounds__(TILES_THREADS) run_tiles_kernel(const int32_t* counts, int groups,
+                                                                  int max_tiles, int tile_rows,
+                                                                  int32_t* start,
+                                                                  int32_t* tiles) {
+  __shared__ int warp_tot[TILES_THREADS / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_launch_dependents();
   pdl_wait();
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int row = 0, n = 0;
-  for (int g = 0; g < groups; ++g) {
-    start[g] = row;
-    for (int left = counts[g]; left > 0 && n < max_tiles; left -= GG_BM, ++n) {
-      tiles[n * 3] = g;
-      tiles[n * 3 + 1] = row;
-      tiles[n * 3 + 2] = left < GG_BM ? left : GG_BM;
-      row += GG_BM;
+  int base = 0;                         // tiles of the groups before this round's
+  for (int g0 = 0; g0 < groups; g0 += TILES_THREADS) {
+    const int g = g0 + threadIdx.x;
+    const int rows = g < groups ? counts[g] : 0;
+    const int own = (rows + tile_rows - 1) / tile_rows;
+    int upto = own;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += n;
     }
+    if (lane == 31) warp_tot[warp] = upto;
+    __syncthreads();
+    int first = base + upto - own;
+#pragma unroll
+    for (int w = 0; w < TILES_THREADS / 32; ++w) {
+      if (w < warp) first += warp_tot[w];
+      base += warp_tot[w];
+    }
+    // a list that is too short cuts the runs off where it ends
+    if (g < groups) start[g] = min(first, max_tiles) * tile_rows;
+    for (int j = 0; j < own && first + j < max_tiles; ++j) {
+      int32_t* tile = tiles + 3 * (first + j);
+      tile[0] = g;
+      tile[1] = (first + j) * tile_rows;
+      tile[2] = min(tile_rows, rows - j * tile_rows);
+    }
+    __syncthreads();                    // warp_tot is written again
   }
-  for (; n < max_tiles; ++n) {
-    tiles[n * 3] = -1;
-    tiles[n * 3 + 1] = 0;
-    tiles[n * 3 + 2] = 0;
+  for (int i = min(base, max_tiles) + threadIdx.x; i < max_tiles; i += TILES_THREADS) {
+    tiles[3 * i] = -1;
+    tiles[3 * i + 1] = 0;
+    tiles[3 * i + 2] = 0;
   }
 }
 }  // namespace
@@ -287,9 +312,10 @@ PBE_EXPORT int pbe_grouped_gemm(const void* a, int a_dtype, int lda, long long a
   return launch_status();
 }
 
-PBE_EXPORT int pbe_run_tiles(const int32_t* counts, int groups, int max_tiles, int32_t* start, int32_t* tiles,
-                             cudaStream_t stream) {
+PBE_EXPORT int pbe_run_tiles(const int32_t* counts, int groups, int max_tiles, int tile_rows, int32_t* start,
+                             int32_t* tiles, cudaStream_t stream) {
   if (groups <= 0 || max_tiles <= 0) return 0;
-  launch_k(run_tiles_kernel, 1, 32, 0, stream, counts, groups, max_tiles, start, tiles);
+  if (tile_rows <= 0) return (int)cudaErrorInvalidValue;
+  launch_k(run_tiles_kernel, 1, TILES_THREADS, 0, stream, counts, groups, max_tiles, tile_rows, start, tiles);
   return launch_status();
 }

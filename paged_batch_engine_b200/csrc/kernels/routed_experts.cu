@@ -338,68 +338,142 @@ __global__ void combine_kernel(const float* __restrict__ part, const T* __restri
 // (count_kernel), then the runs' starts on the host or by a scan, then place_kernel hands the
 // places out in (t, k) order inside every expert's run: a single block walks the pairs of an
 // expert in order, so the order inside a run is the tokens' own and nothing depends on timing.
-__global__ void place_kernel(const int32_t* __restrict__ chosen, int pairs, int E, int32_t* __restrict__ counts,
-                             int32_t* __restrict__ place) {
-  // block e: places of the pairs that chose expert e, in pair order
-  __shared__ int base;
-  __shared__ int warp_tot[32];
+// Block e reads all pairs, a thread PLACE_PER neighbouring ones: each counts its own, one scan over the block turns
+// the counts into places.  8,192 pairs, 32 experts: 21.9 us with a pair a thread and three barriers for every 256
+// pairs, about 6 now.
+// (No __restrict__ on what a kernel before wrote: these kernels are resident before that one has ended, and loads that
+// may be taken for read-only are not ordered behind the wait.)
+constexpr int PLACE_THREADS = 512, PLACE_PER = 16;
+
+__global__ void __launch_bounds__(PLACE_THREADS) place_kernel(const int32_t* chosen, int pairs, int E,
+                                                              int32_t* counts, int32_t* place) {
+  __shared__ int warp_tot[PLACE_THREADS / 32];
   const int e = blockIdx.x;
-  if (threadIdx.x == 0) base = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
-  for (int i0 = 0; i0 < pairs; i0 += blockDim.x) {
-    const int i = i0 + threadIdx.x;
-    const bool mine = i < pairs && chosen[i] == e;
-    const unsigned ballot = __ballot_sync(0xffffffffu, mine);
-    if (lane == 0) warp_tot[warp] = __popc(ballot);
-    __syncthreads();
-    int before = base;
-    for (int w = 0; w < warp; ++w) before += warp_tot[w];
-    if (mine) place[i] = before + __popc(ballot & ((1u << lane) - 1u));
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int tot = 0;
-      for (int w = 0; w < warps; ++w) tot += warp_tot[w];
-      base += tot;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  pdl_launch_dependents();
+  pdl_wait();
+  const bool aligned = ((uintptr_t)chosen & 15) == 0;      // then every sixteenth pair lies on a 16-byte boundary
+  int base = 0;
+  for (long long first = 0; first < pairs; first += PLACE_THREADS * PLACE_PER) {
+    const long long i0 = first + (long long)threadIdx.x * PLACE_PER;
+    unsigned mine = 0;                       // bit j: pair i0 + j chose this block's expert
+    if (aligned && i0 + PLACE_PER <= pairs) {
+#pragma unroll
+      for (int j = 0; j < PLACE_PER; j += 4) {
+        const int4 c = *reinterpret_cast<const int4*>(chosen + i0 + j);
+        mine |= (unsigned)(c.x == e) << j | (unsigned)(c.y == e) << (j + 1) | (unsigned)(c.z == e) << (j + 2) |
+                (unsigned)(c.w == e) << (j + 3);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < PLACE_PER; ++j)
+        if (i0 + j < pairs) mine |= (unsigned)(chosen[i0 + j] == e) << j;
     }
+    int upto = __popc(mine);                 // inclusive scan: of the warp, then of the block
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int n = __shfl_up_sync(0xffffffffu, upto, o);
+      if (lane >= o) upto += n;
+    }
+    if (lane == 31) warp_tot[warp] = upto;
     __syncthreads();
+    int at = base + upto - __popc(mine);
+#pragma unroll
+    for (int w = 0; w < PLACE_THREADS / 32; ++w) {
+      if (w < warp) at += warp_tot[w];
+      base += warp_tot[w];
+    }
+    for (unsigned left = mine; left; left &= left - 1) place[i0 + __ffs(left) - 1] = at++;
+    __syncthreads();                         // warp_tot is written again
   }
   if (threadIdx.x == 0) counts[e] = base;
 }
 
-// gathered[start[e] + place] = x[t] for every pair; and the way back, weighted:
-template <typename T>
-__global__ void gather_rows_kernel(const T* __restrict__ x, const int32_t* __restrict__ chosen,
-                                   const int32_t* __restrict__ place, const int32_t* __restrict__ start,
-                                   const float* __restrict__ weights, T* __restrict__ gathered, int top, int W) {
+// gathered[start[e] + place] = x[t] for every pair; and the way back, weighted.  VEC values a thread and access
+// (eight bfloat16 or four floats where the rows lie on 16-byte boundaries): the sum of 8,192 rows of 2,048 bfloat16
+// values into 2,048 took 23.7 us with a value a thread, 12.3 now.
+template <typename T, int VEC>
+struct __align__(sizeof(T) * VEC) RowPiece {
+  T v[VEC];
+};
+
+template <typename T, int VEC>
+__global__ void gather_rows_kernel(const T* x, const int32_t* chosen,
+                                   const int32_t* place, const int32_t* start,
+                                   const float* weights, T* gathered, int top, int W) {
+  using P = RowPiece<T, VEC>;
+  pdl_launch_dependents();
+  pdl_wait();
   const int pair = blockIdx.x;
-  const int t = pair / top;
-  const size_t dst = (size_t)(start[chosen[pair]] + place[pair]) * W;
-  if (weights) {
-    const float f = weights[pair];
-    for (int i = threadIdx.x; i < W; i += blockDim.x)
-      gathered[dst + i] = from_float<T>(f * to_float(x[(size_t)t * W + i]));
-    return;
+  const P* src = reinterpret_cast<const P*>(x + (size_t)(pair / top) * W);
+  P* dst = reinterpret_cast<P*>(gathered + (size_t)(start[chosen[pair]] + place[pair]) * W);
+  const float f = weights ? weights[pair] : 1.0f;
+  for (int i = threadIdx.x; i < W / VEC; i += blockDim.x) {
+    P p = src[i];
+    if (weights) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) p.v[j] = from_float<T>(f * to_float(p.v[j]));
+    }
+    dst[i] = p;
   }
-  for (int i = threadIdx.x; i < W; i += blockDim.x) gathered[dst + i] = x[(size_t)t * W + i];
+}
+
+template <typename T, int VEC>
+__global__ void scatter_rows_kernel(const T* y, const int32_t* chosen,
+                                    const int32_t* place, const int32_t* start,
+                                    const float* weights, const T* addend,
+                                    const float* gate, int ld_gate, T* out, int top, int W) {
+  using P = RowPiece<T, VEC>;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int t = blockIdx.x;
+  const float factor = addend_factor(gate, ld_gate, t);
+  for (int i = threadIdx.x; i < W / VEC; i += blockDim.x) {
+    float a[VEC];
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) a[j] = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < top; ++k) {
+      const int pair = t * top + k;
+      const float f = weights ? weights[pair] : 1.0f;
+      const P p = reinterpret_cast<const P*>(y + (size_t)(start[chosen[pair]] + place[pair]) * W)[i];
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) a[j] += f * to_float(p.v[j]);
+    }
+    if (addend) {
+      const P p = reinterpret_cast<const P*>(addend + (size_t)t * W)[i];
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) a[j] = fmaf(factor, to_float(p.v[j]), a[j]);
+    }
+    P o;
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) o.v[j] = from_float<T>(a[j]);
+    reinterpret_cast<P*>(out + (size_t)t * W)[i] = o;
+  }
+}
+
+inline bool on_16_bytes(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+template <typename T>
+void gather_rows(const void* x, const int32_t* chosen, const int32_t* place, const int32_t* start, const float* weights,
+                 void* gathered, int T_, int top, int W, cudaStream_t stream) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  if (W % VEC == 0 && on_16_bytes(x) && on_16_bytes(gathered))
+    launch_k(gather_rows_kernel<T, VEC>, T_ * top, 128, 0, stream, (const T*)x, chosen, place, start, weights, (T*)gathered, top, W);
+  else
+    launch_k(gather_rows_kernel<T, 1>, T_ * top, 128, 0, stream, (const T*)x, chosen, place, start, weights, (T*)gathered, top, W);
 }
 
 template <typename T>
-__global__ void scatter_rows_kernel(const T* __restrict__ y, const int32_t* __restrict__ chosen,
-                                    const int32_t* __restrict__ place, const int32_t* __restrict__ start,
-                                    const float* __restrict__ weights, const T* __restrict__ addend,
-                                    const float* __restrict__ gate, int ld_gate, T* __restrict__ out, int top, int W) {
-  const int t = blockIdx.x;
-  const float factor = addend_factor(gate, ld_gate, t);
-  for (int i = threadIdx.x; i < W; i += blockDim.x) {
-    float a = 0.f;
-    for (int k = 0; k < top; ++k) {
-      const int pair = t * top + k;
-      a += (weights ? weights[pair] : 1.0f) * to_float(y[(size_t)(start[chosen[pair]] + place[pair]) * W + i]);
-    }
-    if (addend) a = fmaf(factor, to_float(addend[(size_t)t * W + i]), a);
-    out[(size_t)t * W + i] = from_float<T>(a);
-  }
+void scatter_rows(const void* y, const int32_t* chosen, const int32_t* place, const int32_t* start, const float* weights,
+                  const void* addend, const float* gate, int ld_gate, void* out, int T_, int top, int W, cudaStream_t stream) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  if (W % VEC == 0 && on_16_bytes(y) && on_16_bytes(out) && on_16_bytes(addend))
+    launch_k(scatter_rows_kernel<T, VEC>, T_, 128, 0, stream, (const T*)y, chosen, place, start, weights, (const T*)addend,
+             gate, ld_gate, (T*)out, top, W);
+  else
+    launch_k(scatter_rows_kernel<T, 1>, T_, 128, 0, stream, (const T*)y, chosen, place, start, weights, (const T*)addend,
+             gate, ld_gate, (T*)out, top, W);
 }
 }  // namespace
 
@@ -456,7 +530,7 @@ PBE_EXPORT int pbe_expert_rows(const void* x, const void* w_gate, const void* w_
 PBE_EXPORT int pbe_expert_places(const int32_t* chosen, int pairs, int E, int32_t* counts, int32_t* place,
                                  cudaStream_t stream) {
   if (pairs <= 0) return 0;
-  place_kernel<<<E, 256, 0, stream>>>(chosen, pairs, E, counts, place);
+  launch_k(place_kernel, E, PLACE_THREADS, 0, stream, chosen, pairs, E, counts, place);
   return launch_status();
 }
 
@@ -464,11 +538,8 @@ PBE_EXPORT int pbe_expert_gather(const void* x, const int32_t* chosen, const int
                                  const float* weights, void* gathered, int dtype, int T, int top, int W,
                                  cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (dtype == PBE_F32)
-    gather_rows_kernel<float><<<T * top, 128, 0, stream>>>((const float*)x, chosen, place, start, weights, (float*)gathered, top, W);
-  else
-    gather_rows_kernel<__nv_bfloat16><<<T * top, 128, 0, stream>>>((const __nv_bfloat16*)x, chosen, place, start, weights,
-                                                                  (__nv_bfloat16*)gathered, top, W);
+  if (dtype == PBE_F32) gather_rows<float>(x, chosen, place, start, weights, gathered, T, top, W, stream);
+  else gather_rows<__nv_bfloat16>(x, chosen, place, start, weights, gathered, T, top, W, stream);
   return launch_status();
 }
 
@@ -476,12 +547,7 @@ PBE_EXPORT int pbe_expert_scatter(const void* y, const int32_t* chosen, const in
                                   const float* weights, void* out, int dtype, int T, int top, int W,
                                   const void* addend, const float* addend_gate, int ld_gate, cudaStream_t stream) {
   if (T <= 0) return 0;
-  if (dtype == PBE_F32)
-    scatter_rows_kernel<float><<<T, 128, 0, stream>>>((const float*)y, chosen, place, start, weights,
-                                                     (const float*)addend, addend_gate, ld_gate, (float*)out, top, W);
-  else
-    scatter_rows_kernel<__nv_bfloat16><<<T, 128, 0, stream>>>((const __nv_bfloat16*)y, chosen, place, start, weights,
-                                                             (const __nv_bfloat16*)addend, addend_gate, ld_gate,
-                                                             (__nv_bfloat16*)out, top, W);
+  if (dtype == PBE_F32) scatter_rows<float>(y, chosen, place, start, weights, addend, addend_gate, ld_gate, out, T, top, W, stream);
+  else scatter_rows<__nv_bfloat16>(y, chosen, place, start, weights, addend, addend_gate, ld_gate, out, T, top, W, stream);
   return launch_status();
 }

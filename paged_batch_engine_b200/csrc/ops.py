@@ -1950,16 +1950,16 @@ def grouped_heads(a: torch.Tensor, lda: int, head_stride: int, K: int, w: torch.
                     gate, rot, rot_dims, inv_freq, positions, rot_scale, gate_each)
 
 
-def run_tiles(counts: torch.Tensor, max_tiles: int):
+def run_tiles(counts: torch.Tensor, max_tiles: int, tile_rows: int = GROUP_TILE_ROWS):
     """(start int32 [G], tiles int32 [max_tiles, 3]) for rows sorted by group with every group's run
-    padded to whole tiles of ``GROUP_TILE_ROWS``: a group's first row, and per tile (group, first
-    row, rows), idle tiles with group -1."""
+    padded to whole tiles of ``tile_rows``: a group's first row, and per tile (group, first
+    row, rows), idle tiles with group -1 behind all others."""
     _need_cuda(counts)
     G = counts.numel()
     start = torch.empty(G, dtype=torch.int32, device=counts.device)
     tiles = torch.empty((max_tiles, 3), dtype=torch.int32, device=counts.device)
-    fn = _fn("grouped_gemm", "pbe_run_tiles", [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p])
-    _check(fn(_ptr(counts), G, int(max_tiles), _ptr(start), _ptr(tiles), _stream()), "run_tiles")
+    fn = _fn("grouped_gemm", "pbe_run_tiles", [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    _check(fn(_ptr(counts), G, int(max_tiles), int(tile_rows), _ptr(start), _ptr(tiles), _stream()), "run_tiles")
     return start, tiles
 
 
@@ -1974,6 +1974,44 @@ def grouped_runs(a: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, out_dtyp
         raise KernelError("grouped_runs: the weights are [G, N, K]")
     out = torch.empty((rows, N), dtype=out_dtype, device=a.device)
     return _grouped(a, K, 0, w, N * K, 1, K, out, N, 0, rows, K, N, G, tiles, tiles.shape[0], activation=activation)
+
+
+GROUPED_TC5_ROWS = 128       # rows of a tile of the tcgen05 form
+GROUPED_TC5_EPILOGUES = {None: 0, "relu2": 1, "silu": 2, "capped_swish": 3}
+
+
+def grouped_tc5_applies(x: torch.Tensor, *weights: torch.Tensor) -> bool:
+    """Whether the experts' products over these rows take the tcgen05 form: bfloat16 rows and matrices whose rows
+    lie on 16-byte boundaries (the TMA unit's rule)."""
+    return x.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 and w.shape[2] % 8 == 0 and w.data_ptr() % 16 == 0
+                                             for w in weights)
+
+
+def grouped_runs_tc5(a: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, activation: Optional[str] = None,
+                     limit: float = 0.0, alpha: float = 1.0) -> torch.Tensor:
+    """``grouped_runs`` on tcgen05 (``tiles`` of ``GROUPED_TC5_ROWS`` rows, bfloat16 result), with the activation as
+    the epilogue: "relu2" squares the relu; "silu" and "capped_swish" take ``w`` [G, 2 * I, K] as gate rows followed
+    by up rows and give [rows, I] as ``gated_activation`` does."""
+    _need_cuda(a, w, tiles)
+    _need_contiguous(a, w, tiles)
+    rows, K = a.shape
+    G, N, _ = w.shape
+    if w.shape[2] != K or not grouped_tc5_applies(a, w):
+        raise KernelError("grouped_runs_tc5: bfloat16 rows [rows, K] and weights [G, N, K], K a multiple of eight")
+    if activation not in GROUPED_TC5_EPILOGUES:
+        raise KernelError(f"grouped_runs_tc5: no epilogue {activation!r}")
+    kind = GROUPED_TC5_EPILOGUES[activation]
+    if kind >= 2 and N % 2:
+        raise KernelError("grouped_runs_tc5: a gated product has as many gate rows as up rows")
+    out = torch.empty((rows, N // 2 if kind >= 2 else N), dtype=a.dtype, device=a.device)
+    err = _tc5_err.get(a.device)
+    if err is None:
+        err = _tc5_err[a.device] = torch.zeros(1, dtype=torch.int32, device=a.device)
+    fn = _fn("grouped_tc5", "pbe_grouped_tc5", [c_void_p] * 3 + [c_int] * 4 + [c_void_p, c_int, c_int, c_float, c_float,
+                                                                             c_void_p, c_void_p])
+    _check(fn(_ptr(a), _ptr(w), _ptr(out), rows, K, N, G, _ptr(tiles), tiles.shape[0], kind, float(limit), float(alpha),
+              _ptr(err), _stream()), "grouped_runs_tc5")
+    return out
 
 
 # ------------------------------------------------------------------ norms with one learned number, mix over depth

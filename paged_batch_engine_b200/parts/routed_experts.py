@@ -86,7 +86,7 @@ class RoutedExperts(FeedForward):
                                             tensor_names=dict(up="up", down="down"), weight_suffix="")
 
     def kernel_libraries(self, dtype):
-        tiled = [("grouped_gemm", None)] if dtype == torch.bfloat16 else []
+        tiled = [("grouped_gemm", None), ("grouped_tc5", None)] if dtype == torch.bfloat16 else []
         shared = self.shared.kernel_libraries(dtype) if self.shared is not None else []
         return [("routed_experts", None), ("elementwise", None)] + tiled + ops.gemm_libraries(dtype) + shared
 
@@ -153,10 +153,16 @@ class RoutedExperts(FeedForward):
         launch per projection that multiplies every tile with its expert's matrix on the tensor
         cores.  Nothing is read on the host."""
         T = x.shape[0]
+        tc5 = ops.grouped_tc5_applies(x, self.w_gate_up, self.w_down)
+        tile_rows = ops.GROUPED_TC5_ROWS if tc5 else ops.GROUP_TILE_ROWS
         counts, place = ops.expert_places(chosen, self.num_experts)
-        max_tiles = (T * self.top + ops.GROUP_TILE_ROWS - 1) // ops.GROUP_TILE_ROWS + self.num_experts
-        start, tiles = ops.run_tiles(counts, max_tiles)
-        rows, weights = self._gathered(x, chosen, place, start, weights, total_rows=max_tiles * ops.GROUP_TILE_ROWS)
+        max_tiles = (T * self.top + tile_rows - 1) // tile_rows + self.num_experts
+        start, tiles = ops.run_tiles(counts, max_tiles, tile_rows)
+        rows, weights = self._gathered(x, chosen, place, start, weights, total_rows=max_tiles * tile_rows)
+        if tc5:
+            hidden = ops.grouped_runs_tc5(rows, self.w_gate_up, tiles, self.activation, self.limit, self.alpha)
+            out = ops.grouped_runs_tc5(hidden, self.w_down, tiles)
+            return ops.expert_scatter(out, chosen, place, start, weights, T, **shared)
         if self.gated:
             gu = ops.grouped_runs(rows, self.w_gate_up, tiles, self.dtype)
             hidden = torch.empty((rows.shape[0], self.intermediate_size), dtype=self.dtype, device=x.device)
