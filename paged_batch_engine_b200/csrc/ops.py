@@ -565,6 +565,52 @@ def pooled_attention(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, num_tiles: in
     return out
 
 
+POOLED_MMA_ROWS = 16        # rows of a tile of the tensor-core form
+
+
+def _pm_defines(key_dim: int, value_dim: int) -> dict:
+    return {"PBE_PM_D": int(key_dim), "PBE_PM_E": int(value_dim)}
+
+
+def pooled_mma_applies(dtype: torch.dtype, heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether the tensor-core form of the pooled attention is built for these sizes (a warp a head, sixteen at
+    most; head widths in whole steps of the products)."""
+    return dtype == torch.bfloat16 and heads <= 16 and all(d % 16 == 0 and d <= 128 for d in (key_dim, value_dim))
+
+
+def pooled_mma_fits(heads: int, kv_heads: int, key_dim: int, value_dim: int) -> bool:
+    """Whether its tiles of all key/value heads fit a block's shared memory."""
+    fn = _fn("pooled_attention_mma", "pbe_pooled_attention_mma_keys", [c_int, c_int], _pm_defines(key_dim, value_dim))
+    return fn(int(heads), int(kv_heads)) > 0
+
+
+def pooled_attention_mma(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, num_tiles: int, q_start, q_len, seq_len, bt_tok,
+                         bt_pool, heads: int, kv_heads: int, scale: float, window: int, pool: int,
+                         page_tokens: int) -> torch.Tensor:
+    """``pooled_attention`` on the tensor cores, over row tiles of ``POOLED_MMA_ROWS`` (bfloat16, sizes for which
+    ``pooled_mma_applies`` and ``pooled_mma_fits`` hold)."""
+    _need_cuda(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, q_start, q_len, seq_len, bt_tok, bt_pool)
+    _need_contiguous(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, q_start, q_len, seq_len, bt_tok, bt_pool)
+    T = q.shape[0]
+    D, E = k_tok.shape[3], v_tok.shape[3]
+    if q.shape[1] != heads * D or k_tok.shape[1] != kv_heads or any(
+            x is not None and x.dtype != torch.bfloat16 for x in (q, k_tok, v_tok, k_pool, v_pool)):
+        raise KernelError("pooled_attention_mma: shapes or dtypes do not agree")
+    if talk is not None and (talk.dtype != torch.float32 or tuple(talk.shape) != (heads, heads)):
+        raise KernelError("pooled_attention_mma: the mixing matrix is float32 [heads, heads]")
+    if pool and (k_pool is None or bt_pool is None):
+        raise KernelError("pooled_attention_mma: pooled blocks need their pages and block table")
+    out = torch.empty((T, heads * E), dtype=q.dtype, device=q.device)
+    fn = _fn("pooled_attention_mma", "pbe_pooled_attention_mma",
+             [c_void_p] * 8 + [c_int] + [c_void_p] * 4 + [c_int, c_void_p, c_int] + [c_int] * 5 + [c_float, c_void_p],
+             _pm_defines(D, E))
+    _check(fn(_ptr(q), _ptr(k_tok), _ptr(v_tok), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(talk), _ptr(tiles), num_tiles,
+              _ptr(q_start), _ptr(q_len), _ptr(seq_len), _ptr(bt_tok), bt_tok.shape[1], _ptr(bt_pool),
+              bt_pool.shape[1] if bt_pool is not None else 0, heads, kv_heads, page_tokens, int(window), int(pool or 0),
+              float(scale), _stream()), "pooled_attention_mma")
+    return out
+
+
 # ------------------------------------------------------------------ rope + cache write
 def rope_kv_write(qkv: torch.Tensor, bias: Optional[torch.Tensor], q_out: torch.Tensor,
                   k_cache: Optional[torch.Tensor], v_cache: Optional[torch.Tensor],

@@ -63,6 +63,7 @@ class PooledWindowAttention(Mixer):
             self.rotary_dim = dims
         self.w_qkv = self.w_o = self.q_gain = self.k_gain = self.talk = None
         self._tile_rows = None
+        self._mma = False         # whether prompt portions take the tensor-core form (known once the kernels are loaded)
 
     # ---- what it keeps
     def cache_need(self):
@@ -76,7 +77,9 @@ class PooledWindowAttention(Mixer):
         return CompositeNeed.of(tokens=tokens, pooled=PagedNeed(pair, window=None, stride=self.pool))
 
     def kernel_libraries(self, dtype):
-        return [("pooled_attention", {"PBE_PA_F32": 1 if dtype == torch.float32 else 0})] + ops.gemm_libraries(dtype)
+        mma = [("pooled_attention_mma", ops._pm_defines(self.key_dim, self.value_dim))] \
+            if ops.pooled_mma_applies(dtype, self.num_heads, self.key_dim, self.value_dim) else []
+        return [("pooled_attention", {"PBE_PA_F32": 1 if dtype == torch.float32 else 0})] + mma + ops.gemm_libraries(dtype)
 
     # ---- tensors
     def param_specs(self, prefix):
@@ -124,8 +127,21 @@ class PooledWindowAttention(Mixer):
                                 bt_pool, self.pool, ctx.page_tokens)
         if self._tile_rows is None:
             self._tile_rows = ops.pooled_attention_tile_rows(H, E, 16, self.dtype)
+            self._mma = ops.pooled_mma_applies(self.dtype, H, D, E) and ops.pooled_mma_fits(H, G, D, E)
         # decoded tokens only (always so in a captured step): a row a tile
         single = getattr(ctx, "captured", False) or int(ctx.q_len_host.max(initial=1)) == 1
+        # Prompt portions take the tensor-core form, whose blocks walk all keys of sixteen rows (25 us and 0.24 us a
+        # key).  A short portion behind a long context leaves most of the GPU idle that way: there the split form is
+        # ahead (1,088 keys: 24 rows 131 against 270 us, 48 rows 227 / 262, 96 rows 331 / 267; up to 400 keys it never
+        # is).
+        longest = int(ctx.seq_len_host.max(initial=1))
+        seen = min(longest, self.window + ops.POOLED_MMA_ROWS) + (longest // self.pool if self.pool else 0)
+        if self._mma and not single and (ctx.num_tokens >= 64 or seen <= 400):
+            tiles, n_tiles = ctx.row_tiles(ops.POOLED_MMA_ROWS)
+            out = ops.pooled_attention_mma(q, tok.k, tok.v, k_pool, v_pool, self.talk, tiles, n_tiles, ctx.q_start,
+                                           ctx.q_len, ctx.seq_len, gt.block_table, bt_pool, H, G, self.scale,
+                                           self.window, self.pool, ctx.page_tokens)
+            return ops.linear(out, self.w_o, None, out_dtype=self.dtype, kind=2)
         rows = 1 if single else self._tile_rows
         tiles, n_tiles = ctx.row_tiles(rows)
         # few row tiles (decoded tokens, short portions): the keys are split over more blocks; a
