@@ -25,7 +25,8 @@
 //    k staged in shared memory k-major through registers (the next tile's loads are in flight
 //    while this one is multiplied), slice sums in registers, the running totals in shared
 //    memory (they are touched once per slice), which leaves room for two blocks a
-//    multiprocessor.  With few output tiles the slices become blocks of their own (grid z) and
+//    multiprocessor.  Two columns' multiply-adds are one instruction (fma.rn.f32x2: 2,048 rows, 1,536 -> 17,920 2,443 -> 2,280 us,
+//    49 TFLOP/s).  With few output tiles the slices become blocks of their own (grid z) and
 //    the last block of a tile adds them in order.
 #include "common.cuh"
 
@@ -267,6 +268,23 @@ __device__ __forceinline__ float4 load4(const TX* __restrict__ base, size_t row_
   return v;
 }
 
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2 pack2(float x, float y) {
+  f32x2 d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(x), "f"(y));
+  return d;
+}
+__device__ __forceinline__ float half_of(f32x2 v, int second) {
+  float x, y;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+  return second ? y : x;
+}
+
 template <int BM>
 constexpr int tiled_dyn_smem() { return (BM / 16) * 8 * 256 * (int)sizeof(float); }
 
@@ -291,11 +309,13 @@ sgemm_tiled_kernel(const TX* __restrict__ X, const float* __restrict__ W, const 
   const int k_lo = SPLIT ? blockIdx.z * SLICE : 0;
   const int k_hi = SPLIT ? min(K, k_lo + SLICE) : K;
 
-  float sl[TM][TN];
+  // the slice sums, two neighbouring columns in a register pair: fma.rn.f32x2 is two fused multiply-adds, each
+  // rounded as fmaf rounds, in one issue slot
+  f32x2 sl[TM][TN / 2];
 #pragma unroll
   for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < TN; ++j) sl[i][j] = 0.f;
+    for (int j = 0; j < TN / 2; ++j) sl[i][j] = 0ull;
 
   float4 ra[A_LOADS], rb[B_LOADS];
   auto fetch = [&](int k0) {
@@ -342,7 +362,7 @@ sgemm_tiled_kernel(const TX* __restrict__ X, const float* __restrict__ W, const 
     if (t + 1 < ntiles) fetch(k_lo + (t + 1) * BK);
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      float a[TM], b[TN];
+      float a[TM];
       if constexpr (TM == 8) {
         const float4 a0 = *reinterpret_cast<const float4*>(&As[buf][k][ty * 4]);
         const float4 a1 = *reinterpret_cast<const float4*>(&As[buf][k][64 + ty * 4]);
@@ -355,14 +375,16 @@ sgemm_tiled_kernel(const TX* __restrict__ X, const float* __restrict__ W, const 
         const float2 a0 = *reinterpret_cast<const float2*>(&As[buf][k][ty * 2]);
         a[0] = a0.x; a[1] = a0.y;
       }
-      const float4 b0 = *reinterpret_cast<const float4*>(&Bs[buf][k][tx * 4]);
-      const float4 b1 = *reinterpret_cast<const float4*>(&Bs[buf][k][64 + tx * 4]);
-      b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w;
-      b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
+      const ulonglong2 b0 = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k][tx * 4]);
+      const ulonglong2 b1 = *reinterpret_cast<const ulonglong2*>(&Bs[buf][k][64 + tx * 4]);
 #pragma unroll
-      for (int i = 0; i < TM; ++i)
-#pragma unroll
-        for (int j = 0; j < TN; ++j) sl[i][j] = fmaf(a[i], b[j], sl[i][j]);
+      for (int i = 0; i < TM; ++i) {
+        const f32x2 aa = pack2(a[i], a[i]);
+        sl[i][0] = fma2(aa, b0.x, sl[i][0]);
+        sl[i][1] = fma2(aa, b0.y, sl[i][1]);
+        sl[i][2] = fma2(aa, b1.x, sl[i][2]);
+        sl[i][3] = fma2(aa, b1.y, sl[i][3]);
+      }
     }
     if (!SPLIT && (((t + 1) * BK) % SLICE == 0 || t + 1 == ntiles)) {
       // a slice ends: add it to the totals (each thread touches only its own words)
@@ -371,8 +393,9 @@ sgemm_tiled_kernel(const TX* __restrict__ X, const float* __restrict__ W, const 
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
           float* slot = &tot_s[(i * TN + j) * 256 + tid];
-          *slot = slices_done == 0 ? sl[i][j] : *slot + sl[i][j];
-          sl[i][j] = 0.f;
+          const float x = half_of(sl[i][j / 2], j & 1);
+          *slot = slices_done == 0 ? x : *slot + x;
+          if (j & 1) sl[i][j / 2] = 0ull;
         }
       ++slices_done;
     }
@@ -407,7 +430,7 @@ sgemm_tiled_kernel(const TX* __restrict__ X, const float* __restrict__ W, const 
 #pragma unroll
     for (int j = 0; j < TN; ++j) {
       const int n = col_of(j);
-      if (n < N) part[((size_t)blockIdx.z * M + m) * N + n] = sl[i][j];
+      if (n < N) part[((size_t)blockIdx.z * M + m) * N + n] = half_of(sl[i][j / 2], j & 1);
     }
   }
   __threadfence();
@@ -508,6 +531,18 @@ inline bool tiled_split(int M, int N, int K) {
   return K > SLICE && tiles < 2 * 148;
 }
 
+// Up to sixteen rows behind the last whole tile of 128 go through the weight-streaming kernel (a row's result is the
+// same, bit for bit), where a tile row of their own would not find multiprocessors idle: it costs the multiply-adds of
+// 128 rows, about four times the reading of the weights (8,960 -> 1,536: 1,028 rows 791 -> 653 us, 140 rows 225 -> 185;
+// with the GPU half empty, 140 rows of 1,536 -> 2,048, it would be 68 -> 88).
+inline int rows_behind_tiles(int M, int N, int K) {
+  const int rest = M % 128;
+  if (M <= 128 || rest < 1 || rest > 16) return 0;
+  const long long tiles = (long long)((N + BN - 1) / BN) * ((M + 127) / 128);
+  const long long blocks = tiled_split(M, N, K) ? tiles * ((K + SLICE - 1) / SLICE) : tiles;
+  return blocks > 2 * 148 ? rest : 0;
+}
+
 template <int BM, bool SPLIT, typename TX, typename TY>
 int launch_tiled(const TX* X, const float* W, const float* bias, TY* Y, float* part, int* tickets, int M, int N, int K,
                  int ldx, int ldy, int vec_x, int vec_w, cudaStream_t stream) {
@@ -544,9 +579,14 @@ int tiled_dispatch(const TX* X, const float* W, const float* bias, TY* Y, float*
 template <typename TX, typename TY>
 int sgemm_dispatch(const TX* X, const float* W, const float* bias, TY* Y, float* part, int* tickets, int M, int N, int K,
                    int ldx, int ldy, cudaStream_t stream) {
-  if (M <= 16) {
-    const bool vec = K % 4 == 0 && ((uintptr_t)W % 16) == 0;
-    return skinny_dispatch<TX, TY>(X, W, bias, part, Y, tickets, M, N, K, ldx, ldy, vec, stream);
+  const bool vec = K % 4 == 0 && ((uintptr_t)W % 16) == 0;
+  if (M <= 16) return skinny_dispatch<TX, TY>(X, W, bias, part, Y, tickets, M, N, K, ldx, ldy, vec, stream);
+  if (const int rest = rows_behind_tiles(M, N, K)) {
+    const int whole = M - rest;
+    const int rc = tiled_dispatch<TX, TY>(X, W, bias, Y, part, tickets, whole, N, K, ldx, ldy, stream);
+    if (rc != 0) return rc;
+    return skinny_dispatch<TX, TY>(X + (size_t)whole * ldx, W, bias, part, Y + (size_t)whole * ldy, tickets, rest, N, K,
+                                   ldx, ldy, vec, stream);
   }
   return tiled_dispatch<TX, TY>(X, W, bias, Y, part, tickets, M, N, K, ldx, ldy, stream);
 }
@@ -561,15 +601,21 @@ PBE_EXPORT long long pbe_sgemm_scratch_floats(int M, int N, int K, int* tickets)
   if (tickets) *tickets = 0;
   if (M <= 0 || N <= 0 || K <= SLICE) return 0;
   const long long slices = (K + SLICE - 1) / SLICE;
-  if (M <= 16) {
+  const int rest = M <= 16 ? M : rows_behind_tiles(M, N, K), whole = M - rest;      // rows of either kernel, one after the other
+  long long floats = 0;
+  int groups = 0;
+  if (rest > 0) {
     const int rows = skinny_wide(N, K) ? 64 : 32;
-    if (tickets) *tickets = (N + rows - 1) / rows;
-    return slices * M * N;
+    groups = (N + rows - 1) / rows;
+    floats = slices * rest * N;
   }
-  if (!tiled_split(M, N, K)) return 0;
-  const int bm = tiled_bm(M);
-  if (tickets) *tickets = ((N + BN - 1) / BN) * ((M + bm - 1) / bm);
-  return slices * M * N;
+  if (whole > 0 && tiled_split(whole, N, K)) {
+    const int bm = tiled_bm(whole), tiles = ((N + BN - 1) / BN) * ((whole + bm - 1) / bm);
+    if (tiles > groups) groups = tiles;
+    if (slices * whole * N > floats) floats = slices * whole * N;
+  }
+  if (tickets) *tickets = groups;
+  return floats;
 }
 
 PBE_EXPORT int pbe_sgemm_nt(const void* X, int x_dtype, const float* W, const float* bias, void* Y,
