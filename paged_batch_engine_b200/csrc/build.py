@@ -202,13 +202,22 @@ def _load_library(name: str, defines: Optional[Dict[str, object]] = None,
         return lib
 
 
+_found: Dict[tuple, str] = {}        # (name, defines) -> path, of what compile_many has built or found
+
+
 def compile_many(jobs: Iterable[Tuple[str, Optional[Dict[str, object]]]], workers: int = 0) -> List[str]:
     """Build several libraries side by side (used by the build check and before a model's
-    first step so that its kernels compile in parallel)."""
+    first step so that its kernels compile in parallel).  A library that this process has built or
+    found is not looked up again (its sources were hashed then, as ``load_library`` does once)."""
     jobs = list(jobs)
-    workers = workers or min(len(jobs), os.cpu_count() or 4) or 1
-    with ThreadPoolExecutor(max_workers=workers) as ex:
-        return list(ex.map(lambda j: compile_library(j[0], j[1]), jobs))
+    requests = [(name, tuple(sorted((defines or {}).items()))) for name, defines in jobs]
+    new = [(r, j) for r, j in zip(requests, jobs) if not os.path.isfile(_found.get(r, ""))]
+    if new:
+        workers = workers or min(len(new), os.cpu_count() or 4) or 1
+        with ThreadPoolExecutor(max_workers=workers) as ex:
+            for (request, _), path in zip(new, ex.map(lambda n: compile_library(n[1][0], n[1][1]), new)):
+                _found[request] = path
+    return [_found[r] for r in requests]
 
 
 # ------------------------------------------------------------------ host libraries (plain C++)
