@@ -200,6 +200,84 @@ __global__ void gated_rms_kernel(GatedRmsParams p) {
   const float scale = rsqrtf(block_sum(ss, red) / (float)N + p.eps);
   for (int c = threadIdx.x; c < N; c += blockDim.x) finish(c, scale);
 }
+
+// The same over each head, heads of whole groups of four values: a warp a head of a row, four neighbouring values a
+// lane and access, everything of a head requested at once and kept in registers between the sum and the result (the
+// kernel above reads every value and makes every gate twice, 4 bytes an access: 2,048 rows of 4,096 in eight parts
+// 45 -> 15 us).  Gates of rows that are rounded to bfloat16 take the fast exponential and division.
+constexpr int GR_WARPS = 8;
+
+__device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load_four(const __nv_bfloat16* p) {
+  const uint2 w = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
+                     __uint_as_float(w.y & 0xffff0000u));
+}
+__device__ __forceinline__ void store_four(float* p, const float (&v)[4]) {
+  *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+__device__ __forceinline__ void store_four(__nv_bfloat16* p, const float (&v)[4]) {
+  const __nv_bfloat162 a = __floats2bfloat162_rn(v[0], v[1]), b = __floats2bfloat162_rn(v[2], v[3]);
+  *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const unsigned*>(&a), *reinterpret_cast<const unsigned*>(&b));
+}
+
+template <typename T, typename TG, int QUADS>       // groups of four a lane holds at most
+__global__ void __launch_bounds__(32 * GR_WARPS) gated_rms_heads_kernel(GatedRmsParams p, int rows) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int lane = threadIdx.x & 31;
+  const long long rh = (long long)blockIdx.x * GR_WARPS + (threadIdx.x >> 5);
+  if (rh >= (long long)rows * p.H) return;
+  const int t = (int)(rh / p.H), h = (int)(rh - (long long)t * p.H), E = p.E;
+  const float* o = p.o + (size_t)rh * E;
+  const TG* g = (const TG*)p.gate + (size_t)t * p.ld_gate + (size_t)h * E;
+  const float* gain = p.gain ? p.gain + (size_t)h * E : nullptr;
+  float v[QUADS][4], gate[QUADS][4];
+#pragma unroll
+  for (int i = 0; i < QUADS; ++i) {
+    const int e = (i * 32 + lane) * 4;
+    const float4 x = e < E ? load_four(o + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 y = e < E ? load_four(g + e) : make_float4(0.f, 0.f, 0.f, 0.f);
+    v[i][0] = x.x; v[i][1] = x.y; v[i][2] = x.z; v[i][3] = x.w;
+    gate[i][0] = y.x; gate[i][1] = y.y; gate[i][2] = y.z; gate[i][3] = y.w;
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < QUADS; ++i)
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float gv = gate[i][k];
+      const float sg = sizeof(T) == 2 ? __fdividef(1.0f, 1.0f + __expf(-gv)) : 1.0f / (1.0f + expf(-gv));
+      gate[i][k] = p.gate_act ? gv * sg : sg;
+      if (p.gate_first) v[i][k] *= gate[i][k];
+      ss += v[i][k] * v[i][k];
+    }
+  const float scale = rsqrtf(warp_sum(ss) / (float)E + p.eps);
+  T* out = (T*)p.out + (size_t)rh * E;
+#pragma unroll
+  for (int i = 0; i < QUADS; ++i) {
+    const int e = (i * 32 + lane) * 4;
+    if (e >= E) break;
+    const float4 w = gain ? load_four(gain + e) : make_float4(1.f, 1.f, 1.f, 1.f);
+    const float ws[4] = {w.x, w.y, w.z, w.w};
+    float y[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      y[k] = v[i][k] * scale * ws[k];
+      if (!p.gate_first) y[k] *= gate[i][k];
+    }
+    store_four(out + e, y);
+  }
+}
+
+template <typename T, typename TG>
+void launch_gated_heads(const GatedRmsParams& p, int rows, cudaStream_t stream) {
+  const long long warps = (long long)rows * p.H;
+  const int blocks = (int)((warps + GR_WARPS - 1) / GR_WARPS);
+  if (p.E <= 128) launch_k(gated_rms_heads_kernel<T, TG, 1>, blocks, 32 * GR_WARPS, 0, stream, p, rows);
+  else if (p.E <= 256) launch_k(gated_rms_heads_kernel<T, TG, 2>, blocks, 32 * GR_WARPS, 0, stream, p, rows);
+  else launch_k(gated_rms_heads_kernel<T, TG, 4>, blocks, 32 * GR_WARPS, 0, stream, p, rows);
+}
 }  // namespace
 
 PBE_EXPORT int pbe_stream_norm(float* streams, const void* y, int y_dtype, const float* mix, const float* beta,
@@ -252,6 +330,15 @@ PBE_EXPORT int pbe_gated_rms(const float* o, const void* gate, int gate_dtype, i
                              cudaStream_t stream) {
   if (T <= 0) return 0;
   GatedRmsParams p{o, gate, gain, out, ld_gate, H, E, eps, per_head, gate_act, gate_dtype == PBE_F32 ? 1 : 0, gate_first};
+  // heads of up to 512 values in groups of four that lie on the boundaries of such a group's access
+  const uintptr_t at = (uintptr_t)o | (uintptr_t)gain | (dtype == PBE_F32 ? (uintptr_t)out : (uintptr_t)out << 1) |
+                       (p.gate_f32 ? (uintptr_t)gate : (uintptr_t)gate << 1);
+  if (per_head && E % 4 == 0 && E <= 512 && ld_gate % 4 == 0 && (at & 15) == 0 && (long long)T * H < (1LL << 33)) {
+    if (dtype == PBE_F32) launch_gated_heads<float, float>(p, T, stream);
+    else if (p.gate_f32) launch_gated_heads<__nv_bfloat16, float>(p, T, stream);
+    else launch_gated_heads<__nv_bfloat16, __nv_bfloat16>(p, T, stream);
+    return launch_status();
+  }
   const int threads = H * E >= 512 ? 256 : 128;
   if (dtype == PBE_F32) launch_k(gated_rms_kernel<float>, T, threads, 0, stream, p);
   else launch_k(gated_rms_kernel<__nv_bfloat16>, T, threads, 0, stream, p);
