@@ -233,12 +233,24 @@ __global__ void chunk_scan_kernel(ScanParams p) {
   if (!p.chunk_decay)
     for (int j = 0; j < d[3]; ++j) lam_n *= lam;
   float S = p.state[((size_t)d[0] * p.H + h) * per_head + i];
-  for (int c = 0; c < d[2]; ++c) {
-    float* u = p.scratch + ((size_t)(d[1] + c) * p.H + h) * per_head + i;
-    const float own = c + 1 < d[2] ? *u : 0.f;
-    if (p.chunk_decay && c + 1 < d[2]) lam_n = p.chunk_decay[(size_t)(d[1] + c) * p.H + h];
-    *u = S;
-    S = fmaf(lam_n, S, own);
+  // eight entries' contributions are in flight together: their order binds only the additions
+  constexpr int AHEAD = 8;
+  const int last = d[2] - 1;                     // the last chunk leaves no contribution
+  for (int c0 = 0; c0 <= last; c0 += AHEAD) {
+    float own[AHEAD], keep[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+      const bool live = c0 + j < last;
+      const size_t entry = (size_t)(d[1] + c0 + j) * p.H + h;
+      own[j] = live ? p.scratch[entry * per_head + i] : 0.f;
+      keep[j] = live && p.chunk_decay ? p.chunk_decay[entry] : lam_n;
+    }
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+      if (c0 + j > last) break;
+      p.scratch[((size_t)(d[1] + c0 + j) * p.H + h) * per_head + i] = S;
+      S = fmaf(keep[j], S, own[j]);
+    }
   }
 }
 

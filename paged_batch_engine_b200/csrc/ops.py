@@ -365,11 +365,23 @@ def _column_slice(x: torch.Tensor, what: str):
         raise KernelError(f"{what}: operands are column slices of a row-major matrix")
 
 
+def linear_attention_matrix_applies(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, key_dim: int,
+                                    value_dim: int) -> bool:
+    """Whether the tensor-core form of ``linear_attention`` takes these operands: bfloat16 rows on 16-byte boundaries
+    and widths that it is built for.  It forms logarithms of the decays, so they must not be negative."""
+    if q.dtype != torch.bfloat16 or any(x.data_ptr() % 16 or (x.stride(0) % 8 and x.shape[0] > 1) for x in (q, k, v)):
+        return False
+    if q.shape[0] == 1 and q.stride(0) % 8:
+        return False
+    fn = _fn("linear_attention_mma", "pbe_linear_attention_mma_widths", [c_int, c_int])
+    return fn(int(key_dim), int(value_dim)) == 1
+
+
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, decay: torch.Tensor,
                      q_start: torch.Tensor, q_len: torch.Tensor, slots: torch.Tensor, num_requests: int,
                      heads: int, k_scale: float = 1.0, silu: bool = False, plan=None,
                      tok_decay: Optional[torch.Tensor] = None, tok_scale: Optional[torch.Tensor] = None,
-                     skip: Optional[torch.Tensor] = None, kq_share: int = 1) -> torch.Tensor:
+                     skip: Optional[torch.Tensor] = None, kq_share: int = 1, matrix: bool = False) -> torch.Tensor:
     """o_t = S_t^T q_t with S_t = decay_h S_{t-1} + k_t v_t^T per head, request by request over
     the rows each brings (``q_start``, ``q_len`` int32 [R]); ``state`` float32 [slots, H, D, E]
     is read at ``slots[r]`` and left updated.  q, k [T, H*D] and v [T, H*E] are column slices of
@@ -378,7 +390,8 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: t
     the chunks' own contributions.  The selective form: ``tok_decay`` float32 [T, H] replaces the
     heads' constant decays (``decay`` may then be None), ``tok_scale`` float32 [T, H] multiplies v
     as it enters the state, ``skip`` float32 [H] adds skip_h v_t to the output, and ``kq_share``
-    neighbouring heads read one q and k (q, k are then [T, H / kq_share * D]).
+    neighbouring heads read one q and k (q, k are then [T, H / kq_share * D]).  ``matrix``: run it as
+    products of matrices on the tensor cores (see ``linear_attention_matrix_applies``).
     Returns float32 [T, H*E]."""
     _need_cuda(q, k, v, state, decay, q_start, q_len, slots, tok_decay, tok_scale, skip)
     _need_contiguous(tok_decay, tok_scale, skip)
@@ -417,8 +430,19 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: t
                                                                              c_void_p, c_void_p, c_void_p, c_int,
                                                                              c_void_p, c_void_p])
     chunk_decay = None
+    if matrix and (silu or not linear_attention_matrix_applies(q, k, v, D, E)):
+        raise KernelError("linear_attention: no products of matrices for these operands")
+    fm = _fn("linear_attention_mma", "pbe_linear_attention_mma",
+             [c_void_p, c_void_p, c_void_p, c_int] + [c_void_p] * 8 + [c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                                                      c_void_p, c_void_p, c_int, c_void_p, c_void_p]) \
+        if matrix else None
 
     def launch(result, items, scratch, n):
+        if matrix:
+            _check(fm(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(result), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(q_len),
+                      _ptr(slots), _ptr(items), _ptr(scratch), n, heads, D, E, float(k_scale), _ptr(tok_decay),
+                      _ptr(tok_scale), _ptr(skip), int(kq_share), _ptr(chunk_decay), _stream()), "linear_attention")
+            return
         _check(fn(_ptr(q), _ptr(k), _ptr(v), ld, _dtype_code(q), _ptr(result), _ptr(state), _ptr(decay), _ptr(q_start),
                   _ptr(q_len), _ptr(slots), _ptr(items), _ptr(scratch), n, heads, D, E, float(k_scale),
                   1 if silu else 0, _ptr(tok_decay), _ptr(tok_scale), _ptr(skip), int(kq_share), _ptr(chunk_decay),

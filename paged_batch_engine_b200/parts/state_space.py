@@ -60,7 +60,8 @@ class SelectiveStateSpace(Mixer):
         return CompositeNeed.of(**need)
 
     def kernel_libraries(self, dtype):
-        return [("short_conv", None), ("linear_attention", None), ("streams", None)] + ops.gemm_libraries(dtype)
+        matrix = [("linear_attention_mma", None)] if dtype == torch.bfloat16 else []
+        return [("short_conv", None), ("linear_attention", None), ("streams", None)] + matrix + ops.gemm_libraries(dtype)
 
     def param_specs(self, prefix):
         n, w = self.names, self.hidden_size
@@ -80,11 +81,12 @@ class SelectiveStateSpace(Mixer):
         self.conv_wt = self.conv_w.t().contiguous()        # [taps, C]: the layout the eight-channel kernel reads
         self.dt_bias, self.a_log, self.skip, self.gain = f32("dt_bias"), f32("a_log"), f32("skip"), f32("norm")
 
-    def chunk_rows(self, rows: int) -> int:
+    def chunk_rows(self, rows: int, matrix: bool = False) -> int:
         """Rows of a chunk when a long portion's recurrence runs as chunks side by side: so long that
-        the chunks of all heads and column slices fill the GPU about once, a power of two, 64 to 512."""
-        blocks_per_chunk = self.num_heads * ((self.head_dim + 31) // 32)
-        want = rows * blocks_per_chunk // 1024
+        the chunks of all heads and column slices fill the GPU about once, a power of two, 64 to 512.
+        ``matrix``: the tensor-core form, whose blocks take all columns of a head."""
+        blocks_per_chunk = self.num_heads * (1 if matrix else (self.head_dim + 31) // 32)
+        want = rows * blocks_per_chunk // (512 if matrix else 1024)
         chunk = 64
         while chunk < want and chunk < 512:
             chunk *= 2
@@ -104,10 +106,13 @@ class SelectiveStateSpace(Mixer):
                              weight_t=self.conv_wt)
         dt, decay = ops.step_sizes(dt_in, self.dt_bias, self.a_log)
         xs, B, Cm = xbc[:, :inner], xbc[:, inner:inner + G * N], xbc[:, inner + G * N:]
-        plan = None if getattr(ctx, "captured", False) else ctx.recurrence_plan(self.chunk_rows(ctx.num_tokens))
+        # prompt portions on the tensor cores, in chunks of 64 tokens; a step of mostly single tokens is faster as the
+        # plain recurrence
+        matrix = ctx.num_tokens >= 8 * ctx.num_requests and ops.linear_attention_matrix_applies(Cm, B, xs, N, P)
+        plan = None if getattr(ctx, "captured", False) else ctx.recurrence_plan(self.chunk_rows(ctx.num_tokens, matrix))
         y = ops.linear_attention(Cm, B, xs, cache.sub["ssm"].state, None, ctx.q_start, ctx.q_len, ctx.state_slots,
                                  ctx.num_requests, H, 1.0, False, plan, tok_decay=decay, tok_scale=dt,
-                                 skip=self.skip, kq_share=H // G)
+                                 skip=self.skip, kq_share=H // G, matrix=matrix)
         u = ops.gated_rms(y, z, self.gain, self.norm_groups, self.eps, True, "silu", self.dtype, gate_first=True)
         return ops.linear(u, self.w_o, None, out_dtype=self.dtype, kind=2)
 

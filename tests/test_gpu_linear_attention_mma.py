@@ -1,0 +1,77 @@
+"""The decayed recurrence as products of matrices (chunks of 64 tokens) against the recurrence in float64: edges of
+chunks and work items, strong decays and ones that underflow, states that are carried on; and the gated norm per head."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("D,E", [(128, 64), (64, 64), (64, 128)])
+@pytest.mark.parametrize("lens,chunk,decays", [([1], None, "mild"), ([63, 64, 65], None, "mild"), ([200, 17], None, "strong"),
+                                               ([300, 40, 129], 64, "mild"), ([700], 128, "strong")])
+def test_matrix_form(D, E, lens, chunk, decays):
+    from paged_batch_engine_b200.csrc import ops
+    from paged_batch_engine_b200.engine.batch import RecurrencePlan, recurrence_plan_arrays
+    H, share, T = 4, 2, sum(lens)
+    g = torch.Generator(device=DEV).manual_seed(T + D)
+    q, k = (torch.randn(T, H // share * D, device=DEV, generator=g).bfloat16() / D ** 0.25 for _ in range(2))
+    v = torch.randn(T, H * E, device=DEV, generator=g).bfloat16()
+    wide = torch.cat([q, k, v], 1).contiguous()
+    q, k, v = wide[:, :q.shape[1]], wide[:, q.shape[1]:2 * q.shape[1]], wide[:, 2 * q.shape[1]:]
+    dt = torch.rand(T, H, device=DEV, generator=g) * 0.2
+    rate = torch.tensor([0.5, 2.0, 8.0, 40.0], device=DEV) * (1.0 if decays == "mild" else 30.0)
+    if decays == "strong":       # some tokens keep everything, some nothing at all
+        dt = torch.where(torch.rand(T, H, device=DEV, generator=g) < 0.5, dt * 1e-6, dt)
+    a = torch.exp(-rate * dt)
+    skip = torch.randn(H, device=DEV, generator=g)
+    state = torch.randn(len(lens) + 1, H, D, E, device=DEV, generator=g)
+    start = state.double().clone()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+    starts = [sum(lens[:i]) for i in range(len(lens))]
+    slots = list(range(len(lens)))[::-1]
+    plan = None
+    if chunk:
+        first, scan, second, entries = recurrence_plan_arrays(starts, lens, slots, chunk)
+        plan = RecurrencePlan(entries, i32(first), len(first), i32(scan), len(scan), i32(second), len(second), rows_per_chunk=chunk)
+    out = ops.linear_attention(q, k, v, state, None, i32(starts), i32(lens), i32(slots), len(lens), H, plan=plan,
+                               tok_decay=a, tok_scale=dt, skip=skip, kq_share=share, matrix=True)
+    qd, kd = (x.double().view(T, H // share, D).repeat_interleave(share, 1) for x in (q, k))
+    vd = v.double().view(T, H, E)
+    want = torch.empty(T, H, E, dtype=torch.float64, device=DEV)
+    size = torch.empty_like(want)         # the same sums over absolute values: what the errors are relative to
+    for s0, n, slot in zip(starts, lens, slots):
+        S, A = start[slot], start[slot].abs()
+        for t in range(s0, s0 + n):
+            w = a[t].double()[:, None, None]
+            write = kd[t][:, :, None] * (dt[t].double()[:, None] * vd[t])[:, None, :]
+            S, A = w * S + write, w * A + write.abs()
+            want[t] = torch.einsum("hde,hd->he", S, qd[t]) + skip.double()[:, None] * vd[t]
+            size[t] = torch.einsum("hde,hd->he", A, qd[t].abs()) + (skip.double()[:, None] * vd[t]).abs()
+        assert ((state[slot].double() - S).abs() <= 2 ** -15 * A + 1e-12).all()
+    # state, weights and scaled values enter products with seventeen bits (2^-17 of each addend), sums are float32
+    assert ((out.double().view(T, H, E) - want).abs() <= 2 ** -15 * size).all()
+    assert torch.equal(state[len(lens)].double(), start[len(lens)])
+
+
+@pytest.mark.parametrize("E", [4, 64, 100, 128, 256, 512, 132])
+@pytest.mark.parametrize("gate_first", [False, True])
+@pytest.mark.parametrize("dtype,gate_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
+                                              (torch.bfloat16, torch.float32)])
+def test_gated_norm_per_head(E, gate_first, dtype, gate_dtype):
+    from paged_batch_engine_b200.csrc import ops
+    T, H = 13, 3
+    g = torch.Generator(device=DEV).manual_seed(E)
+    o = torch.randn(T, H * E, device=DEV, generator=g) * 3
+    wide = torch.randn(T, 2 * H * E + 4, device=DEV, generator=g).to(gate_dtype)
+    gain = torch.randn(H * E, device=DEV, generator=g)
+    for off in (0, 4, 1):               # 1: a gate that lies on no boundary
+        gate = wide[:, off:off + H * E]
+        for act in ("silu", "sigmoid"):
+            got = ops.gated_rms(o, gate, gain, H, 1e-6, True, act, dtype, gate_first).double()
+            s = torch.sigmoid(gate.double()) * (gate.double() if act == "silu" else 1.0)
+            u = o.double() * s if gate_first else o.double()
+            n = u.view(T, H, E) / torch.sqrt((u.view(T, H, E) ** 2).mean(-1, keepdim=True) + 1e-6)
+            want = n.reshape(T, H * E) * gain.double() * (1.0 if gate_first else s)
+            tol = 2 ** -8 if dtype == torch.bfloat16 else 2e-6
+            assert ((got - want).abs() <= tol * (want.abs() + 1e-3)).all()
