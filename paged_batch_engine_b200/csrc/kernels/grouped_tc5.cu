@@ -40,7 +40,8 @@ struct GroupedParams {
   int N;               // rows of a group's matrix
   int N_out;           // columns of the output (N, or N / 2 with a gate)
   int K;
-  const int32_t* tiles;   // [max_tiles, 3]: group (-1: idle, behind all live ones), first row, rows
+  const int32_t* tiles;   // [max_tiles, 3]: group (-1: idle, behind all live ones), first row, rows; null: one group, all rows
+  int rows;
   int max_tiles;
   float limit, alpha;     // of the capped gate
   int* err;
@@ -107,7 +108,7 @@ grouped_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   pdl_wait();          // the tile list and the rows come from the kernels before
   // the live tiles stand at the front of the list
   for (int i = threadIdx.x; i < p.max_tiles; i += NTHREADS)
-    if (p.tiles[3 * i] >= 0) atomicAdd(&live_smem, 1);
+    if (p.tiles == nullptr || p.tiles[3 * i] >= 0) atomicAdd(&live_smem, 1);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -121,10 +122,10 @@ grouped_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
       int it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < num_tiles && ok; t += gridDim.x) {
-        const int32_t* tile = p.tiles + 3 * (t % live);
+        const int32_t* tile = p.tiles ? p.tiles + 3 * (t % live) : nullptr;
         const int n0 = (t / live) * COLS;
-        const int m0 = tile[1];
-        const int wrow0 = tile[0] * p.N + n0;
+        const int m0 = tile ? tile[1] : (t % live) * BM;
+        const int wrow0 = (tile ? tile[0] * p.N : 0) + n0;
         const int wrow1 = wrow0 + (GLU ? p.N_out : 128);
         for (int kb = 0; kb < kblocks; ++kb, ++it) {
           const int s = it % STAGES;
@@ -174,17 +175,19 @@ grouped_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     const bool aligned = (p.N_out % 8) == 0;
     int j = 0;
     for (int t = blockIdx.x; t < num_tiles; t += gridDim.x, ++j) {
-      const int32_t* tile = p.tiles + 3 * (t % live);
+      const int32_t* tile = p.tiles ? p.tiles + 3 * (t % live) : nullptr;
       const int n0 = (t / live) * COLS;
+      const int m0 = tile ? tile[1] : (t % live) * BM;
+      const int rows = tile ? tile[2] : min(BM, p.rows - m0);
       const int buf = j & 1;
       const int r = quarter * 32 + lane;
-      const bool row_live = r < tile[2];
-      bf16* yrow = p.out + (size_t)(tile[1] + r) * p.N_out;
+      const bool row_live = r < rows;
+      bf16* yrow = p.out + (size_t)(m0 + r) * p.N_out;
       if (!mbar_wait(&acc_full[buf], (j >> 1) & 1, p.err)) break;      // flagged; the roles run to their end
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN;
       // rows beyond the tile's are padding: a warp without a live row reads nothing back
-      if (quarter * 32 < tile[2]) {
+      if (quarter * 32 < rows) {
 #pragma unroll 1
         for (int c = 0; c < COLS / 32; ++c) {
           const int col = n0 + c * 32;
@@ -245,12 +248,13 @@ void launch_grouped(const CUtensorMap& map_a, const CUtensorMap& map_w, const Gr
 
 PBE_EXPORT int pbe_grouped_tc5_tile_rows() { return BM; }
 
-// a [rows, K], w [groups, N, K], out [rows, N or N / 2], all bfloat16; tiles as the kernel's; epilogue as enumerated.
+// a [rows, K], w [groups, N, K], out [rows, N or N / 2], all bfloat16; tiles as the kernel's (null: all rows are group
+// 0's); epilogue as enumerated.
 // err: device int, set to 1 if a bounded wait ran out (the result is then invalid).
 PBE_EXPORT int pbe_grouped_tc5(const void* a, const void* w, void* out, int rows, int K, int N, int groups,
                                const int32_t* tiles, int max_tiles, int epilogue, float limit, float alpha, int* err,
                                cudaStream_t stream) {
-  if (rows <= 0 || N <= 0 || groups <= 0 || max_tiles <= 0) return 0;
+  if (rows <= 0 || N <= 0 || groups <= 0 || (tiles && max_tiles <= 0)) return 0;
   if (K <= 0 || (K & 7) || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || ((uintptr_t)out & 15))
     return (int)cudaErrorInvalidValue;
   const bool glu = epilogue == SILU_GLU || epilogue == CAPPED_GLU;
@@ -260,7 +264,7 @@ PBE_EXPORT int pbe_grouped_tc5(const void* a, const void* w, void* out, int rows
   int rc = make_map(&map_a, a, rows, K);
   if (rc == 0) rc = make_map(&map_w, w, groups * N, K);
   if (rc != 0) return rc;
-  GroupedParams p{(bf16*)out, N, glu ? N / 2 : N, K, tiles, max_tiles, limit, alpha, err};
+  GroupedParams p{(bf16*)out, N, glu ? N / 2 : N, K, tiles, rows, tiles ? max_tiles : (rows + BM - 1) / BM, limit, alpha, err};
   switch (epilogue) {
     case RELU2: launch_grouped<RELU2>(map_a, map_w, p, stream); break;
     case SILU_GLU: launch_grouped<SILU_GLU>(map_a, map_w, p, stream); break;

@@ -1602,6 +1602,59 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, sink: Optional[torch.
     return out
 
 
+LATENT_TC5_ROWS = 128       # rows of a tile of the expanded form
+LATENT_TC5_BYTES = 1 << 29  # of a step's expanded keys and values at most
+
+
+def latent_expands(dtype: torch.dtype, head_dim: int, rot_dim: int, value_dim: int, kv_rank: int, scale: float) -> bool:
+    """Whether prompt portions can expand their keys and values and run on tcgen05: bfloat16, heads of 128 + 64
+    rotated with values of 128."""
+    return (dtype == torch.bfloat16 and head_dim == 128 and rot_dim == 64 and value_dim == 128 and kv_rank % 8 == 0
+            and scale > 0)
+
+
+def latent_attention_expanded(q: torch.Tensor, pages: torch.Tensor, w_kv: torch.Tensor, total_keys: int, most_keys: int,
+                              num_row_tiles: int, group, seq_len, q_start, q_len, positions, num_heads: int, kv_rank: int, scale: float,
+                              window: Optional[int], page_tokens: int, inv_freq: Optional[torch.Tensor], rot_dims: int,
+                              rot_scale: float, sink: Optional[torch.Tensor], gate: Optional[torch.Tensor],
+                              gate_each: bool) -> torch.Tensor:
+    """Attention over one cached latent per token with the heads' keys and values expanded from the latents first:
+    the keys that the step's rows see (``total_keys``, of one request ``most_keys`` at most) are gathered from the pages,
+    multiplied by ``w_kv`` [2 * H * 128, kv_rank] (the key maps of all heads, then the value
+    maps) and attended to by ``q`` bfloat16 [T, H * (128 + 64)], whose rotated part is turned on the way.  Returns
+    bfloat16 [T, H * 128], gates applied.  Queries, expanded keys and expanded values are bfloat16, softmax weights
+    two bfloat16 terms, everything else float32."""
+    _need_cuda(q, pages, w_kv, seq_len, q_start, q_len, positions, inv_freq, sink, gate)
+    _need_contiguous(q, pages, w_kv, positions, inv_freq, sink)
+    T, H, R = q.shape[0], num_heads, q_len.numel()
+    if (q.dtype != torch.bfloat16 or pages.dtype != torch.bfloat16 or w_kv.dtype != torch.bfloat16 or q.shape[1] != H * 192
+            or tuple(w_kv.shape) != (2 * H * 128, kv_rank) or pages.shape[-1] != kv_rank + 64):
+        raise KernelError("latent_attention_expanded: shapes or dtypes do not agree")
+    if gate is not None and (gate.dtype != torch.bfloat16 or gate.stride(1) != 1):
+        raise KernelError("latent_attention_expanded: the gate is a bfloat16 column slice")
+    lib = {"PBE_X_LATENT": 1}
+    c = torch.empty((total_keys, kv_rank), dtype=torch.bfloat16, device=q.device)
+    kr = torch.empty((total_keys, 64), dtype=torch.bfloat16, device=q.device)
+    gather = _fn("attention_tc5_wide", "pbe_gather_latents",
+                 [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
+                  c_void_p], lib)
+    _check(gather(_ptr(pages), _ptr(group.block_table), int(group.bt_stride), int(page_tokens), int(kv_rank), _ptr(q_len),
+                  _ptr(seq_len), R, int(window or 0), int(most_keys), _ptr(c), _ptr(kr), _stream()), "gather_latents")
+    kv = grouped_runs_tc5(c, w_kv.unsqueeze(0), None)
+    out = torch.empty((T, H * 128), dtype=torch.bfloat16, device=q.device)
+    ldg = 0
+    if gate is not None:
+        ldg = gate.stride(0) if T > 1 else max(gate.stride(0), H * (128 if gate_each else 1))
+    fn = _fn("attention_tc5_wide", "pbe_latent_attention_tc5",
+             [c_void_p] * 4 + [c_ll, c_int, c_int] + [c_void_p] * 5 + [c_int, c_float, c_void_p, c_void_p, c_int, c_int,
+                                                                        c_int, c_int, c_float, c_void_p, c_void_p], lib)
+    _check(fn(_ptr(q), _ptr(kv), _ptr(kr), _ptr(out), int(total_keys), int(num_row_tiles), R, _ptr(q_start),
+              _ptr(q_len), _ptr(seq_len), _ptr(positions), _ptr(inv_freq),
+              int(rot_dims), float(rot_scale), _ptr(sink), _ptr(gate), int(ldg), 1 if gate_each else 0, H, int(window or 0),
+              float(scale), _ptr(tc5_attention_error_buffer(q.device)), _stream()), "latent_attention_tc5")
+    return out
+
+
 # ------------------------------------------------------------------ masked attention (head norms, bias, sink, gate)
 MASKED_TILE_ROWS = 16     # packed rows (row x head of a key/value group) a block of the float32 masked attention takes
 MASKED_MMA_TILE_ROWS = 64  # and a block of the tensor-core one
@@ -1620,11 +1673,20 @@ def masked_tile_rows(dtype: torch.dtype, key_dim: int, value_dim: int) -> int:
     return MASKED_MMA_TILE_ROWS if masked_mma_applies(dtype, key_dim, value_dim) else MASKED_TILE_ROWS
 
 
+def masked_tc5_applies(dtype: torch.dtype, key_dim: int, value_dim: int, page_tokens: int, scale: float) -> bool:
+    """Whether prompt portions can take the tcgen05 form: bfloat16 pages of 128-wide keys and values that its copies
+    can fetch in whole boxes, and a positive scale (it compares scores before they are scaled)."""
+    return (masked_mma_applies(dtype, key_dim, value_dim) and key_dim == 128 and value_dim == 128 and scale > 0
+            and tc5_attention_applies(128, page_tokens))
+
+
 def masked_libraries(dtype: torch.dtype, key_dim: int, value_dim: int):
     """The (library, defines) pairs of the masked attention for these pages (for parallel builds)."""
     jobs = [("masked_attention", None)]
     if masked_mma_applies(dtype, key_dim, value_dim):
         jobs.append(("masked_attention_mma", {"PBE_MA_D": int(key_dim), "PBE_MA_E": int(value_dim)}))
+        if key_dim == value_dim == 128:
+            jobs.append(("attention_tc5_wide", {"PBE_X_LATENT": 0}))
     return jobs
 
 
@@ -1766,7 +1828,8 @@ def masked_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
                      num_kv_heads: int, scale: float, mask: Optional[str], mask_size: Optional[int],
                      page_tokens: int, bias: Optional[torch.Tensor] = None, unit_sink: bool = False,
                      gate: Optional[torch.Tensor] = None, sink: Optional[torch.Tensor] = None,
-                     softcap: Optional[float] = None, turn: Optional[torch.Tensor] = None) -> torch.Tensor:
+                     softcap: Optional[float] = None, turn: Optional[torch.Tensor] = None,
+                     tcgen05: bool = False) -> torch.Tensor:
     """Softmax attention of every row over its request's pages.  ``q`` float32 [T, H * D]; pages
     [page, G, page_tokens, D] and [page, G, page_tokens, E].  ``mask``: None / "causal" (every earlier
     key), "window" (the last ``mask_size`` keys) or "chunk" (the earlier keys of the row's own chunk of
@@ -1775,7 +1838,8 @@ def masked_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
     ``unit_sink``: one more term e^0 in the denominator; ``sink`` float32 [H]: one more term e^sink[h].
     ``turn`` (from ``head_norm_write``): every head's output is turned back by its row's angles, before
     the gate.  ``gate`` [T, >= H * E] (a column slice in the pages' dtype): the output times its sigmoid.  ``meta``: the step's work list
-    for (group, H / G, ``masked_tile_rows(dtype, D, E)``, ``mask_size``).  Returns [T, H * E] in the
+    for (group, H / G, ``masked_tile_rows(dtype, D, E)``, ``mask_size``).  ``tcgen05``: the form for prompt
+    portions (``masked_tc5_applies``, no bias).  Returns [T, H * E] in the
     pages' dtype.  Arithmetic is float32 throughout; on the tensor-core path the float32 queries and
     softmax weights enter the products as two bfloat16 numbers each."""
     _need_cuda(q, k_pages, v_pages, bias, gate, sink, turn)
@@ -1820,7 +1884,16 @@ def masked_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         num_heads=int(H), num_kv_heads=int(G), page_tokens=int(page_tokens),
         window=int(mask_size or 0), split_keys=int(meta.split_keys), max_splits=int(meta.max_splits),
         tile_rows=int(meta.tile_rows), scale=float(scale), kinds=0, num_pages=int(k_pages.shape[0]))
-    if masked_mma_applies(k_pages.dtype, D, E):
+    if tcgen05:
+        if bias is not None or not masked_tc5_applies(k_pages.dtype, D, E, page_tokens, scale):
+            raise KernelError("masked_attention: the tcgen05 form does not take these operands")
+        fn = _fn("attention_tc5_wide", "pbe_masked_attention_tc5",
+                 [ctypes.POINTER(AttnParams), c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p,
+                  c_void_p], {"PBE_X_LATENT": 0})
+        _check(fn(ctypes.byref(p), MASK_KINDS[mask], has_sink, _ptr(sink), float(softcap or 0.0), _ptr(turn), _ptr(gate),
+                  int(ldg), int(meta.num_work), _ptr(tc5_attention_error_buffer(q.device)), _stream()),
+               "masked_attention_tc5")
+    elif masked_mma_applies(k_pages.dtype, D, E):
         fn = _fn("masked_attention_mma", "pbe_masked_attention_mma",
                  [ctypes.POINTER(AttnParams), c_void_p, c_int, c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int,
                   c_int, c_void_p],
@@ -2057,16 +2130,16 @@ def grouped_tc5_applies(x: torch.Tensor, *weights: torch.Tensor) -> bool:
                                              for w in weights)
 
 
-def grouped_runs_tc5(a: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, activation: Optional[str] = None,
+def grouped_runs_tc5(a: torch.Tensor, w: torch.Tensor, tiles: Optional[torch.Tensor], activation: Optional[str] = None,
                      limit: float = 0.0, alpha: float = 1.0) -> torch.Tensor:
     """``grouped_runs`` on tcgen05 (``tiles`` of ``GROUPED_TC5_ROWS`` rows, bfloat16 result), with the activation as
     the epilogue: "relu2" squares the relu; "silu" and "capped_swish" take ``w`` [G, 2 * I, K] as gate rows followed
-    by up rows and give [rows, I] as ``gated_activation`` does."""
+    by up rows and give [rows, I] as ``gated_activation`` does.  ``tiles`` None: all rows belong to one group."""
     _need_cuda(a, w, tiles)
     _need_contiguous(a, w, tiles)
     rows, K = a.shape
     G, N, _ = w.shape
-    if w.shape[2] != K or not grouped_tc5_applies(a, w):
+    if w.shape[2] != K or not grouped_tc5_applies(a, w) or (tiles is None and G != 1):
         raise KernelError("grouped_runs_tc5: bfloat16 rows [rows, K] and weights [G, N, K], K a multiple of eight")
     if activation not in GROUPED_TC5_EPILOGUES:
         raise KernelError(f"grouped_runs_tc5: no epilogue {activation!r}")
@@ -2079,7 +2152,7 @@ def grouped_runs_tc5(a: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, acti
         err = _tc5_err[a.device] = torch.zeros(1, dtype=torch.int32, device=a.device)
     fn = _fn("grouped_tc5", "pbe_grouped_tc5", [c_void_p] * 3 + [c_int] * 4 + [c_void_p, c_int, c_int, c_float, c_float,
                                                                              c_void_p, c_void_p])
-    _check(fn(_ptr(a), _ptr(w), _ptr(out), rows, K, N, G, _ptr(tiles), tiles.shape[0], kind, float(limit), float(alpha),
+    _check(fn(_ptr(a), _ptr(w), _ptr(out), rows, K, N, G, _ptr(tiles), tiles.shape[0] if tiles is not None else 0, kind, float(limit), float(alpha),
               _ptr(err), _stream()), "grouped_runs_tc5")
     return out
 

@@ -88,7 +88,7 @@ class LatentAttention(Mixer):
             self.inv_freq = freq.to(torch.float32).to(device)
             self.rot_dims = dims
         self.tile_rows = ops.latent_tile_rows(num_heads)
-        self.w_down = self.w_uq = self.w_uk = self.w_uv = self.w_o = None
+        self.w_down = self.w_uq = self.w_uk = self.w_uv = self.w_kv = self.w_o = None
         self.q_gain = self.c_gain = self.sink_logits = None
 
     # ---- what it keeps: one row [c | kr] per token, shared by all heads
@@ -100,6 +100,8 @@ class LatentAttention(Mixer):
 
     def kernel_libraries(self, dtype):
         tiled = [("grouped_gemm", None)] if dtype == torch.bfloat16 else []
+        if ops.latent_expands(dtype, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank, self.scale):
+            tiled += [("grouped_tc5", None), ("attention_tc5_wide", {"PBE_X_LATENT": 1})]
         return [("latent_attention", None)] + tiled + ops.gemm_libraries(dtype)
 
     # ---- tensors
@@ -128,8 +130,11 @@ class LatentAttention(Mixer):
         self.w_down = torch.cat(ws, dim=0).contiguous()
         del ws
         self.w_uq = tensors.pop(prefix + n["uq"]).contiguous()
-        self.w_uk = tensors.pop(prefix + n["uk"]).contiguous()      # [H, D, kv_rank]: applied to q as it lies
-        self.w_uv = tensors.pop(prefix + n["uv"]).contiguous()      # [H, V, kv_rank]
+        uk, uv = tensors.pop(prefix + n["uk"]).contiguous(), tensors.pop(prefix + n["uv"]).contiguous()
+        if uk.dtype == uv.dtype:            # one matrix for the keys and values of prompt portions, and its two halves
+            self.w_kv = torch.cat([uk, uv], dim=0).contiguous()
+            uk, uv = self.w_kv[:uk.shape[0]], self.w_kv[uk.shape[0]:]
+        self.w_uk, self.w_uv = uk, uv       # [H, D, kv_rank]: applied to q as it lies; [H, V, kv_rank]
         self.w_o = tensors.pop(prefix + n["o"]).contiguous()
         self.q_gain = tensors.pop(prefix + n["dq_norm"]).to(torch.float32).contiguous()
         self.c_gain = tensors.pop(prefix + n["dkv_norm"]).to(torch.float32).contiguous()
@@ -137,6 +142,30 @@ class LatentAttention(Mixer):
             self.sink_logits = tensors.pop(prefix + n["sink"]).to(torch.float32).contiguous()
 
     # ---- compute
+    ROWS_A_KEY = 8          # rows that see a key, on average, from which on expanding it pays
+    EXPANDED_ROWS = 16      # rows of a step at least
+
+    def _expanded_keys(self, ctx, q, pages):
+        """The keys that each request's rows see, when the step's keys and values are worth expanding, else None.  A
+        pair of row and key costs a head 448 multiply-adds on expanded keys and values against 1,600 on the latents,
+        and every key 2 x 128 x kv_rank for its expansion."""
+        if getattr(ctx, "captured", False) or ctx.num_tokens < self.EXPANDED_ROWS or self.w_kv is None or not ops.latent_expands(
+                self.w_kv.dtype, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank, self.scale):
+            return None
+        if q.dtype != torch.bfloat16 or pages.dtype != torch.bfloat16 or not ops.grouped_tc5_applies(q, self.w_kv[None]):
+            return None
+        window = self.window or 1 << 60
+        lens, keys = ctx.q_len_host.tolist(), []
+        for n, before in zip(lens, ctx.context_before_host.tolist()):
+            keys.append(before + n - max(0, before - window + 1))
+        total = sum(keys)
+        # 16 rows behind 2,048 tokens 180 -> 98 us, 64 and four decoded tokens there 504 -> 162; but 32 requests of 2
+        # rows each behind 512 would take 152 -> 197, and 16 rows alone behind 8,192, which the splits of the other
+        # form spread over the GPU, 180 -> 258
+        worth = sum(n * k for n, k in zip(lens, keys)) >= self.ROWS_A_KEY * total and \
+            (ctx.num_tokens >= 32 or max(keys) <= 4096)
+        return keys if worth and total * self.num_heads * 512 <= ops.LATENT_TC5_BYTES else None
+
     def forward(self, x, ctx, cache):
         T = x.shape[0]
         H, D, R, V, rank, qr = self.num_heads, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank, self.q_rank
@@ -148,6 +177,15 @@ class LatentAttention(Mixer):
                                    self.rot_dims, ctx.positions, group.slots if cache.writes else None,
                                    pages if cache.writes else None, self.eps, rot_scale=self.rot_scale)
         q = ops.linear(q_lat, self.w_uq, None, out_dtype=self.dtype, kind=16)           # [T, H * (D + R)]
+        keys = self._expanded_keys(ctx, q, pages)
+        if keys:
+            out = ops.latent_attention_expanded(
+                q, pages, self.w_kv, sum(keys), max(keys), sum((n + ops.LATENT_TC5_ROWS - 1) // ops.LATENT_TC5_ROWS
+                                                               for n in ctx.q_len_host.tolist()),
+                group, ctx.seq_len, ctx.q_start, ctx.q_len, ctx.positions, H, rank, self.scale, self.window,
+                ctx.page_tokens, self.inv_freq, self.rot_dims, self.rot_scale, self.sink_logits,
+                down[:, qr + dk:] if self.out_gate else None, self.out_gate == "each")
+            return ops.linear(out, self.w_o, None, out_dtype=self.dtype, kind=2)
         # the heads' key maps applied to the queries, the rotated part behind: float32 [T, H, rank + R]
         q_full = torch.empty((T, H, dk), dtype=torch.float32, device=x.device)
         # bfloat16 steps of more than a few rows: the per-head products on the tensor cores

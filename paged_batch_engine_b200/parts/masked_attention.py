@@ -219,6 +219,19 @@ class MaskedAttention(Mixer):
             self.bias_by_distance = rel[rows].t().contiguous()      # [H, mask_size]
 
     # ---- compute
+    def _long_rows(self, ctx) -> bool:
+        """Whether a portion's row sees enough keys for the tcgen05 form's larger start to pay: 100 rows without a
+        context 41 us on mma.sync and 43 there, 300 rows 62 and 50, 64 rows behind 2,048 134 and 87, but behind 2,048
+        in chunks of 512 (64 keys) 41 and 49."""
+        size = self.mask_size or 1 << 60
+        for n, length in zip(ctx.q_len_host.tolist(), ctx.seq_len_host.tolist()):
+            keys = min(length, size)
+            if self.mask == "chunk" and (length - 1) // size == (length - n) // size:
+                keys = (length - 1) % size + 1
+            if keys >= 192 and n * (self.num_heads // self.num_kv_heads) > 16:
+                return True
+        return False
+
     def forward(self, x, ctx, cache):
         H, G, D, E = self.num_heads, self.num_kv_heads, self.key_dim, self.value_dim
         q_off, k_off, v_off, g_off = self._columns()
@@ -246,11 +259,14 @@ class MaskedAttention(Mixer):
                                     positions=ctx.position_ids if self.rot_dims else None,
                                     rot_freq=self.rot_freq, value_freq=self.value_freq)
         q, turn = q if self.rotate_values else (q, None)
+        # prompt portions on tcgen05, but for the distance bias, whose loads a softmax thread a row would wait for
+        tc5 = (self.bias_by_distance is None and not getattr(ctx, "captured", False)
+               and ops.masked_tc5_applies(cache.k.dtype, D, E, ctx.page_tokens, self.scale) and self._long_rows(ctx))
         meta = ctx.attention_work(cache.group, H // G, self.tile_rows, self.mask_size, H, E)
         gate = proj[:, g_off:] if self.out_gate else None
         out = ops.masked_attention(q, cache.k, cache.v, meta, H, G, self.scale, self.mask, self.mask_size,
                                    ctx.page_tokens, bias=self.bias_by_distance, unit_sink=self.unit_sink, gate=gate,
-                                   sink=self.sink_scores, softcap=self.softcap, turn=turn)
+                                   sink=self.sink_scores, softcap=self.softcap, turn=turn, tcgen05=tc5)
         return ops.linear(out, self.w_o, self.b_o, out_dtype=self.dtype, kind=2)
 
 
