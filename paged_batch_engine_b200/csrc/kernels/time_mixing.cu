@@ -18,6 +18,7 @@
 //   formed, so nothing can overflow.
 // The state is laid out [head][column][key channel]: the lanes of a column move consecutive 16-byte pieces.
 #include "chunk_scan.cuh"
+#include "chunk_scan_mma.cuh"
 #include "common.cuh"
 #include "pdl.cuh"
 
@@ -343,6 +344,7 @@ struct Segments {
   float* scratch;            // [entries, H, E, D]
   float* own_decay;          // [entries, H, D]
   const int32_t* request_of_row;
+  bool matrix;               // the scans' products on the tensor cores (see chunk_scan_mma.cuh)
 };
 
 template <typename T, int RPT, int CPT, int WARPS>
@@ -365,7 +367,12 @@ int launch_chunks(const WkvParams& g, float* records, int count, const Segments&
   ChunkScanParams<T> p{records, (const T*)g.v, g.ld_v, g.out, g.state, g.q_start, g.q_len, g.slots,
                        g.H, g.D, g.E, g.write_state};
   const int slices = (g.E + COLS - 1) / COLS;
+  bool matrix = false;
+  if constexpr (DP <= 128 && sizeof(T) == 2) matrix = s.matrix && g.D % 2 == 0;
   if (s.second == nullptr) {
+    if constexpr (DP <= 128 && sizeof(T) == 2) {
+      if (matrix) return scan_mma::launch<DP, false, false, T>(p, g.R, stream);
+    }
     launch_spread(scan_chunks_kernel<RPT, CPT, WARPS, false, false, T>, dim3(g.R, g.H, slices), 32 * WARPS, smem_p,
                   stream, p);
     return launch_status();
@@ -374,15 +381,23 @@ int launch_chunks(const WkvParams& g, float* records, int count, const Segments&
   p.own_decay = s.own_decay;
   p.request_of_row = s.request_of_row;
   p.items = s.first;
-  launch_spread(scan_chunks_kernel<RPT, CPT, WARPS, false, true, T>, dim3(s.n_first, g.H, slices), 32 * WARPS, smem_p,
-                stream, p);
-  err = launch_status();
+  if constexpr (DP <= 128 && sizeof(T) == 2) {
+    if (matrix) err = scan_mma::launch<DP, false, true, T>(p, s.n_first, stream);
+  }
+  if (!matrix) {
+    launch_spread(scan_chunks_kernel<RPT, CPT, WARPS, false, true, T>, dim3(s.n_first, g.H, slices), 32 * WARPS, smem_p,
+                  stream, p);
+    err = launch_status();
+  }
   if (err != 0) return err;
   launch_k(segment_starts_kernel, dim3(s.n_starts, g.H, (unsigned)(((size_t)g.D * g.E + 255) / 256)), 256, 0, stream,
            (const float*)g.state, s.scratch, (const float*)s.own_decay, s.starts, g.H, g.D, g.E);
   err = launch_status();
   if (err != 0) return err;
   p.items = s.second;
+  if constexpr (DP <= 128 && sizeof(T) == 2) {
+    if (matrix) return scan_mma::launch<DP, false, false, T>(p, s.n_second, stream);
+  }
   launch_spread(scan_chunks_kernel<RPT, CPT, WARPS, false, false, T>, dim3(s.n_second, g.H, slices), 32 * WARPS, smem_p,
                 stream, p);
   return launch_status();
@@ -464,18 +479,19 @@ PBE_EXPORT int pbe_wkv_chunk_tokens() { return CH; }
 
 // The same for steps with prompt portions, sixteen tokens of a request at a time: two launches.
 // records: [T / 16 + R][H][pbe_wkv_record_floats(D)] floats of scratch memory.  With `second` (segments of whole
-// chunks, see chunk_scan.cuh) long portions run as segments side by side: two launches more.
+// chunks, see chunk_scan.cuh) long portions run as segments side by side: two launches more.  matrix: bfloat16 rows'
+// scans on the tensor cores, every float32 factor as two bfloat16 terms.
 PBE_EXPORT int pbe_wkv_chunks(const void* r, const void* k, const void* v, int ld_r, int ld_k, int ld_v, int dtype,
                               const float* decay, const float* bonus, float* out, float* state, float* records,
                               const int32_t* q_start, const int32_t* q_len, const int32_t* slots, int T, int R, int H,
                               int D, int E, int write_state, const int32_t* first, int n_first, const int32_t* starts,
                               int n_starts, const int32_t* second, int n_second, float* scratch, float* own_decay,
-                              const int32_t* request_of_row, cudaStream_t stream) {
+                              const int32_t* request_of_row, int matrix, cudaStream_t stream) {
   if (R <= 0 || T <= 0) return 0;
   if (second != nullptr && (!first || !starts || !scratch || !own_decay || !request_of_row || n_first < 1 || n_starts < 1))
     return (int)cudaErrorInvalidValue;
   if (((uintptr_t)scratch & 15) != 0) return (int)cudaErrorMisalignedAddress;
-  const Segments s{first, n_first, starts, n_starts, second, n_second, scratch, own_decay, request_of_row};
+  const Segments s{first, n_first, starts, n_starts, second, n_second, scratch, own_decay, request_of_row, matrix != 0};
   if (D < 1 || D > 256 || E < 1 || H < 1 || records == nullptr) return (int)cudaErrorInvalidValue;
   if ((((uintptr_t)state | (uintptr_t)records | (uintptr_t)decay) & 15) != 0) return (int)cudaErrorMisalignedAddress;
   WkvParams p{r, k, v, ld_r, ld_k, ld_v, decay, bonus, out, state, q_start, q_len, slots, R, H, D, E, write_state};

@@ -2410,12 +2410,13 @@ DELTA_CHUNK_MAX_DIM = 256     # wider key heads always run token by token
 def delta_scan(qk: torch.Tensor, kq: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor,
                state: torch.Tensor, q_start: torch.Tensor, q_len: torch.Tensor, slots: torch.Tensor, num_requests: int,
                update_state: bool = True, zero_out: bool = False,
-               chunked: bool = False) -> torch.Tensor:
+               chunked: bool = False, matrix: bool = False) -> torch.Tensor:
     """The gated delta rule request by request over the rows each brings: S <- g S,
     u = beta (v - S^T k), S <- S + k u^T, o = S^T q, with the inputs of ``delta_inputs`` and ``state``
     float32 [slots, H, E, D] (S transposed: a value column's key channels side by side), read at
     ``slots[r]`` and left updated.  ``chunked``: sixteen tokens at a time
-    (prompt portions: two launches, v is overwritten), else one by one.  Returns o, float32 [T, H * E]."""
+    (prompt portions: two launches, v is overwritten), else one by one.  ``matrix``: the chunks' scan on the tensor
+    cores, every float32 factor as two bfloat16 terms (bfloat16 runs).  Returns o, float32 [T, H * E]."""
     _need_cuda(qk, kq, v, beta, decay, state, q_start, q_len, slots)
     _need_contiguous(qk, kq, v, beta, decay, state)
     T, G, _, D = qk.shape
@@ -2436,11 +2437,11 @@ def delta_scan(qk: torch.Tensor, kq: torch.Tensor, v: torch.Tensor, beta: torch.
         size = _fn("delta_rule", "pbe_delta_record_floats", [c_int])(D)
         ct = _fn("delta_rule", "pbe_delta_chunk_tokens", [])()
         records = torch.empty((T // ct + int(num_requests), H, size), dtype=torch.float32, device=v.device)
-        fn = _fn("delta_rule", "pbe_delta_scan_chunks", [c_void_p] * 4 + [c_int] + [c_void_p] * 6 + [c_int] * 7 + [c_void_p])
+        fn = _fn("delta_rule", "pbe_delta_scan_chunks", [c_void_p] * 4 + [c_int] + [c_void_p] * 6 + [c_int] * 8 + [c_void_p])
         global _launches
         _check(fn(_ptr(qk), _ptr(v), _ptr(beta), _ptr(decay), 1 if per_channel else 0, _ptr(out), _ptr(state),
                   _ptr(records), _ptr(q_start), _ptr(q_len), _ptr(slots), T, int(num_requests), G, H, D, E,
-                  1 if update_state else 0, _stream()), "delta_scan_chunks")
+                  1 if update_state else 0, 1 if matrix else 0, _stream()), "delta_scan_chunks")
         _launches += 1
         return out
     fn = _fn("delta_rule", "pbe_delta_scan", [c_void_p] * 5 + [c_int] + [c_void_p] * 5 + [c_int] * 6 + [c_void_p])
@@ -2498,14 +2499,15 @@ WKV_CHUNK_MAX_DIM = 256       # wider key heads always run token by token
 def wkv(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, bonus: torch.Tensor,
         state: torch.Tensor, q_start: torch.Tensor, q_len: torch.Tensor, slots: torch.Tensor, num_requests: int,
         heads: int, update_state: bool = True, zero_out: bool = False, chunked: bool = False, plan=None,
-        request_of_row: Optional[torch.Tensor] = None) -> torch.Tensor:
+        request_of_row: Optional[torch.Tensor] = None, matrix: bool = False) -> torch.Tensor:
     """o_t = (S + diag(bonus) k_t v_t^T)^T r_t, S <- diag(decay_t) S + k_t v_t^T per head, request by request over
     the rows each brings: ``r``, ``k`` [T, H * D] and ``v`` [T, H * E] column slices in one dtype, ``decay`` float32
     [T, H * D] (numbers in [0, 1]), ``bonus`` float32 [H * D], ``state`` float32 [slots, H, E, D] (S transposed: a
     value column's key channels side by side), read at ``slots[r]`` and left updated.  ``chunked``: sixteen
     tokens at a time (prompt portions: two launches), else one by one.  ``plan`` (a ``RecurrencePlan`` of the step
     whose chunks are multiples of sixteen rows; with ``request_of_row`` int32 [T]): chunked portions of several
-    such lengths run as segments side by side (two launches more).  Returns o, float32 [T, H * E]."""
+    such lengths run as segments side by side (two launches more).  ``matrix``: the chunks' scans of bfloat16 rows on
+    the tensor cores, every float32 factor as two bfloat16 terms.  Returns o, float32 [T, H * E]."""
     _need_cuda(r, k, v, decay, bonus, state, q_start, q_len, slots)
     _need_contiguous(decay, bonus, state)
     for x in (r, k, v):
@@ -2545,10 +2547,10 @@ def wkv(r: torch.Tensor, k: torch.Tensor, v: torch.Tensor, decay: torch.Tensor, 
                         _ptr(plan.second_pass), plan.num_second_pass, _ptr(scratch), _ptr(own_decay),
                         _ptr(request_of_row)]
         fn = _fn("time_mixing", "pbe_wkv_chunks", types + [c_void_p] * 4 + [c_int] * 6 + [c_void_p, c_int] * 3
-                 + [c_void_p] * 4)
+                 + [c_void_p] * 3 + [c_int, c_void_p])
         global _launches
         _check(fn(*heads_of, _ptr(records), _ptr(q_start), _ptr(q_len), _ptr(slots), T, int(num_requests), H, D, E,
-                  1 if update_state else 0, *segments, _stream()), "wkv_chunks")
+                  1 if update_state else 0, *segments, 1 if matrix else 0, _stream()), "wkv_chunks")
         _launches += 1 if segments[4] is None else 3
         return out
     fn = _fn("time_mixing", "pbe_wkv_steps", types + [c_void_p] * 3 + [c_int] * 5 + [c_void_p])

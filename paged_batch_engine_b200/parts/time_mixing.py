@@ -109,7 +109,7 @@ class TimeMixing(Mixer):
         plan = None if single else ctx.recurrence_plan(self.segment_rows(ctx.num_tokens))
         o = ops.wkv(r, k, v, decay, self.bonus, cache.sub["wkv"].state, ctx.q_start, ctx.q_len, ctx.state_slots,
                     ctx.num_requests, H, update_state=cache.writes, zero_out=captured, chunked=not single,
-                    plan=plan, request_of_row=ctx.request_of_row)
+                    plan=plan, request_of_row=ctx.request_of_row, matrix=self.dtype == torch.bfloat16)
         y = ops.gated_rms(o, g, self.gain, H, self.eps, True, "silu", self.dtype)
         return ops.linear(y, self.w_o, None, out_dtype=self.dtype, kind=2)
 
