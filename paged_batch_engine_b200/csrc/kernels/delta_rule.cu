@@ -65,6 +65,7 @@ struct InputParams {
   const int32_t* slots;
   int T, R, G, H, D, E, taps, update;
   float q_scale, unit_eps;
+  int moves_from;            // delta_conv_state moves the state on for requests of at least so many tokens
 };
 
 __device__ __forceinline__ float softplus_(float x) { return x > 20.f ? x : log1pf(expf(x)); }
@@ -181,7 +182,8 @@ __global__ void __launch_bounds__(IN_WARPS * 32) delta_inputs_kernel(InputParams
   }
 }
 
-// The convolution state after a portion of two or more tokens (one token: delta_inputs did it).
+// The convolution state after a portion of two or more tokens (one token: delta_inputs did it; after
+// delta_inputs_rows, which writes no state, of one or more).
 template <typename T>
 __global__ void delta_conv_state_kernel(InputParams p) {
   pdl_launch_dependents();
@@ -190,14 +192,151 @@ __global__ void delta_conv_state_kernel(InputParams p) {
   const int C = 2 * p.G * p.D + p.H * p.E;
   const int c = blockIdx.y * blockDim.x + threadIdx.x;
   const int n = p.q_len[r];
-  if (c >= C || n <= 1) return;
+  if (c >= C || n < p.moves_from) return;
   const int keep = p.taps - 1;
   float* st = p.conv_state + (size_t)p.slots[r] * keep * C + c;
   const T* in = (const T*)p.proj + c;
   const int t0 = p.q_start[r];
-  for (int i = 0; i < keep; ++i) {                 // ascending: entry i + n > i is still the old one
+  float fresh[MAX_TAPS];                           // all requested before the first is written
+#pragma unroll
+  for (int i = 0; i < MAX_TAPS; ++i) {
+    if (i >= keep) break;
     const int li = n - keep + i;
-    st[(size_t)i * C] = li >= 0 ? to_float(in[(size_t)(t0 + li) * p.ld]) : st[(size_t)(i + n) * C];
+    fresh[i] = li >= 0 ? to_float(in[(size_t)(t0 + li) * p.ld]) : st[(size_t)(i + n) * C];
+  }
+#pragma unroll
+  for (int i = 0; i < MAX_TAPS; ++i) {
+    if (i >= keep) break;
+    st[(size_t)i * C] = fresh[i];
+  }
+}
+
+// delta_inputs for steps of many rows with a decay per channel, TAPS taps and heads of up to 128 in groups of four: a warp
+// takes one head of IN_ROWS rows of the step, a lane four of its channels, whose inputs of the rows before stay in
+// registers; the decays have blocks of their own, a thread four channels of IN_ROWS rows.  What bounds it is the
+// exponentials and the float32 stores.  2,048 rows, 8 + 8 + 16 heads of 128: 59 -> 45 us (a row a warp, one block a row for
+// its 2,048 decays, which was the last to end); the step's convolution state, requested at once, 16 -> 12 us.
+constexpr int IN_ROWS = 8;
+
+template <typename T, int TAPS>
+__global__ void __launch_bounds__(IN_WARPS * 32) delta_inputs_rows_kernel(InputParams p, int head_blocks) {
+  pdl_launch_dependents();
+  pdl_wait();
+  const int G = p.G, H = p.H, D = p.D, E = p.E;
+  const int C = 2 * G * D + H * E;
+  const int first = blockIdx.x * IN_ROWS;
+  const int rows = min(IN_ROWS, p.T - first);
+  auto alive = [&](int t) {
+    const int r = p.request_of_row[t];
+    return r >= 0 && r < p.R && p.q_len[r] > 0;
+  };
+  if ((int)blockIdx.y >= head_blocks) {
+    if ((int)blockIdx.y == head_blocks) {                    // beta
+      for (int i = threadIdx.x; i < rows * H; i += blockDim.x) {
+        const int t = first + i / H, h = i % H;
+        const bool live = alive(t);
+        const float b = live ? p.small[(size_t)t * p.ld_small + h] : 0.f;
+        p.beta[(size_t)t * H + h] = 1.0f / (1.0f + expf(-b));
+      }
+      return;
+    }
+    const int c = (((int)blockIdx.y - head_blocks - 1) * (int)blockDim.x + (int)threadIdx.x) * 4;
+    if (c >= H * D) return;
+    float bias[4], rate[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      bias[k] = p.dt_bias[c + k];
+      rate[k] = -expf(p.a_log[(c + k) / D]);
+    }
+    for (int n = 0; n < rows; ++n) {
+      const int t = first + n;
+      const bool live = alive(t);
+      float a[4], y[4];
+      load_v<4>(p.chan + (size_t)t * p.ld_chan + c, a);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[k] = expf(rate[k] * softplus_(live ? a[k] + bias[k] : 0.f));
+      put_v<4>(p.decay + (size_t)t * H * D + c, y);
+    }
+    return;
+  }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int head = blockIdx.y * IN_WARPS + warp;
+  if (head >= G + H) return;
+  const bool is_qk = head < G;
+  const int h = head - G, d = lane * 4;
+  const bool mine = d < (is_qk ? D : E);
+  // the channel of the value, or of the query; the key's lies G * D further
+  const int c0 = mine ? (is_qk ? head * D + d : 2 * G * D + h * E + d) : 0;
+  const T* in = (const T*)p.proj + c0;
+  constexpr int PARTS = 2;
+  float w[PARTS][TAPS][4], u[PARTS][TAPS][4];             // u: the rows t - (TAPS - 1) .. t
+#pragma unroll
+  for (int x = 0; x < PARTS; ++x) {
+    if (x == 1 && !is_qk) break;
+#pragma unroll
+    for (int j = 0; j < TAPS; ++j) {
+      load_v<4>(p.conv_t + (size_t)j * C + c0 + x * G * D, w[x][j]);
+      const int t = first - TAPS + j;                      // moved on by one before the first row
+      if (j > 0 && t >= 0) load_v<4>(in + (size_t)t * p.ld + x * G * D, u[x][j]);
+      else u[x][j][0] = u[x][j][1] = u[x][j][2] = u[x][j][3] = 0.f;
+    }
+  }
+  for (int n = 0; n < rows; ++n) {
+    const int t = first + n;
+    const int r = p.request_of_row[t];
+    const bool live = r >= 0 && r < p.R && p.q_len[r] > 0;
+    const int place = live ? t - p.q_start[r] : 0;
+    float y[PARTS][4];
+#pragma unroll
+    for (int x = 0; x < PARTS; ++x) {
+      if (x == 1 && !is_qk) break;
+#pragma unroll
+      for (int j = 0; j + 1 < TAPS; ++j)
+#pragma unroll
+        for (int k = 0; k < 4; ++k) u[x][j][k] = u[x][j + 1][k];
+      load_v<4>(in + (size_t)t * p.ld + x * G * D, u[x][TAPS - 1]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[x][k] = 0.f;
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) {
+        const int off = place - (TAPS - 1) + j;            // the input's place among this step's rows; negative: before them
+        float in_j[4];
+        if (off >= 0 || !live) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) in_j[k] = u[x][j][k];
+        } else {
+          load_v<4>(p.conv_state + ((size_t)p.slots[r] * (TAPS - 1) + TAPS - 1 + off) * C + c0 + x * G * D, in_j);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) y[x][k] = fmaf(w[x][j][k], in_j[k], y[x][k]);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) y[x][k] = mine && live ? y[x][k] / (1.0f + expf(-y[x][k])) : 0.f;
+    }
+    if (is_qk) {
+      float qq = 0.f, kk = 0.f, dot = 0.f;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        qq = fmaf(y[0][k], y[0][k], qq);
+        kk = fmaf(y[1][k], y[1][k], kk);
+      }
+      const float qs = p.q_scale / sqrtf(warp_sum(qq) + p.unit_eps), ks = 1.0f / sqrtf(warp_sum(kk) + p.unit_eps);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        y[0][k] *= qs;
+        y[1][k] *= ks;
+        dot = fmaf(y[0][k], y[1][k], dot);
+      }
+      float* out = p.qk + ((size_t)t * G + head) * 2 * D;
+      if (mine) {
+        put_v<4>(out + d, y[0]);
+        put_v<4>(out + D + d, y[1]);
+      }
+      dot = warp_sum(dot);
+      if (lane == 0) p.kq[(size_t)t * G + head] = dot;
+    } else if (mine) {
+      put_v<4>(p.v + (size_t)t * H * E + h * E + d, y[0]);
+    }
   }
 }
 
@@ -573,11 +712,22 @@ void launch_scan(const ScanParams& p, int R, bool chan, cudaStream_t stream) {
 }
 
 template <typename T, int V>
-int launch_inputs(const InputParams& p, bool many, cudaStream_t stream) {
+int launch_inputs(InputParams p, bool many, cudaStream_t stream) {
   const int wide = p.D > p.E ? p.D : p.E;
   dim3 grid(p.T, (p.G + p.H + IN_WARPS - 1) / IN_WARPS + 1);
   const int per = (wide + 32 * V - 1) / (32 * V);
-  if (per <= 1) launch_k(delta_inputs_kernel<T, V, 1>, grid, IN_WARPS * 32, 0, stream, p);
+  // steps with prompt portions and a decay per channel, launch and state included (row a warp -> rows a warp): 256 rows
+  // 24.8 -> 26.6 us, 512 32.8 -> 28.7, 1,024 43.0 -> 36.9, 2,048 70.5 -> 57.4; requests of two rows 27 -> 29.  With a decay
+  // per head the row a warp stays (512 rows 20.6 -> 28.7, 2,048 45 -> 41), for other numbers of taps and wider heads too.
+  if (V == 4 && many && p.chan && per <= 1 && p.taps == 4 && p.T >= IN_ROWS * 64 && p.T >= IN_ROWS * p.R &&
+      p.ld_chan % 4 == 0 && (((uintptr_t)p.chan | (uintptr_t)p.decay) & 15) == 0) {
+    p.moves_from = 1;
+    const int head_blocks = (p.G + p.H + IN_WARPS - 1) / IN_WARPS;
+    const int decay_blocks = (p.H * p.D / 4 + IN_WARPS * 32 - 1) / (IN_WARPS * 32);
+    if constexpr (V == 4)
+      launch_k(delta_inputs_rows_kernel<T, 4>, dim3((p.T + IN_ROWS - 1) / IN_ROWS, head_blocks + 1 + decay_blocks),
+               IN_WARPS * 32, 0, stream, p, head_blocks);
+  } else if (per <= 1) launch_k(delta_inputs_kernel<T, V, 1>, grid, IN_WARPS * 32, 0, stream, p);
   else if (per <= 2) launch_k(delta_inputs_kernel<T, V, 2>, grid, IN_WARPS * 32, 0, stream, p);
   else if (per <= 4) launch_k(delta_inputs_kernel<T, V, 4>, grid, IN_WARPS * 32, 0, stream, p);
   else if (per <= 16 / V) launch_k(delta_inputs_kernel<T, V, 16 / V>, grid, IN_WARPS * 32, 0, stream, p);
@@ -601,7 +751,7 @@ PBE_EXPORT int pbe_delta_inputs(const void* proj, int ld, int dtype, const float
   if (taps < 1 || taps > MAX_TAPS || D < 1 || E < 1 || D > MAX_HEAD || E > MAX_HEAD || G < 1 || H % G != 0)
     return (int)cudaErrorInvalidValue;
   InputParams p{proj, ld, conv_t, conv_state, small, ld_small, chan, ld_chan, dt_bias, a_log, qk, kq, v, beta, decay,
-                request_of_row, q_start, q_len, slots, T, R, G, H, D, E, taps, update, q_scale, unit_eps};
+                request_of_row, q_start, q_len, slots, T, R, G, H, D, E, taps, update, q_scale, unit_eps, 2};
   const bool vec4 = D % 4 == 0 && E % 4 == 0 && ld % 4 == 0 &&
                     (((uintptr_t)conv_t | (uintptr_t)conv_state | (uintptr_t)qk | (uintptr_t)v) & 15) == 0 &&
                     ((uintptr_t)proj & (dtype == PBE_F32 ? 15 : 7)) == 0;
