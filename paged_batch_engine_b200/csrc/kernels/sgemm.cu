@@ -288,13 +288,15 @@ __device__ __forceinline__ float half_of(f32x2 v, int second) {
 template <int BM>
 constexpr int tiled_dyn_smem() { return (BM / 16) * 8 * 256 * (int)sizeof(float); }
 
+// only_if: nothing is done where it points to a zero.
 // SPLIT: every block multiplies one K slice (blockIdx.z) and writes its sums to `part`; the block
 // that finishes an output tile last (a ticket per tile) adds the slices in order.
 template <int BM, bool SPLIT, typename TX, typename TY>
 __global__ void __launch_bounds__(256, 2)
 sgemm_tiled_kernel(const TX* __restrict__ X, const float* __restrict__ W, const float* __restrict__ bias,
                    TY* __restrict__ Y, float* __restrict__ part, int* __restrict__ tickets, int M, int N, int K,
-                   int ldx, int ldy, int vec_x, int vec_w) {
+                   int ldx, int ldy, int vec_x, int vec_w, const int* only_if) {
+  if (only_if != nullptr && *only_if == 0) return;
   constexpr int TM = BM / 16, TN = 8;
   constexpr int A_LOADS = (BM * BK / 4 + 255) / 256;     // float4 loads of the X tile per thread
   constexpr int B_LOADS = BN * BK / 4 / 256;
@@ -545,7 +547,7 @@ inline int rows_behind_tiles(int M, int N, int K) {
 
 template <int BM, bool SPLIT, typename TX, typename TY>
 int launch_tiled(const TX* X, const float* W, const float* bias, TY* Y, float* part, int* tickets, int M, int N, int K,
-                 int ldx, int ldy, int vec_x, int vec_w, cudaStream_t stream) {
+                 int ldx, int ldy, int vec_x, int vec_w, cudaStream_t stream, const int* only_if = nullptr) {
   auto kern = sgemm_tiled_kernel<BM, SPLIT, TX, TY>;
   const int smem = SPLIT ? 0 : tiled_dyn_smem<BM>();
   static bool attr_set = false;
@@ -556,7 +558,8 @@ int launch_tiled(const TX* X, const float* W, const float* bias, TY* Y, float* p
   }
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, SPLIT ? (K + SLICE - 1) / SLICE : 1);
   if (grid.y > 65535 || grid.z > 65535) return (int)cudaErrorInvalidValue;
-  kern<<<grid, 256, smem, stream>>>(X, W, bias, Y, part, tickets, M, N, K, ldx, ldy, vec_x, vec_w);
+  kern<<<grid, 256, smem, stream>>>(X, W, bias, Y, part, tickets, M, N, K, ldx, ldy, vec_x, vec_w,
+                                       only_if);
   return launch_status();
 }
 
@@ -633,4 +636,14 @@ PBE_EXPORT int pbe_sgemm_nt(const void* X, int x_dtype, const float* W, const fl
   if (x_dtype == PBE_BF16 && y_dtype == PBE_F32)
     return sgemm_dispatch<bf16, float>((const bf16*)X, W, bias, (float*)Y, scratch, tickets, M, N, K, ldx, ldy, stream);
   return (int)cudaErrorInvalidValue;          // float32 rows in, bfloat16 rows out: nothing asks for it
+}
+
+// The float32 product where *only_if is not zero when the kernel starts, else nothing; no scratch memory.
+PBE_EXPORT int pbe_sgemm_nt_if(const float* X, const float* W, const float* bias, float* Y, int M, int N, int K,
+                               const int* only_if, cudaStream_t stream) {
+  if (M <= 0 || N <= 0) return 0;
+  if (K <= 0 || only_if == nullptr) return (int)cudaErrorInvalidValue;
+  const int vec = K % 4 == 0;
+  return launch_tiled<128, false, float, float>(X, W, bias, Y, nullptr, nullptr, M, N, K, K, N,
+                                                vec && (uintptr_t)X % 16 == 0, vec && (uintptr_t)W % 16 == 0, stream, only_if);
 }

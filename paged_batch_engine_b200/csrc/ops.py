@@ -705,6 +705,43 @@ def sgemm_nt(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out
     return out
 
 
+def sgemm_tc5_applies(x: torch.Tensor, w: torch.Tensor) -> bool:
+    """Whether a float32 product takes tcgen05 (multiply-adds -> tcgen05): with more than 64 rows it is 1.2 (K = 256,
+    33 -> 27 us) to 4.2 times faster at every size from 64 x 256 up; with 64 rows, where the multiply-adds' tiles are
+    smaller, 1.06 to 1.18 times, with 16 or fewer the weights' streaming is the better one."""
+    return x.dtype == torch.float32 and x.shape[0] > 64 and w.shape[0] >= 64 and w.shape[1] >= 256
+
+
+def sgemm_tc5(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor):
+    """``sgemm_nt`` of float32 rows on tcgen05: every operand as three bfloat16 terms, which hold its 24 bits, and the
+    six products that count; no further from the exact result than the multiply-adds, in another order of addition.
+    Operands that are not finite, or beyond the largest bfloat16, take the multiply-adds (found on the device)."""
+    _need_cuda(x, w, bias, out)
+    _need_contiguous(x, w, bias, out)
+    M, K = x.shape
+    N = w.shape[0]
+    if x.dtype != torch.float32 or w.dtype != torch.float32 or out.dtype != torch.float32 or w.shape[1] != K or \
+            out.shape != (M, N):
+        raise KernelError("sgemm_tc5: shapes or dtypes do not agree")
+    if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
+        raise KernelError("sgemm_tc5: bias must be float32 [N]")
+    tiled = int(_fn("sgemm_tc5", "pbe_sgemm_tc5_rows", [c_int] * 3)(M, N, K))
+    if tiled < M:
+        sgemm_nt(x[tiled:], w, bias, out[tiled:])
+        M = tiled
+    need = _fn("sgemm_tc5", "pbe_sgemm_tc5_scratch", [c_int, c_int, c_int])
+    need.restype = c_ll
+    scratch = torch.empty(int(need(M, N, K)), dtype=torch.uint8, device=x.device)
+    err = _tc5_err.get(x.device)
+    if err is None:
+        err = _tc5_err[x.device] = torch.zeros(1, dtype=torch.int32, device=x.device)
+    fn = _fn("sgemm_tc5", "pbe_sgemm_tc5", [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 3)
+    _check(fn(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), M, N, K, _ptr(scratch), _ptr(err), _stream()), "sgemm_tc5")
+    again = _fn("sgemm", "pbe_sgemm_nt_if", [c_void_p] * 4 + [c_int] * 3 + [c_void_p] * 2)
+    _check(again(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), M, N, K, _ptr(scratch), _stream()), "sgemm_nt_if")
+    return out
+
+
 _sgemm_tickets = {}      # per device: zeroed int32 tickets shared by the float32 products of the stream
 
 
@@ -894,7 +931,7 @@ def gemm_libraries(dtype: torch.dtype, largest_weight: int = 0):
     """The matrix-product libraries a part of this dtype launches whose largest matrix has that
     many elements (for parallel builds)."""
     if dtype == torch.float32:
-        return [("sgemm", None)]
+        return [("sgemm", None), ("sgemm_tc5", None)]
     return [("gemm_skinny", None)] + ([("gemm_stream", None)] if stream_wanted(largest_weight) else []) + \
         ([("gemm_tc5", None)] if TC5_MASK else [])
 
@@ -914,6 +951,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor] = None
     out_dtype = out_dtype or x.dtype
     if w.dtype == torch.float32:
         out = torch.empty((x.shape[0], w.shape[0]), dtype=out_dtype, device=x.device)
+        if sgemm_tc5_applies(x, w) and out_dtype == torch.float32:
+            return sgemm_tc5(x, w, bias, out)
         return sgemm_nt(x, w, bias, out)
     if x.dtype != torch.bfloat16:
         raise KernelError("a bfloat16 weight takes bfloat16 activations")

@@ -1,0 +1,76 @@
+"""The float32 product on tcgen05 (three bfloat16 terms an operand) against 64 bits and against the multiply-adds: edges of
+its tiles, K blocks and parts of K, rows behind the last whole tile, columns multiplied in several goes, numbers that are
+not finite, and which products take it."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _ops():
+    from paged_batch_engine_b200.csrc import ops
+    return ops
+
+
+def _inputs(M, N, K):
+    g = torch.Generator(device=DEV).manual_seed(M + N + K)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    return rand(M, K), rand(N, K), rand(N)
+
+
+def _product(fn, x, w, b):
+    out = torch.full((x.shape[0], w.shape[0]), float("nan"), device=DEV)
+    fn(x, w, b, out)
+    return out
+
+
+@pytest.mark.parametrize("M,N,K", [(65, 64, 256), (128, 256, 320), (129, 257, 333), (144, 130, 1100), (300, 2049, 63),
+                                   (513, 128, 8960), (1028, 1536, 2112), (66, 6000, 8200), (1, 1, 1)])
+def test_against_64_bits(M, N, K):
+    x, w, b = _inputs(M, N, K)
+    got, fma = _product(_ops().sgemm_tc5, x, w, b), _product(_ops().sgemm_nt, x, w, b)
+    want, size = x.double() @ w.double().t() + b.double(), x.double().abs() @ w.double().abs().t() + b.double().abs()
+    # left out: 2^-26 of a product's size.  In a block of 64 k at most 24 additions are cut off at 2^-23 of what they
+    # add to; the blocks' sums, the parts and the bias are added with less than 2^-24 each, 32 + K / 2048 + 9 of them in
+    # a row at most
+    assert ((got.double() - want).abs() <= size * (2.0 ** -26 + 24 * 2.0 ** -23 + (41 + K / 2048) * 2.0 ** -24)).all()
+    if K >= 256:                    # and no further off than the multiply-adds
+        assert (got.double() - want).norm() <= (fma.double() - want).norm()
+
+
+def test_numbers_that_are_not_finite():
+    ops = _ops()
+    x, w, b = _inputs(130, 200, 300)
+    for value in (float("inf"), float("nan"), 3.4e38):
+        x2, w2 = x.clone(), w.clone()
+        x2[5, 7] = value
+        w2[11, 299] = -value
+        for xs, ws in ((x2, w), (x, w2), (x2, w2)):
+            got, want = _product(ops.sgemm_tc5, xs, ws, b), _product(ops.sgemm_nt, xs, ws, b)
+            assert torch.equal(got.nan_to_num(1.25), want.nan_to_num(1.25)) and torch.equal(got.isnan(), want.isnan())
+    assert torch.isfinite(_product(ops.sgemm_tc5, x, w, b)).all()       # nothing is left behind
+
+
+def test_captured():
+    ops = _ops()
+    x, w, b = _inputs(150, 256, 512)
+    out = torch.empty(150, 256, device=DEV)
+    ops.sgemm_tc5(x, w, b, out)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ops.sgemm_tc5(x, w, b, out)
+    for value in (float("inf"), 1.0):
+        x[3, 3] = value
+        graph.replay()
+        assert torch.equal(out.nan_to_num(1.25), _product(ops.sgemm_tc5, x, w, b).nan_to_num(1.25))
+
+
+def test_which_products_take_it():
+    ops = _ops()
+    x, w, b = _inputs(80, 64, 256)
+    assert torch.equal(ops.linear(x[:64], w, b), _product(ops.sgemm_nt, x[:64], w, b))
+    assert torch.equal(ops.linear(x[:65], w, b), _product(ops.sgemm_tc5, x[:65], w, b))
+    assert torch.equal(ops.linear(x, w[:63], b[:63]), _product(ops.sgemm_nt, x, w[:63], b[:63]))
+    assert ops.linear(x.bfloat16(), w).dtype == torch.bfloat16          # rows of 16 bits stay with the multiply-adds
