@@ -260,8 +260,8 @@ class MaskedAttention(Mixer):
                                     rot_freq=self.rot_freq, value_freq=self.value_freq)
         q, turn = q if self.rotate_values else (q, None)
         # prompt portions on tcgen05, but for the distance bias, whose loads a softmax thread a row would wait for
-        tc5 = (self.bias_by_distance is None and not getattr(ctx, "captured", False)
-               and ops.masked_tc5_applies(cache.k.dtype, D, E, ctx.page_tokens, self.scale) and self._long_rows(ctx))
+        tc5 = (D == E == 128 and self.bias_by_distance is None and not getattr(ctx, "captured", False)
+               and self._long_rows(ctx) and ops.masked_tc5_applies(cache.k.dtype, D, E, ctx.page_tokens, self.scale))
         meta = ctx.attention_work(cache.group, H // G, self.tile_rows, self.mask_size, H, E)
         gate = proj[:, g_off:] if self.out_gate else None
         out = ops.masked_attention(q, cache.k, cache.v, meta, H, G, self.scale, self.mask, self.mask_size,
