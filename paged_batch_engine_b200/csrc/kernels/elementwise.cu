@@ -11,8 +11,8 @@ using namespace pbe;
 
 // ---------------------------------------------------------------- embedding
 template <typename TW>
-__global__ void embedding_kernel(float* __restrict__ out, const TW* __restrict__ table,
-                                 const int32_t* __restrict__ ids, int d, int vocab) {
+__global__ void embedding_kernel(float* out, const TW* __restrict__ table,
+                                 const int32_t* ids, int d, int vocab) {
   pdl_launch_dependents();   // the next kernel may fetch what does not depend on this one
   pdl_wait();
   const int t = blockIdx.x;
@@ -67,9 +67,9 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&a)[4]) {
 // residual is left alone (the final norm before the LM head, on the wanted rows only).
 // y_i = (w_i * x_i) * rsqrt(mean(x^2) + eps), the product order of the reference.
 template <typename TD, typename TO>
-__global__ void add_rmsnorm_kernel(float* __restrict__ residual, const TD* __restrict__ delta,
-                                   const float* __restrict__ gain, TO* __restrict__ out,
-                                   const int32_t* __restrict__ row_index, int d, float eps) {
+__global__ void add_rmsnorm_kernel(float* residual, const TD* delta,
+                                   const float* __restrict__ gain, TO* out,
+                                   const int32_t* row_index, int d, float eps) {
   __shared__ float red[33];
   pdl_launch_dependents();   // the next kernel may fetch what does not depend on this one
   // the gains are weights: a thread's first two vectors of them are fetched before the wait
@@ -171,10 +171,10 @@ PBE_EXPORT int pbe_add_rmsnorm(float* residual, const void* delta, int delta_dty
 // with the one r = rsqrt(mean(x^2) + eps) both norms share.  g2 == nullptr: one output only.
 // delta_scale m: x += m * (a + b) (a design that scales its branches before the residual sum).
 template <typename TD, typename TO>
-__global__ void add2_rmsnorm2_kernel(float* __restrict__ residual, const TD* __restrict__ delta_a,
-                                     const TD* __restrict__ delta_b, const float* __restrict__ gain1,
-                                     const float* __restrict__ gain2, TO* __restrict__ out1, TO* __restrict__ out2,
-                                     const int32_t* __restrict__ row_index, int d, float eps,
+__global__ void add2_rmsnorm2_kernel(float* residual, const TD* delta_a,
+                                     const TD* delta_b, const float* __restrict__ gain1,
+                                     const float* __restrict__ gain2, TO* out1, TO* out2,
+                                     const int32_t* row_index, int d, float eps,
                                      float delta_scale) {
   __shared__ float red[33];
   extern __shared__ __align__(16) float row[];
@@ -234,7 +234,7 @@ PBE_EXPORT int pbe_add2_rmsnorm2(float* residual, const void* delta_a, const voi
 
 // ---------------------------------------------------------------- relu(x)^2, and scaled soft-capped logits
 template <typename T>
-__global__ void relu_squared_kernel(const T* __restrict__ in, T* __restrict__ out, size_t total) {
+__global__ void relu_squared_kernel(const T* in, T* out, size_t total) {
   pdl_launch_dependents();
   pdl_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -254,7 +254,7 @@ PBE_EXPORT int pbe_relu_squared(const void* in, void* out, int dtype, long long 
 }
 
 // x <- x * scale, then (cap > 0) x <- cap * tanh(x / cap); float32 logits in place
-__global__ void scale_softcap_kernel(float* __restrict__ x, size_t total, float scale, float cap) {
+__global__ void scale_softcap_kernel(float* x, size_t total, float scale, float cap) {
   pdl_launch_dependents();
   pdl_wait();
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -275,7 +275,7 @@ PBE_EXPORT int pbe_scale_softcap(float* x, long long total, float scale, float c
 // ---------------------------------------------------------------- SiLU(gate) * up
 // in: [rows, 2*inter], gate in columns [0, inter), up in [inter, 2*inter); out [rows, inter].
 template <typename T>
-__global__ void silu_mul_kernel(const T* __restrict__ in, T* __restrict__ out, int inter,
+__global__ void silu_mul_kernel(const T* in, T* out, int inter,
                                 size_t total) {
   pdl_launch_dependents();   // the next kernel may fetch what does not depend on this one
   pdl_wait();
@@ -292,7 +292,7 @@ __global__ void silu_mul_kernel(const T* __restrict__ in, T* __restrict__ out, i
 
 // the same, four columns a thread (inter a multiple of 4)
 template <typename T>
-__global__ void silu_mul_vec4_kernel(const T* __restrict__ in, T* __restrict__ out, int inter,
+__global__ void silu_mul_vec4_kernel(const T* in, T* out, int inter,
                                      size_t total4) {
   pdl_launch_dependents();   // the next kernel may fetch what does not depend on this one
   pdl_wait();
@@ -317,7 +317,7 @@ __global__ void silu_mul_vec4_kernel(const T* __restrict__ in, T* __restrict__ o
 // the up projection, one 16-byte store; a block row per batch row, so no division per element.
 // The sigmoid is 1 / (1 + 2^(-g log2 e)) in float32 with the fast exponential and reciprocal;
 // the result is rounded to bfloat16 anyway.
-__global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+__global__ void silu_mul_bf16x8_kernel(const __nv_bfloat16* in, __nv_bfloat16* out,
                                        int inter, int rows) {
   pdl_launch_dependents();   // the next kernel may fetch what does not depend on this one
   pdl_wait();
@@ -379,9 +379,9 @@ PBE_EXPORT int pbe_silu_mul(const void* in, void* out, int dtype, int rows, int 
 // out[t] = table[ids[t]] * scale + pos_table[positions[t]] (the position row unscaled), float32; `lp`
 // (or null) receives a copy in bfloat16.
 template <typename TW>
-__global__ void embedding_pos_kernel(float* __restrict__ out, __nv_bfloat16* __restrict__ lp,
-                                     const TW* __restrict__ table, const int32_t* __restrict__ ids, float scale, const TW* __restrict__ pos_table,
-                                     const int32_t* __restrict__ positions, int max_pos, int d, int vocab) {
+__global__ void embedding_pos_kernel(float* out, __nv_bfloat16* lp,
+                                     const TW* __restrict__ table, const int32_t* ids, float scale, const TW* __restrict__ pos_table,
+                                     const int32_t* positions, int max_pos, int d, int vocab) {
   pdl_launch_dependents();
   pdl_wait();
   const int t = blockIdx.x;
@@ -417,18 +417,33 @@ PBE_EXPORT int pbe_embedding_pos(float* out, void* lp, const void* table, int ta
 // out[t] = [residual[t] + delta_scale * (a[t] + b[t]) | first[t]], both halves d wide, in the run
 // dtype: the operand of a projection that reads the current residual beside the embedding output.
 template <typename TD, typename TO>
-__global__ void fold_pair_kernel(const float* __restrict__ residual, const TD* __restrict__ delta_a,
-                                 const TD* __restrict__ delta_b, float delta_scale, const float* __restrict__ first,
-                                 TO* __restrict__ out, int d) {
+__global__ void fold_pair_kernel(const float* residual, const TD* delta_a,
+                                 const TD* delta_b, float delta_scale, const float* first,
+                                 TO* out, int d) {
   pdl_launch_dependents();
   pdl_wait();
   const size_t t = blockIdx.x;
-  for (int i = threadIdx.x; i < d; i += blockDim.x) {
-    float add = 0.f;
-    if (delta_a) add = to_float(delta_a[t * d + i]);
-    if (delta_b) add += to_float(delta_b[t * d + i]);
-    out[t * 2 * d + i] = from_float<TO>(fmaf(delta_scale, add, residual[t * d + i]));
-    out[t * 2 * d + d + i] = from_float<TO>(first[t * d + i]);
+  // four elements' loads are requested before the first of them is written
+  constexpr int AHEAD = 4;
+  for (int i0 = threadIdx.x; i0 < d; i0 += AHEAD * blockDim.x) {
+    float sum[AHEAD], own[AHEAD];
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+      const int i = i0 + j * blockDim.x;
+      if (i >= d) break;
+      float add = 0.f;
+      if (delta_a) add = to_float(delta_a[t * d + i]);
+      if (delta_b) add += to_float(delta_b[t * d + i]);
+      sum[j] = fmaf(delta_scale, add, residual[t * d + i]);
+      own[j] = first[t * d + i];
+    }
+#pragma unroll
+    for (int j = 0; j < AHEAD; ++j) {
+      const int i = i0 + j * blockDim.x;
+      if (i >= d) break;
+      out[t * 2 * d + i] = from_float<TO>(sum[j]);
+      out[t * 2 * d + d + i] = from_float<TO>(own[j]);
+    }
   }
 }
 
@@ -453,7 +468,7 @@ PBE_EXPORT int pbe_fold_pair(const float* residual, const void* delta_a, const v
 // kind 2 (gelu, tanh form): y = gelu_tanh(g) * u.  kind 3 (relu): y = max(g, 0) * u.
 // bias (float32 [2*inter], optional) is added to both first.
 template <typename T>
-__global__ void glu_act_kernel(const T* __restrict__ in, const float* __restrict__ bias, T* __restrict__ out, int inter,
+__global__ void glu_act_kernel(const T* in, const float* __restrict__ bias, T* out, int inter,
                                size_t total, int kind, float limit, float alpha) {
   pdl_launch_dependents();
   pdl_wait();
@@ -486,7 +501,7 @@ __global__ void glu_act_kernel(const T* __restrict__ in, const float* __restrict
 // The capped swish on bfloat16 rows, eight values a thread (16-byte loads and stores) as the silu
 // kernel above; float32 arithmetic with the fast exponential and reciprocal, the result is rounded
 // to bfloat16 anyway.
-__global__ void capped_swish_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out,
+__global__ void capped_swish_bf16x8_kernel(const __nv_bfloat16* in, __nv_bfloat16* out,
                                            int inter, int rows, float limit, float alpha) {
   pdl_launch_dependents();
   pdl_wait();
@@ -516,7 +531,7 @@ __global__ void capped_swish_bf16x8_kernel(const __nv_bfloat16* __restrict__ in,
 }
 
 // gelu_tanh(g) * u on bfloat16 rows, eight values a thread
-__global__ void gelu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __nv_bfloat16* __restrict__ out, int inter,
+__global__ void gelu_mul_bf16x8_kernel(const __nv_bfloat16* in, __nv_bfloat16* out, int inter,
                                        int rows) {
   pdl_launch_dependents();
   pdl_wait();
@@ -540,8 +555,8 @@ __global__ void gelu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, __n
 }
 
 // max(g, 0) * u on bfloat16 rows with optional biases, eight values a thread
-__global__ void relu_mul_bf16x8_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ bias,
-                                       __nv_bfloat16* __restrict__ out, int inter, int rows) {
+__global__ void relu_mul_bf16x8_kernel(const __nv_bfloat16* in, const float* __restrict__ bias,
+                                       __nv_bfloat16* out, int inter, int rows) {
   pdl_launch_dependents();
   const int chunk = blockIdx.x * blockDim.x + threadIdx.x;
   float bg[8], bu[8];

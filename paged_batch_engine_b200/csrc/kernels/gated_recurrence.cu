@@ -205,8 +205,8 @@ __global__ void gated_scan_kernel(ScanParams p) {
 // scan entry (state row, first scratch entry, chunks, rows a chunk): chunk k's scratch entry holds
 // what the chunk adds from zero (q_k) and its product of a (P_k); it gets the chunk's start value,
 // s_0 = the state row, s_(k+1) = P_k s_k + q_k.  The last chunk left nothing: it only gets its start.
-__global__ void chunk_starts_kernel(const int32_t* __restrict__ scan, const float* __restrict__ state,
-                                    float* __restrict__ scratch_s, const float* __restrict__ scratch_p, int C) {
+__global__ void chunk_starts_kernel(const int32_t* scan, const float* state,
+                                    float* scratch_s, const float* scratch_p, int C) {
   pdl_launch_dependents();
   pdl_wait();
   const int c = blockIdx.y * blockDim.x + threadIdx.x;

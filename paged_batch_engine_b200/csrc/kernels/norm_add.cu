@@ -48,8 +48,8 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float (&a)[4]) {
 
 // VPT: groups of four elements a thread holds
 template <typename T, int VPT>
-__global__ void norm_add_kernel(float* __restrict__ x, const T* __restrict__ y, const float* __restrict__ gain,
-                                T* __restrict__ lp, int d, float eps) {
+__global__ void norm_add_kernel(float* x, const T* y, const float* __restrict__ gain,
+                                T* lp, int d, float eps) {
   __shared__ float red[33];
   pdl_launch_dependents();
   float g[VPT][4];
@@ -91,8 +91,8 @@ __global__ void norm_add_kernel(float* __restrict__ x, const T* __restrict__ y, 
 
 // any width: the row of y waits in shared memory
 template <typename T>
-__global__ void norm_add_any_kernel(float* __restrict__ x, const T* __restrict__ y, const float* __restrict__ gain,
-                                    T* __restrict__ lp, int d, float eps) {
+__global__ void norm_add_any_kernel(float* x, const T* y, const float* __restrict__ gain,
+                                    T* lp, int d, float eps) {
   __shared__ float red[33];
   extern __shared__ __align__(16) float held[];
   pdl_launch_dependents();

@@ -3,7 +3,10 @@
 // pdl_wait(), which returns once the previous kernel has completed and its writes are
 // visible; everything a kernel reads from or writes to activations, the cache or any
 // other buffer of the step comes after that call.  What does not depend on the previous
-// kernel (weights, above all) may be fetched before it.  pdl_launch_dependents() tells
+// kernel (weights, above all) may be fetched before it.  The order of loads and the wait is the compiler's
+// to keep, and it need not keep it for pointers marked __restrict__ (nothing else may write what they
+// name, so neither may the wait), nor for loads through the read-only cache: in a kernel that waits
+// only weights are marked so (tests/test_kernel_sources.py).  pdl_launch_dependents() tells
 // the next kernel it may begin launching: the weight-streaming kernels call it where their
 // blocks have issued most of their memory traffic, the short kernels between them (norms,
 // position encoding, merge, activation, sampling) at their very top, before their own

@@ -319,8 +319,8 @@ __device__ __forceinline__ float addend_factor(const float* gate, int ld_gate, s
 }
 
 template <typename T>
-__global__ void combine_kernel(const float* __restrict__ part, const T* __restrict__ addend,
-                               const float* __restrict__ gate, int ld_gate, T* __restrict__ out, int top, int W,
+__global__ void combine_kernel(const float* part, const T* addend,
+                               const float* gate, int ld_gate, T* out, int top, int W,
                                size_t total) {
   pdl_launch_dependents();
   pdl_wait();

@@ -242,7 +242,7 @@ __device__ void block_argmax(const float* row, int V, Shared& sh, float* out_max
 }
 
 __global__ void __launch_bounds__(THREADS)
-argmax_kernel(const float* __restrict__ logits, size_t ld, int V, int32_t* __restrict__ out) {
+argmax_kernel(const float* logits, size_t ld, int V, int32_t* out) {
   __shared__ Shared sh;
   pdl_launch_dependents();   // the next kernel may fetch what does not depend on this one
   pdl_wait();
@@ -259,7 +259,7 @@ argmax_kernel(const float* __restrict__ logits, size_t ld, int V, int32_t* __res
 constexpr int ARGMAX_CLUSTER = 8;
 
 __global__ void __cluster_dims__(ARGMAX_CLUSTER, 1, 1) __launch_bounds__(THREADS)
-argmax_cluster_kernel(const float* __restrict__ logits, size_t ld, int V, int32_t* __restrict__ out) {
+argmax_cluster_kernel(const float* logits, size_t ld, int V, int32_t* out) {
   namespace cg = cooperative_groups;
   __shared__ Shared sh;
   __shared__ float part_v[ARGMAX_CLUSTER];
@@ -574,10 +574,10 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
 // mode 1: the radix descent only (for tests that compare the two ways).
 template <int CL>
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(const float* __restrict__ logits, size_t ld, int V,
-              const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
-              const float* __restrict__ top_p, const float* __restrict__ uniform,
-              int32_t* __restrict__ out, int mode) {
+sample_kernel(const float* logits, size_t ld, int V,
+              const float* temperature, const int32_t* top_k,
+              const float* top_p, const float* uniform,
+              int32_t* out, int mode) {
   __shared__ Shared sh;
   extern __shared__ __align__(16) unsigned char quick_raw[];
   Quick& q = *reinterpret_cast<Quick*>(quick_raw);

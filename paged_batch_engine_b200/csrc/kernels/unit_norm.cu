@@ -148,8 +148,8 @@ __global__ void unit_norm_kernel(UnitNormParams p) {
 }
 
 template <typename TW, typename TO>
-__global__ void embedding_unit_norm_kernel(float* __restrict__ out, TO* __restrict__ lp, const TW* __restrict__ table,
-                                           const int32_t* __restrict__ ids, const float* __restrict__ gain, int d,
+__global__ void embedding_unit_norm_kernel(float* out, TO* lp, const TW* __restrict__ table,
+                                           const int32_t* ids, const float* __restrict__ gain, int d,
                                            int vocab, float eps) {
   __shared__ float red[33];
   extern __shared__ __align__(16) float row[];

@@ -61,3 +61,36 @@ def test_sorted_rows_through_the_experts(T, K, N, E, top, activation):
         back = ops.expert_scatter(y, chosen, place, start, weights, T).float()
         plain = (y[at].float().view(T, top, N) * weights[..., None]).sum(1)
         assert ((back - plain).abs() <= 2 ** -8 * (plain.abs() + 1e-3)).all()
+
+
+@pytest.mark.parametrize("W", [128, 2052, 2048])
+def test_what_reads_the_result_next(W):
+    """The kernels that read the experts' result start while it is written: over inputs that change from call to call,
+    with the same buffers handed out again, each of them sees the call's own result."""
+    from paged_batch_engine_b200.csrc import ops
+    T, top, E = 257, 3, 5
+    g = torch.Generator(device=DEV).manual_seed(W)
+    chosen = torch.rand(T, E, device=DEV, generator=g).topk(top, -1).indices.to(torch.int32).contiguous()
+    counts, place = ops.expert_places(chosen, E)
+    max_tiles = (T * top + 127) // 128 + E
+    start, _ = ops.run_tiles(counts, max_tiles, 128)
+    weights = torch.rand(T, top, device=DEV, generator=g)
+    gain = torch.rand(W, device=DEV, generator=g)
+    ys = [torch.randn(max_tiles * 128, W, device=DEV, generator=g).bfloat16() for _ in range(3)]
+    xs = [torch.randn(T, W, device=DEV, generator=g) for _ in range(3)]
+
+    def chain(i, wait):
+        def scattered():
+            y = ops.expert_scatter(ys[i % 3], chosen, place, start, weights, T)
+            if wait:
+                torch.cuda.synchronize()
+            return y
+        x1, x2 = xs[i % 3].clone(), xs[(i + 1) % 3].clone()
+        out = [*ops.add2_rmsnorm2(x1, scattered(), None, gain, gain, 1e-5, torch.bfloat16), x1]
+        out.append(ops.norm_add(x2, scattered(), gain, 1e-5, torch.bfloat16))
+        out.append(ops.fold_pair(xs[i % 3], scattered(), None, 0.5, xs[2], torch.bfloat16))
+        return out
+    want = [chain(i, True) for i in range(3)]
+    got = [chain(i, False) for i in range(30)]
+    for i, outs in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(outs, want[i % 3])), i
