@@ -9,6 +9,10 @@
 // accumulators.  Sums of logarithms and their differences are taken in double (a decay of zero counts as 2^-400),
 // so a weight keeps float32's accuracy however strong the decays before it are.
 //
+// A product multiplies the zero weight of a later token with that token's values too, so values that are not finite would
+// reach back to the tokens before theirs: a chunk that has some takes the products of a row tile with its own tokens one
+// by one.
+//
 // One block per (work item or request, head), four warps: a warp makes sixteen rows of o and keeps D / 4 rows of the
 // state in registers; o's weights pass from score accumulators to operands in registers.  Two blocks a multiprocessor
 // (99 KB at 128 x 64) fill each other's barriers and copies.  Work items cut long portions as in
@@ -200,7 +204,15 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
     const float keep = exp2f((float)total);
     log_all += total;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    __syncthreads();
+    bool odd = false;                                  // values that are not finite, among those this thread fetched
+    for (int i = tid; i < L * (E / 8); i += THREADS) {
+      const int row = i / (E / 8);
+      const uint4 raw = *reinterpret_cast<const uint4*>(Vs + row * VSTR + (i - row * (E / 8)) * 8);
+      const unsigned x[4] = {raw.x, raw.y, raw.z, raw.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) odd = odd || (x[k] & 0x7f80u) == 0x7f80u || (x[k] & 0x7f800000u) == 0x7f800000u;
+    }
+    odd = __syncthreads_or(odd) != 0;
     // v times its weight in the new state
     for (int i = tid; i < L * (E / 8); i += THREADS) {
       const int row = i / (E / 8), at = row * VSTR + (i - row * (E / 8)) * 8;
@@ -262,6 +274,27 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
           }
           split2(g[t][0], g[t][1], hi[2 * t], lo[2 * t]);
           split2(g[t][2], g[t][3], hi[2 * t + 1], lo[2 * t + 1]);
+        }
+        if (odd && jt == warp) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {               // token j's weights lie in the quad's lane (j % 8) / 2
+            const int from_lane = (lane & ~3) | ((j & 7) >> 1);
+            const float w0 = __shfl_sync(0xffffffffu, g[j >> 3][j & 1], from_lane);
+            const float w1 = __shfl_sync(0xffffffffu, g[j >> 3][2 + (j & 1)], from_lane);
+#pragma unroll
+            for (int c = 0; c < E / 8; ++c) {
+              const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Vs + (jt * 16 + j) * VSTR + c * 8 + q2));
+              if (j <= g8) {
+                o[c][0] = fmaf(w0, x.x, o[c][0]);
+                o[c][1] = fmaf(w0, x.y, o[c][1]);
+              }
+              if (j <= g8 + 8) {
+                o[c][2] = fmaf(w1, x.x, o[c][2]);
+                o[c][3] = fmaf(w1, x.y, o[c][3]);
+              }
+            }
+          }
+          break;
         }
 #pragma unroll
         for (int j = 0; j < E / 16; ++j) {

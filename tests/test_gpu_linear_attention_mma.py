@@ -54,6 +54,37 @@ def test_matrix_form(D, E, lens, chunk, decays):
     assert torch.equal(state[len(lens)].double(), start[len(lens)])
 
 
+@pytest.mark.parametrize("D,E", [(128, 64), (64, 64), (64, 128)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("at", [0, 13, 15, 16, 70, 99])
+def test_what_is_not_finite_stays_behind_its_token(D, E, value, at):
+    """A token's value reaches its own output and later ones, as in the recurrence token by token, never an earlier one."""
+    from paged_batch_engine_b200.csrc import ops
+    T, H = 100, 2
+    g = torch.Generator(device=DEV).manual_seed(at + D)
+    rand = lambda *s: torch.randn(*s, device=DEV, generator=g)
+    q, k, v = (rand(T, H * D).bfloat16(), rand(T, H * D).bfloat16(), rand(T, H * E).bfloat16())
+    a, dt = torch.exp(-0.1 * rand(T, H).abs()), rand(T, H).abs()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)
+
+    def run(v, matrix):
+        state = torch.zeros(1, H, D, E, device=DEV)
+        wide = torch.cat([q, k, v], 1).contiguous()
+        parts = wide[:, :H * D], wide[:, H * D:2 * H * D], wide[:, 2 * H * D:]
+        o = ops.linear_attention(*parts, state, None, i32([0]), i32([T]), i32([0]), 1, H, tok_decay=a, tok_scale=dt,
+                                 matrix=matrix)
+        return o.view(T, H, E), state
+    clean, _ = run(v, True)
+    v2 = v.clone()
+    v2.view(T, H, E)[at, 1, 5] = value
+    got, state = run(v2, True)
+    want, want_state = run(v2, False)
+    # the tokens of its tile of sixteen are added one by one, in float32 rather than as terms of it: 2^-15 as above
+    assert ((got[:at] - clean[:at]).abs() <= 2 ** -15 * clean.abs().max()).all()
+    assert torch.equal(got.isfinite(), want.isfinite()) and torch.equal(state.isfinite(), want_state.isfinite())
+    assert torch.equal(got[:, 0], clean[:, 0])             # nor another head's
+
+
 @pytest.mark.parametrize("E", [4, 64, 100, 128, 256, 512, 132])
 @pytest.mark.parametrize("gate_first", [False, True])
 @pytest.mark.parametrize("dtype,gate_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16),
