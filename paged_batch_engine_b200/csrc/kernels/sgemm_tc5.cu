@@ -1,7 +1,7 @@
 // The float32 product Y[M, N] = X[M, K] * W[N, K]^T (+ bias[N]) of many rows on the fifth-generation tensor cores, with
-// float32's precision: every operand is cut into three bfloat16 terms, x = h + m + l, which hold all of its 24 bits, and
-// the six products hh, hm, mh, mm, hl, lh are added; those left out are at most 2^-26 of a product, less than the
-// rounding of the multiply-add that they stand for.
+// float32's precision: every operand is cut into three bfloat16 terms, x = h + m + l, |m| <= 2^-8 |x| and |l| <= 2^-17 |x|,
+// which hold all of its 24 bits, and the six products hh, hm, mh, mm, hl, lh are added; ml and lm, which are left out, are
+// 2^-25 of a product each at most, together as large as the rounding of the multiply-add that they stand for.
 //
 // The tensor cores add in float32 but cut off what does not fit instead of rounding it, so a sum is not left to them
 // for long: after every 64 k the accumulator in tensor memory starts anew, the small products are issued before hh, and the epilogue's warps add its contents to the tile's running sums in registers, with a rounding
@@ -12,9 +12,10 @@
 //
 // Two kernels a product:
 //  * split3: an operand's three terms as bfloat16 matrices one below the other, rows padded with zeros to 64 k; bound by
-//    memory (4 bytes in, 6 out).  It also tells whether an element is beyond the largest bfloat16 or not finite: such a
-//    product is left to sgemm.cu, whose kernel is launched behind and looks at the flag (an infinity times a term that
-//    is zero would be no number).
+//    memory (4 bytes in, 6 out).  It also tells whether an element is other than zero or of a size from SMALLEST to
+//    LARGEST: such a product is left to sgemm.cu, whose kernel is launched behind and looks at the flag.  A smaller one's
+//    third term would fall under bfloat16's smallest normal number, larger ones' products could overflow with either sign
+//    where their sum does not, and an infinity times a term that is zero would be no number.
 //  * the product: persistent blocks walk over tiles of 128 x BN, or over parts of K of such tiles where there are too few
 //    (a small kernel adds the parts in order); warp 0 is the TMA producer, warp 1 issues the MMAs (128 x BN x 16), warps
 //    2-9 hold the running sums, half a tile row a thread, and write them out.  Two accumulators alternate.  What bounds
@@ -40,9 +41,12 @@ typedef __nv_bfloat16 bf16;
 constexpr int BM = 128, BK = 64, UMMA_K = 16, TERMS = 3;
 constexpr int SLICE = 2048 / BK;                  // K blocks whose sums are added in one chain
 constexpr int EPI_WARPS = 8, NTHREADS = 64 + 32 * EPI_WARPS;
-constexpr float LARGEST = 3.38953139e38f;          // of bfloat16
+constexpr float SMALLEST = 0x1p-102f;              // its last bit, 2^-125, is a bfloat16 number
+constexpr float LARGEST = 0x1p47f;                 // a sum of 2^31 products of two such numbers stays below 2^127
 
 // ------------------------------------------------------------------ the terms
+__device__ __forceinline__ bool whole_in_terms(float x) { return x == 0.f || (fabsf(x) >= SMALLEST && fabsf(x) <= LARGEST); }
+
 // planes [TERMS][rows][Kp]; a thread takes eight k of a row
 __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* planes, int rows, int K, int Kp, int vec, int* flag) {
   const int pieces = Kp / 8;
@@ -63,7 +67,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* plane
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float a = v[2 * i], b = v[2 * i + 1];
-    plain = plain && fabsf(a) <= LARGEST && fabsf(b) <= LARGEST;
+    plain = plain && whole_in_terms(a) && whole_in_terms(b);
 #pragma unroll
     for (int t = 0; t < TERMS; ++t) {
       const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
@@ -368,7 +372,7 @@ PBE_EXPORT long long pbe_sgemm_tc5_scratch(int M, int N, int K) {
 }
 
 // X [M, K], W [N, K], Y [M, N], float32, contiguous.  Afterwards the first int of scratch says whether an element was not
-// finite or too large: Y is then to be made by pbe_sgemm_nt_if.
+// finite, too large or too small: Y is then to be made by pbe_sgemm_nt_if.
 // err: device int, set to 1 if a bounded wait ran out (the result is then invalid).
 PBE_EXPORT int pbe_sgemm_tc5(const float* X, const float* W, const float* bias, float* Y, int M, int N, int K, void* scratch,
                              int* err, cudaStream_t stream) {

@@ -715,7 +715,8 @@ def sgemm_tc5_applies(x: torch.Tensor, w: torch.Tensor) -> bool:
 def sgemm_tc5(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], out: torch.Tensor):
     """``sgemm_nt`` of float32 rows on tcgen05: every operand as three bfloat16 terms, which hold its 24 bits, and the
     six products that count; no further from the exact result than the multiply-adds, in another order of addition.
-    Operands that are not finite, or beyond the largest bfloat16, take the multiply-adds (found on the device)."""
+    Operands with an element that is not zero and not of a size from 2^-102 to 2^47 take the multiply-adds (found on
+    the device)."""
     _need_cuda(x, w, bias, out)
     _need_contiguous(x, w, bias, out)
     M, K = x.shape

@@ -31,10 +31,10 @@ def test_against_64_bits(M, N, K):
     x, w, b = _inputs(M, N, K)
     got, fma = _product(_ops().sgemm_tc5, x, w, b), _product(_ops().sgemm_nt, x, w, b)
     want, size = x.double() @ w.double().t() + b.double(), x.double().abs() @ w.double().abs().t() + b.double().abs()
-    # left out: 2^-26 of a product's size.  In a block of 64 k at most 24 additions are cut off at 2^-23 of what they
+    # left out: 2^-24 of a product's size.  In a block of 64 k at most 24 additions are cut off at 2^-23 of what they
     # add to; the blocks' sums, the parts and the bias are added with less than 2^-24 each, 32 + K / 2048 + 9 of them in
     # a row at most
-    assert ((got.double() - want).abs() <= size * (2.0 ** -26 + 24 * 2.0 ** -23 + (41 + K / 2048) * 2.0 ** -24)).all()
+    assert ((got.double() - want).abs() <= size * (2.0 ** -24 + 24 * 2.0 ** -23 + (41 + K / 2048) * 2.0 ** -24)).all()
     if K >= 256:                    # and no further off than the multiply-adds
         assert (got.double() - want).norm() <= (fma.double() - want).norm()
 
@@ -50,6 +50,30 @@ def test_numbers_that_are_not_finite():
             got, want = _product(ops.sgemm_tc5, xs, ws, b), _product(ops.sgemm_nt, xs, ws, b)
             assert torch.equal(got.nan_to_num(1.25), want.nan_to_num(1.25)) and torch.equal(got.isnan(), want.isnan())
     assert torch.isfinite(_product(ops.sgemm_tc5, x, w, b)).all()       # nothing is left behind
+
+
+@pytest.mark.parametrize("x_value,w_value", [(1e-36, 1.0), (-3e-39, 2.0), (1e25, 1e25), (2.0 ** 70, -1.0), (1.0, 1e-33)])
+def test_numbers_that_three_terms_do_not_hold(x_value, w_value):
+    """Beside ordinary numbers: products that overflow stay the infinity that the multiply-adds make of them, and the last
+    bits of tiny numbers are not lost."""
+    ops = _ops()
+    x, w, b = _inputs(130, 200, 300)
+    x[5] = 0.0
+    x[5, 7], w[:, 7] = x_value * 1.2345678, w_value * 1.1234567
+    got, want = _product(ops.sgemm_tc5, x, w, None), _product(ops.sgemm_nt, x, w, None)
+    assert torch.equal(got[5], want[5]) and not want[5].isnan().any()
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("x_scale,w_scale", [(2.0 ** -60, 2.0 ** -55), (2.0 ** -65, 2.0 ** -60), (2.0 ** 40, 2.0 ** 42), (2.0 ** -85, 2.0 ** 45)])
+def test_sizes_of_the_operands(x_scale, w_scale):
+    ops = _ops()
+    x, w, _ = _inputs(130, 200, 300)
+    x, w = x.sign() * x.abs().clamp(min=1e-3) * x_scale, w.sign() * w.abs().clamp(min=1e-3) * w_scale
+    got = _product(ops.sgemm_tc5, x, w, None)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    # as above, and the smallest float32 number for each of the sums that may end below 2^-126
+    assert ((got.double() - want).abs() <= size * (2.0 ** -24 + 24 * 2.0 ** -23 + 41 * 2.0 ** -24) + 200 * 2.0 ** -149).all()
 
 
 def test_captured():
