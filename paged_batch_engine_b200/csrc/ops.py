@@ -2133,6 +2133,13 @@ def grouped_heads(a: torch.Tensor, lda: int, head_stride: int, K: int, w: torch.
                     gate, rot, rot_dims, inv_freq, positions, rot_scale, gate_each)
 
 
+def most_run_tiles(rows: int, groups: int, tile_rows: int) -> int:
+    """The most tiles that ``rows`` rows fill when each of them belongs to one of ``groups`` groups: a tile with one row
+    for every group that can have some, and a whole tile's rows more for each further one."""
+    some = min(rows, groups)
+    return some + (rows - some) // tile_rows
+
+
 def run_tiles(counts: torch.Tensor, max_tiles: int, tile_rows: int = GROUP_TILE_ROWS):
     """(start int32 [G], tiles int32 [max_tiles, 3]) for rows sorted by group with every group's run
     padded to whole tiles of ``tile_rows``: a group's first row, and per tile (group, first

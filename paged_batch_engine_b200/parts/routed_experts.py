@@ -156,7 +156,7 @@ class RoutedExperts(FeedForward):
         tc5 = ops.grouped_tc5_applies(x, self.w_gate_up, self.w_down)
         tile_rows = ops.GROUPED_TC5_ROWS if tc5 else ops.GROUP_TILE_ROWS
         counts, place = ops.expert_places(chosen, self.num_experts)
-        max_tiles = (T * self.top + tile_rows - 1) // tile_rows + self.num_experts
+        max_tiles = ops.most_run_tiles(T * self.top, self.num_experts, tile_rows)
         start, tiles = ops.run_tiles(counts, max_tiles, tile_rows)
         rows, weights = self._gathered(x, chosen, place, start, weights, total_rows=max_tiles * tile_rows)
         if tc5:

@@ -1,5 +1,7 @@
 """Which matrix-product kernel a projection of a step goes to: decided from the step's rows, the
 projection and the size of the matrix alone (no GPU needed to check the rule)."""
+import itertools
+
 import torch
 
 from paged_batch_engine_b200.csrc import ops
@@ -47,3 +49,19 @@ def test_skinny_and_tc5_rules(monkeypatch):
     monkeypatch.setattr(ops, "TC5_MASK", 4)
     assert ops.tc5_applies(_bf16(2048, 3584), w, 4) and not ops.tc5_applies(_bf16(2048, 3584), w, 1)
     assert not ops.tc5_applies(_bf16(ops.TC5_MIN_ROWS - 1, 3584), w, 4)
+
+
+def test_padded_rows_of_the_experts_are_as_many_as_can_be_filled():
+    """Few rows of many experts: a tile for every expert that a row can have chosen, not for every expert there is."""
+    def tiles(counts, rows):
+        return sum((c + rows - 1) // rows for c in counts)
+    for rows in (1, 3, 8):
+        for groups in (1, 2, 5):
+            for pairs in range(1, 30):
+                most = 0
+                for cut in itertools.combinations(range(pairs + groups - 1), groups - 1):     # all ways to share them out
+                    ends = (-1,) + cut + (pairs + groups - 1,)
+                    most = max(most, tiles([b - a - 1 for a, b in zip(ends, ends[1:])], rows))
+                assert ops.most_run_tiles(pairs, groups, rows) == most
+    assert ops.most_run_tiles(16 * 8, 512, 128) == 128                  # 16 rows, 8 of 512 experts
+    assert ops.most_run_tiles(2048 * 4, 32, 128) == 32 + (8192 - 32) // 128
