@@ -323,6 +323,15 @@ int columns_at_a_time(int N, int Kp) {
   return most < 256 ? (N < 256 ? N : 256) : (int)(N < most ? N : most);
 }
 
+// Rows of X whose terms are made at a time: all, unless they would take more than 256 MB, else groups of whole tiles and about
+// one size (2,304 rows and more for K up to 18,944, so that making W's terms once more for each costs a tenth at most).
+int rows_at_a_time(int M, int Kp) {
+  const long long most = (256LL << 20) / ((long long)TERMS * Kp * 2) / BM * BM;
+  if (M <= most || M <= BM) return M;
+  const long long groups = most < BM ? (M + BM - 1) / BM : (M + most - 1) / most;
+  return (int)(((M + groups - 1) / groups + BM - 1) / BM * BM);
+}
+
 // How M x N outputs over K are cut: the tiles' columns and the parts of K that take least by this count (microseconds, as
 // measured: a K block of a tile, its start and end, the parts' way through memory).
 struct Plan {
@@ -360,15 +369,18 @@ PBE_EXPORT int pbe_sgemm_tc5_rows(int M, int N, int K) {
   return plan_of(M - rest, N, Kp).us + stream_us < plan_of(M, N, Kp).us ? M - rest : M;
 }
 
-// Bytes of scratch memory, 256-byte aligned, that pbe_sgemm_tc5 needs: the flag, X's terms, W's terms, the parts' sums.
+// Bytes of scratch memory, 256-byte aligned, that pbe_sgemm_tc5 needs: the flag, X's terms, W's terms, the parts' sums; at
+// most 256 + 256 + 128 MB whatever M and N are (K up to 174,762, where 256 rows' or columns' terms take 256 MB).
 PBE_EXPORT long long pbe_sgemm_tc5_scratch(int M, int N, int K) {
-  const int Kp = padded(K), step = columns_at_a_time(N, Kp), last = N % step;
-  long long parts = part_bytes(plan_of(M, step, Kp), M, step);
-  if (last > 0) {
-    const long long more = part_bytes(plan_of(M, last, Kp), M, last);
-    if (more > parts) parts = more;
-  }
-  return 256 + aligned256((long long)M * TERMS * Kp * 2) + aligned256((long long)step * TERMS * Kp * 2) + parts;
+  const int Kp = padded(K), columns = columns_at_a_time(N, Kp), rows = rows_at_a_time(M, Kp);
+  long long parts = 0;
+  for (const int m : {rows, M % rows})                   // the groups' sizes
+    for (const int n : {columns, N % columns})
+      if (m > 0 && n > 0) {
+        const long long bytes = part_bytes(plan_of(m, n, Kp), m, n);
+        if (bytes > parts) parts = bytes;
+      }
+  return 256 + aligned256((long long)rows * TERMS * Kp * 2) + aligned256((long long)columns * TERMS * Kp * 2) + parts;
 }
 
 // X [M, K], W [N, K], Y [M, N], float32, contiguous.  Afterwards the first int of scratch says whether an element was not
@@ -380,32 +392,37 @@ PBE_EXPORT int pbe_sgemm_tc5(const float* X, const float* W, const float* bias, 
   if (K <= 0 || scratch == nullptr || ((uintptr_t)scratch & 255)) return (int)cudaErrorInvalidValue;
   if ((long long)M * TERMS > 0x7fffffffLL - 512 || (long long)N * TERMS > 0x7fffffffLL - 512 || K > 0x7fffffff - BK)
     return (int)cudaErrorInvalidValue;
-  const int Kp = padded(K), step = columns_at_a_time(N, Kp);
+  const int Kp = padded(K), columns = columns_at_a_time(N, Kp), rows = rows_at_a_time(M, Kp);
   int* flag = (int*)scratch;
   bf16* xt = (bf16*)((char*)scratch + 256);
-  bf16* wt = (bf16*)((char*)xt + aligned256((long long)M * TERMS * Kp * 2));
-  float* sums = (float*)((char*)wt + aligned256((long long)step * TERMS * Kp * 2));
+  bf16* wt = (bf16*)((char*)xt + aligned256((long long)rows * TERMS * Kp * 2));
+  float* sums = (float*)((char*)wt + aligned256((long long)columns * TERMS * Kp * 2));
   const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), stream);
   if (e != cudaSuccess) return (int)e;
-  int rc = split3(X, xt, M, K, Kp, flag, stream);
+  int rc = 0;
   CUtensorMap map_a, map_w;
-  if (rc == 0) rc = make_map(&map_a, xt, M * TERMS, Kp, BM);
-  for (int n0 = 0; n0 < N && rc == 0; n0 += step) {
-    const int n = N - n0 < step ? N - n0 : step;
-    rc = split3(W + (size_t)n0 * K, wt, n, K, Kp, flag, stream);
-    const Plan plan = plan_of(M, n, Kp);
-    if (rc == 0) rc = make_map(&map_w, wt, n * TERMS, Kp, plan.bn);
-    if (rc != 0) break;
-    const bool parts = plan.parts > 1;
-    float* y = parts ? sums : Y + n0;
-    const int ldy = parts ? n : N;
-    const float* b = bias ? bias + n0 : nullptr;
-    const ProductParams p{parts ? nullptr : b, y, M, n, Kp, ldy, (ldy % 4 == 0 && ((uintptr_t)y & 15) == 0) ? 1 : 0, plan.parts,
-                          plan.part_blocks, err};
-    rc = plan.bn == 128 ? launch_product<128>(map_a, map_w, p, stream) : launch_product<256>(map_a, map_w, p, stream);
-    if (rc == 0 && parts) {
-      add_parts_kernel<<<(unsigned)(((long long)M * n + 255) / 256), 256, 0, stream>>>(sums, plan.parts, b, Y + n0, M, n, N);
-      rc = launch_status();
+  for (int m0 = 0; m0 < M && rc == 0; m0 += rows) {
+    const int m = M - m0 < rows ? M - m0 : rows;
+    rc = split3(X + (size_t)m0 * K, xt, m, K, Kp, flag, stream);
+    if (rc == 0) rc = make_map(&map_a, xt, m * TERMS, Kp, BM);
+    for (int n0 = 0; n0 < N && rc == 0; n0 += columns) {
+      const int n = N - n0 < columns ? N - n0 : columns;
+      if (m0 == 0 || columns < N) rc = split3(W + (size_t)n0 * K, wt, n, K, Kp, flag, stream);
+      const Plan plan = plan_of(m, n, Kp);
+      if (rc == 0) rc = make_map(&map_w, wt, n * TERMS, Kp, plan.bn);
+      if (rc != 0) break;
+      const bool parts = plan.parts > 1;
+      float* out = Y + (size_t)m0 * N + n0;
+      float* y = parts ? sums : out;
+      const int ldy = parts ? n : N;
+      const float* b = bias ? bias + n0 : nullptr;
+      const ProductParams p{parts ? nullptr : b, y, m, n, Kp, ldy, (ldy % 4 == 0 && ((uintptr_t)y & 15) == 0) ? 1 : 0,
+                            plan.parts, plan.part_blocks, err};
+      rc = plan.bn == 128 ? launch_product<128>(map_a, map_w, p, stream) : launch_product<256>(map_a, map_w, p, stream);
+      if (rc == 0 && parts) {
+        add_parts_kernel<<<(unsigned)(((long long)m * n + 255) / 256), 256, 0, stream>>>(sums, plan.parts, b, out, m, n, N);
+        rc = launch_status();
+      }
     }
   }
   return rc;

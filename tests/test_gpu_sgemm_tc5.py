@@ -39,6 +39,26 @@ def test_against_64_bits(M, N, K):
         assert (got.double() - want).norm() <= (fma.double() - want).norm()
 
 
+@pytest.mark.parametrize("M,N,K", [(2433, 130, 18944), (4700, 3000, 18944), (1000, 64, 50000)])
+def test_rows_whose_terms_are_made_in_several_goes(M, N, K):
+    x, w, b = _inputs(M, N, K)
+    got = _product(_ops().sgemm_tc5, x, w, b)
+    want = torch.cat([x[i:i + 500].double() @ w.double().t() + b.double() for i in range(0, M, 500)])
+    # sums of K products of normal numbers, off by the roundings' random walk: see the first test for the worst
+    assert float((got.double() - want).norm() / want.norm()) <= 4e-7
+
+
+def test_scratch_memory_is_bounded():
+    """However many rows a step brings, and however many columns the matrix has."""
+    ops = _ops()
+    need = ops._fn("sgemm_tc5", "pbe_sgemm_tc5_scratch", [ops.c_int] * 3)
+    need.restype = ops.c_ll
+    for M in (65, 1000, 4096, 4097, 100000, 1 << 24):
+        for N in (64, 5000, 152064):
+            for K in (256, 1536, 18944, 65536):
+                assert need(M, N, K) <= (640 << 20) + 4096, (M, N, K)
+
+
 def test_numbers_that_are_not_finite():
     ops = _ops()
     x, w, b = _inputs(130, 200, 300)
