@@ -614,8 +614,12 @@ int map_rows(CUtensorMap* map, const void* at, long long rows, int columns, long
 int launch_wide(const CUtensorMap& a, const CUtensorMap& b, const AttnParams& p, const MaskedExtra& x, const LatentExtra& y,
                 long long blocks, int* err, cudaStream_t stream) {
   if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
-  const cudaError_t e = cudaFuncSetAttribute(attention_tc5_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-  if (e != cudaSuccess) return (int)e;
+  static bool opted = false;
+  if (!opted) {
+    const cudaError_t e = cudaFuncSetAttribute(attention_tc5_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
+    if (e != cudaSuccess) return (int)e;
+    opted = true;
+  }
   launch_k(attention_tc5_wide_kernel, (int)blocks, NTHREADS, SMEM_BYTES, stream, a, b, p, x, y, err);
   return launch_status();
 }

@@ -1925,7 +1925,8 @@ def masked_attention(q: torch.Tensor, k_pages: torch.Tensor, v_pages: torch.Tens
         window=int(mask_size or 0), split_keys=int(meta.split_keys), max_splits=int(meta.max_splits),
         tile_rows=int(meta.tile_rows), scale=float(scale), kinds=0, num_pages=int(k_pages.shape[0]))
     if tcgen05:
-        if bias is not None or not masked_tc5_applies(k_pages.dtype, D, E, page_tokens, scale):
+        if (bias is not None or k_pages.dtype != torch.bfloat16 or D != 128 or E != 128 or not scale > 0
+                or not tc5_attention_applies(128, page_tokens)):
             raise KernelError("masked_attention: the tcgen05 form does not take these operands")
         fn = _fn("attention_tc5_wide", "pbe_masked_attention_tc5",
                  [ctypes.POINTER(AttnParams), c_int, c_int, c_void_p, c_float, c_void_p, c_void_p, c_int, c_int, c_void_p,

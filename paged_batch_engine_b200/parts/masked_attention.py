@@ -120,6 +120,8 @@ class MaskedAttention(Mixer):
         self.dtype, self.device = dtype, device
         self.rot_freq = self.value_freq = self.sink_scores = None
         self.tile_rows = ops.masked_tile_rows(dtype, key_dim, value_dim)
+        # whether prompt portions can take the tcgen05 form, whatever the pages' size
+        self.tcgen05 = ops.masked_tc5_applies(dtype, key_dim, value_dim, 64, self.scale)
         self.w_in = self.b_in = self.w_o = self.b_o = self.q_gain = self.k_gain = self.bias_by_distance = None
         self.q_head_scale = None
 
@@ -220,17 +222,27 @@ class MaskedAttention(Mixer):
 
     # ---- compute
     def _long_rows(self, ctx) -> bool:
-        """Whether a portion's row sees enough keys for the tcgen05 form's larger start to pay: 100 rows without a
-        context 41 us on mma.sync and 43 there, 300 rows 62 and 50, 64 rows behind 2,048 134 and 87, but behind 2,048
-        in chunks of 512 (64 keys) 41 and 49."""
-        size = self.mask_size or 1 << 60
-        for n, length in zip(ctx.q_len_host.tolist(), ctx.seq_len_host.tolist()):
-            keys = min(length, size)
-            if self.mask == "chunk" and (length - 1) // size == (length - n) // size:
-                keys = (length - 1) % size + 1
-            if keys >= 192 and n * (self.num_heads // self.num_kv_heads) > 16:
-                return True
-        return False
+        """Whether a portion's row sees enough keys for the tcgen05 form's larger start to pay.  Layers of 16 heads over two
+        key/value heads, on the device (mma.sync -> tcgen05): 100 rows without a context 27 us and 28, 192 rows 37 and 29,
+        64 rows behind 2,048 68 and 47; in chunks of 512 with a gate 150 rows 42 and 43, 192 rows 43.5 and 42.9, 256 rows 48
+        and 44, 128 rows behind 2,048 (128 keys) 38 and 41, and with a single block a head group 16 rows behind 300 41 and
+        43, 17 rows behind 2,000 (481 keys) 47 and 40.  Asked once a step for all layers with this mask: a step of few rows
+        waits for the host, and each layer's look at the lengths was 3 us of 82."""
+        ratio = self.num_heads // self.num_kv_heads
+        kept = ctx.__dict__.setdefault("_long_rows", {})
+        kind = self.mask, self.mask_size, ratio, self.out_gate
+        long = kept.get(kind)
+        if long is None:
+            size, long = self.mask_size or 1 << 60, False
+            for n, length in zip(ctx.q_len_host.tolist(), ctx.seq_len_host.tolist()):
+                keys = min(length, size)
+                if self.mask == "chunk" and (length - 1) // size == (length - n) // size:
+                    keys = (length - 1) % size + 1
+                if keys >= (384 if self.out_gate and n * ratio <= 128 else 192) and n * ratio > 16:
+                    long = True
+                    break
+            kept[kind] = long
+        return long
 
     def forward(self, x, ctx, cache):
         H, G, D, E = self.num_heads, self.num_kv_heads, self.key_dim, self.value_dim
@@ -260,8 +272,8 @@ class MaskedAttention(Mixer):
                                     rot_freq=self.rot_freq, value_freq=self.value_freq)
         q, turn = q if self.rotate_values else (q, None)
         # prompt portions on tcgen05, but for the distance bias, whose loads a softmax thread a row would wait for
-        tc5 = (D == E == 128 and self.bias_by_distance is None and not getattr(ctx, "captured", False)
-               and self._long_rows(ctx) and ops.masked_tc5_applies(cache.k.dtype, D, E, ctx.page_tokens, self.scale))
+        tc5 = (self.tcgen05 and self.bias_by_distance is None and not getattr(ctx, "captured", False)
+               and self._long_rows(ctx) and ops.tc5_attention_applies(128, ctx.page_tokens))
         meta = ctx.attention_work(cache.group, H // G, self.tile_rows, self.mask_size, H, E)
         gate = proj[:, g_off:] if self.out_gate else None
         out = ops.masked_attention(q, cache.k, cache.v, meta, H, G, self.scale, self.mask, self.mask_size,

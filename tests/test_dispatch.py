@@ -1,7 +1,10 @@
 """Which matrix-product kernel a projection of a step goes to: decided from the step's rows, the
 projection and the size of the matrix alone (no GPU needed to check the rule)."""
 import itertools
+from types import SimpleNamespace
 
+import numpy as np
+import pytest
 import torch
 
 from paged_batch_engine_b200.csrc import ops
@@ -65,3 +68,46 @@ def test_padded_rows_of_the_experts_are_as_many_as_can_be_filled():
                 assert ops.most_run_tiles(pairs, groups, rows) == most
     assert ops.most_run_tiles(16 * 8, 512, 128) == 128                  # 16 rows, 8 of 512 experts
     assert ops.most_run_tiles(2048 * 4, 32, 128) == 32 + (8192 - 32) // 128
+
+
+def _masked_part(**options):
+    from paged_batch_engine_b200.config import PartSpec
+    from paged_batch_engine_b200.parts import build_part
+    return build_part("mixer", PartSpec("masked_attention", dict(
+        hidden_size=256, num_heads=16, num_kv_heads=2, key_dim=128, value_dim=128, scale=128 ** -0.5, eps=1e-6, **options)),
+        torch.bfloat16, torch.device("cpu"))
+
+
+def _lengths(rows, before):
+    return SimpleNamespace(q_len_host=np.array(rows), seq_len_host=np.array(rows) + np.array(before))
+
+
+@pytest.mark.parametrize("options,rows,before,long", [
+    (dict(mask="chunk", mask_size=512, out_gate=True), [150], [0], False),
+    (dict(mask="chunk", mask_size=512, out_gate=True), [192], [0], True),
+    (dict(mask="chunk", mask_size=512, out_gate=True), [16], [300], False),        # one block a head group, 316 keys
+    (dict(mask="chunk", mask_size=512, out_gate=True), [17], [2000], True),        # 481 of the chunk
+    (dict(mask="chunk", mask_size=512, out_gate=True), [128], [2048], False),      # a chunk of its own
+    (dict(mask="chunk", mask_size=512, out_gate=True), [100, 100, 1, 100], [0, 0, 4000, 0], False),
+    (dict(mask="window", mask_size=1024), [16], [300], True),
+    (dict(mask="window", mask_size=128), [700], [0], False),
+    (dict(), [1, 1, 2], [5000, 4000, 3000], False),
+    (dict(), [1, 64], [5000, 2048], True),
+])
+def test_masked_prompts_that_take_the_form_for_long_rows(options, rows, before, long):
+    part = _masked_part(**options)
+    assert part.tcgen05 and part._long_rows(_lengths(rows, before)) is long
+
+
+def test_a_steps_lengths_are_looked_at_once_for_all_layers():
+    """Not once a layer: a step of few rows waits for the host."""
+    class Lengths:
+        looks = 0
+
+        def tolist(self):
+            Lengths.looks += 1
+            return [300]
+    ctx = SimpleNamespace(q_len_host=Lengths(), seq_len_host=Lengths())
+    layers = [_masked_part() for _ in range(4)]
+    assert all(layer._long_rows(ctx) for layer in layers) and Lengths.looks == 2
+    assert not _masked_part(mask="window", mask_size=64)._long_rows(ctx) and Lengths.looks == 4     # another mask
