@@ -363,19 +363,18 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
 template <int D, int E>
 int launch_ssd(const SsdParams& p, int R, cudaStream_t stream) {
   const int smem = (int)ssd_smem<D, E>();
-  const cudaError_t e = cudaFuncSetAttribute(linear_attention_mma_kernel<D, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return (int)e;
+  static bool opted = false;
+  if (!opted) {
+    const cudaError_t e = cudaFuncSetAttribute(linear_attention_mma_kernel<D, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    opted = true;
+  }
   // without the programmatic dependency: few long-running blocks, which would else be placed several to a
   // multiprocessor while the kernel before still fills the others
   linear_attention_mma_kernel<D, E><<<dim3(R, p.H), THREADS, smem, stream>>>(p);
   return launch_status();
 }
 }  // namespace
-
-// Whether the kernel is there for these widths.
-PBE_EXPORT int pbe_linear_attention_mma_widths(int D, int E) {
-  return (D == 128 && E == 64) || (D == 64 && E == 64) || (D == 64 && E == 128) ? 1 : 0;
-}
 
 PBE_EXPORT int pbe_linear_attention_mma(const void* q, const void* k, const void* v, int ld, float* out, float* state,
                                         const float* decay, const int32_t* q_start, const int32_t* q_len,

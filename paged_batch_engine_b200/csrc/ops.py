@@ -365,16 +365,8 @@ def _column_slice(x: torch.Tensor, what: str):
         raise KernelError(f"{what}: operands are column slices of a row-major matrix")
 
 
-def linear_attention_matrix_applies(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, key_dim: int,
-                                    value_dim: int) -> bool:
-    """Whether the tensor-core form of ``linear_attention`` takes these operands: bfloat16 rows on 16-byte boundaries
-    and widths that it is built for.  It forms logarithms of the decays, so they must not be negative."""
-    if q.dtype != torch.bfloat16 or any(x.data_ptr() % 16 or (x.stride(0) % 8 and x.shape[0] > 1) for x in (q, k, v)):
-        return False
-    if q.shape[0] == 1 and q.stride(0) % 8:
-        return False
-    fn = _fn("linear_attention_mma", "pbe_linear_attention_mma_widths", [c_int, c_int])
-    return fn(int(key_dim), int(value_dim)) == 1
+# (key, value) widths of the tensor-core form's instances; it forms logarithms of the decays, so they must not be negative
+MATRIX_WIDTHS = ((128, 64), (64, 64), (64, 128))
 
 
 def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor, decay: torch.Tensor,
@@ -391,7 +383,7 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: t
     heads' constant decays (``decay`` may then be None), ``tok_scale`` float32 [T, H] multiplies v
     as it enters the state, ``skip`` float32 [H] adds skip_h v_t to the output, and ``kq_share``
     neighbouring heads read one q and k (q, k are then [T, H / kq_share * D]).  ``matrix``: run it as
-    products of matrices on the tensor cores (see ``linear_attention_matrix_applies``).
+    products of matrices on the tensor cores (bfloat16 rows on 16-byte boundaries, ``MATRIX_WIDTHS``).
     Returns float32 [T, H*E]."""
     _need_cuda(q, k, v, state, decay, q_start, q_len, slots, tok_decay, tok_scale, skip)
     _need_contiguous(tok_decay, tok_scale, skip)
@@ -425,21 +417,21 @@ def linear_attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: t
     if D > 512:
         raise KernelError(f"linear_attention: key width {D} per head is beyond 512")
     out = torch.empty((T, heads * E), dtype=torch.float32, device=q.device)
-    fn = _fn("linear_attention", "pbe_linear_attention",
-             [c_void_p, c_void_p, c_void_p, c_int, c_int] + [c_void_p] * 8 + [c_int, c_int, c_int, c_int, c_float, c_int,
-                                                                             c_void_p, c_void_p, c_void_p, c_int,
-                                                                             c_void_p, c_void_p])
     chunk_decay = None
-    if matrix and (silu or not linear_attention_matrix_applies(q, k, v, D, E)):
-        raise KernelError("linear_attention: no products of matrices for these operands")
-    fm = _fn("linear_attention_mma", "pbe_linear_attention_mma",
-             [c_void_p, c_void_p, c_void_p, c_int] + [c_void_p] * 8 + [c_int, c_int, c_int, c_int, c_float, c_void_p,
-                                                                      c_void_p, c_void_p, c_int, c_void_p, c_void_p]) \
-        if matrix else None
+    if matrix:                      # that its rows lie on 16-byte boundaries the launch checks
+        if silu or q.dtype != torch.bfloat16 or (D, E) not in MATRIX_WIDTHS:
+            raise KernelError("linear_attention: no products of matrices for these operands")
+        fn = _fn("linear_attention_mma", "pbe_linear_attention_mma",
+                 [c_void_p, c_void_p, c_void_p, c_int] + [c_void_p] * 8 + [c_int, c_int, c_int, c_int, c_float, c_void_p,
+                                                                          c_void_p, c_void_p, c_int, c_void_p, c_void_p])
+    else:
+        fn = _fn("linear_attention", "pbe_linear_attention",
+                 [c_void_p, c_void_p, c_void_p, c_int, c_int] + [c_void_p] * 8
+                 + [c_int, c_int, c_int, c_int, c_float, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p])
 
     def launch(result, items, scratch, n):
         if matrix:
-            _check(fm(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(result), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(q_len),
+            _check(fn(_ptr(q), _ptr(k), _ptr(v), ld, _ptr(result), _ptr(state), _ptr(decay), _ptr(q_start), _ptr(q_len),
                       _ptr(slots), _ptr(items), _ptr(scratch), n, heads, D, E, float(k_scale), _ptr(tok_decay),
                       _ptr(tok_scale), _ptr(skip), int(kq_share), _ptr(chunk_decay), _stream()), "linear_attention")
             return

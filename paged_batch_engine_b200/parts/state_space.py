@@ -50,6 +50,8 @@ class SelectiveStateSpace(Mixer):
         self.inner = num_heads * head_dim
         self.conv_channels = self.inner + 2 * groups * state_dim
         self.dtype, self.device = dtype, device
+        # whether prompt portions take the tensor-core form: its widths put every row of x, B and C on 16-byte boundaries
+        self.matrix = dtype == torch.bfloat16 and (state_dim, head_dim) in ops.MATRIX_WIDTHS
         self.w_in = self.w_o = self.conv_w = self.conv_b = self.dt_bias = self.a_log = self.skip = self.gain = None
 
     def cache_need(self):
@@ -60,7 +62,7 @@ class SelectiveStateSpace(Mixer):
         return CompositeNeed.of(**need)
 
     def kernel_libraries(self, dtype):
-        matrix = [("linear_attention_mma", None)] if dtype == torch.bfloat16 else []
+        matrix = [("linear_attention_mma", None)] if self.matrix else []
         return [("short_conv", None), ("linear_attention", None), ("streams", None)] + matrix + ops.gemm_libraries(dtype)
 
     def param_specs(self, prefix):
@@ -108,7 +110,7 @@ class SelectiveStateSpace(Mixer):
         xs, B, Cm = xbc[:, :inner], xbc[:, inner:inner + G * N], xbc[:, inner + G * N:]
         # prompt portions on the tensor cores, in chunks of 64 tokens; a step of mostly single tokens is faster as the
         # plain recurrence
-        matrix = ctx.num_tokens >= 8 * ctx.num_requests and ops.linear_attention_matrix_applies(Cm, B, xs, N, P)
+        matrix = self.matrix and ctx.num_tokens >= 8 * ctx.num_requests
         plan = None if getattr(ctx, "captured", False) else ctx.recurrence_plan(self.chunk_rows(ctx.num_tokens, matrix))
         y = ops.linear_attention(Cm, B, xs, cache.sub["ssm"].state, None, ctx.q_start, ctx.q_len, ctx.state_slots,
                                  ctx.num_requests, H, 1.0, False, plan, tok_decay=decay, tok_scale=dt,

@@ -111,3 +111,18 @@ def test_a_steps_lengths_are_looked_at_once_for_all_layers():
     layers = [_masked_part() for _ in range(4)]
     assert all(layer._long_rows(ctx) for layer in layers) and Lengths.looks == 2
     assert not _masked_part(mask="window", mask_size=64)._long_rows(ctx) and Lengths.looks == 4     # another mask
+
+
+@pytest.mark.parametrize("state,head,dtype,matrix", [(128, 64, torch.bfloat16, True), (64, 64, torch.bfloat16, True),
+                                                     (64, 128, torch.bfloat16, True), (128, 128, torch.bfloat16, False),
+                                                     (128, 64, torch.float32, False), (32, 64, torch.bfloat16, False)])
+def test_state_space_form_is_known_from_the_widths(state, head, dtype, matrix):
+    """At construction: a step's rows lie on 16-byte boundaries for these widths, and looking was 10 us of a layer's 120."""
+    from paged_batch_engine_b200.config import PartSpec
+    from paged_batch_engine_b200.parts import build_part
+    part = build_part("mixer", PartSpec("selective_state_space", dict(
+        hidden_size=256, num_heads=4, head_dim=head, state_dim=state, groups=1, conv_taps=4, norm_groups=4, eps=1e-6)),
+        dtype, torch.device("cpu"))
+    assert part.matrix is matrix
+    assert (("linear_attention_mma", None) in part.kernel_libraries(dtype)) is matrix
+    assert not matrix or all(n % 8 == 0 for n in (part.inner, part.groups * state, part.conv_channels))
