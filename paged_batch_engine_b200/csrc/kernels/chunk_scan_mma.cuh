@@ -297,8 +297,12 @@ template <int DP, bool CORRECT, bool OWN, typename TU>
 int launch(const ChunkScanParams<TU>& p, int items, cudaStream_t stream) {
   constexpr int smem = 2 * buffer_bytes<DP, CORRECT>();
   auto kernel = scan_chunks_mma_kernel<DP, CORRECT, OWN, TU>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return (int)e;
+  static bool opted = false;
+  if (!opted) {
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;
+    opted = true;
+  }
   launch_spread(kernel, dim3(items, p.H, (p.E + COLS - 1) / COLS), 256, smem, stream, p);
   return launch_status();
 }
