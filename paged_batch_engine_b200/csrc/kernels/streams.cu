@@ -204,7 +204,7 @@ __global__ void gated_rms_kernel(GatedRmsParams p) {
 // The same over each head, heads of whole groups of four values: a warp a head of a row, four neighbouring values a
 // lane and access, everything of a head requested at once and kept in registers between the sum and the result (the
 // kernel above reads every value and makes every gate twice, 4 bytes an access: 2,048 rows of 4,096 in eight parts
-// 45 -> 15 us).  Gates of rows that are rounded to bfloat16 take the fast exponential and division.
+// 45 -> 16 us).
 constexpr int GR_WARPS = 8;
 
 __device__ __forceinline__ float4 load_four(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(32 * GR_WARPS) gated_rms_heads_kernel(GatedRms
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       const float gv = gate[i][k];
-      const float sg = sizeof(T) == 2 ? __fdividef(1.0f, 1.0f + __expf(-gv)) : 1.0f / (1.0f + expf(-gv));
+      const float sg = 1.0f / (1.0f + expf(-gv));
       gate[i][k] = p.gate_act ? gv * sg : sg;
       if (p.gate_first) v[i][k] *= gate[i][k];
       ss += v[i][k] * v[i][k];

@@ -106,3 +106,21 @@ def test_gated_norm_per_head(E, gate_first, dtype, gate_dtype):
             want = n.reshape(T, H * E) * gain.double() * (1.0 if gate_first else s)
             tol = 2 ** -8 if dtype == torch.bfloat16 else 2e-6
             assert ((got - want).abs() <= tol * (want.abs() + 1e-3)).all()
+
+
+@pytest.mark.parametrize("E", [64, 512])
+@pytest.mark.parametrize("gate_dtype", [torch.float32, torch.bfloat16])
+def test_gates_that_are_almost_closed(E, gate_dtype):
+    """Gates so negative that their sigmoid is close to float32's smallest normal number, with rows that are rounded to
+    bfloat16 and bring the result back to an ordinary size."""
+    from paged_batch_engine_b200.csrc import ops
+    T, H = 5, 2
+    g = torch.Generator(device=DEV).manual_seed(E)
+    gate = (-80.0 - 8.5 * torch.rand(T, H * E, device=DEV, generator=g)).to(gate_dtype)
+    o = torch.rand(T, H * E, device=DEV, generator=g) + 0.5
+    gain = torch.full((H * E,), 1e30, device=DEV)
+    got = ops.gated_rms(o, gate, gain, H, 1e-6, True, "silu", torch.bfloat16).double()
+    n = o.double().view(T, H, E) / torch.sqrt((o.double().view(T, H, E) ** 2).mean(-1, keepdim=True) + 1e-6)
+    want = n.reshape(T, H * E) * 1e30 * gate.double() * torch.sigmoid(gate.double())
+    # the sigmoid may lie just below 2^-126, where a number holds 22 bits and more; the result is rounded to bfloat16
+    assert ((got - want).abs() <= (2 ** -8 + 2 ** -16) * want.abs()).all()
