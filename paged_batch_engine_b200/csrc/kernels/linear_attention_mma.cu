@@ -5,9 +5,10 @@
 //   o_i = 2^c_i S^T q_i + sum_{j<=i} (q_i . k_j) 2^(c_i - c_j) s_j v_j + skip v_i
 //   S  <- 2^c_last S + sum_j k_j (2^(c_last - c_j) s_j v_j)^T
 // q, k and v are bfloat16 and exact in the products; what is float32 (the state as it is read, the weights of the
-// second sum, the scaled v) enters them as two bfloat16 terms, hi + lo, and the state itself stays in float32
-// accumulators.  Sums of logarithms and their differences are taken in double (a decay of zero counts as 2^-400),
-// so a weight keeps float32's accuracy however strong the decays before it are.
+// second sum, the weighted k of the third) enters them as three bfloat16 terms, which hold all of its 24 bits, and the
+// state itself stays in float32: products are summed from zero, four or twelve of them, and added with one rounding.  Sums of
+// logarithms and their differences are taken in double (a decay of zero counts as 2^-400), so a weight keeps float32's
+// accuracy however strong the decays before it are.
 //
 // A product multiplies the zero weight of a later token with that token's values too, so values that are not finite would
 // reach back to the tokens before theirs: a chunk that has some takes the products of a row tile with its own tokens one
@@ -17,19 +18,20 @@
 // state in registers; o's weights pass from score accumulators to operands in registers.  Two blocks a multiprocessor
 // (99 KB at 128 x 64) fill each other's barriers and copies.  Work items cut long portions as in
 // linear_attention.cu: a pass without outputs leaves each item's own contribution and decay product.
-// 2,048 tokens, 64 heads of 128 x 64 over 8 groups (both passes): 104 us against 823 of the recurrence token by token;
-// 512 tokens 113 us the whole layer, 100 tokens 55.
-#include <cuda_bf16.h>
-
+// 2,048 tokens, 64 heads of 128 x 64 over 8 groups (both passes): 148 us against 823 of the recurrence token by token.  Two
+// terms a factor, the weighted v in shared memory, took 104, but outputs and state were 10 to 30 times further off 64 bits
+// than the recurrence's (1 to 3e-7); now they are 0.6 to 1.2 times.
 #include "common.cuh"
+#include "mma_sync.cuh"
 #include "pdl.cuh"
 
 using namespace pbe;
+using namespace pbe::mma_sync;
 
 namespace {
-typedef __nv_bfloat16 bf16;
 constexpr int L = 64;                     // tokens of a chunk
 constexpr int THREADS = 128;
+constexpr int RUN = 4;                    // products a sum is left to the tensor cores for, which cut off what does not fit it
 constexpr double LOG2_ZERO = -400.0;      // of a decay that has underflowed: 2^-400 is 0 in float32
 
 struct SsdParams {
@@ -54,34 +56,9 @@ struct SsdParams {
   float* chunk_decay;       // [entries, H] or null
 };
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void ldm4(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)) : "memory");
-}
-__device__ __forceinline__ void ldm4t(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)) : "memory");
-}
-__device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void split2(float x, float y, unsigned& hi, unsigned& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  const float2 f = __bfloat1622float2(h);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-  hi = *reinterpret_cast<const unsigned*>(&h);
-  lo = *reinterpret_cast<const unsigned*>(&l);
-}
-
 template <int D, int E>
 constexpr size_t ssd_smem() {
-  return 2 * (2 * (size_t)L * (D + 8) + 3 * (size_t)L * (E + 8) + 2 * (size_t)D * (E + 8));
+  return 2 * (2 * (size_t)L * (D + 8) + (size_t)L * (E + 8) + TERMS * (size_t)D * (E + 8));
 }
 
 template <int D, int E>
@@ -93,13 +70,11 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
   bf16* Qs = reinterpret_cast<bf16*>(smem_raw);        // [L][QSTR]
   bf16* Ks = Qs + L * QSTR;
   bf16* Vs = Ks + L * QSTR;                            // [L][VSTR]
-  bf16* Vh = Vs + L * VSTR;                            // v times its weight in the state, hi and lo
-  bf16* Vl = Vh + L * VSTR;
-  bf16* Sh = Vl + L * VSTR;                            // [D][VSTR] the state at the chunk's start, hi and lo
-  bf16* Sl = Sh + D * VSTR;
+  bf16* Ss = Vs + L * VSTR;                            // [TERMS][D][VSTR] the terms of the state at the chunk's start
   __shared__ float cs_hi[L], cs_lo[L];                 // the sums of logarithms, as two floats
   __shared__ float factor[L], into[L], from[L];        // s_j; its weight in the new state; 2^c_i
   __shared__ double half_total, total;
+  __shared__ float keep_all;                           // 2^total
 
   const int h = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -184,24 +159,27 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
         for (int j = 0; j < E / 8; ++j)
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            unsigned hi, lo;
-            split2(S[m][j][2 * hh], S[m][j][2 * hh + 1], hi, lo);
+            unsigned t[TERMS];
+            split3(S[m][j][2 * hh], S[m][j][2 * hh + 1], t);
             const int at = (warp * (D / 4) + m * 16 + g8 + hh * 8) * VSTR + j * 8 + q2;
-            *reinterpret_cast<unsigned*>(Sh + at) = hi;
-            *reinterpret_cast<unsigned*>(Sl + at) = lo;
+#pragma unroll
+            for (int i = 0; i < TERMS; ++i) *reinterpret_cast<unsigned*>(Ss + i * D * VSTR + at) = t[i];
           }
     }
     __syncthreads();
     if (tid < L) {
       if (tid >= 32) c += half_total;
-      if (tid == L - 1) total = c;
+      if (tid == L - 1) {
+        total = c;
+        keep_all = (float)exp2(c);
+      }
       cs_hi[tid] = (float)c;
       cs_lo[tid] = (float)(c - (double)(float)c);
-      from[tid] = exp2f((float)c);
+      from[tid] = (float)exp2(c);
     }
     __syncthreads();
-    if (tid < L) into[tid] = factor[tid] * exp2f((float)(total - c));
-    const float keep = exp2f((float)total);
+    if (tid < L) into[tid] = factor[tid] * (float)exp2(total - c);
+    const float keep = keep_all;
     log_all += total;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     bool odd = false;                                  // values that are not finite, among those this thread fetched
@@ -213,37 +191,37 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
       for (int k = 0; k < 4; ++k) odd = odd || (x[k] & 0x7f80u) == 0x7f80u || (x[k] & 0x7f800000u) == 0x7f800000u;
     }
     odd = __syncthreads_or(odd) != 0;
-    // v times its weight in the new state
-    for (int i = tid; i < L * (E / 8); i += THREADS) {
-      const int row = i / (E / 8), at = row * VSTR + (i - row * (E / 8)) * 8;
-      const float w = into[row];
-      const uint4 raw = *reinterpret_cast<const uint4*>(Vs + at);
-      const unsigned x[4] = {raw.x, raw.y, raw.z, raw.w};
-      unsigned hi[4], lo[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) split2(__uint_as_float(x[k] << 16) * w, __uint_as_float(x[k] & 0xffff0000u) * w, hi[k], lo[k]);
-      *reinterpret_cast<uint4*>(Vh + at) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-      *reinterpret_cast<uint4*>(Vl + at) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
-    }
     if (outputs && warp * 16 < left) {
       const int r0 = warp * 16 + g8;                   // this thread's rows: r0 and r0 + 8
-      unsigned q[D / 16][4];
+      auto queries = [&](unsigned (&q)[RUN][4], int k0) {
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk) ldm4(q[kk], Qs + (warp * 16 + lrow) * QSTR + kk * 16 + lcol);
+        for (int k = 0; k < RUN; ++k) ldm4(q[k], Qs + (warp * 16 + lrow) * QSTR + (k0 + k) * 16 + lcol);
+      };
       float o[E / 8][4];
 #pragma unroll
       for (int j = 0; j < E / 8; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+#pragma unroll 1
+      for (int i = TERMS - 1; i >= 0; --i)             // the small terms' sums first
+#pragma unroll 1
+        for (int k0 = 0; k0 < D / 16; k0 += RUN) {
+          unsigned q[RUN][4];
+          queries(q, k0);
 #pragma unroll
-      for (int kk = 0; kk < D / 16; ++kk)
+          for (int j = 0; j < E / 16; ++j) {
+            float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-        for (int j = 0; j < E / 16; ++j) {
-          unsigned b[4], d[4];
-          ldm4t(b, Sh + (kk * 16 + lrow) * VSTR + j * 16 + lcol);
-          ldm4t(d, Sl + (kk * 16 + lrow) * VSTR + j * 16 + lcol);
-          mma(o[2 * j], q[kk], b[0], b[1]);
-          mma(o[2 * j + 1], q[kk], b[2], b[3]);
-          mma(o[2 * j], q[kk], d[0], d[1]);
-          mma(o[2 * j + 1], q[kk], d[2], d[3]);
+            for (int k = 0; k < RUN; ++k) {
+              unsigned b[4];
+              ldm4t(b, Ss + i * D * VSTR + ((k0 + k) * 16 + lrow) * VSTR + j * 16 + lcol);
+              mma(y[0], q[k], b[0], b[1]);
+              mma(y[1], q[k], b[2], b[3]);
+            }
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+              o[2 * j][c] += y[0][c];
+              o[2 * j + 1][c] += y[1][c];
+            }
+          }
         }
       const float f0 = from[r0], f1 = from[r0 + 8];
 #pragma unroll
@@ -256,13 +234,24 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
       for (int jt = 0; jt <= warp; ++jt) {             // sixteen tokens j at a time, up to the rows' own
         float g[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-        for (int kk = 0; kk < D / 16; ++kk) {
-          unsigned b[4];
-          ldm4(b, Ks + (jt * 16 + krow) * QSTR + kk * 16 + kcol);
-          mma(g[0], q[kk], b[0], b[1]);
-          mma(g[1], q[kk], b[2], b[3]);
+        for (int k0 = 0; k0 < D / 16; k0 += RUN) {
+          unsigned q[RUN][4];
+          queries(q, k0);
+          float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+          for (int k = 0; k < RUN; ++k) {
+            unsigned b[4];
+            ldm4(b, Ks + (jt * 16 + krow) * QSTR + (k0 + k) * 16 + kcol);
+            mma(y[0], q[k], b[0], b[1]);
+            mma(y[1], q[k], b[2], b[3]);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            g[0][c] += y[0][c];
+            g[1][c] += y[1][c];
+          }
         }
-        unsigned hi[4], lo[4];
+        unsigned w[TERMS][4];
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
           const int j = jt * 16 + t * 8 + q2;
@@ -272,8 +261,13 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
             g[t][x] = j + x <= r0 ? g[t][x] * (s * exp2f((hi0 - chi) + (lo0 - clo))) : 0.f;
             g[t][2 + x] = j + x <= r0 + 8 ? g[t][2 + x] * (s * exp2f((hi1 - chi) + (lo1 - clo))) : 0.f;
           }
-          split2(g[t][0], g[t][1], hi[2 * t], lo[2 * t]);
-          split2(g[t][2], g[t][3], hi[2 * t + 1], lo[2 * t + 1]);
+#pragma unroll
+          for (int hh = 0; hh < 2; ++hh) {
+            unsigned terms[TERMS];
+            split3(g[t][2 * hh], g[t][2 * hh + 1], terms);
+#pragma unroll
+            for (int i = 0; i < TERMS; ++i) w[i][2 * t + hh] = terms[i];
+          }
         }
         if (odd && jt == warp) {
 #pragma unroll
@@ -300,10 +294,17 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
         for (int j = 0; j < E / 16; ++j) {
           unsigned b[4];
           ldm4t(b, Vs + (jt * 16 + lrow) * VSTR + j * 16 + lcol);
-          mma(o[2 * j], hi, b[0], b[1]);
-          mma(o[2 * j + 1], hi, b[2], b[3]);
-          mma(o[2 * j], lo, b[0], b[1]);
-          mma(o[2 * j + 1], lo, b[2], b[3]);
+          float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+          for (int i = TERMS - 1; i >= 0; --i) {
+            mma(y[0], w[i], b[0], b[1]);
+            mma(y[1], w[i], b[2], b[3]);
+          }
+#pragma unroll
+          for (int c = 0; c < 4; ++c) {
+            o[2 * j][c] += y[0][c];
+            o[2 * j + 1][c] += y[1][c];
+          }
         }
       }
 #pragma unroll
@@ -318,31 +319,42 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
         }
       }
     }
-    __syncthreads();                                   // the weighted v
+    // the chunk's writes: k times its weight in the new state, split in registers, times v
 #pragma unroll
-    for (int m = 0; m < MT; ++m)
+    for (int m = 0; m < MT; ++m) {
+      unsigned a[L / 16][TERMS][4];
 #pragma unroll
-      for (int j = 0; j < E / 8; ++j)
+      for (int kk = 0; kk < L / 16; ++kk) {
+        if (kk * 16 >= left) break;                    // tokens that do not exist weigh nothing
+        unsigned x[4];
+        ldm4t(x, Ks + (kk * 16 + krow) * QSTR + warp * (D / 4) + m * 16 + kcol);
 #pragma unroll
-        for (int x = 0; x < 4; ++x) S[m][j][x] *= keep;
+        for (int c = 0; c < 4; ++c) {
+          const int t = kk * 16 + (c >> 1) * 8 + q2;         // the tokens of this register's pair
+          unsigned terms[TERMS];
+          split3(__uint_as_float(x[c] << 16) * into[t], __uint_as_float(x[c] & 0xffff0000u) * into[t + 1], terms);
 #pragma unroll
-    for (int kk = 0; kk < L; kk += 16) {
-      if (kk >= left) break;                           // tokens that do not exist weigh nothing
-      unsigned a[MT][4];
-#pragma unroll
-      for (int m = 0; m < MT; ++m) ldm4t(a[m], Ks + (kk + krow) * QSTR + warp * (D / 4) + m * 16 + kcol);
+          for (int i = 0; i < TERMS; ++i) a[kk][i][c] = terms[i];
+        }
+      }
 #pragma unroll
       for (int j = 0; j < E / 16; ++j) {
-        unsigned b[4], d[4];
-        ldm4t(b, Vh + (kk + lrow) * VSTR + j * 16 + lcol);
-        ldm4t(d, Vl + (kk + lrow) * VSTR + j * 16 + lcol);
+        float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-        for (int m = 0; m < MT; ++m) {
-          mma(S[m][2 * j], a[m], b[0], b[1]);
-          mma(S[m][2 * j + 1], a[m], b[2], b[3]);
-          mma(S[m][2 * j], a[m], d[0], d[1]);
-          mma(S[m][2 * j + 1], a[m], d[2], d[3]);
+        for (int kk = 0; kk < L / 16; ++kk) {
+          if (kk * 16 >= left) break;
+          unsigned b[4];
+          ldm4t(b, Vs + (kk * 16 + lrow) * VSTR + j * 16 + lcol);
+#pragma unroll
+          for (int i = TERMS - 1; i >= 0; --i) {
+            mma(y[0], a[kk][i], b[0], b[1]);
+            mma(y[1], a[kk][i], b[2], b[3]);
+          }
         }
+#pragma unroll
+        for (int t = 0; t < 2; ++t)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) S[m][2 * j + t][c] = fmaf(keep, S[m][2 * j + t][c], y[t][c]);
       }
     }
   }
