@@ -1,6 +1,8 @@
 // The scan over chunks of sixteen tokens (chunk_scan.cuh: the same records, the same recurrence) on the tensor cores,
-// for bfloat16 runs: mma.sync m16n8k16, a float32 factor as two bfloat16 terms, a product of two such factors as three
-// (hi hi + hi lo + lo hi, what is left out is 2^-16 of it), float32 sums.
+// for bfloat16 runs: mma.sync m16n8k16, a float32 factor as three bfloat16 terms h + m + l, which hold its 24 bits, a
+// product of two such factors as six (h h, h m, m h, m m, h l, l h; what is left out is 2^-24 of it at most), float32 sums.
+// The tensor cores cut off what does not fit a sum instead of rounding it, so the state is not left to them: what a chunk
+// writes is summed from zero and added to the state with one rounding.
 //
 // A block takes 64 columns of a head's state: warps 0-3 compute, sixteen columns each, whose [16, D] piece of S^T stays in
 // float32 accumulators and turns into an operand in registers; warps 4-7 fetch the next chunk's record and values,
@@ -8,57 +10,57 @@
 //   [W | QG]: S^T (as it lies) times the records' vectors, two tiles of eight tokens each;
 //   u = U - S^T W;   o = S^T QG + u MQ;   S^T <- decays S^T + u KD.
 // What binds the scan of chunk_scan.cuh is the shared-memory pipe (every half warp reads the whole record for its
-// two or four columns); here sixteen columns share each fragment.  Delta rule, 1,100 + 37 + 911 tokens, 16 heads of
-// 128 x 128: 264 -> 91 us (the longest request's 69 chunks, 1.3 us each); time mixing, 2,048 tokens in segments, both
-// passes: 118 -> 77 us.  Against 64 bits on given inputs the read-outs are 5e-6 off (1e-7 in float32 multiply-adds);
-// the layers, whose inputs are bfloat16, 0.004 either way.
+// two or four columns); here sixteen columns share each fragment, and the 300 products of a chunk and computing warp bind.
+// Delta rule, 1,100 + 37 + 911 tokens, 16 heads of 128 x 128: 264 -> 157 us (the longest request's 69 chunks, 2.3 us each);
+// time mixing, 2,048 tokens in segments, both passes: 118 -> 95 us.  Two terms a factor took 91 and 77, but read-outs and
+// state were 5e-6 off 64 bits on given inputs; the multiply-adds are 0.5e-7 to 5e-7 off and this 0.6 to 1.4 times that.
 #pragma once
-#include <cuda_bf16.h>
-
 #include "chunk_scan.cuh"
+#include "mma_sync.cuh"
 
 namespace pbe {
 namespace scan_mma {
 
-typedef __nv_bfloat16 bf16;
+using namespace mma_sync;
+
 constexpr int COLS = 64;                 // columns of a block
 constexpr int USTR = COLS + 4;           // floats a row of U: four rows apart start in different banks
 constexpr int MSTR = CH + 8;             // elements a row of MQ
 
 template <int DP>
 __host__ __device__ constexpr int row_elems() { return DP + 8; }
-// one buffer: QG, KD and W as hi and lo [CH][DP + 8], MQ as hi and lo [CH][MSTR], the decays [DP], U [CH][USTR]
+// one buffer: QG, KD and W as terms [CH][DP + 8], MQ as terms [CH][MSTR], the decays [DP], U [CH][USTR]
 template <int DP, bool CORRECT>
 __host__ __device__ constexpr int buffer_bytes() {
-  return 2 * 2 * ((CORRECT ? 3 : 2) * CH * row_elems<DP>() + CH * MSTR) + 4 * (DP + CH * USTR);
+  return 2 * TERMS * ((CORRECT ? 3 : 2) * CH * row_elems<DP>() + CH * MSTR) + 4 * (DP + CH * USTR);
 }
 
-__device__ __forceinline__ unsigned at_smem(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void ldm4(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at_smem(p)) : "memory");
-}
-__device__ __forceinline__ void ldm4t(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(at_smem(p)) : "memory");
-}
-__device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-__device__ __forceinline__ void split2(float x, float y, unsigned& hi, unsigned& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  hi = *reinterpret_cast<const unsigned*>(&h);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(x - __uint_as_float(hi << 16), y - __uint_as_float(hi & 0xffff0000u));
-  lo = *reinterpret_cast<const unsigned*>(&l);
-}
 // two tiles of eight columns of C as the A operand of sixteen steps of k
-__device__ __forceinline__ void as_operand(const float (&c0)[4], const float (&c1)[4], unsigned (&hi)[4], unsigned (&lo)[4]) {
-  split2(c0[0], c0[1], hi[0], lo[0]);
-  split2(c0[2], c0[3], hi[1], lo[1]);
-  split2(c1[0], c1[1], hi[2], lo[2]);
-  split2(c1[2], c1[3], hi[3], lo[3]);
+__device__ __forceinline__ void as_operand(const float (&c0)[4], const float (&c1)[4], unsigned (&a)[TERMS][4]) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    unsigned t[TERMS];
+    split3(k < 2 ? c0[2 * k] : c1[2 * k - 4], k < 2 ? c0[2 * k + 1] : c1[2 * k - 3], t);
+#pragma unroll
+    for (int i = 0; i < TERMS; ++i) a[i][k] = t[i];
+  }
+}
+// The products of terms x of A and y of B that count, x + y < 3: the small ones are added apart from h h, so that they are
+// not cut off against it.  B: sixteen k times sixteen columns, its terms `apart` elements from one another.
+template <bool TRANSPOSED, bool A_EXACT = false>
+__device__ __forceinline__ void products(float (&big)[2][4], float (&small)[2][4], const unsigned (&a)[TERMS][4], const bf16* at,
+                                         int apart) {
+#pragma unroll
+  for (int y = TERMS - 1; y >= 0; --y) {
+    unsigned b[4];
+    if (TRANSPOSED) ldm4t(b, at + y * apart);
+    else ldm4(b, at + y * apart);
+#pragma unroll
+    for (int x = (A_EXACT ? 0 : TERMS - 1 - y); x >= 0; --x) {
+      mma(x + y == 0 ? big[0] : small[0], a[x], b[0], b[1]);
+      mma(x + y == 0 ? big[1] : small[1], a[x], b[2], b[3]);
+    }
+  }
 }
 
 template <int DP, bool CORRECT, bool OWN, typename TU>
@@ -69,7 +71,7 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
   constexpr int BYTES = buffer_bytes<DP, CORRECT>();
   constexpr int PER = (REC / 4 + 127) / 128;             // float4s of a record a fetching thread takes
   constexpr int UPER = CH * COLS / 128;
-  constexpr bool U_EXACT = sizeof(TU) == 2 && !CORRECT;  // u is a bfloat16 number: its second term is zero
+  constexpr bool U_EXACT = sizeof(TU) == 2 && !CORRECT;  // u is a bfloat16 number: its other terms are zero
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_launch_dependents();
   pdl_wait();
@@ -92,10 +94,10 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
   const int q0 = p.q_start[r];
   const float* rec0 = p.records + ((size_t)(first_record(q0, r) + (t0 - q0) / CH) * H + h) * REC;
   auto matrix = [&](int buf, int which, int term) {
-    return reinterpret_cast<bf16*>(smem_raw + buf * BYTES) + (which * 2 + term) * CH * STR;
+    return reinterpret_cast<bf16*>(smem_raw + buf * BYTES) + (which * TERMS + term) * CH * STR;
   };
-  auto mixed = [&](int buf, int term) { return reinterpret_cast<bf16*>(smem_raw + buf * BYTES) + MATS * 2 * CH * STR + term * CH * MSTR; };
-  auto decays = [&](int buf) { return reinterpret_cast<float*>(smem_raw + buf * BYTES + 2 * 2 * (MATS * CH * STR + CH * MSTR)); };
+  auto mixed = [&](int buf, int term) { return reinterpret_cast<bf16*>(smem_raw + buf * BYTES) + MATS * TERMS * CH * STR + term * CH * MSTR; };
+  auto decays = [&](int buf) { return reinterpret_cast<float*>(smem_raw + buf * BYTES + 2 * TERMS * (MATS * CH * STR + CH * MSTR)); };
   auto values = [&](int buf) { return decays(buf) + DP; };
 
   if (tid >= 128) {
@@ -119,20 +121,20 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
       for (int i = 0; i < PER; ++i) {
         const int x = (ft + i * 128) * 4;
         if (x >= REC) break;
-        uint2 hi, lo;
-        split2(raw[i].x, raw[i].y, hi.x, lo.x);
-        split2(raw[i].z, raw[i].w, hi.y, lo.y);
+        unsigned t0[TERMS], t1[TERMS];
+        split3(raw[i].x, raw[i].y, t0);
+        split3(raw[i].z, raw[i].w, t1);
         if (x < rec_decay(DP) || (CORRECT && x >= rec_w(DP))) {
           const int y = x < rec_decay(DP) ? x : x - rec_w(DP) + 2 * CH * DP;       // QG, KD, W in a row
           const int which = y / (CH * DP), row = (y / DP) % CH, at = row * STR + y % DP;
-          *reinterpret_cast<uint2*>(matrix(buf, which, 0) + at) = hi;
-          *reinterpret_cast<uint2*>(matrix(buf, which, 1) + at) = lo;
+#pragma unroll
+          for (int t = 0; t < TERMS; ++t) *reinterpret_cast<uint2*>(matrix(buf, which, t) + at) = make_uint2(t0[t], t1[t]);
         } else if (x < rec_mq(DP)) {
           *reinterpret_cast<float4*>(decays(buf) + x - rec_decay(DP)) = raw[i];
         } else {
           const int y = x - rec_mq(DP), at = (y / CH) * MSTR + y % CH;
-          *reinterpret_cast<uint2*>(mixed(buf, 0) + at) = hi;
-          *reinterpret_cast<uint2*>(mixed(buf, 1) + at) = lo;
+#pragma unroll
+          for (int t = 0; t < TERMS; ++t) *reinterpret_cast<uint2*>(mixed(buf, t) + at) = make_uint2(t0[t], t1[t]);
         }
       }
 #pragma unroll
@@ -182,8 +184,7 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
 #pragma unroll 1
   for (int c = 0; c < nc; ++c) {
     const int buf = c & 1;
-    // S^T times the records' vectors; sums of the leading products and of the corrections apart, so that fewer wait
-    // for one another
+    // S^T times the records' vectors
     float w[2][4], q[2][4], wc[2][4], qc[2][4];
 #pragma unroll
     for (int t = 0; t < 2; ++t)
@@ -192,28 +193,11 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
     if (CORRECT || !OWN) {
 #pragma unroll
       for (int kk = 0; kk < DP / 16; ++kk) {
-        unsigned hi[4], lo[4], b[4], d[4];
-        as_operand(S[2 * kk], S[2 * kk + 1], hi, lo);
-        if (CORRECT) {
-          ldm4(b, matrix(buf, 2, 0) + krow * STR + kk * 16 + kcol);
-          ldm4(d, matrix(buf, 2, 1) + krow * STR + kk * 16 + kcol);
-          mma(w[0], hi, b[0], b[1]);
-          mma(w[1], hi, b[2], b[3]);
-          mma(wc[0], hi, d[0], d[1]);
-          mma(wc[1], hi, d[2], d[3]);
-          mma(wc[0], lo, b[0], b[1]);
-          mma(wc[1], lo, b[2], b[3]);
-        }
-        if (!OWN) {
-          ldm4(b, matrix(buf, 0, 0) + krow * STR + kk * 16 + kcol);
-          ldm4(d, matrix(buf, 0, 1) + krow * STR + kk * 16 + kcol);
-          mma(q[0], hi, b[0], b[1]);
-          mma(q[1], hi, b[2], b[3]);
-          mma(qc[0], hi, d[0], d[1]);
-          mma(qc[1], hi, d[2], d[3]);
-          mma(qc[0], lo, b[0], b[1]);
-          mma(qc[1], lo, b[2], b[3]);
-        }
+        unsigned a[TERMS][4];
+        as_operand(S[2 * kk], S[2 * kk + 1], a);
+        const int at = krow * STR + kk * 16 + kcol;
+        if (CORRECT) products<false>(w, wc, a, matrix(buf, 2, 0) + at, CH * STR);
+        if (!OWN) products<false>(q, qc, a, matrix(buf, 0, 0) + at, CH * STR);
       }
     }
     // u: token 8 t + q2 (+ 1) of columns g8 (+ 8)
@@ -223,46 +207,23 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
     for (int t = 0; t < 2; ++t)
 #pragma unroll
       for (int k = 0; k < 4; ++k) u[t][k] = U[(t * 8 + q2 + (k & 1)) * USTR + (k >> 1) * 8] - (w[t][k] + wc[t][k]);
-    unsigned uh[4], ul[4];
-    as_operand(u[0], u[1], uh, ul);
-    if (!OWN) {
-      unsigned b[4], d[4];
-      ldm4t(b, mixed(buf, 0) + lrow * MSTR + lcol);
-      ldm4t(d, mixed(buf, 1) + lrow * MSTR + lcol);
-      mma(q[0], uh, b[0], b[1]);
-      mma(q[1], uh, b[2], b[3]);
-      mma(qc[0], uh, d[0], d[1]);
-      mma(qc[1], uh, d[2], d[3]);
-      if (!U_EXACT) {
-        mma(qc[0], ul, b[0], b[1]);
-        mma(qc[1], ul, b[2], b[3]);
-      }
-    }
+    unsigned ua[TERMS][4];
+    as_operand(u[0], u[1], ua);
+    if (!OWN) products<true, U_EXACT>(q, qc, ua, mixed(buf, 0) + lrow * MSTR + lcol, CH * MSTR);
     const float* decay = decays(buf) + q2;
 #pragma unroll
-    for (int j = 0; j < DP / 8; ++j) {
-      const float2 f = *reinterpret_cast<const float2*>(decay + j * 8);
-      if (OWN) {
-        product[j][0] *= f.x;
-        product[j][1] *= f.y;
-      }
-      S[j][0] *= f.x;
-      S[j][1] *= f.y;
-      S[j][2] *= f.x;
-      S[j][3] *= f.y;
-    }
-#pragma unroll
     for (int j = 0; j < DP / 16; ++j) {
-      unsigned b[4], d[4];
-      ldm4t(b, matrix(buf, 1, 0) + lrow * STR + j * 16 + lcol);
-      ldm4t(d, matrix(buf, 1, 1) + lrow * STR + j * 16 + lcol);
-      mma(S[2 * j], uh, b[0], b[1]);
-      mma(S[2 * j + 1], uh, b[2], b[3]);
-      mma(S[2 * j], uh, d[0], d[1]);
-      mma(S[2 * j + 1], uh, d[2], d[3]);
-      if (!U_EXACT) {
-        mma(S[2 * j], ul, b[0], b[1]);
-        mma(S[2 * j + 1], ul, b[2], b[3]);
+      float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, yc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+      products<true, U_EXACT>(y, yc, ua, matrix(buf, 1, 0) + lrow * STR + j * 16 + lcol, CH * STR);
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const float2 f = *reinterpret_cast<const float2*>(decay + (2 * j + t) * 8);
+        if (OWN) {
+          product[2 * j + t][0] *= f.x;
+          product[2 * j + t][1] *= f.y;
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) S[2 * j + t][k] = fmaf(k & 1 ? f.y : f.x, S[2 * j + t][k], y[t][k] + yc[t][k]);
       }
     }
     if (!OWN) {
