@@ -4,30 +4,30 @@
 //
 // A block takes sixteen rows of a request and all heads, a warp a head.  Pass 1 walks the key tiles and keeps every
 // (row, head)'s running maximum and sum in registers.  Pass 2 walks them again: the probabilities, normalised, go to
-// shared memory as two bfloat16 terms, hi + lo (seventeen bits of a number in [0, 1]; queries, keys and values are
-// bfloat16 and exact), every warp mixes the heads of one row, W = M P, as a product over the sixteen heads
-// (M also hi + lo: three products), and head h's warp adds W_hi V + W_lo V to its 16 x E outputs, which stay in
-// registers.  Scores are computed twice because the mixture needs normalised probabilities of all heads
+// shared memory as three bfloat16 terms, which hold their 24 bits (queries, keys and values are bfloat16 and exact),
+// every warp mixes the heads of one row, W = M P, as a product over the sixteen heads (M as three terms too: the six
+// products that count), and head h's warp adds a tile's W V, three products summed from zero, to its 16 x E outputs,
+// which stay in registers (the tensor cores cut off what does not fit a sum, so the outputs are not left to them).  Scores are computed twice because the mixture needs normalised probabilities of all heads
 // before any value is weighted; keeping the heads' values apart until the end would take G times the value products.
 //
 // What bounds it: the shared-memory pipe (every head's warp reads its key/value head's tile: 3 x 8 KB a warp and
-// tile) and three block barriers a tile with one block a multiprocessor (181 KB).  A key tile travels while the
+// tile) and three block barriers a tile with one block a multiprocessor (202 KB).  A key tile travels while the
 // tile before it is mixed, a value tile while its scores are made, so one buffer of each is enough.
 // A 2,048-token prompt, sixteen heads of 128 over four key/value heads, window 1,024, blocks of 64: 4,336 us in
-// float32 multiply-adds, 243 us here (tensor pipe and shared memory both under half busy: the barriers' latencies).
-#include <cuda_bf16.h>
-
+// float32 multiply-adds, 292 us here.  Two terms took 243; where the mixture nearly cancels they were further off 64 bits
+// than the multiply-adds (5e-4 of the bfloat16 result's own rounding), three are as close to seven digits.
 #include "common.cuh"
+#include "mma_sync.cuh"
 #include "pdl.cuh"
 
 using namespace pbe;
+using namespace pbe::mma_sync;
 
 #if !defined(PBE_PM_D) || !defined(PBE_PM_E)
 #error "PBE_PM_D (key width) and PBE_PM_E (value width) must be defined"
 #endif
 
 namespace {
-typedef __nv_bfloat16 bf16;
 constexpr int D = PBE_PM_D, E = PBE_PM_E;
 static_assert(D % 16 == 0 && E % 16 == 0 && D <= 128 && E <= 128, "head widths are multiples of 16 up to 128");
 constexpr int BM = 16, HEADS = 16;         // rows of a block, most heads
@@ -52,41 +52,12 @@ struct PmParams {
   float scale_log2;         // scale * log2(e): scores in units of the exponential's base
 };
 
-__device__ __forceinline__ unsigned smem_addr(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void cp16(void* dst, const void* src, bool live) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(live ? 16 : 0) : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void ldm4(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)) : "memory");
-}
-__device__ __forceinline__ void ldm4t(unsigned (&r)[4], const bf16* p) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(smem_addr(p)) : "memory");
-}
-__device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
-// x and y as bfloat16 pairs, hi + lo
-__device__ __forceinline__ void split2(float x, float y, unsigned& hi, unsigned& lo) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  const float2 f = __bfloat1622float2(h);
-  const __nv_bfloat162 l = __floats2bfloat162_rn(x - f.x, y - f.y);
-  hi = *reinterpret_cast<const unsigned*>(&h);
-  lo = *reinterpret_cast<const unsigned*>(&l);
-}
-
 // The probabilities' buffer: [head][row][key], rows and heads padded so that eight rows of a head and eight heads of
 // a row both start in different banks
 template <int BN> __host__ __device__ constexpr int p_row() { return BN + 8; }
 template <int BN> __host__ __device__ constexpr int p_head() { return BM * p_row<BN>() + 8; }
 template <int BN> __host__ __device__ constexpr size_t pm_smem(int H, int G) {
-  return 2 * ((size_t)H * BM * KSTR + (size_t)G * BN * (2 * (KSTR > VSTR ? KSTR : VSTR)) + 2 * (size_t)HEADS * p_head<BN>());
+  return 2 * ((size_t)H * BM * KSTR + (size_t)G * BN * (2 * (KSTR > VSTR ? KSTR : VSTR)) + TERMS * (size_t)HEADS * p_head<BN>());
 }
 
 template <int N>
@@ -104,8 +75,7 @@ __global__ void __launch_bounds__(32 * HEADS, 1) pooled_attention_mma_kernel(PmP
   bf16* Qs = reinterpret_cast<bf16*>(smem_raw);            // [H][BM][KSTR]
   bf16* const buf0 = Qs + H * BM * KSTR;                   // [G][BN][KSTR]
   bf16* const buf1 = buf0 + G * BN * TILE;                 // [G][BN][VSTR]; pass 1: the other key buffer
-  bf16* Phi = buf1 + G * BN * TILE;                        // [HEADS] of PH
-  bf16* Plo = Phi + HEADS * PH;
+  bf16* Ps = buf1 + G * BN * TILE;                         // [TERMS][HEADS] of PH
   const int tid = threadIdx.x, NT = blockDim.x, warp = tid >> 5, lane = tid & 31;
   const int g8 = lane >> 2, q2 = (lane & 3) * 2;
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;     // ldmatrix: A operands, and B transposed
@@ -163,14 +133,19 @@ __global__ void __launch_bounds__(32 * HEADS, 1) pooled_attention_mma_kernel(PmP
     *reinterpret_cast<uint4*>(Qs + (h * BM + row) * KSTR + piece * 8) = v;
   }
   // heads that do not exist take part in the mixture as zeros
-  for (int i = tid; i < (HEADS - H) * PH; i += NT) Phi[H * PH + i] = Plo[H * PH + i] = __float2bfloat16_rn(0.f);
-  unsigned mix_hi[4] = {0u, 0u, 0u, 0u}, mix_lo[4] = {0u, 0u, 0u, 0u};     // M as the A operand
+  for (int i = tid; i < (HEADS - H) * PH; i += NT)
+#pragma unroll
+    for (int t = 0; t < TERMS; ++t) Ps[(t * HEADS + H) * PH + i] = __float2bfloat16_rn(0.f);
+  unsigned mix[TERMS][4] = {};                             // M as the A operand
   if (p.talk) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int h = g8 + (i & 1) * 8, g = q2 + (i >> 1) * 8;
       const float x = h < H && g < H ? p.talk[h * H + g] : 0.f, y = h < H && g + 1 < H ? p.talk[h * H + g + 1] : 0.f;
-      split2(x, y, mix_hi[i], mix_lo[i]);
+      unsigned terms[TERMS];
+      split3(x, y, terms);
+#pragma unroll
+      for (int t = 0; t < TERMS; ++t) mix[t][i] = terms[t];
     }
   }
   const bf16* Qh = Qs + warp * BM * KSTR;
@@ -281,11 +256,11 @@ __global__ void __launch_bounds__(32 * HEADS, 1) pooled_attention_mma_kernel(PmP
     for (int j = 0; j < BN / 8; ++j)
 #pragma unroll
       for (int hh = 0; hh < 2; ++hh) {
-        unsigned hi, lo;
-        split2(exp2f(s[j][2 * hh] - m[hh]) * inv[hh], exp2f(s[j][2 * hh + 1] - m[hh]) * inv[hh], hi, lo);
+        unsigned terms[TERMS];
+        split3(exp2f(s[j][2 * hh] - m[hh]) * inv[hh], exp2f(s[j][2 * hh + 1] - m[hh]) * inv[hh], terms);
         const int at = warp * PH + (g8 + hh * 8) * PR + j * 8 + q2;
-        *reinterpret_cast<unsigned*>(Phi + at) = hi;
-        *reinterpret_cast<unsigned*>(Plo + at) = lo;
+#pragma unroll
+        for (int t = 0; t < TERMS; ++t) *reinterpret_cast<unsigned*>(Ps + t * HEADS * PH + at) = terms[t];
       }
     if (tid < BN) ring[(kt + 2) & 3][tid] = ahead;
     __syncthreads();                                       // all heads' probabilities; the key buffer is free
@@ -293,29 +268,26 @@ __global__ void __launch_bounds__(32 * HEADS, 1) pooled_attention_mma_kernel(PmP
     cp_commit();
     if (p.talk) {
       for (int row = warp; row < BM; row += NT / 32) {     // in place: nobody else touches this row now
-        unsigned hi[BN / 16][4], lo[BN / 16][4];
+        unsigned b[BN / 16][TERMS][4];
 #pragma unroll
-        for (int j = 0; j < BN / 16; ++j) {                // B operands: k the heads, n sixteen keys
-          const int at = lrow * PH + row * PR + j * 16 + lcol;
-          ldm4t(hi[j], Phi + at);
-          ldm4t(lo[j], Plo + at);
-        }
+        for (int j = 0; j < BN / 16; ++j)                  // B operands: k the heads, n sixteen keys
+#pragma unroll
+          for (int t = 0; t < TERMS; ++t) ldm4t(b[j][t], Ps + (t * HEADS + lrow) * PH + row * PR + j * 16 + lcol);
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < BN / 8; ++j) {
-          const unsigned h0 = hi[j / 2][(j & 1) * 2], h1 = hi[j / 2][(j & 1) * 2 + 1];
-          const unsigned l0 = lo[j / 2][(j & 1) * 2], l1 = lo[j / 2][(j & 1) * 2 + 1];
           float w[4] = {0.f, 0.f, 0.f, 0.f};
-          mma(w, mix_lo, h0, h1);
-          mma(w, mix_hi, l0, l1);
-          mma(w, mix_hi, h0, h1);
+#pragma unroll
+          for (int sum = TERMS - 1; sum >= 0; --sum)       // the small products first
+#pragma unroll
+            for (int t = 0; t <= sum; ++t) mma(w, mix[t], b[j / 2][sum - t][(j & 1) * 2], b[j / 2][sum - t][(j & 1) * 2 + 1]);
 #pragma unroll
           for (int hh = 0; hh < 2; ++hh) {
-            unsigned x, y;
-            split2(w[2 * hh], w[2 * hh + 1], x, y);
+            unsigned terms[TERMS];
+            split3(w[2 * hh], w[2 * hh + 1], terms);
             const int at = (g8 + hh * 8) * PH + row * PR + j * 8 + q2;
-            *reinterpret_cast<unsigned*>(Phi + at) = x;
-            *reinterpret_cast<unsigned*>(Plo + at) = y;
+#pragma unroll
+            for (int t = 0; t < TERMS; ++t) *reinterpret_cast<unsigned*>(Ps + t * HEADS * PH + at) = terms[t];
           }
         }
       }
@@ -323,19 +295,28 @@ __global__ void __launch_bounds__(32 * HEADS, 1) pooled_attention_mma_kernel(PmP
     cp_wait<1>();
     __syncthreads();                                       // mixed; the values of tile kt have landed
     const bf16* Vh = buf1 + kv * BN * VSTR;
+    unsigned a[BN / 16][TERMS][4];
 #pragma unroll
-    for (int kk = 0; kk < BN; kk += 16) {
-      unsigned hi[4], lo[4];
-      ldm4(hi, Phi + warp * PH + lrow * PR + kk + lcol);
-      ldm4(lo, Plo + warp * PH + lrow * PR + kk + lcol);
+    for (int kk = 0; kk < BN / 16; ++kk)
 #pragma unroll
-      for (int j = 0; j < E / 16; ++j) {
+      for (int t = 0; t < TERMS; ++t) ldm4(a[kk][t], Ps + (t * HEADS + warp) * PH + lrow * PR + kk * 16 + lcol);
+#pragma unroll
+    for (int j = 0; j < E / 16; ++j) {
+      float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
+#pragma unroll
+      for (int kk = 0; kk < BN / 16; ++kk) {
         unsigned b[4];
-        ldm4t(b, Vh + (kk + lrow) * VSTR + j * 16 + lcol);
-        mma(o[2 * j], hi, b[0], b[1]);
-        mma(o[2 * j + 1], hi, b[2], b[3]);
-        mma(o[2 * j], lo, b[0], b[1]);
-        mma(o[2 * j + 1], lo, b[2], b[3]);
+        ldm4t(b, Vh + (kk * 16 + lrow) * VSTR + j * 16 + lcol);
+#pragma unroll
+        for (int t = TERMS - 1; t >= 0; --t) {
+          mma(y[0], a[kk][t], b[0], b[1]);
+          mma(y[1], a[kk][t], b[2], b[3]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        o[2 * j][c] += y[0][c];
+        o[2 * j + 1][c] += y[1][c];
       }
     }
     cp_wait<0>();

@@ -130,13 +130,13 @@ class PooledWindowAttention(Mixer):
             self._mma = ops.pooled_mma_applies(self.dtype, H, D, E) and ops.pooled_mma_fits(H, G, D, E)
         # decoded tokens only (always so in a captured step): a row a tile
         single = getattr(ctx, "captured", False) or int(ctx.q_len_host.max(initial=1)) == 1
-        # Prompt portions take the tensor-core form, whose blocks walk all keys of sixteen rows (25 us and 0.24 us a
+        # Prompt portions take the tensor-core form, whose blocks walk all keys of sixteen rows (30 us and 0.25 us a
         # key).  A short portion behind a long context leaves most of the GPU idle that way: there the split form is
-        # ahead (1,088 keys: 24 rows 131 against 270 us, 48 rows 227 / 262, 96 rows 331 / 267; up to 400 keys it never
-        # is).
+        # ahead (1,073 keys: 64 rows 225 against 303 us, 80 rows 319 / 303; 648 keys: 48 rows 117 / 187, 64 rows 198 /
+        # 188; 394 keys: 48 rows 126 / 132; 335 keys: 16 rows 115 / 101).
         longest = int(ctx.seq_len_host.max(initial=1))
         seen = min(longest, self.window + ops.POOLED_MMA_ROWS) + (longest // self.pool if self.pool else 0)
-        if self._mma and not single and (ctx.num_tokens >= 64 or seen <= 400):
+        if self._mma and not single and (ctx.num_tokens >= (80 if seen > 700 else 64) or seen <= 350):
             tiles, n_tiles = ctx.row_tiles(ops.POOLED_MMA_ROWS)
             out = ops.pooled_attention_mma(q, tok.k, tok.v, k_pool, v_pool, self.talk, tiles, n_tiles, ctx.q_start,
                                            ctx.q_len, ctx.seq_len, gt.block_table, bt_pool, H, G, self.scale,
