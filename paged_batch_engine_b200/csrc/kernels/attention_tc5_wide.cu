@@ -62,7 +62,8 @@ static_assert(2 * (SMEM_BYTES + 1024) <= 228 * 1024, "two blocks a multiprocesso
 
 struct LatentExtra {
   const bf16* q;             // [T, H * (128 + 64)]
-  int num_tiles, R;          // row tiles of all requests, requests
+  const int32_t* list;       // the requests whose keys are expanded, ascending; null: all of the step
+  int num_tiles, R;          // their row tiles, their number
   const int32_t* positions;  // [T]
   const float* inv_freq;     // [rot_dims / 2] or null
   int rot_dims;
@@ -131,20 +132,22 @@ __device__ __forceinline__ uint32_t pack2(float x, float y) {
 __device__ __forceinline__ float low_of(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float high_of(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
-// The expanded matrix holds the keys that the step's rows can see, request after request.
+// The expanded matrix holds the keys that the rows of a list of the step's requests can see, request after request.
 __device__ __forceinline__ int lowest_key(int seq_len, int q_len, int window) {
   return window > 0 ? max(0, seq_len - q_len - window + 1) : 0;
 }
-// By a warp: the request that row tile `index` of the step belongs to (tiles: all requests' rows in tiles of BM; -1: every
-// request is passed), its first tile, and the expanded row of the first key of request `r` (of that request if r < 0).
+// By a warp, over the list's requests (null: all of the step): the request that row tile `index` belongs to (tiles: their
+// rows in tiles of BM; -1: every request is passed), its first tile, and the expanded row of the first key of place `at`
+// of the list (of that request if at < 0).
 struct Located { int r, first_tile, key_base; };
-__device__ Located locate(int index, int r, int R, const int32_t* q_len, const int32_t* seq_len, int window) {
+__device__ Located locate(int index, int at, const int32_t* list, int R, const int32_t* q_len, const int32_t* seq_len, int window) {
   const int lane = threadIdx.x & 31;
   int tiles_before = 0, keys_before = 0;
   for (int i0 = 0; i0 < R; i0 += 32) {
     const int i = i0 + lane;
-    const int n = i < R ? q_len[i] : 0;
-    const int keys = i < R ? seq_len[i] - lowest_key(seq_len[i], n, window) : 0;
+    const int r = i < R ? (list ? list[i] : i) : 0;
+    const int n = i < R ? q_len[r] : 0;
+    const int keys = i < R ? seq_len[r] - lowest_key(seq_len[r], n, window) : 0;
     const int tiles = (n + BM - 1) / BM;
     int t = tiles, k = keys;
 #pragma unroll
@@ -152,11 +155,11 @@ __device__ Located locate(int index, int r, int R, const int32_t* q_len, const i
       const int ut = __shfl_up_sync(0xffffffffu, t, o), uk = __shfl_up_sync(0xffffffffu, k, o);
       if (lane >= o) { t += ut; k += uk; }
     }
-    const unsigned hit = __ballot_sync(0xffffffffu, r >= 0 ? i == r : (i < R && index >= 0 && index < tiles_before + t));
+    const unsigned hit = __ballot_sync(0xffffffffu, at >= 0 ? i == at : (i < R && index >= 0 && index < tiles_before + t));
     if (hit) {
-      const int at = __ffs(hit) - 1;
-      return Located{i0 + at, tiles_before + __shfl_sync(0xffffffffu, t - tiles, at),
-                     keys_before + __shfl_sync(0xffffffffu, k - keys, at)};
+      const int from = __ffs(hit) - 1;
+      return Located{__shfl_sync(0xffffffffu, r, from), tiles_before + __shfl_sync(0xffffffffu, t - tiles, from),
+                     keys_before + __shfl_sync(0xffffffffu, k - keys, from)};
     }
     tiles_before += __shfl_sync(0xffffffffu, t, 31);
     keys_before += __shfl_sync(0xffffffffu, k, 31);
@@ -187,7 +190,7 @@ attention_tc5_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   if (LATENT) {
     // the last row tiles of a request have the most keys: they come first
     const int index = y.num_tiles - 1 - (int)(blockIdx.x / KV);
-    const Located at = locate(index, -1, y.R, p.q_len, p.seq_len, p.window);
+    const Located at = locate(index, -1, y.list, y.R, p.q_len, p.seq_len, p.window);
     r = at.r;
     if (r < 0) return;
     pr0 = (index - at.first_tile) * BM;
@@ -649,9 +652,9 @@ PBE_EXPORT int pbe_masked_attention_tc5(const AttnParams* params, int mask_kind,
 }
 #else
 // The latent attention over expanded keys and values: kv [keys, 2 * H * 128] (K of all heads, then V of all heads),
-// kr [keys, 64]; rows in tiles of 128 of one request.
+// kr [keys, 64]; rows in tiles of 128 of one request.  Only the list's requests' rows of out are written.
 PBE_EXPORT int pbe_latent_attention_tc5(const void* q, const void* kv, const void* kr, void* out, long long num_keys,
-                                        int num_tiles, int R, const int32_t* q_start, const int32_t* q_len,
+                                        int num_tiles, const int32_t* list, int R, const int32_t* q_start, const int32_t* q_len,
                                         const int32_t* seq_len, const int32_t* positions, const float* inv_freq, int rot_dims, float rot_scale,
                                         const float* sink, const void* gate, int ldg, int gate_each, int H, int window,
                                         float scale, int* err, cudaStream_t stream) {
@@ -674,24 +677,25 @@ PBE_EXPORT int pbe_latent_attention_tc5(const void* q, const void* kv, const voi
   p.scale = scale;
   MaskedExtra x = {};
   x.mask_kind = window > 0 ? 1 : 0;
-  LatentExtra y{(const bf16*)q, num_tiles, R, positions, inv_freq, rot_dims, rot_scale, sink,
+  LatentExtra y{(const bf16*)q, list, num_tiles, R, positions, inv_freq, rot_dims, rot_scale, sink,
                 (const bf16*)gate, ldg, gate_each};
   return launch_wide(map_kv, map_kr, p, x, y, (long long)num_tiles * H, err, stream);
 }
 
-// The latents and rotated parts of the keys that the step's rows can see, gathered from the pages, request after
-// request: c [keys, rank], kr [keys, 64].  grid.y: the request; a warp a key, 16-byte pieces.
+// The latents and rotated parts of the keys that the list's requests' rows can see, gathered from the pages, request after
+// request: c [keys, rank], kr [keys, 64].  grid.y: the place in the list; a warp a key, 16-byte pieces.
 namespace {
 __global__ void __launch_bounds__(256) gather_latents_kernel(const bf16* pages, const int32_t* block_table, int bt_stride,
                                                              int page_tokens, int rank, const int32_t* q_len,
-                                                             const int32_t* seq_len, int R, int window, bf16* c, bf16* kr) {
+                                                             const int32_t* seq_len, const int32_t* list, int R, int window,
+                                                             bf16* c, bf16* kr) {
   pdl_launch_dependents();
   pdl_wait();
-  const int r = blockIdx.y, lane = threadIdx.x & 31;
+  const int r = list ? list[blockIdx.y] : (int)blockIdx.y, lane = threadIdx.x & 31;
   const int low = lowest_key(seq_len[r], q_len[r], window);
   const int key = low + blockIdx.x * 8 + (threadIdx.x >> 5);
   if (key >= seq_len[r]) return;
-  const size_t row = (size_t)(locate(-1, r, R, q_len, seq_len, window).key_base + key - low);
+  const size_t row = (size_t)(locate(-1, (int)blockIdx.y, list, R, q_len, seq_len, window).key_base + key - low);
   const int page = block_table[(size_t)r * bt_stride + key / page_tokens];
   const int width = rank + ROT;
   const bf16* src = pages + ((size_t)max(page, 0) * page_tokens + key % page_tokens) * width;
@@ -704,12 +708,12 @@ __global__ void __launch_bounds__(256) gather_latents_kernel(const bf16* pages, 
 }  // namespace
 
 PBE_EXPORT int pbe_gather_latents(const void* pages, const int32_t* block_table, int bt_stride, int page_tokens, int rank,
-                                  const int32_t* q_len, const int32_t* seq_len, int R, int window, int most_keys, void* c,
-                                  void* kr, cudaStream_t stream) {
+                                  const int32_t* q_len, const int32_t* seq_len, const int32_t* list, int R, int window,
+                                  int most_keys, void* c, void* kr, cudaStream_t stream) {
   if (R <= 0 || most_keys <= 0) return 0;
   if (rank % 8 || (((uintptr_t)pages | (uintptr_t)c | (uintptr_t)kr) & 15) || R > 65535) return (int)cudaErrorInvalidValue;
   launch_k(gather_latents_kernel, dim3((most_keys + 7) / 8, R), 256, 0, stream, (const bf16*)pages, block_table, bt_stride,
-           page_tokens, rank, q_len, seq_len, R, window, (bf16*)c, (bf16*)kr);
+           page_tokens, rank, q_len, seq_len, list, R, window, (bf16*)c, (bf16*)kr);
   return launch_status();
 }
 #endif

@@ -1,6 +1,7 @@
 // Attention over a compressed latent: every token keeps one row [c | kr] in the paged cache (c: a
 // normed latent of `rank` values from which all heads' keys and values are linear maps; kr: one
-// rotated key part of `rot` values that all heads share).  Keys and values are never expanded:
+// rotated key part of `rot` values that all heads share).  These kernels never expand keys and values
+// (long portions do, see attention_tc5_wide.cu):
 // the heads' key maps are applied to the queries instead and the heads' value maps to the
 // attention's output,
 //   score_h(i, j) = ((U_k,h^T q_h,i) . c_j + rope(q'_h,i) . kr_j) * scale,

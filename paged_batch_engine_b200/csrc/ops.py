@@ -1602,7 +1602,7 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, sink: Optional[torch.
     mode = 0 if (LATENT_FMA or cache.dtype != torch.bfloat16 or dk % 16) else (1 if meta.decode_rows > 0 else 2)
     # steps of decoded tokens in which every row's keys are split: four blocks share each split, so
     # that few long requests still fill the GPU (8 requests at 2,048 keys: 64 -> 256 blocks)
-    sub = LATENT_SUB if (mode == 1 and meta.num_split_rows == T and meta.split_keys % (LATENT_SUB * 32) == 0) else 1
+    sub = LATENT_SUB if (mode == 1 and meta.num_split_rows == meta.decode_rows and meta.split_keys % (LATENT_SUB * 32) == 0) else 1
     slots = meta.max_splits * sub
     part_o = part_ml = None
     if meta.num_split_rows:
@@ -1635,7 +1635,7 @@ def latent_attention(q: torch.Tensor, cache: torch.Tensor, sink: Optional[torch.
 
 
 LATENT_TC5_ROWS = 128       # rows of a tile of the expanded form
-LATENT_TC5_BYTES = 1 << 29  # of a step's expanded keys and values at most
+LATENT_TC5_BYTES = 1 << 29  # of the expanded keys and values that are there at a time
 
 
 def latent_expands(dtype: torch.dtype, head_dim: int, rot_dim: int, value_dim: int, kv_rank: int, scale: float) -> bool:
@@ -1649,38 +1649,45 @@ def latent_attention_expanded(q: torch.Tensor, pages: torch.Tensor, w_kv: torch.
                               num_row_tiles: int, group, seq_len, q_start, q_len, positions, num_heads: int, kv_rank: int, scale: float,
                               window: Optional[int], page_tokens: int, inv_freq: Optional[torch.Tensor], rot_dims: int,
                               rot_scale: float, sink: Optional[torch.Tensor], gate: Optional[torch.Tensor],
-                              gate_each: bool) -> torch.Tensor:
+                              gate_each: bool, requests: Optional[torch.Tensor] = None,
+                              out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention over one cached latent per token with the heads' keys and values expanded from the latents first:
-    the keys that the step's rows see (``total_keys``, of one request ``most_keys`` at most) are gathered from the pages,
+    the keys that the rows of ``requests`` (ascending int32 places in the step; None: all) see (``total_keys``, of one
+    request ``most_keys`` at most) are gathered from the pages,
     multiplied by ``w_kv`` [2 * H * 128, kv_rank] (the key maps of all heads, then the value
-    maps) and attended to by ``q`` bfloat16 [T, H * (128 + 64)], whose rotated part is turned on the way.  Returns
-    bfloat16 [T, H * 128], gates applied.  Queries, expanded keys and expanded values are bfloat16, softmax weights
+    maps) and attended to by ``q`` bfloat16 [T, H * (128 + 64)], whose rotated part is turned on the way (their rows: ``num_row_tiles``
+    tiles of ``LATENT_TC5_ROWS``).  Returns bfloat16 [T, H * 128], gates applied, in ``out`` where given; only those rows
+    are written.  Queries, expanded keys and expanded values are bfloat16, softmax weights
     two bfloat16 terms, everything else float32."""
-    _need_cuda(q, pages, w_kv, seq_len, q_start, q_len, positions, inv_freq, sink, gate)
-    _need_contiguous(q, pages, w_kv, positions, inv_freq, sink)
-    T, H, R = q.shape[0], num_heads, q_len.numel()
+    _need_cuda(q, pages, w_kv, seq_len, q_start, q_len, positions, inv_freq, sink, gate, requests, out)
+    _need_contiguous(q, pages, w_kv, positions, inv_freq, sink, requests, out)
+    T, H, R = q.shape[0], num_heads, q_len.numel() if requests is None else requests.numel()
     if (q.dtype != torch.bfloat16 or pages.dtype != torch.bfloat16 or w_kv.dtype != torch.bfloat16 or q.shape[1] != H * 192
             or tuple(w_kv.shape) != (2 * H * 128, kv_rank) or pages.shape[-1] != kv_rank + 64):
         raise KernelError("latent_attention_expanded: shapes or dtypes do not agree")
     if gate is not None and (gate.dtype != torch.bfloat16 or gate.stride(1) != 1):
         raise KernelError("latent_attention_expanded: the gate is a bfloat16 column slice")
+    if (requests is not None and requests.dtype != torch.int32) or (
+            out is not None and (out.dtype != torch.bfloat16 or tuple(out.shape) != (T, H * 128))):
+        raise KernelError("latent_attention_expanded: requests are int32, the result bfloat16 [T, H * 128]")
     lib = {"PBE_X_LATENT": 1}
     c = torch.empty((total_keys, kv_rank), dtype=torch.bfloat16, device=q.device)
     kr = torch.empty((total_keys, 64), dtype=torch.bfloat16, device=q.device)
     gather = _fn("attention_tc5_wide", "pbe_gather_latents",
-                 [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p,
-                  c_void_p], lib)
+                 [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p,
+                  c_void_p, c_void_p], lib)
     _check(gather(_ptr(pages), _ptr(group.block_table), int(group.bt_stride), int(page_tokens), int(kv_rank), _ptr(q_len),
-                  _ptr(seq_len), R, int(window or 0), int(most_keys), _ptr(c), _ptr(kr), _stream()), "gather_latents")
+                  _ptr(seq_len), _ptr(requests), R, int(window or 0), int(most_keys), _ptr(c), _ptr(kr), _stream()), "gather_latents")
     kv = grouped_runs_tc5(c, w_kv.unsqueeze(0), None)
-    out = torch.empty((T, H * 128), dtype=torch.bfloat16, device=q.device)
+    if out is None:
+        out = torch.empty((T, H * 128), dtype=torch.bfloat16, device=q.device)
     ldg = 0
     if gate is not None:
         ldg = gate.stride(0) if T > 1 else max(gate.stride(0), H * (128 if gate_each else 1))
     fn = _fn("attention_tc5_wide", "pbe_latent_attention_tc5",
-             [c_void_p] * 4 + [c_ll, c_int, c_int] + [c_void_p] * 5 + [c_int, c_float, c_void_p, c_void_p, c_int, c_int,
-                                                                        c_int, c_int, c_float, c_void_p, c_void_p], lib)
-    _check(fn(_ptr(q), _ptr(kv), _ptr(kr), _ptr(out), int(total_keys), int(num_row_tiles), R, _ptr(q_start),
+             [c_void_p] * 4 + [c_ll, c_int, c_void_p, c_int] + [c_void_p] * 5
+             + [c_int, c_float, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p], lib)
+    _check(fn(_ptr(q), _ptr(kv), _ptr(kr), _ptr(out), int(total_keys), int(num_row_tiles), _ptr(requests), R, _ptr(q_start),
               _ptr(q_len), _ptr(seq_len), _ptr(positions), _ptr(inv_freq),
               int(rot_dims), float(rot_scale), _ptr(sink), _ptr(gate), int(ldg), 1 if gate_each else 0, H, int(window or 0),
               float(scale), _ptr(tc5_attention_error_buffer(q.device)), _stream()), "latent_attention_tc5")

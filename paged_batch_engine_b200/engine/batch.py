@@ -111,7 +111,7 @@ def attention_work_arrays(q_len: np.ndarray, seq_len: np.ndarray, q_start: np.nd
     pos0 = seq_len - q_len
     lo_req = np.maximum(0, pos0 - window + 1) if window else np.zeros(R, dtype=np.int64)
     span_splits = (seq_len + split_keys - 1) // split_keys - lo_req // split_keys
-    can_split = (m_tiles <= MAX_SPLIT_TILES) & (span_splits > 1)
+    can_split = (m_tiles <= MAX_SPLIT_TILES) & (span_splits > 1) & (m_tiles > 0)
     n_splits = np.where(can_split, span_splits, 1)
     if fixed_splits:
         if (n_splits > fixed_splits).any() or (m_tiles != 1).any():
@@ -146,7 +146,7 @@ def attention_work_arrays(q_len: np.ndarray, seq_len: np.ndarray, q_start: np.nd
         lo = np.maximum(0, p0 + (mt * tile_rows) // group_size - window + 1) if window else 0
         cost = np.where(ns > 1, np.minimum(split_keys, hi - lo), hi - lo)
         work = work[np.argsort(-cost, kind="stable")]
-    T = int(q_len.sum())
+    T = int((q_start + q_len).max(initial=0))      # a request without rows (another form's) leaves its places unused
     tok_split_row = np.full(T, -1, dtype=np.int32)
     is_split = (n_splits > 1) | force_split
     split_req = np.nonzero(is_split)[0]
@@ -404,6 +404,32 @@ class StepContext:
                 host = host.pin_memory()
             got = self._row_tiles[tile_rows] = (host.to(self.device, non_blocking=True), len(tiles), host)
         return got[0], got[1]
+
+    def attention_work_of(self, group: int, group_size: int, tile_rows: int, window, some) -> AttentionWork:
+        """The work list of the requests in ``some`` (a bool per request) only, made on first use; the other requests' rows
+        are in no tile."""
+        kept = self.__dict__.setdefault("_work_of_some", {})
+        key = (group, group_size, tile_rows, window, np.asarray(some).tobytes())
+        got = kept.get(key)
+        if got is None:
+            q_len = np.where(some, self.q_len_host, 0)
+            work, tsr, st, sc, max_splits = attention_work_arrays(q_len, self.seq_len_host, self.q_start_host, group_size,
+                                                                  tile_rows, window, split_keys=self.split_keys)
+            pk = _Packer()
+            iw, it, ist, isc = pk.add(work), pk.add(tsr), pk.add(st), pk.add(sc)
+            pk.upload(self.device)
+            kinds, small_items = work_kinds(work, q_len, group_size, tile_rows)
+            g, single = self._groups[group], int(q_len.max(initial=0)) == 1
+            got = AttentionWork(
+                q_start=self.q_start, q_len=self.q_len, seq_len=self.seq_len, block_table=g.block_table,
+                bt_stride=g.bt_stride, work=pk.view(iw), num_work=len(work), tok_split_row=pk.view(it),
+                split_tokens=pk.view(ist) if len(st) else None, split_counts=pk.view(isc) if len(st) else None,
+                num_split_rows=len(st), max_splits=max_splits, split_keys=self.split_keys, tile_rows=tile_rows,
+                kinds=kinds, small_items=small_items, decode_rows=int(np.sum(some)) if single else 0,
+                longest_keys=int(np.where(some, self.seq_len_host, 0).max(initial=0)))
+            kept[key] = got
+            self.__dict__.setdefault("_plan_hosts", []).append(pk)       # pinned until the step is done
+        return got
 
     def attention_work(self, group: int, group_size: int, tile_rows: int, window, num_heads: int,
                        head_dim: int) -> AttentionWork:

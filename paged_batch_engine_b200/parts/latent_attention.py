@@ -5,6 +5,7 @@ import math
 import os
 from typing import Optional
 
+import numpy as np
 import torch
 
 from ..csrc import ops
@@ -43,10 +44,10 @@ class LatentAttention(Mixer):
     output is multiplied (``out_gate``) by sigmoid(W_g x)_h (``out_gate`` "each": W_g is [H*V, hidden]
     and every output value has a gate of its own); then the output projection.
 
-    Keys and values are never expanded here: U_k,h^T is applied to q_plain (the score becomes a
-    product with c) and U_v,h to the attention's output over c, so attention reads the cached rows
-    alone.  Rotation: pairs (2i, 2i + 1) of the first ``rotary["dims"]`` values of the rotated
-    part turn by position * base^(-2i / dims).  ``rotary["scaling"]`` = dict(factor, original, fast,
+    The cache holds no expanded keys and values.  Decoded tokens and short portions read the cached rows alone:
+    U_k,h^T is applied to q_plain (the score becomes a product with c) and U_v,h to the attention's output over c.
+    Longer portions expand the keys and values that they see for the time of the call.  Rotation: pairs (2i, 2i + 1) of
+    the first ``rotary["dims"]`` values of the rotated part turn by position * base^(-2i / dims).  ``rotary["scaling"]`` = dict(factor, original, fast,
     slow) stretches the slow pairs (``yarn_frequencies``) and multiplies cos and sin by 0.1 ln(factor)
     + 1; ``scale`` is used as given.
 
@@ -142,29 +143,68 @@ class LatentAttention(Mixer):
             self.sink_logits = tensors.pop(prefix + n["sink"]).to(torch.float32).contiguous()
 
     # ---- compute
-    ROWS_A_KEY = 8          # rows that see a key, on average, from which on expanding it pays
-    EXPANDED_ROWS = 16      # rows of a step at least
+    ROWS_A_KEY = 8          # rows of a portion from which on its keys are worth expanding
 
     def _expanded_keys(self, ctx, q, pages):
-        """The keys that each request's rows see, when the step's keys and values are worth expanding, else None.  A
-        pair of row and key costs a head 448 multiply-adds on expanded keys and values against 1,600 on the latents,
-        and every key 2 x 128 x kv_rank for its expansion."""
-        if getattr(ctx, "captured", False) or ctx.num_tokens < self.EXPANDED_ROWS or self.w_kv is None or not ops.latent_expands(
-                self.w_kv.dtype, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank, self.scale):
+        """Per request the number of keys that its rows see where keys and values are expanded for it, else 0; None where
+        they are for no request.  A pair of row and key costs a head 448 multiply-adds on expanded keys and values against
+        1,600 on the latents, and every key 2 x 128 x kv_rank for its expansion.
+
+        Each request is looked at by itself: the two forms round different factors to bfloat16 (see
+        ``ops.latent_attention_expanded``), and what a request computes is not to follow from which others share its
+        step.  A decoded token always takes the latents."""
+        if getattr(ctx, "captured", False) or int(ctx.q_len_host.max()) < self.ROWS_A_KEY or self.w_kv is None or \
+                not ops.latent_expands(self.w_kv.dtype, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank, self.scale):
             return None
         if q.dtype != torch.bfloat16 or pages.dtype != torch.bfloat16 or not ops.grouped_tc5_applies(q, self.w_kv[None]):
             return None
-        window = self.window or 1 << 60
-        lens, keys = ctx.q_len_host.tolist(), []
-        for n, before in zip(lens, ctx.context_before_host.tolist()):
-            keys.append(before + n - max(0, before - window + 1))
-        total = sum(keys)
-        # 16 rows behind 2,048 tokens 180 -> 98 us, 64 and four decoded tokens there 504 -> 162; but 32 requests of 2
-        # rows each behind 512 would take 152 -> 197, and 16 rows alone behind 8,192, which the splits of the other
-        # form spread over the GPU, 180 -> 258
-        worth = sum(n * k for n, k in zip(lens, keys)) >= self.ROWS_A_KEY * total and \
-            (ctx.num_tokens >= 32 or max(keys) <= 4096)
-        return keys if worth and total * self.num_heads * 512 <= ops.LATENT_TC5_BYTES else None
+        kept = ctx.__dict__.setdefault("_expanded_keys", {})       # looked at once a step for all such layers
+        kind = self.window, self.num_heads
+        if kind not in kept:
+            window = self.window or 1 << 60
+            keys = [self.expanded(n, before + n - max(0, before - window + 1))
+                    for n, before in zip(ctx.q_len_host.tolist(), ctx.context_before_host.tolist())]
+            kept[kind] = keys if any(keys) else None
+        return kept[kind]
+
+    def expanded(self, rows: int, keys: int) -> int:
+        """``keys`` where a portion of ``rows`` rows that see them takes the expanded form, else 0.  Layers of 16 heads: 8
+        rows alone 70 -> 43 us, 16 rows behind 2,000 tokens 173 -> 89, behind 4,000 172 -> 143; behind 6,000, which the
+        splits of the other form spread over the GPU, 16 rows would take 172 -> 191, 24 rows 1,210 -> 196."""
+        few = rows < self.ROWS_A_KEY or (rows < 32 and keys > 4096)
+        return 0 if few or keys * self.num_heads * 512 > ops.LATENT_TC5_BYTES else keys
+
+    def _goes(self, ctx, keys):
+        """The expanding requests in goes whose expanded keys and values stay within ``ops.LATENT_TC5_BYTES``: tuples of
+        (requests on the device or None for all of the step, keys, most keys of one, row tiles).  Made once a step for all
+        layers of one kind."""
+        made = ctx.__dict__.setdefault("_latent_goes", {})
+        got = made.get((self.window, self.num_heads))
+        if got is None:
+            goes, room = [], 0
+            for r, n in enumerate(keys):
+                if n == 0:
+                    continue
+                if n > room:
+                    goes.append([])
+                    room = ops.LATENT_TC5_BYTES // (self.num_heads * 512)
+                goes[-1].append(r)
+                room -= n
+            lists = torch.tensor([r for go in goes for r in go], dtype=torch.int32)
+            if len(goes) > 1 or len(lists) < len(keys):
+                host = lists.pin_memory() if torch.cuda.is_available() else lists
+                ctx.__dict__.setdefault("_plan_hosts", []).append(host)      # pinned until the step is done
+                lists = host.to(ctx.device, non_blocking=True)
+            else:
+                lists = None
+            got, first = [], 0
+            for go in goes:
+                rows = [(int(ctx.q_len_host[r]) + ops.LATENT_TC5_ROWS - 1) // ops.LATENT_TC5_ROWS for r in go]
+                got.append((lists[first:first + len(go)] if lists is not None else None, sum(keys[r] for r in go),
+                            max(keys[r] for r in go), sum(rows)))
+                first += len(go)
+            made[(self.window, self.num_heads)] = got
+        return got
 
     def forward(self, x, ctx, cache):
         T = x.shape[0]
@@ -178,31 +218,42 @@ class LatentAttention(Mixer):
                                    pages if cache.writes else None, self.eps, rot_scale=self.rot_scale)
         q = ops.linear(q_lat, self.w_uq, None, out_dtype=self.dtype, kind=16)           # [T, H * (D + R)]
         keys = self._expanded_keys(ctx, q, pages)
-        if keys:
-            out = ops.latent_attention_expanded(
-                q, pages, self.w_kv, sum(keys), max(keys), sum((n + ops.LATENT_TC5_ROWS - 1) // ops.LATENT_TC5_ROWS
-                                                               for n in ctx.q_len_host.tolist()),
-                group, ctx.seq_len, ctx.q_start, ctx.q_len, ctx.positions, H, rank, self.scale, self.window,
-                ctx.page_tokens, self.inv_freq, self.rot_dims, self.rot_scale, self.sink_logits,
-                down[:, qr + dk:] if self.out_gate else None, self.out_gate == "each")
+        out = torch.empty((T, H * V), dtype=self.dtype, device=x.device)
+        gate = down[:, qr + dk:] if self.out_gate else None
+        if keys is None:
+            self._on_latents(q, pages, ctx, ctx.attention_work(cache.group, H, self.tile_rows, self.window, H, rank), 0, T,
+                             gate, out)
             return ops.linear(out, self.w_o, None, out_dtype=self.dtype, kind=2)
+        if not all(keys):
+            # the other requests' rows, and those that lie between them, which the expanded form then writes over
+            rest = [r for r, n in enumerate(keys) if n == 0]
+            first, last = int(ctx.q_start_host[rest[0]]), int(ctx.q_start_host[rest[-1]] + ctx.q_len_host[rest[-1]])
+            self._on_latents(q, pages, ctx, ctx.attention_work_of(cache.group, H, self.tile_rows, self.window,
+                                                                  np.array(keys) == 0), first, last, gate, out)
+        for requests, total, most, row_tiles in self._goes(ctx, keys):
+            ops.latent_attention_expanded(
+                q, pages, self.w_kv, total, most, row_tiles, group, ctx.seq_len, ctx.q_start, ctx.q_len, ctx.positions, H,
+                rank, self.scale, self.window, ctx.page_tokens, self.inv_freq, self.rot_dims, self.rot_scale,
+                self.sink_logits, gate, self.out_gate == "each", requests, out)
+        return ops.linear(out, self.w_o, None, out_dtype=self.dtype, kind=2)
+
+    def _on_latents(self, q, pages, ctx, meta, first: int, last: int, gate, out):
+        """The rows ``first`` to ``last`` of the step that are in the work list ``meta``, on the cached latents."""
+        H, D, R, V, rank = self.num_heads, self.head_dim, self.rot_dim, self.value_dim, self.kv_rank
+        T, dk, n = q.shape[0], rank + R, last - first
+        cut = (lambda t: t) if n == T else (lambda t: t if t is None else t[first:last])
         # the heads' key maps applied to the queries, the rotated part behind: float32 [T, H, rank + R]
-        q_full = torch.empty((T, H, dk), dtype=torch.float32, device=x.device)
+        q_full = torch.empty((T, H, dk), dtype=torch.float32, device=q.device)
         # bfloat16 steps of more than a few rows: the per-head products on the tensor cores
-        product = ops.grouped_heads if (T > self.FEW_ROWS and self.w_uk.dtype == torch.bfloat16
+        product = ops.grouped_heads if (n > self.FEW_ROWS and self.w_uk.dtype == torch.bfloat16
                                         and q.dtype == torch.bfloat16) else ops.head_product
-        product(q, H * (D + R), D + R, D, self.w_uk, D * rank, rank, 1, rank, q_full, H * dk, dk, T, H,
-                rot=R, rot_dims=self.rot_dims, inv_freq=self.inv_freq, positions=ctx.positions,
-                rot_scale=self.rot_scale)
-        meta = ctx.attention_work(cache.group, H, self.tile_rows, self.window, H, rank)
+        product(cut(q), H * (D + R), D + R, D, self.w_uk, D * rank, rank, 1, rank, cut(q_full), H * dk, dk, n, H, rot=R,
+                rot_dims=self.rot_dims, inv_freq=self.inv_freq, positions=cut(ctx.positions), rot_scale=self.rot_scale)
         mixed = ops.latent_attention(q_full, pages, self.sink_logits, meta, H, rank, self.scale, self.window,
                                      ctx.page_tokens)                                   # float32 [T, H, rank]
         # the heads' value maps applied to the attention's output, times the heads' gates
-        out = torch.empty((T, H * V), dtype=self.dtype, device=x.device)
-        gate = down[:, qr + dk:] if self.out_gate else None
-        product(mixed, H * rank, rank, rank, self.w_uv, V * rank, 1, rank, V, out, H * V, V, T, H, gate=gate,
+        product(cut(mixed), H * rank, rank, rank, self.w_uv, V * rank, 1, rank, V, cut(out), H * V, V, n, H, gate=cut(gate),
                 gate_each=self.out_gate == "each")
-        return ops.linear(out, self.w_o, None, out_dtype=self.dtype, kind=2)
 
 
 register_part("mixer", "latent_attention", LatentAttention, replace=True)

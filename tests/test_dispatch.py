@@ -126,3 +126,55 @@ def test_state_space_form_is_known_from_the_widths(state, head, dtype, matrix):
     assert part.matrix is matrix
     assert (("linear_attention_mma", None) in part.kernel_libraries(dtype)) is matrix
     assert not matrix or all(n % 8 == 0 for n in (part.inner, part.groups * state, part.conv_channels))
+
+
+def _latent_part(heads):
+    from paged_batch_engine_b200.config import PartSpec
+    from paged_batch_engine_b200.parts import build_part
+    return build_part("mixer", PartSpec("latent_attention", dict(
+        hidden_size=256, num_heads=heads, head_dim=128, rot_dim=64, value_dim=128, kv_rank=512, q_rank=192, scale=192 ** -0.5,
+        eps=1e-6, rotary=dict(base=1e4, dims=64))), torch.bfloat16, torch.device("cpu"))
+
+
+def test_portions_that_expand_their_latents(monkeypatch):
+    """Decided for each request by its own rows and keys, on either side of every threshold."""
+    part = _latent_part(16)
+    assert [part.expanded(n, k) for n, k in ((7, 500), (8, 500), (8, 4096), (8, 4097), (31, 4097), (32, 4097))] \
+        == [0, 500, 4096, 0, 0, 4097]
+    assert part.expanded(512, 65536) == 65536 and part.expanded(512, 65537) == 0       # 512 MB of keys and values
+    assert _latent_part(128).expanded(512, 8192) == 8192 and _latent_part(128).expanded(512, 8193) == 0
+    rows, before = np.array([1, 300, 7, 16, 40, 1]), np.array([9000, 0, 30, 4081, 100, 20])
+    step = SimpleNamespace(q_len_host=rows, context_before_host=before)
+    assert part.ROWS_A_KEY == 8
+    operands = torch.empty(1, 16 * 192, dtype=torch.bfloat16), torch.empty(1, 1, 16, 576, dtype=torch.bfloat16)
+    assert part._expanded_keys(step, *operands) is None                                 # no weights yet
+    part.w_kv = torch.empty(2 * 16 * 128, 512, dtype=torch.bfloat16)
+    assert part._expanded_keys(step, *operands) == [0, 300, 0, 0, 140, 0]
+    alone = [SimpleNamespace(q_len_host=rows[i:i + 1], context_before_host=before[i:i + 1]) for i in range(6)]
+    assert [(part._expanded_keys(one, *operands) or [0])[0] for one in alone] == [0, 300, 0, 0, 140, 0]
+    part.window = 50
+    assert part._expanded_keys(step, *operands) == [0, 300, 0, 65, 89, 0]               # the keys that the rows see
+    part.window = None
+    step.device = torch.device("cpu")
+    step2 = SimpleNamespace(q_len_host=np.array([70, 1, 200, 64, 33]), device=torch.device("cpu"))
+    monkeypatch.setattr(ops, "LATENT_TC5_BYTES", 400 * 16 * 512)
+    goes = part._goes(step2, [70, 0, 300, 71, 283])
+    assert [(g[0].tolist(),) + g[1:] for g in goes] == [([0, 2], 370, 300, 1 + 2), ([3, 4], 354, 283, 1 + 1)]
+    assert part._goes(step2, [70, 0, 300, 71, 283]) is goes                             # once a step
+    assert part._goes(SimpleNamespace(q_len_host=np.array([300, 20]), device=torch.device("cpu")), [310, 50]) \
+        == [(None, 360, 310, 3 + 1)]
+
+
+def test_a_work_list_of_some_requests():
+    """The same tiles and key splits that these requests have in a list of all."""
+    from paged_batch_engine_b200.engine.batch import attention_work_arrays
+    q_len, seq_len = np.array([1, 300, 3, 1, 700]), np.array([2000, 300, 900, 5, 900])
+    q_start = np.cumsum(q_len) - q_len
+    some = np.array([True, False, True, True, False])
+    every = attention_work_arrays(q_len, seq_len, q_start, 16, 16, None)
+    part = attention_work_arrays(np.where(some, q_len, 0), seq_len, q_start, 16, 16, None)
+    assert sorted(map(tuple, part[0])) == sorted(tuple(w) for w in every[0] if some[w[0]])
+    split = [t for t in every[2].tolist() if some[np.searchsorted(q_start, t, side="right") - 1]]
+    assert part[2].tolist() == split and (part[1][split] >= 0).all() and part[4] == every[0][np.isin(every[0][:, 0], [0, 2, 3]), 3].max()
+    none = attention_work_arrays(np.zeros(5, dtype=np.int64), seq_len, q_start, 16, 16, None)
+    assert len(none[0]) == 0 and len(none[2]) == 0
