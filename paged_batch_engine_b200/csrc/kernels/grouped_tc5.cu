@@ -246,8 +246,6 @@ void launch_grouped(const CUtensorMap& map_a, const CUtensorMap& map_w, const Gr
 }
 }  // namespace
 
-PBE_EXPORT int pbe_grouped_tc5_tile_rows() { return BM; }
-
 // a [rows, K], w [groups, N, K], out [rows, N or N / 2], all bfloat16; tiles as the kernel's (null: all rows are group
 // 0's); epilogue as enumerated.
 // err: device int, set to 1 if a bounded wait ran out (the result is then invalid).

@@ -88,8 +88,8 @@ class TimeMixing(Mixer):
         """Rows of a segment when a long portion's recurrence is cut to run side by side: so long that the
         segments of all heads and column slices fill the GPU a few times over, a power of two, 64 to 1,024.  The
         scans on the tensor cores are short enough that segments of 64 rows pay more for the states between them than
-        they gain: 128 rows and more there (2,048 rows of 8 heads of 128: 173 -> 157 us a layer, 200 rows of 16 heads
-        135 -> 123, 2,048 rows of 16 heads, already 128, 247)."""
+        they gain: 128 rows and more there (2,048 rows of 8 heads of 128: 185 -> 169 us a layer, 200 rows of 16 heads
+        138 -> 129, 2,048 rows of 16 heads, already 128, 265)."""
         want = rows * self.num_heads * ((self.value_dim + 31) // 32) // 1024
         segment = 128 if self.dtype == torch.bfloat16 and self.key_dim <= 128 else 64
         while segment < want and segment < 1024:
