@@ -534,15 +534,24 @@ inline bool tiled_split(int M, int N, int K) {
 }
 
 // Up to sixteen rows behind the last whole tile of 128 go through the weight-streaming kernel (a row's result is the
-// same, bit for bit), where a tile row of their own would not find multiprocessors idle: it costs the multiply-adds of
-// 128 rows, about four times the reading of the weights (8,960 -> 1,536: 1,028 rows 791 -> 653 us, 140 rows 225 -> 185;
-// with the GPU half empty, 140 rows of 1,536 -> 2,048, it would be 68 -> 88).
+// same, bit for bit), where a tile row of their own would take another wave of blocks or there are so many that their ends
+// blur: it costs the multiply-adds of 128 rows, about four times the reading of the weights.  What comes here with that many
+// rows are the products side by side of float32 time mixing (2,048 -> 2,048, 515 rows 171 -> 138 us, 2,052 rows 414 -> 388;
+// 1,028 rows, whose two waves have room for the rest, would be 223 -> 241) and bfloat16 rows times float32 weights
+// (4,096 -> 4,096, 132 rows 234 -> 169 us).
+constexpr int WAVE = 2 * 148;               // blocks of 128-row tiles that run at a time
+inline long long tiled_blocks(int M, int N, int K) {
+  const long long tiles = (long long)((N + BN - 1) / BN) * ((M + 127) / 128);
+  return tiled_split(M, N, K) ? tiles * ((K + SLICE - 1) / SLICE) : tiles;
+}
+// waves of blocks, times the slices of K that each multiplies
+inline long long tiled_waves(int M, int N, int K) {
+  return (tiled_blocks(M, N, K) + WAVE - 1) / WAVE * (tiled_split(M, N, K) ? 1 : (K + SLICE - 1) / SLICE);
+}
 inline int rows_behind_tiles(int M, int N, int K) {
   const int rest = M % 128;
   if (M <= 128 || rest < 1 || rest > 16) return 0;
-  const long long tiles = (long long)((N + BN - 1) / BN) * ((M + 127) / 128);
-  const long long blocks = tiled_split(M, N, K) ? tiles * ((K + SLICE - 1) / SLICE) : tiles;
-  return blocks > 2 * 148 ? rest : 0;
+  return tiled_waves(M, N, K) > tiled_waves(M - rest, N, K) || tiled_blocks(M, N, K) > 7 * WAVE / 2 ? rest : 0;
 }
 
 template <int BM, bool SPLIT, typename TX, typename TY>
