@@ -4,28 +4,36 @@
 // 2^-25 of a product each at most, together as large as the rounding of the multiply-add that they stand for.
 //
 // The tensor cores add in float32 but cut off what does not fit instead of rounding it, so a sum is not left to them
-// for long: after every 64 k the accumulator in tensor memory starts anew, the small products are issued before hh, and the epilogue's warps add its contents to the tile's running sums in registers, with a rounding
-// add each; after 2,048 k the running sums are added to the output.  Against 64 bits, relative root mean square error of
-// sgemm.cu's multiply-adds -> this: normal numbers 4.1e-7 -> 1.2e-7 (K = 1,536) and 1.4e-7 (8,960, 19,200), positive ones
-// 2.1e-7 -> 1.1e-7 and 1.1e-7 -> 1.0e-7; a float32 model's logits after 1,028 prompt tokens 2.8e-6 -> 2.5e-6.  Where single
-// products outweigh all others (factors spread over e^3) both are at the last bit: 0.5-1.5e-7 and 0.7-1.4e-7.
+// for long: after every 64 k the accumulator in tensor memory starts anew, the small products are issued before hh, and the
+// epilogue's warps add its contents to the tile's running sums in registers, with a rounding add each; after 1,792 k at most the
+// running sums are added to the output.  Against 64 bits, relative root mean square error of sgemm.cu's multiply-adds -> this: normal
+// numbers 4.1e-7 -> 1.2e-7 (K = 1,536) and 1.3e-7 (8,960), positive ones 2.1e-7 -> 1.1e-7 and 1.1e-7 -> 1.0e-7; a float32 model's
+// logits after 1,028 prompt tokens 2.8e-6 -> 2.5e-6.  Where single products outweigh all others (factors spread over e^3) both
+// are at the last bit: 0.5-1.5e-7 and 0.7-1.4e-7.
 //
 // Two kernels a product:
-//  * split3: an operand's three terms as bfloat16 matrices one below the other, rows padded with zeros to 64 k; bound by
-//    memory (4 bytes in, 6 out).  It also tells whether an element is other than zero or of a size from SMALLEST to
-//    LARGEST: such a product is left to sgemm.cu, whose kernel is launched behind and looks at the flag.  A smaller one's
-//    third term would fall under bfloat16's smallest normal number, larger ones' products could overflow with either sign
-//    where their sum does not, and an infinity times a term that is zero would be no number.
-//  * the product: persistent blocks walk over tiles of 128 x BN, or over parts of K of such tiles where there are too few
-//    (a small kernel adds the parts in order); warp 0 is the TMA producer, warp 1 issues the MMAs (128 x BN x 16), warps
-//    2-9 hold the running sums, half a tile row a thread, and write them out.  Two accumulators alternate.  What bounds
-//    it is the tensor pipe, six products of the bfloat16 rate.  A slot of the ring holds one term of A and of W, 64 k
-//    wide (boxes 32 k wide, a stage with all terms a slot, were bound by the TMA unit, two cycles a row of 64 bytes:
-//    1,028 x 17,920 x 1,536 395 us); the terms come in the order l, h, m, so that a slot is free again after 8, 20 and 24
-//    of a block's 24 MMAs and each load has the time of a dozen MMAs or more.
-// Multiply-adds -> this, all launches: 1,028 rows 1,536 -> 17,920 1,190 -> 342 us, 8,960 -> 1,536 652 -> 223; 2,048 rows
-// 1,536 -> 17,920 2,278 -> 543 (208 TFLOP/s of float32, 1.25 PFLOP/s of bfloat16 products; a tile's operands out of L2 are
-// the next bound: 24 blocks of one wave take 1.6 us each, of eight waves 2.4); 65 rows 1,024 -> 1,024 66 -> 39.
+//  * split3: X's three terms as bfloat16 matrices one below the other, rows padded with zeros to 64 k.
+//  * the product, of tiles of 128 rows of W by up to 192 rows of X, as many X tiles as there have to be and of one size (a multiple
+//    of 16: 1,028 rows are six tiles of 176, where tiles of 128 rows of X leave four rows to a tile of their own).  W comes as it
+//    is: warp 14 fetches 128 rows x 64 k by TMA, warps 0-3 cut them into terms, a row a thread, and write these to tensor memory,
+//    where the MMAs take A from (terms written out by a kernel of their own took 47 us of 345 for 1,028 x 17,920 x 1,536, and are
+//    6 bytes an element to fetch instead of 4).  Warp 12 fetches X's terms, two sets of three; warp 13 issues the MMAs in
+//    the order l h, h l, m m, m h, h m, h h; warps 4-11 hold the running sums, a row of W and half of the tile's rows of X a
+//    thread, and write them out, 32 neighbouring columns of Y a warp.  Two accumulators alternate, and two of W's terms h; l and
+//    m are written while the products that do not need them run.  Persistent blocks walk over tiles, or over parts of K of
+//    tiles where there are too few (a small kernel adds the parts in order).
+// Either kernel also tells whether an element is other than zero or of a size from SMALLEST to LARGEST: such a product is left to
+// sgemm.cu, whose kernel is launched behind and looks at the flag.  A smaller one's third term would fall under bfloat16's
+// smallest normal number, larger ones' products could overflow with either sign where their sum does not, and an infinity
+// times a term that is zero would be no number.
+//
+// What bounds it is the tensor pipe, 2,112 clocks a K block of 176 rows (2,340 measured), and, where a wave of blocks ends, the
+// outputs' way to memory (350 clocks a K block on average).  The split has to be free of branches: with a test a number it took
+// 4,700 clocks a K block and bound everything.  A pair of blocks with cta_group::2 (half of X's rows a block) was slower, 305 us
+// against 258: the hand-over of W's terms then crosses blocks.
+// Terms of both operands written out and tiles of 128 x 256 -> this, all launches: 1,028 rows 1,536 -> 17,920 345 -> 254 us,
+// 8,960 -> 1,536 224 -> 166; 2,048 rows 1,536 -> 17,920 547 -> 480 (235 TFLOP/s of float32, 1.4 PFLOP/s of bfloat16 products);
+// 65 rows 1,536 -> 17,920 102 -> 57, 1,024 -> 1,024 37 -> 31.  Multiply-adds: 1,028 rows 1,190 and 652 us, 2,048 rows 2,278.
 //
 // Every wait on an mbarrier is bounded; one that runs out sets *err and the block goes on to its end.
 #include <cuda_bf16.h>
@@ -39,13 +47,26 @@ using namespace pbe::tc5;
 namespace {
 typedef __nv_bfloat16 bf16;
 constexpr int BM = 128, BK = 64, UMMA_K = 16, TERMS = 3;
-constexpr int SLICE = 2048 / BK;                  // K blocks whose sums are added in one chain
-constexpr int EPI_WARPS = 8, NTHREADS = 64 + 32 * EPI_WARPS;
+constexpr int SLICE = 28;                         // K blocks whose sums are added in one chain, at most
+constexpr int MAX_BN = 192;                       // rows of X a tile has at most
+constexpr int SPLIT_WARPS = 4, EPI_WARPS = 8, X_WARP = 12, MMA_WARP = 13, W_WARP = 14, NTHREADS = 32 * 15;
 constexpr float SMALLEST = 0x1p-102f;              // its last bit, 2^-125, is a bfloat16 number
 constexpr float LARGEST = 0x1p47f;                 // a sum of 2^31 products of two such numbers stays below 2^127
 
 // ------------------------------------------------------------------ the terms
-__device__ __forceinline__ bool whole_in_terms(float x) { return x == 0.f || (fabsf(x) >= SMALLEST && fabsf(x) <= LARGEST); }
+// Are numbers zero, or of a size from SMALLEST to LARGEST?  Without a branch a number: the largest size and the smallest that is not zero, as integers (zero less
+// one is the largest integer; infinities and what is no number are above LARGEST).
+struct Sizes {
+  uint32_t largest = 0, smallest = 0xffffffffu;
+  __device__ __forceinline__ void add(float x) {
+    const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
+    largest = max(largest, u);
+    smallest = min(smallest, u - 1u);
+  }
+  __device__ __forceinline__ bool whole() const {
+    return largest <= __float_as_uint(LARGEST) && smallest >= __float_as_uint(SMALLEST) - 1u;
+  }
+};
 
 // planes [TERMS][rows][Kp]; a thread takes eight k of a row
 __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* planes, int rows, int K, int Kp, int vec, int* flag) {
@@ -62,12 +83,13 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* plane
 #pragma unroll
     for (int i = 0; i < 8; ++i) v[i] = k + i < K ? src[i] : 0.f;
   }
-  bool plain = true;
+  Sizes sizes;
   unsigned out[TERMS][4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float a = v[2 * i], b = v[2 * i + 1];
-    plain = plain && whole_in_terms(a) && whole_in_terms(b);
+    sizes.add(a);
+    sizes.add(b);
 #pragma unroll
     for (int t = 0; t < TERMS; ++t) {
       const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
@@ -76,7 +98,7 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* plane
       b -= __high2float(p);
     }
   }
-  if (!plain) *flag = 1;
+  if (!sizes.whole()) *flag = 1;
 #pragma unroll
   for (int t = 0; t < TERMS; ++t)
     *reinterpret_cast<uint4*>(planes + ((size_t)t * rows + row) * Kp + k) = make_uint4(out[t][0], out[t][1], out[t][2], out[t][3]);
@@ -86,192 +108,308 @@ __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* plane
 struct ProductParams {
   const float* bias;       // [N] or null
   float* Y;                // [parts, M, ldy]
-  int M, N, Kp, ldy, aligned;
+  int M, N, Kp, ldy;
+  int bn;                  // rows of X a tile, a multiple of 16 up to MAX_BN
   int parts, part_blocks;  // of K, and K blocks a part
+  int* flag;               // set when an element of W is not whole in its terms
   int* err;
 };
 
-template <int BN> __host__ __device__ constexpr int slot_bytes() { return (BM + BN) * BK * 2; }
-template <int BN> __host__ __device__ constexpr int num_slots() { return BN == 256 ? 4 : 6; }
+constexpr int XB = MAX_BN * BK * 2, WB = BM * BK * 4;            // a slot of X's terms, a stage of W
+constexpr int X_SLOTS = 2 * TERMS, W_STAGES = 2;
+constexpr int PRODUCT_SMEM = X_SLOTS * XB + W_STAGES * WB + 1024;
+constexpr int A_COL = 2 * MAX_BN, TMEM_COLS = 512;               // the accumulators, then W's terms: l, m, h and the next h
+static_assert(A_COL + 4 * (BK / 2) <= TMEM_COLS && PRODUCT_SMEM <= 226 * 1024, "tensor and shared memory");
+__device__ __forceinline__ int slot_l() { return 0; }
+__device__ __forceinline__ int slot_m() { return 1; }
+__device__ __forceinline__ int slot_h(int block) { return 2 + (block & 1); }
 
-template <int BN>
+// acc_full, a K block's end, also gives back what it read: W's term h and X's terms, of which there are two sets
+struct ProductBarriers {
+  uint64_t w_full[W_STAGES], w_empty[W_STAGES], a_lh_full, a_m_full, l_empty, m_empty, x_full[2], acc_full[2], acc_empty[2];
+  uint32_t tmem_base;
+};
+
+// A from tensor memory (128 lanes x 8 columns of two bfloat16 per k-step), B from shared memory
+__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+}
+__device__ __forceinline__ void tmem_st32_nowait(uint32_t taddr, const uint32_t* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
+        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
+        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
+        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+  uint32_t r[16];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr) : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+// two numbers' next terms; what is left of them stays in x and y (exact: it has fewer bits than they had)
+__device__ __forceinline__ uint32_t next_term(float& x, float& y) {
+  const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&p);
+  x -= __uint_as_float(w << 16);
+  y -= __uint_as_float(w & 0xffff0000u);
+  return w;
+}
+
 __global__ void __launch_bounds__(NTHREADS, 1)
-sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, ProductParams p) {
-  constexpr int SLOTS = num_slots<BN>(), A_BYTES = BM * BK * 2, SLOT_BYTES = slot_bytes<BN>();
-  constexpr int TMEM_COLS = 2 * BN, HALF = BN / 2;
+sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, ProductParams p) {
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* slots = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  __shared__ __align__(8) uint64_t full_bar[SLOTS];
-  __shared__ __align__(8) uint64_t empty_bar[SLOTS];
-  __shared__ __align__(8) uint64_t acc_full[2];
-  __shared__ __align__(8) uint64_t acc_empty[2];
-  __shared__ uint32_t tmem_base_smem;
+  unsigned char* Ws = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);   // [stage][32 k][128 rows][128 B]
+  unsigned char* Xs = Ws + W_STAGES * WB;                                                                  // [slot][bn rows][128 B]
+  __shared__ ProductBarriers bar;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int kblocks = p.Kp / BK;
-  const int mtiles = (p.M + BM - 1) / BM, num_tiles = mtiles * ((p.N + BN - 1) / BN), items = num_tiles * p.parts;
+  const int kblocks = p.Kp / BK, bn = p.bn;
+  const int mtiles = (p.M + bn - 1) / bn, num_tiles = mtiles * ((p.N + BM - 1) / BM), items = num_tiles * p.parts;
+  auto first_block = [&](int t) { return t / num_tiles * p.part_blocks; };
+  auto last_block = [&](int t) { return min(first_block(t) + p.part_blocks, kblocks); };
 
   if (threadIdx.x == 0) {
-#pragma unroll
-    for (int s = 0; s < SLOTS; ++s) {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], 1);
+    for (int i = 0; i < W_STAGES; ++i) {
+      mbar_init(&bar.w_full[i], 1);
+      mbar_init(&bar.w_empty[i], SPLIT_WARPS);
     }
-#pragma unroll
-    for (int b = 0; b < 2; ++b) {
-      mbar_init(&acc_full[b], 1);
-      mbar_init(&acc_empty[b], EPI_WARPS);
+    mbar_init(&bar.a_lh_full, SPLIT_WARPS);
+    mbar_init(&bar.a_m_full, SPLIT_WARPS);
+    mbar_init(&bar.l_empty, 1);
+    mbar_init(&bar.m_empty, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&bar.x_full[i], 1);
+      mbar_init(&bar.acc_full[i], 1);
+      mbar_init(&bar.acc_empty[i], EPI_WARPS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) {
+  if (warp == MMA_WARP) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
-                 ::"r"(smem_u32(&tmem_base_smem)), "r"(TMEM_COLS) : "memory");
+                 ::"r"(smem_u32(&bar.tmem_base)), "r"(TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem_base = tmem_base_smem;
+  const uint32_t tmem_base = bar.tmem_base;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      // ------------------------------------------------------------ TMA producer
-      int it = 0;                                   // slots filled
-      bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        const int tile = t % num_tiles, k0 = t / num_tiles * p.part_blocks, k1 = min(k0 + p.part_blocks, kblocks);
-        const int m0 = (tile % mtiles) * BM, n0 = (tile / mtiles) * BN;
-        for (int kb = k0; kb < k1 && ok; ++kb) {
+  if (warp < SPLIT_WARPS) {
+    // -------------------------------------------------------------- W into terms: a row (tensor-memory lane) a thread
+    const int row = warp * 32 + lane;
+    const uint32_t a_addr = tmem_base + ((uint32_t)(warp * 32) << 16) + A_COL;
+    int b = 0;                                        // K blocks so far
+    bool ok = true;
+    Sizes sizes;
+    for (int t = blockIdx.x; t < items && ok; t += gridDim.x)
+      for (int kb = first_block(t); kb < last_block(t); ++kb, ++b) {
+        const int st = b % W_STAGES;
+        ok = mbar_wait(&bar.w_full[st], (b / W_STAGES) & 1, p.err);
+        if (!ok) break;
+        uint32_t w[TERMS][BK / 2];
 #pragma unroll
-          for (int i = 0; i < TERMS; ++i, ++it) {
-            const int term = i == 0 ? 2 : i - 1;    // l, h, m
-            const int s = it % SLOTS;
-            ok = mbar_wait(&empty_bar[s], ((it / SLOTS) & 1) ^ 1, p.err);
-            if (!ok) break;
-            unsigned char* a = slots + (size_t)s * SLOT_BYTES;
-            mbar_expect_tx(&full_bar[s], SLOT_BYTES);
-            // rows behind an operand's last belong to its next term (or are zeros): they reach no output that is written
-            tma_load_2d(a + A_BYTES, &map_w, kb * BK, term * p.N + n0, &full_bar[s]);
-            tma_load_2d(a, &map_a, kb * BK, term * p.M + m0, &full_bar[s]);
+        for (int c = 0; c < BK / 4; ++c) {
+          const unsigned char* at = Ws + st * WB + (c >> 3) * (BM * 128) + row * 128 + (((c & 7) ^ (row & 7)) << 4);
+          float4 v = *reinterpret_cast<const float4*>(at);
+          sizes.add(v.x);
+          sizes.add(v.y);
+          sizes.add(v.z);
+          sizes.add(v.w);
+#pragma unroll
+          for (int i = 0; i < TERMS; ++i) {
+            w[i][2 * c] = next_term(v.x, v.y);
+            w[i][2 * c + 1] = next_term(v.z, v.w);
           }
         }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.w_empty[st]);
+        const int h = slot_h(b);
+        // the term h of two blocks before is given back with that block's accumulator
+        ok = mbar_wait(&bar.l_empty, (b & 1) ^ 1, p.err) && mbar_wait(&bar.acc_full[b & 1], ((b >> 1) & 1) ^ 1, p.err);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_st32_nowait(a_addr + slot_l() * (BK / 2), w[2]);
+        tmem_st32_nowait(a_addr + h * (BK / 2), w[0]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.a_lh_full);
+        ok = mbar_wait(&bar.m_empty, (b & 1) ^ 1, p.err);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_st32_nowait(a_addr + slot_m() * (BK / 2), w[1]);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&bar.a_m_full);
       }
-      // the commits that release the last slots arrive on this block's barriers: it stays until they have
-      for (int q = it > SLOTS ? it - SLOTS : 0; q < it && ok; ++q)
-        ok = mbar_wait(&empty_bar[q % SLOTS], (q / SLOTS) & 1, p.err);
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      // ------------------------------------------------------------ MMA issuer: an accumulator a K block
-      const uint32_t idesc = make_idesc(BM, BN);
-      int it = 0, blocks = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
-        const int k0 = t / num_tiles * p.part_blocks, k1 = min(k0 + p.part_blocks, kblocks);
-        for (int kb = k0; kb < k1; ++kb, ++blocks, it += TERMS) {
-          const int buf = blocks & 1, sl = it % SLOTS, sh = (it + 1) % SLOTS, sm = (it + 2) % SLOTS;
-          ok = mbar_wait(&acc_empty[buf], ((blocks >> 1) & 1) ^ 1, p.err) &&
-               mbar_wait(&full_bar[sl], (it / SLOTS) & 1, p.err) &&
-               mbar_wait(&full_bar[sh], ((it + 1) / SLOTS) & 1, p.err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t tmem_d = tmem_base + buf * BN, base = smem_u32(slots);
-          const uint32_t l = base + sl * SLOT_BYTES, h = base + sh * SLOT_BYTES, m = base + sm * SLOT_BYTES;
-          auto product = [&](uint32_t a, uint32_t b, bool fresh) {
-#pragma unroll
-            for (int k = 0; k < BK / UMMA_K; ++k)
-              umma(tmem_d, make_desc(a + k * UMMA_K * 2), make_desc(b + A_BYTES + k * UMMA_K * 2), idesc, fresh && k == 0 ? 0u : 1u);
-          };
-          product(l, h, true);
-          product(h, l, false);
-          umma_commit(&empty_bar[sl]);
-          ok = mbar_wait(&full_bar[sm], ((it + 2) / SLOTS) & 1, p.err);
-          if (!ok) break;
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          product(m, m, false);
-          product(m, h, false);
-          product(h, m, false);
-          umma_commit(&empty_bar[sm]);
-          product(h, h, false);
-          umma_commit(&empty_bar[sh]);
-          umma_commit(&acc_full[buf]);
-        }
-      }
-    }
-  } else {
-    // -------------------------------------------------------------- running sums, warps 2..9
-    const int quarter = warp & 3;                   // the tensor-memory lanes this warp may read
-    const int half = (warp - 2) >> 2;               // of the tile's columns
+    if (!sizes.whole()) *p.flag = 1;
+    // the commits that release the last terms arrive on this block's barriers: it stays until they have
+    if (ok && b > 0) mbar_wait(&bar.l_empty, (b - 1) & 1, p.err) && mbar_wait(&bar.m_empty, (b - 1) & 1, p.err);
+  } else if (warp < SPLIT_WARPS + EPI_WARPS) {
+    // -------------------------------------------------------------- running sums: a row of W, half the tile's rows of X a thread
+    const int quarter = warp & 3, half = (warp - SPLIT_WARPS) >> 2;
+    constexpr int CHUNKS = MAX_BN / 32;
+    const int chunks = bn / 16, mine = half ? chunks / 2 : (chunks + 1) / 2, c0 = half ? (chunks + 1) / 2 : 0;
+    const uint32_t addr0 = tmem_base + ((uint32_t)(quarter * 32) << 16) + c0 * 16;
     int it = 0;
     bool ok = true;
     for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
       const int tile = t % num_tiles, part = t / num_tiles;
-      const int row = (tile % mtiles) * BM + quarter * 32 + lane, n0 = (tile / mtiles) * BN + half * HALF;
-      const int begin = part * p.part_blocks, end = min(begin + p.part_blocks, kblocks);
-      float* y = p.Y + ((size_t)part * p.M + row) * p.ldy + n0;
-      for (int k0 = begin; k0 < end && ok; k0 += SLICE) {
-        float acc[HALF];
+      const int n = (tile / mtiles) * BM + quarter * 32 + lane, m0 = (tile % mtiles) * bn + c0 * 16;
+      const int begin = first_block(t), end = last_block(t);
+      const int rows = n < p.N ? min(p.M - m0, mine * 16) : 0;
+      const int slices = (end - begin + SLICE - 1) / SLICE, slice = (end - begin + slices - 1) / slices;
+      for (int k0 = begin; k0 < end && ok; k0 += slice) {
+        float acc[CHUNKS * 16];
 #pragma unroll
-        for (int i = 0; i < HALF; ++i) acc[i] = 0.f;
-        const int k1 = min(k0 + SLICE, end);
+        for (int i = 0; i < CHUNKS * 16; ++i) acc[i] = 0.f;
+        const int k1 = min(k0 + slice, end);
         for (int kb = k0; kb < k1; ++kb, ++it) {
           const int buf = it & 1;
-          ok = mbar_wait(&acc_full[buf], (it >> 1) & 1, p.err);
+          ok = mbar_wait(&bar.acc_full[buf], (it >> 1) & 1, p.err);
           if (!ok) break;                             // flagged; the roles run to their end
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN + half * HALF;
 #pragma unroll
-          for (int c = 0; c < HALF / 32; ++c) {
-            float v[32];
-            tmem_ld32(addr + c * 32, v);
+          for (int c = 0; c < CHUNKS; ++c) {
+            if (c < mine) {
+              float v[16];
+              tmem_ld16(addr0 + buf * MAX_BN + c * 16, v);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) acc[c * 32 + i] += v[i];
+              for (int i = 0; i < 16; ++i) acc[c * 16 + i] += v[i];
+            }
           }
           asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
           __syncwarp();
-          if (lane == 0) mbar_arrive(&acc_empty[buf]);
+          if (lane == 0) mbar_arrive(&bar.acc_empty[buf]);
         }
-        if (!ok || row >= p.M) continue;
-        // the slices before lie in Y, written by this thread
-        const bool first = k0 == begin, last = k1 == end;
+        if (!ok) break;
+        // the slices before lie in Y, written by this thread; 32 neighbouring columns a warp and row
+        float* y = p.Y + ((size_t)part * p.M + m0) * p.ldy + n;
+        const bool first = k0 == begin;
+        const float bias = k1 == end && p.bias && n < p.N ? p.bias[n] : 0.f;
+        const bool add = k1 == end && p.bias != nullptr;
 #pragma unroll
-        for (int i = 0; i < HALF; i += 4) {
-          if (n0 + i >= p.N) break;
-          if (p.aligned && n0 + i + 4 <= p.N) {
-            float4* at = reinterpret_cast<float4*>(y + i);
-            float4 v = make_float4(acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
-            if (!first) {
-              const float4 u = *at;
-              v = make_float4(u.x + v.x, u.y + v.y, u.z + v.z, u.w + v.w);
-            }
-            if (last && p.bias) {
-              v.x += p.bias[n0 + i];
-              v.y += p.bias[n0 + i + 1];
-              v.z += p.bias[n0 + i + 2];
-              v.w += p.bias[n0 + i + 3];
-            }
-            *at = v;
-          } else {
+        for (int i = 0; i < CHUNKS * 16; i += 8) {
+          if (i >= rows) continue;
+          float before[8];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              if (n0 + i + j >= p.N) break;
-              float v = first ? acc[i + j] : y[i + j] + acc[i + j];
-              if (last && p.bias) v += p.bias[n0 + i + j];
-              y[i + j] = v;
+          for (int k = 0; k < 8; ++k) before[k] = !first && i + k < rows ? y[(size_t)k * p.ldy] : 0.f;
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            if (i + k < rows) {
+              float v = first ? acc[i + k] : before[k] + acc[i + k];
+              if (add) v += bias;
+              *y = v;
             }
+            y += p.ldy;
           }
+          asm volatile("" ::: "memory");              // eight loads ahead, not ninety-six
         }
       }
+    }
+  } else if (warp == X_WARP) {
+    if (lane == 0) {
+      // ------------------------------------------------------------ TMA: X's terms
+      int b = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+        const int m0 = (t % num_tiles % mtiles) * bn;
+        for (int kb = first_block(t); kb < last_block(t); ++kb, ++b) {
+          ok = mbar_wait(&bar.acc_full[b & 1], ((b >> 1) & 1) ^ 1, p.err);       // the block two before
+          if (!ok) break;
+          mbar_expect_tx(&bar.x_full[b & 1], TERMS * bn * BK * 2);
+          // rows behind X's last belong to its next term (or are zeros): they reach no output that is written
+          for (int term = 0; term < TERMS; ++term)
+            tma_load_2d(Xs + ((b & 1) * TERMS + term) * XB, &map_x, kb * BK, term * p.M + m0, &bar.x_full[b & 1]);
+        }
+      }
+    }
+  } else if (warp == W_WARP) {
+    if (lane == 0) {
+      // ------------------------------------------------------------ TMA: W as it is
+      int b = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < items && ok; t += gridDim.x) {
+        const int n0 = (t % num_tiles / mtiles) * BM;
+        for (int kb = first_block(t); kb < last_block(t); ++kb, ++b) {
+          const int st = b % W_STAGES;
+          ok = mbar_wait(&bar.w_empty[st], ((b / W_STAGES) & 1) ^ 1, p.err);
+          if (!ok) break;
+          mbar_expect_tx(&bar.w_full[st], WB);
+          tma_load_2d(Ws + st * WB, &map_w, kb * BK, n0, &bar.w_full[st]);
+          tma_load_2d(Ws + st * WB + WB / 2, &map_w, kb * BK + BK / 2, n0, &bar.w_full[st]);
+        }
+      }
+    }
+  } else if (lane == 0) {
+    // -------------------------------------------------------------- MMA issuer: an accumulator a K block
+    const uint32_t idesc = make_idesc(BM, bn);
+    const uint64_t x_desc = make_desc(smem_u32(Xs));
+    int b = 0;
+    bool ok = true;
+    // what block b's first products need; called before the last ones of the block before are issued, which run meanwhile
+    auto ready = [&](int b) {
+      return mbar_wait(&bar.acc_empty[b & 1], ((b >> 1) & 1) ^ 1, p.err) && mbar_wait(&bar.x_full[b & 1], (b >> 1) & 1, p.err) &&
+             mbar_wait(&bar.a_lh_full, b & 1, p.err);
+    };
+    int left = 0;                                     // K blocks this thread block has in all
+    for (int t = blockIdx.x; t < items; t += gridDim.x) left += last_block(t) - first_block(t);
+    if (left > 0) ok = ready(0);
+    for (; b < left && ok; ++b) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tmem_d = tmem_base + (b & 1) * MAX_BN, tmem_a = tmem_base + A_COL;
+      const uint64_t xb = x_desc + (uint64_t)(((b & 1) * TERMS * XB) >> 4);
+      auto product = [&](int a_slot, int x_term, bool fresh) {
+#pragma unroll
+        for (int k = 0; k < BK / UMMA_K; ++k)
+          umma_ts(tmem_d, tmem_a + a_slot * (BK / 2) + k * (UMMA_K / 2), xb + (uint64_t)((x_term * XB + k * UMMA_K * 2) >> 4), idesc,
+                  fresh && k == 0 ? 0u : 1u);
+      };
+      const int h = slot_h(b);
+      product(slot_l(), 0, true);
+      product(h, 2, false);
+      umma_commit(&bar.l_empty);
+      ok = mbar_wait(&bar.a_m_full, b & 1, p.err);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      product(slot_m(), 1, false);
+      product(slot_m(), 0, false);
+      umma_commit(&bar.m_empty);
+      product(h, 1, false);
+      if (b + 1 < left) ok = ready(b + 1);
+      product(h, 0, false);
+      umma_commit(&bar.acc_full[b & 1]);              // the accumulator, its h terms and X's terms
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 1) {
+  if (warp == MMA_WARP) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
   }
+}
+
+// A matrix whose rows the TMA unit cannot take (not of a multiple of 16 bytes, or misaligned), rows padded with zeros to 64 k
+__global__ void __launch_bounds__(256) pad_rows_kernel(const float* w, float* out, long long rows, int K, int Kp) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= rows * Kp) return;
+  const long long row = i / Kp;
+  const int k = (int)(i - row * Kp);
+  out[i] = k < K ? w[row * K + k] : 0.f;
 }
 
 // Y = the parts of K, in order, + bias
@@ -296,14 +434,30 @@ int multiprocessors() {
   return n;
 }
 
-template <int BN>
-int launch_product(const CUtensorMap& map_a, const CUtensorMap& map_w, const ProductParams& p, cudaStream_t stream) {
-  const int smem = num_slots<BN>() * slot_bytes<BN>() + 1024;
-  const cudaError_t e = cudaFuncSetAttribute(sgemm_tc5_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  if (e != cudaSuccess) return (int)e;
-  const long long tiles = (long long)((p.M + BM - 1) / BM) * ((p.N + BN - 1) / BN) * p.parts;
+// [rows, K] row-major float32, rows ld elements apart, boxes of BM rows x 32, 128-byte swizzle, zeros outside
+int make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld) {
+  EncodeTiledFn fn = encode_fn();
+  if (fn == nullptr) return (int)cudaErrorNotSupported;
+  cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+  cuuint64_t strides[1] = {(cuuint64_t)ld * 4};
+  cuuint32_t box[2] = {32, (cuuint32_t)BM};
+  cuuint32_t estr[2] = {1, 1};
+  const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)cudaErrorInvalidValue;
+}
+
+int launch_product(const CUtensorMap& map_w, const CUtensorMap& map_x, const ProductParams& p, cudaStream_t stream) {
+  static bool opted = false;
+  if (!opted) {
+    const cudaError_t e = cudaFuncSetAttribute(sgemm_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PRODUCT_SMEM);
+    if (e != cudaSuccess) return (int)e;
+    opted = true;
+  }
+  const long long tiles = (long long)((p.M + p.bn - 1) / p.bn) * ((p.N + BM - 1) / BM) * p.parts;
   const int blocks = (int)(tiles < multiprocessors() ? tiles : multiprocessors());
-  sgemm_tc5_kernel<BN><<<blocks, NTHREADS, smem, stream>>>(map_a, map_w, p);
+  sgemm_tc5_kernel<<<blocks, NTHREADS, PRODUCT_SMEM, stream>>>(map_w, map_x, p);
   return launch_status();
 }
 
@@ -316,23 +470,21 @@ int split3(const float* x, bf16* planes, int rows, int K, int Kp, int* flag, cud
 
 int padded(int K) { return (K + BK - 1) / BK * BK; }
 
-// Columns of W whose terms are made and multiplied at a time: all, unless the terms would take more than 256 MB (the
-// 1.5B model's gate and up matrix takes 165, a vocabulary of 152 thousand 1,400).
+// Rows of W that are padded and multiplied at a time, where they have to be: all, unless they would take more than 256 MB.
 int columns_at_a_time(int N, int Kp) {
-  const long long most = (256LL << 20) / ((long long)TERMS * Kp * 2) / 256 * 256;
-  return most < 256 ? (N < 256 ? N : 256) : (int)(N < most ? N : most);
+  const long long most = (256LL << 20) / ((long long)Kp * 4) / BM * BM;
+  return most < BM ? (N < BM ? N : BM) : (int)(N < most ? N : most);
 }
 
-// Rows of X whose terms are made at a time: all, unless they would take more than 256 MB, else groups of whole tiles and about
-// one size (2,304 rows and more for K up to 18,944, so that making W's terms once more for each costs a tenth at most).
+// Rows of X whose terms are made at a time: all, unless they would take more than 256 MB, else groups of one size, about.
 int rows_at_a_time(int M, int Kp) {
-  const long long most = (256LL << 20) / ((long long)TERMS * Kp * 2) / BM * BM;
-  if (M <= most || M <= BM) return M;
-  const long long groups = most < BM ? (M + BM - 1) / BM : (M + most - 1) / most;
-  return (int)(((M + groups - 1) / groups + BM - 1) / BM * BM);
+  const long long most = (256LL << 20) / ((long long)TERMS * Kp * 2) / 16 * 16;
+  if (M <= most || M <= 16) return M;
+  const long long groups = most < 16 ? (M + 15) / 16 : (M + most - 1) / most;
+  return (int)(((M + groups - 1) / groups + 15) / 16 * 16);
 }
 
-// How M x N outputs over K are cut: the tiles' columns and the parts of K that take least by this count (microseconds, as
+// How M x N outputs over K are cut: the rows of X a tile has and the parts of K that take least by this count (microseconds, as
 // measured: a K block of a tile, its start and end, the parts' way through memory).
 struct Plan {
   int bn, parts, part_blocks;
@@ -342,14 +494,20 @@ struct Plan {
 Plan plan_of(int M, int N, int Kp) {
   const int kblocks = Kp / BK, sms = multiprocessors();
   Plan best{0, 1, kblocks, 0.f};
-  for (int bn = 256; bn >= 128; bn -= 128) {
-    const long long tiles = (long long)((M + BM - 1) / BM) * ((N + bn - 1) / bn);
+  const int fewest = (M + MAX_BN - 1) / MAX_BN;
+  int before = 0;
+  for (int mtiles = fewest; mtiles < fewest + 4; ++mtiles) {
+    const int bn = ((M + mtiles - 1) / mtiles + 15) / 16 * 16;
+    if (bn == before) continue;
+    before = bn;
+    const long long tiles = (long long)((M + bn - 1) / bn) * ((N + BM - 1) / BM);
+    const float block_us = 1.1f + bn * 0.0025f;
     for (int parts = 1; parts <= 8; ++parts) {
       const int per = (kblocks + parts - 1) / parts;
       const long long bytes = (long long)parts * M * N * 4;
       if (parts > 1 && (per < 8 || (long long)per * (parts - 1) >= kblocks || bytes > (128LL << 20))) continue;
       const long long waves = (tiles * parts + sms - 1) / sms;
-      const float us = (float)waves * ((float)per * (bn == 256 ? 1.9f : 1.0f) + 4.f) + (parts > 1 ? 4.f + (float)bytes * 2.f / 4e6f : 0.f);
+      const float us = (float)waves * (float)per * block_us + 4.f + (parts > 1 ? 4.f + (float)bytes * 2.f / 4e6f : 0.f);
       if (best.bn == 0 || us < best.us) best = Plan{bn, parts, per, us};
     }
   }
@@ -358,21 +516,12 @@ Plan plan_of(int M, int N, int Kp) {
 
 long long aligned256(long long bytes) { return (bytes + 255) / 256 * 256; }
 long long part_bytes(const Plan& plan, int M, int N) { return plan.parts > 1 ? aligned256((long long)plan.parts * M * N * 4) : 0; }
+bool takes_rows(int K) { return K % 4 == 0; }              // can the TMA unit take W's rows where they lie?
 }  // namespace
 
-// Rows of M that pbe_sgemm_tc5 should be given: without those behind the last whole tile of 128, where a tile row of
-// their own would cost more than pbe_sgemm_nt's streaming of the weights for up to sixteen rows.
-PBE_EXPORT int pbe_sgemm_tc5_rows(int M, int N, int K) {
-  const int rest = M % BM, Kp = padded(K);
-  if (M <= BM || rest < 1 || rest > 16) return M;
-  const float stream_us = 8.f + (float)N * (float)K * 4.f / 4.5e6f;
-  return plan_of(M - rest, N, Kp).us + stream_us < plan_of(M, N, Kp).us ? M - rest : M;
-}
-
-// Bytes of scratch memory, 256-byte aligned, that pbe_sgemm_tc5 needs: the flag, X's terms, W's terms, the parts' sums; at
-// most 256 + 256 + 128 MB whatever M and N are (K up to 174,762, where 256 rows' or columns' terms take 256 MB).
-PBE_EXPORT long long pbe_sgemm_tc5_scratch(int M, int N, int K) {
-  const int Kp = padded(K), columns = columns_at_a_time(N, Kp), rows = rows_at_a_time(M, Kp);
+namespace {
+long long scratch_bytes(int M, int N, int K, bool pad) {
+  const int Kp = padded(K), columns = pad ? columns_at_a_time(N, Kp) : N, rows = rows_at_a_time(M, Kp);
   long long parts = 0;
   for (const int m : {rows, M % rows})                   // the groups' sizes
     for (const int n : {columns, N % columns})
@@ -380,8 +529,15 @@ PBE_EXPORT long long pbe_sgemm_tc5_scratch(int M, int N, int K) {
         const long long bytes = part_bytes(plan_of(m, n, Kp), m, n);
         if (bytes > parts) parts = bytes;
       }
-  return 256 + aligned256((long long)rows * TERMS * Kp * 2) + aligned256((long long)columns * TERMS * Kp * 2) + parts;
+  return 256 + aligned256((long long)rows * TERMS * Kp * 2) + (pad ? aligned256((long long)columns * Kp * 4) : 0) + parts;
 }
+}  // namespace
+
+// Bytes of scratch memory, 256-byte aligned, that pbe_sgemm_tc5 needs: the flag, X's terms, W's padded rows where the TMA unit
+// cannot take them where they lie, the parts' sums; at most 256 + 256 + 128 MB whatever M and N are (K up to 500,000, where 128 rows
+// of W and 80 rows' terms take 256 MB).  _padded: for a W that does not start on a 16-byte boundary.
+PBE_EXPORT long long pbe_sgemm_tc5_scratch(int M, int N, int K) { return scratch_bytes(M, N, K, !takes_rows(K)); }
+PBE_EXPORT long long pbe_sgemm_tc5_scratch_padded(int M, int N, int K) { return scratch_bytes(M, N, K, true); }
 
 // X [M, K], W [N, K], Y [M, N], float32, contiguous.  Afterwards the first int of scratch says whether an element was not
 // finite, too large or too small: Y is then to be made by pbe_sgemm_nt_if.
@@ -390,35 +546,40 @@ PBE_EXPORT int pbe_sgemm_tc5(const float* X, const float* W, const float* bias, 
                              int* err, cudaStream_t stream) {
   if (M <= 0 || N <= 0) return 0;
   if (K <= 0 || scratch == nullptr || ((uintptr_t)scratch & 255)) return (int)cudaErrorInvalidValue;
-  if ((long long)M * TERMS > 0x7fffffffLL - 512 || (long long)N * TERMS > 0x7fffffffLL - 512 || K > 0x7fffffff - BK)
-    return (int)cudaErrorInvalidValue;
-  const int Kp = padded(K), columns = columns_at_a_time(N, Kp), rows = rows_at_a_time(M, Kp);
+  if ((long long)M * TERMS > 0x7fffffffLL - 512 || N > 0x7fffffff - 512 || K > 0x7fffffff - BK) return (int)cudaErrorInvalidValue;
+  const bool pad = !takes_rows(K) || ((uintptr_t)W & 15);
+  const int Kp = padded(K), columns = pad ? columns_at_a_time(N, Kp) : N, rows = rows_at_a_time(M, Kp);
   int* flag = (int*)scratch;
   bf16* xt = (bf16*)((char*)scratch + 256);
-  bf16* wt = (bf16*)((char*)xt + aligned256((long long)rows * TERMS * Kp * 2));
-  float* sums = (float*)((char*)wt + aligned256((long long)columns * TERMS * Kp * 2));
+  float* wp = (float*)((char*)xt + aligned256((long long)rows * TERMS * Kp * 2));
+  float* sums = (float*)((char*)wp + (pad ? aligned256((long long)columns * Kp * 4) : 0));
   const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), stream);
   if (e != cudaSuccess) return (int)e;
   int rc = 0;
-  CUtensorMap map_a, map_w;
+  CUtensorMap map_x, map_w;
   for (int m0 = 0; m0 < M && rc == 0; m0 += rows) {
     const int m = M - m0 < rows ? M - m0 : rows;
     rc = split3(X + (size_t)m0 * K, xt, m, K, Kp, flag, stream);
-    if (rc == 0) rc = make_map(&map_a, xt, m * TERMS, Kp, BM);
     for (int n0 = 0; n0 < N && rc == 0; n0 += columns) {
       const int n = N - n0 < columns ? N - n0 : columns;
-      if (m0 == 0 || columns < N) rc = split3(W + (size_t)n0 * K, wt, n, K, Kp, flag, stream);
+      const float* w = W + (size_t)n0 * K;
+      if (pad) {
+        if (m0 == 0 || columns < N) {
+          pad_rows_kernel<<<(unsigned)(((long long)n * Kp + 255) / 256), 256, 0, stream>>>(w, wp, n, K, Kp);
+          rc = launch_status();
+        }
+        w = wp;
+      }
       const Plan plan = plan_of(m, n, Kp);
-      if (rc == 0) rc = make_map(&map_w, wt, n * TERMS, Kp, plan.bn);
+      if (rc == 0) rc = make_map(&map_x, xt, m * TERMS, Kp, plan.bn);
+      if (rc == 0) rc = pad ? make_map_f32(&map_w, w, n, Kp, Kp) : make_map_f32(&map_w, w, n, K, K);
       if (rc != 0) break;
       const bool parts = plan.parts > 1;
       float* out = Y + (size_t)m0 * N + n0;
-      float* y = parts ? sums : out;
-      const int ldy = parts ? n : N;
       const float* b = bias ? bias + n0 : nullptr;
-      const ProductParams p{parts ? nullptr : b, y, m, n, Kp, ldy, (ldy % 4 == 0 && ((uintptr_t)y & 15) == 0) ? 1 : 0,
-                            plan.parts, plan.part_blocks, err};
-      rc = plan.bn == 128 ? launch_product<128>(map_a, map_w, p, stream) : launch_product<256>(map_a, map_w, p, stream);
+      const ProductParams p{parts ? nullptr : b, parts ? sums : out, m, n, Kp, parts ? n : N, plan.bn, plan.parts, plan.part_blocks,
+                            flag, err};
+      rc = launch_product(map_w, map_x, p, stream);
       if (rc == 0 && parts) {
         add_parts_kernel<<<(unsigned)(((long long)m * n + 255) / 256), 256, 0, stream>>>(sums, plan.parts, b, out, m, n, N);
         rc = launch_status();

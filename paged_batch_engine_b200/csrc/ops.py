@@ -718,11 +718,8 @@ def sgemm_tc5(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor], ou
         raise KernelError("sgemm_tc5: shapes or dtypes do not agree")
     if bias is not None and (bias.dtype != torch.float32 or bias.numel() != N):
         raise KernelError("sgemm_tc5: bias must be float32 [N]")
-    tiled = int(_fn("sgemm_tc5", "pbe_sgemm_tc5_rows", [c_int] * 3)(M, N, K))
-    if tiled < M:
-        sgemm_nt(x[tiled:], w, bias, out[tiled:])
-        M = tiled
-    need = _fn("sgemm_tc5", "pbe_sgemm_tc5_scratch", [c_int, c_int, c_int])
+    name = "pbe_sgemm_tc5_scratch" if w.data_ptr() % 16 == 0 else "pbe_sgemm_tc5_scratch_padded"
+    need = _fn("sgemm_tc5", name, [c_int, c_int, c_int])
     need.restype = c_ll
     scratch = torch.empty(int(need(M, N, K)), dtype=torch.uint8, device=x.device)
     err = _tc5_err.get(x.device)
