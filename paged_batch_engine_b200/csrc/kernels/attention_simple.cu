@@ -44,9 +44,15 @@ __device__ __forceinline__ float4 load_row4(const __nv_bfloat16* p) {
   return make_float4(__low2float(lo), __high2float(lo), __low2float(hi), __high2float(hi));
 }
 
+// handed_back (or null): the step is another kernel's (attention_f32_tc5.cu), but for the 128-row tiles and splits whose entry
+// [place of the tile, split, key/value head] is set.
+struct Rest {
+  const int32_t* handed_back;
+};
+
 template <typename T>
 __global__ void __launch_bounds__(NWARPS * 32)
-attn_simple_kernel(AttnParams p) {
+attn_simple_kernel(AttnParams p, Rest rest) {
   extern __shared__ __align__(16) float smem[];
   float* Qs = smem;                       // [BM][HD]
   float* Ks = Qs + BM * HD;               // [BN][HD + 1]
@@ -64,6 +70,9 @@ attn_simple_kernel(AttnParams p) {
   const int n_packed = nq * G;
   const int pr0 = m_tile * BM;
   if (pr0 >= n_packed) return;
+  if (rest.handed_back &&
+      !rest.handed_back[((size_t)((long long)qs * G / 128 + r + pr0 / 128) * p.max_splits + split) * KV + kvh])
+    return;
   const int row_lo = pr0 / G;
   const int last_pr = min(n_packed, pr0 + BM) - 1;
   const int row_hi = last_pr / G;
@@ -294,8 +303,8 @@ PBE_EXPORT int pbe_attn_simple_tile_rows() { return BM; }
 PBE_EXPORT int pbe_attn_simple_key_tile() { return BN; }
 PBE_EXPORT int pbe_attn_simple_head_dim() { return HD; }
 
-PBE_EXPORT int pbe_attn_simple(const AttnParams* params, int num_work, int dtype,
-                               cudaStream_t stream) {
+namespace {
+int launch_simple(const AttnParams* params, int num_work, int dtype, Rest rest, cudaStream_t stream) {
   if (num_work <= 0) return 0;
   AttnParams p = *params;
   if (p.num_heads % p.num_kv_heads != 0 || p.tile_rows != BM || p.split_keys % BN != 0)
@@ -310,15 +319,21 @@ PBE_EXPORT int pbe_attn_simple(const AttnParams* params, int num_work, int dtype
       cudaFuncSetAttribute(attn_simple_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       opted[0] = true;
     }
-    launch_k(attn_simple_kernel<float>, grid, NWARPS * 32, smem, stream, p);
+    launch_k(attn_simple_kernel<float>, grid, NWARPS * 32, smem, stream, p, rest);
   } else {
     if (!opted[1]) {
       cudaFuncSetAttribute(attn_simple_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       opted[1] = true;
     }
-    launch_k(attn_simple_kernel<__nv_bfloat16>, grid, NWARPS * 32, smem, stream, p);
+    launch_k(attn_simple_kernel<__nv_bfloat16>, grid, NWARPS * 32, smem, stream, p, rest);
   }
   return launch_status();
+}
+}  // namespace
+
+PBE_EXPORT int pbe_attn_simple(const AttnParams* params, int num_work, int dtype,
+                               cudaStream_t stream) {
+  return launch_simple(params, num_work, dtype, Rest{nullptr}, stream);
 }
 
 PBE_EXPORT int pbe_attn_merge(const AttnMergeParams* params, int split_rows, int dtype,

@@ -54,8 +54,8 @@ constexpr float SMALLEST = 0x1p-102f;              // its last bit, 2^-125, is a
 constexpr float LARGEST = 0x1p47f;                 // a sum of 2^31 products of two such numbers stays below 2^127
 
 // ------------------------------------------------------------------ the terms
-// Are numbers zero, or of a size from SMALLEST to LARGEST?  Without a branch a number: the largest size and the smallest that is not zero, as integers (zero less
-// one is the largest integer; infinities and what is no number are above LARGEST).
+// Are numbers zero, or of a size from SMALLEST to LARGEST?  Without a branch a number: the largest size and the smallest that is
+// not zero, as integers (zero less one is the largest integer; infinities and what is no number are above LARGEST).
 struct Sizes {
   uint32_t largest = 0, smallest = 0xffffffffu;
   __device__ __forceinline__ void add(float x) {

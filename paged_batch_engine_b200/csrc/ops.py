@@ -1041,6 +1041,23 @@ def _mma_available() -> bool:
     return os.path.isfile(os.path.join(KERNEL_DIR, "attention_mma.cu"))
 
 
+F32_TILE_ROWS = 128     # packed rows per block of the float32 tensor-core kernel, which takes the steps
+F32_SMALL_ROWS = 64     # that have a request of more packed rows than this
+
+
+def attention_f32_tiles(q_len, seq_len, group_size: int, window, split_keys: int) -> int:
+    """Blocks a key/value head that ``attention_f32_tc5.cu`` takes a step in (the requests' lengths as numpy arrays): the row
+    tiles of requests of many rows and the key splits of the others; 0 where it does not take the step."""
+    packed = q_len * group_size
+    wide = packed > F32_SMALL_ROWS
+    if not wide.any():
+        return 0
+    low = (seq_len - q_len - window + 1).clip(0) if window else 0 * seq_len
+    splits = (seq_len + split_keys - 1) // split_keys - low // split_keys
+    tiles = (packed + F32_TILE_ROWS - 1) // F32_TILE_ROWS
+    return int(tiles[wide].sum() + splits[~wide & (packed > 0)].sum())
+
+
 def paged_attention(q, k_cache, v_cache, out, meta, num_heads, num_kv_heads, head_dim, scale, window,
                     page_tokens, kind="simple"):
     """Causal attention of every row of the batch over the paged cache.
@@ -1085,10 +1102,21 @@ def paged_attention(q, k_cache, v_cache, out, meta, num_heads, num_kv_heads, hea
             _check(tfn(ctypes.byref(p), int(meta.num_work), int(k_cache.shape[0]), _ptr(err), _stream()),
                    "paged_attention (tcgen05)")
         p.kinds = (p.kinds | 8) if (p.kinds & 3) else (1 | 8)
-    fn = _fn(lib, "pbe_attn_" + kind, [ctypes.POINTER(AttnParams), c_int, c_int, c_void_p], defines)
-    if kind == "mma":
-        _mma_flag_heads.add(int(head_dim))
-    _check(fn(ctypes.byref(p), int(meta.num_work), _dtype_code(q), _stream()), "paged_attention")
+    wide_tiles = getattr(meta, "wide_tiles", 0)
+    if kind == "simple" and wide_tiles and q.dtype == torch.float32 and head_dim in (64, 128):
+        # a step with prompt portions: on tcgen05, and the row tiles with elements whose terms do not hold them (found on the
+        # device) by the multiply-adds
+        if meta.handed_back is None:
+            places = int(q.shape[0]) * (num_heads // num_kv_heads) // F32_TILE_ROWS + int(meta.q_len.numel()) + 1
+            meta.handed_back = torch.empty(places * num_kv_heads * int(meta.max_splits), dtype=torch.int32, device=q.device)
+        fn = _fn("attention_f32_tc5", "pbe_attn_f32", [ctypes.POINTER(AttnParams)] + [c_int] * 3 + [c_void_p] * 3, defines)
+        _check(fn(ctypes.byref(p), int(meta.num_work), wide_tiles, int(meta.q_len.numel()), _ptr(meta.handed_back),
+                  _ptr(tc5_attention_error_buffer(q.device)), _stream()), "paged_attention (float32, tcgen05)")
+    else:
+        fn = _fn(lib, "pbe_attn_" + kind, [ctypes.POINTER(AttnParams), c_int, c_int, c_void_p], defines)
+        if kind == "mma":
+            _mma_flag_heads.add(int(head_dim))
+        _check(fn(ctypes.byref(p), int(meta.num_work), _dtype_code(q), _stream()), "paged_attention")
     if meta.num_split_rows > 0:
         mp = AttnMergeParams(part_o=meta.part_o.data_ptr(), part_ml=meta.part_ml.data_ptr(),
                              out=out.data_ptr(), split_tokens=meta.split_tokens.data_ptr(),
@@ -1287,6 +1315,8 @@ def raise_on_kernel_status(device) -> None:
 def attention_libraries(head_dim: int, dtype: torch.dtype):
     """The (library, defines) pairs a model with this head size needs, for parallel builds."""
     jobs = [("attention_simple", {"PBE_HEAD_DIM": int(head_dim)})]
+    if dtype == torch.float32 and head_dim in (64, 128):
+        jobs.append(("attention_f32_tc5", {"PBE_HEAD_DIM": int(head_dim)}))
     if dtype == torch.bfloat16 and _mma_available():
         jobs.append(("attention_mma", {"PBE_HEAD_DIM": int(head_dim)}))
         if head_dim in (64, 128) and _attention_choice() != "mma" and _tc5_available():

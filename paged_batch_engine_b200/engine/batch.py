@@ -86,6 +86,8 @@ class AttentionWork:
     small_items: int = 0            # live work items with at most 16 packed rows
     decode_rows: int = 0            # rows of a step of decoded tokens only (0: the step has prompt portions)
     longest_keys: int = 0           # the longest context of the step (a captured step: of its capacity)
+    wide_tiles: int = 0             # blocks of the float32 tensor-core kernel (``ops.attention_f32_tiles``)
+    handed_back: Optional[torch.Tensor] = None      # and what it leaves to the multiply-adds: a flag a block
 
 
 def attention_work_arrays(q_len: np.ndarray, seq_len: np.ndarray, q_start: np.ndarray,
@@ -363,7 +365,9 @@ class StepContext:
                 split_counts=pk.view(isc) if ns else None, num_split_rows=ns, max_splits=max_splits,
                 split_keys=self.split_keys, tile_rows=key[2], kinds=kinds, small_items=small_items,
                 decode_rows=R if int(q_len.max(initial=0)) == 1 and int(q_len.min(initial=1)) == 1 else 0,
-                longest_keys=int(seq_len.max(initial=0)))
+                longest_keys=int(seq_len.max(initial=0)),
+                wide_tiles=ops.attention_f32_tiles(q_len, seq_len, key[1], key[3], self.split_keys)
+                if key[2] == ops.SIMPLE_TILE_ROWS else 0)
 
     def group(self, g: int) -> GroupArrays:
         return self._groups[g]
