@@ -46,7 +46,7 @@ __device__ __forceinline__ float key_value(uint32_t k) {
 // block waiting for the L2's latency 150 times over a vocabulary of 150,000.
 constexpr int LOADS_AHEAD = 8;
 template <typename F>
-__device__ __forceinline__ void for_each_logit(const float* __restrict__ row, int V, F&& f) {
+__device__ __forceinline__ void for_each_logit(const float* row, int V, F&& f) {
   for (int i0 = threadIdx.x; i0 < V; i0 += THREADS * LOADS_AHEAD) {
     float xs[LOADS_AHEAD];
 #pragma unroll
@@ -58,6 +58,47 @@ __device__ __forceinline__ void for_each_logit(const float* __restrict__ row, in
     for (int u = 0; u < LOADS_AHEAD; ++u) {
       const int i = i0 + u * THREADS;
       if (i < V) f(clean(xs[u]), i);
+    }
+  }
+}
+// The same for f with little to do (the row's maximum: bound by memory), as it lies: where the row starts on a 16-byte boundary f gets
+// groups of four neighbours (the last one to three elements one by one), else single elements, filled up with -inf.  The groups of
+// thread t are t, t + THREADS, ...
+constexpr int GROUPS_AHEAD = 4;
+__device__ __forceinline__ bool in_groups(const float* row) { return ((uintptr_t)row & 15) == 0; }
+__device__ __forceinline__ float4 single(float x) { return make_float4(x, -INFINITY, -INFINITY, -INFINITY); }
+template <typename F>
+__device__ __forceinline__ void for_each_group(const float* row, int V, F&& f) {
+  if (in_groups(row)) {
+    const int groups = V / 4;
+    for (int j0 = threadIdx.x; j0 < groups; j0 += THREADS * GROUPS_AHEAD) {
+      float4 xs[GROUPS_AHEAD];
+#pragma unroll
+      for (int u = 0; u < GROUPS_AHEAD; ++u) {
+        const int j = j0 + u * THREADS;
+        xs[u] = j < groups ? *reinterpret_cast<const float4*>(row + 4 * (size_t)j) : single(0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < GROUPS_AHEAD; ++u) {
+        const int j = j0 + u * THREADS;
+        if (j < groups) f(xs[u], 4 * j);
+      }
+    }
+    const int last = 4 * groups + threadIdx.x;
+    if (last < V) f(single(row[last]), last);
+  } else {
+    for (int i0 = threadIdx.x; i0 < V; i0 += THREADS * LOADS_AHEAD) {
+      float xs[LOADS_AHEAD];
+#pragma unroll
+      for (int u = 0; u < LOADS_AHEAD; ++u) {
+        const int i = i0 + u * THREADS;
+        xs[u] = i < V ? row[i] : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < LOADS_AHEAD; ++u) {
+        const int i = i0 + u * THREADS;
+        if (i < V) f(single(xs[u]), i);
+      }
     }
   }
 }
@@ -203,15 +244,26 @@ __device__ Cut select_by_weight(const float* row, int V, float mx, float temp, b
 }
 
 // out_min (optional): the smallest logit above -inf (+inf when there is none)
+// own (optional): the thread's own maximum
 __device__ void block_argmax(const float* row, int V, Shared& sh, float* out_max, int* out_idx,
-                             float* out_min = nullptr) {
+                             float* out_min = nullptr, float* own = nullptr) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   float best = -INFINITY, low = INFINITY;
   int idx = 0x7fffffff;
-  for_each_logit(row, V, [&](float x, int i) {
-    if (x > best || (x == best && i < idx)) { best = x; idx = i; }
-    if (x > -INFINITY) low = fminf(low, x);
+  // a thread meets its elements in rising order, so the first of equal ones stays; fmaxf and fminf pass over what is no number
+  for_each_group(row, V, [&](const float4& x, int i) {
+    const float top = fmaxf(fmaxf(x.x, x.y), fmaxf(x.z, x.w));
+    if (top > best) {
+      best = top;
+      idx = i + (x.x == top ? 0 : x.y == top ? 1 : x.z == top ? 2 : 3);
+    }
+    if (out_min) {
+      low = fminf(fminf(low, x.x > -INFINITY ? x.x : INFINITY), x.y > -INFINITY ? x.y : INFINITY);
+      low = fminf(fminf(low, x.z > -INFINITY ? x.z : INFINITY), x.w > -INFINITY ? x.w : INFINITY);
+    }
   });
+  best += 0.0f;
+  if (own) *own = best;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ob = __shfl_xor_sync(0xffffffffu, best, o);
@@ -321,6 +373,9 @@ struct Quick {
   u64 warp_tot[NWARPS];
   u64 pick_cum;
   int n_list, chosen, first_idx, last_bin;
+  int overflow;                    // the list of the row's block 0 did not hold what the blocks found
+  int n_found;                     // threads of this block whose elements are looked through, in `found`
+  int found[THREADS];
   float part_max[SAMPLE_CLUSTER], part_min[SAMPLE_CLUSTER];
   int part_idx[SAMPLE_CLUSTER];
   Picked picked;
@@ -375,21 +430,22 @@ __device__ u64 block_exclusive_scan(u64 v, Quick& q, u64* total) {
   return before + inc - v;
 }
 
-// The bins of a row: counts, weights and their prefix sums, in every block of the cluster.
+// The bins of a row: weights, where they are asked for counts, and their prefix sums, in every block of the cluster.
 // slice: this block's part of the row (first token `lo`, `n` tokens).
 template <int CL>
-__device__ void fill_bins(const float* slice, int n, float mx, float temp, float scale, Quick& q) {
+__device__ void fill_bins(const float* slice, int n, float mx, float temp, float scale, bool counts, Quick& q) {
   const int tid = threadIdx.x;
   q.cnt_part[tid] = 0;
   q.limb[0][tid] = q.limb[1][tid] = q.limb[2][tid] = 0;
   if (tid == 0) {
-    q.last_bin = 0;
+    q.last_bin = counts ? 0 : NB - 1;
     q.n_list = 0;
+    q.overflow = 0;
   }
   __syncthreads();
   for_each_logit(slice, n, [&](float x, int) {
     const int b = value_bin(x, mx, scale);
-    atomicAdd(&q.cnt_part[b], 1u);
+    if (counts) atomicAdd(&q.cnt_part[b], 1u);
     const u64 w = weight_of(x, mx, temp, false);      // at most 2^40
     const unsigned l0 = (unsigned)w & 0x3fffu, l1 = (unsigned)(w >> 14) & 0x3fffu, l2 = (unsigned)(w >> 28);
     if (l0) atomicAdd(&q.limb[0][b], l0);
@@ -421,6 +477,132 @@ __device__ void fill_bins(const float* slice, int n, float mx, float temp, float
   sync_row<CL>();
 }
 
+// An element into the list of the row's block 0; every block learns if that is full.
+template <int CL>
+__device__ __forceinline__ void push(Quick& q, uint32_t key, int token) {
+  Quick* q0 = of_block<CL>(&q, 0);
+  const int pos = atomicAdd(&q0->n_list, 1);
+  if (pos < LIST_CAP) {
+    q0->list[pos] = ((u64)key << 32) | (u64)(0xffffffffu - (uint32_t)token);
+  } else {
+#pragma unroll
+    for (int r = 0; r < CL; ++r) of_block<CL>(&q, r)->overflow = 1;
+  }
+}
+
+// the list's n elements in descending order; n2: a power of two, 32 or more, from n on, zeros behind the elements
+__device__ void sort_list(Quick& q, int n, int n2) {
+  const int tid = threadIdx.x;
+  if (n2 <= THREADS) {
+    // few elements: every element counts the larger ones (all are different: the token is part
+    // of them) and moves to that place
+    const u64 mine = tid < n2 ? q.list[tid] : 0;
+    int place = 0;
+    if (tid < n) {
+      for (int j = 0; j < n; ++j) place += q.list[j] > mine ? 1 : 0;
+    }
+    __syncthreads();
+    if (tid < n) q.list[place] = mine;
+    __syncthreads();
+  } else {
+    // bitonic sort, descending
+    for (int k = 2; k <= n2; k <<= 1) {
+      for (int j = k >> 1; j > 0; j >>= 1) {
+        for (int i = tid; i < n2; i += THREADS) {
+          const int partner = i ^ j;
+          if (partner > i) {
+            const u64 a = q.list[i], b = q.list[partner];
+            const bool down = (i & k) == 0;
+            if (down ? a < b : a > b) {
+              q.list[i] = b;
+              q.list[partner] = a;
+            }
+          }
+        }
+        __syncthreads();
+      }
+    }
+  }
+}
+
+// The row's first k elements without bins (k up to TOP_MAX): the k largest of a block's threads' own maxima are k elements, so no
+// element below the smallest of these is among the first k, and only the threads whose maximum is not below it have to be looked
+// through again.  The bound is found to TOP_BITS of the key, by halving, and what is not below it goes to block 0's list.
+// What is left is one pass over the row, which memory bounds; bins take four shared-memory atomics a logit, and their elements a pass
+// for each of the three choices.  k = 50, top_p 0.9, launch and all: 64 rows of 152,064 90 -> 27 us, of 32,000 43 -> 19; one row
+// of 152,064 52 -> 25.  The line: with k = 128 86 -> 31 and 43 -> 41 us (64 rows of 152,064, one of 32,000), with 512 one row of 32,000
+// was slower, 35 -> 49 (top_p 1).
+constexpr int TOP_MAX = 128, TOP_BITS = 20;
+template <int CL>
+__device__ void list_top(const float* slice, int lo, int n_slice, int k, float own, Quick& q) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t key = order_key(own);
+  uint32_t bound = 0;
+#pragma unroll 1
+  for (int bit = 31; bit > 31 - TOP_BITS; --bit) {
+    const uint32_t higher = bound | (1u << bit);
+    if (__syncthreads_count(key >= higher) >= k) bound = higher;
+  }
+  if (key >= bound) q.found[atomicAdd(&q.n_found, 1)] = tid;
+  __syncthreads();
+  const int n = q.n_found;
+  auto look = [&](float x, int i) {
+    const uint32_t kx = order_key(clean(x));
+    if (kx >= bound) push<CL>(q, kx, lo + i);
+  };
+  if (in_groups(slice)) {
+    const int groups = n_slice / 4;
+    for (int f = warp; f < n; f += NWARPS) {
+      const int t = q.found[f];
+      for (int j = t + lane * THREADS; j < groups; j += 32 * THREADS) {
+        const float4 x = *reinterpret_cast<const float4*>(slice + 4 * (size_t)j);
+        look(x.x, 4 * j);
+        look(x.y, 4 * j + 1);
+        look(x.z, 4 * j + 2);
+        look(x.w, 4 * j + 3);
+      }
+      if (lane == 0 && 4 * groups + t < n_slice) look(slice[4 * groups + t], 4 * groups + t);
+    }
+  } else {
+    for (int f = warp; f < n; f += NWARPS)
+      for (int i = q.found[f] + lane * THREADS; i < n_slice; i += 32 * THREADS) look(slice[i], i);
+  }
+}
+
+// The token from the row's first k elements (block 0, the list complete): the same sums, targets and choices as by select_quick.
+__device__ int sample_top(int k, int amax, float mx, float temp, float p_in, float u, Quick& q) {
+  const int tid = threadIdx.x, n = q.n_list;
+  int n2 = 32;
+  while (n2 < n) n2 <<= 1;
+  for (int i = n + tid; i < n2; i += THREADS) q.list[i] = 0;     // below every real key
+  __syncthreads();
+  sort_list(q, n, n2);
+  const u64 w = tid < k ? weight_of(key_value((uint32_t)(q.list[tid] >> 32)), mx, temp, false) : 0;
+  u64 kept;
+  const u64 upto = block_exclusive_scan(w, q, &kept) + w;
+  if (kept == 0) return amax;
+  // the first element of positive weight whose running sum reaches `target`: there is one, the target is `kept` at most
+  auto first = [&](u64 target) {
+    __syncthreads();
+    if (tid == 0) q.first_idx = 0x7fffffff;
+    __syncthreads();
+    if (w > 0 && upto >= target) atomicMin(&q.first_idx, tid);
+    __syncthreads();
+    return q.first_idx;
+  };
+  auto share = [](float of_one, u64 all) {                       // ceil: cumulative >= share * total
+    u64 t = (u64)((double)of_one * (double)all);
+    return (double)t < (double)of_one * (double)all ? t + 1 : t;
+  };
+  if (p_in < 1.f) {
+    const int last = first(share(p_in, kept));
+    if (tid == last) q.pick_cum = upto;
+    __syncthreads();
+    kept = q.pick_cum;
+  }
+  return (int)(0xffffffffu - (uint32_t)q.list[first(share(u, kept))]);
+}
+
 // First element of the ordered list, inside the domain, whose weight is positive and whose
 // inclusive cumulative weight (count in count mode) reaches `target`; the domain's last element
 // if there is none: what select_by_weight returns.  In count mode *weight_cum gets the cumulative
@@ -433,7 +615,6 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
                              u64* weight_cum) {
   const int tid = threadIdx.x;
   const int rank = block_rank<CL>();
-  Quick* q0 = of_block<CL>(&q, 0);
   const int last_bin = lim.on ? lim.bin : q.last_bin;
   __syncthreads();
   if (tid == 0) {
@@ -448,7 +629,6 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
   }
   __syncthreads();
   const int bin = q.chosen;
-  if (q.cnt[bin] > (unsigned)LIST_CAP) return false;
   // the bin's elements inside the domain (block 0's counter is zero: it is reset after every use,
   // a row barrier before the next)
   for_each_logit(slice, n_slice, [&](float x, int i) {
@@ -456,10 +636,10 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
     const uint32_t key = order_key(x);
     const int token = lo + i;
     if (lim.on && !(key > lim.key || (key == lim.key && token <= lim.token))) return;
-    const int pos = atomicAdd(&q0->n_list, 1);
-    q0->list[pos] = ((u64)key << 32) | (u64)(0xffffffffu - (uint32_t)token);
+    push<CL>(q, key, token);
   });
   sync_row<CL>();
+  if (q.overflow) return false;
   if (rank == 0) {
     const int n = q.n_list;
     Picked res;
@@ -470,36 +650,7 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
       while (n2 < n) n2 <<= 1;
       for (int i = n + tid; i < n2; i += THREADS) q.list[i] = 0;     // below every real key
       __syncthreads();
-      if (n2 <= THREADS) {
-        // few elements: every element counts the larger ones (all are different: the token is part
-        // of them) and moves to that place
-        const u64 mine = tid < n2 ? q.list[tid] : 0;
-        int place = 0;
-        if (tid < n) {
-          for (int j = 0; j < n; ++j) place += q.list[j] > mine ? 1 : 0;
-        }
-        __syncthreads();
-        if (tid < n) q.list[place] = mine;
-        __syncthreads();
-      } else {
-        // bitonic sort, descending
-        for (int k = 2; k <= n2; k <<= 1) {
-          for (int j = k >> 1; j > 0; j >>= 1) {
-            for (int i = tid; i < n2; i += THREADS) {
-              const int partner = i ^ j;
-              if (partner > i) {
-                const u64 a = q.list[i], b = q.list[partner];
-                const bool down = (i & k) == 0;
-                if (down ? a < b : a > b) {
-                  q.list[i] = b;
-                  q.list[partner] = a;
-                }
-              }
-            }
-            __syncthreads();
-          }
-        }
-      }
+      sort_list(q, n, n2);
       // running sum along the sorted list, a few consecutive elements a thread
       const int ipt = (n2 + THREADS - 1) / THREADS;       // 1 .. LIST_CAP / THREADS
       constexpr int MAX_IPT = LIST_CAP / THREADS;
@@ -571,7 +722,7 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
 
 // One block a row, or a cluster of CL blocks a row (large vocabularies: each block takes a slice
 // of the row for every pass; block 0 sorts the gathered bin and writes the token).
-// mode 1: the radix descent only (for tests that compare the two ways).
+// mode 1: the radix descent only, 2: not by the threads' maxima (for tests that compare the ways).
 template <int CL>
 __global__ void __launch_bounds__(THREADS)
 sample_kernel(const float* logits, size_t ld, int V,
@@ -589,10 +740,15 @@ sample_kernel(const float* logits, size_t ld, int V,
   const int chunk = CL > 1 ? (((V + CL - 1) / CL + 3) & ~3) : V;
   const int lo = min(V, rank * chunk), n_slice = min(V, lo + chunk) - lo;
   const float* slice = row + lo;
-  float mx = -INFINITY, mn = INFINITY;
+  const float t_in = temperature[r];
+  const int k_in = top_k[r];
+  const float p_in = fminf(fmaxf(top_p[r], 0.f), 1.f);
+  const bool top = mode == 0 && k_in > 0 && k_in < V && k_in <= TOP_MAX;
+  if (threadIdx.x == 0) q.n_list = q.n_found = q.overflow = 0;
+  float mx = -INFINITY, mn = INFINITY, own = -INFINITY;
   int amax = 0x7fffffff;
   if (n_slice > 0) {
-    block_argmax(slice, n_slice, sh, &mx, &amax, &mn);
+    block_argmax(slice, n_slice, sh, &mx, &amax, &mn, &own);
     amax += lo;
   }
   if constexpr (CL > 1) {
@@ -614,29 +770,38 @@ sample_kernel(const float* logits, size_t ld, int V,
   }
   if (amax == 0x7fffffff) amax = 0;
   const bool writer = rank == 0 && threadIdx.x == 0;
-  const float t_in = temperature[r];
-  const int k_in = top_k[r];
-  const float p_in = fminf(fmaxf(top_p[r], 0.f), 1.f);
   if ((t_in <= 0.f && k_in <= 0 && p_in >= 1.f) || !(mx > -INFINITY)) {
     if (writer) out[r] = amax;
     return;
   }
   const float temp = fmaxf(t_in, 1e-6f);
   const float u = fminf(fmaxf(uniform[r], 0.f), 0.99999994f);
+  if (top) {
+    list_top<CL>(slice, lo, n_slice, k_in, own, q);
+    sync_row<CL>();
+    if (!q.overflow) {             // else thousands of equal logits
+      if (rank != 0) return;
+      const int token = sample_top(k_in, amax, mx, temp, p_in, u, q);
+      if (writer) out[r] = token;
+      return;
+    }
+    __syncthreads();
+  }
   if (mode != 1 && chunk < (1 << 18)) {      // (the limbs of a bin's weight sum hold 2^18 elements)
     // bins over the logits from the maximum down to the smallest one, but no further than where
     // weights have long vanished (masks of -1e9 would otherwise stretch the bins): what lies
     // below shares the last bin
     const float reach = fminf(mx - mn, fmaxf(64.f * temp, 32.f));
     const float scale = reach > 0.f ? (float)(NB - 1) / reach : 0.f;
-    fill_bins<CL>(slice, n_slice, mx, temp, scale, q);
+    const bool counts = k_in > 0 && k_in < V;
+    fill_bins<CL>(slice, n_slice, mx, temp, scale, counts, q);
     Limit lim;
     lim.on = false; lim.key = 0; lim.token = 0; lim.bin = 0;
     u64 kept = q.cumw[NB];
     bool ok = true;
     Cut c;
     int bin = 0;
-    if (k_in > 0 && k_in < V) {
+    if (counts) {
       u64 wc = 0;
       ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, true, (u64)k_in, lim, q, &c, &bin, &wc);
       if (ok) {
@@ -817,7 +982,7 @@ PBE_EXPORT int pbe_sample(const float* logits, long long ld, int num_rows, int v
   return launch_status();
 }
 
-// 0: the quick way with the radix descent behind it; 1: the radix descent only
+// 0: the quick ways with the radix descent behind them; 1: the radix descent only; 2: bins, with the radix descent behind them
 PBE_EXPORT int pbe_sample_set_mode(int mode) {
   g_sample_mode = mode;
   return 0;

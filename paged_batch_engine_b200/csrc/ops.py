@@ -1383,8 +1383,8 @@ def penalty_seen(logits: torch.Tensor, seen: torch.Tensor, slots: torch.Tensor, 
 
 
 def sample_set_mode(mode: int) -> None:
-    """0 (default): the sampling kernel's binned selection with the radix descent behind it; 1: the
-    radix descent only.  Both give the same token; the switch is for tests that compare them."""
+    """0 (default): the sampling kernel's quick ways with the radix descent behind them; 1: the radix descent only; 2: bins
+    with the radix descent behind them.  All give the same token; the switch is for tests that compare them."""
     _fn("sampling", "pbe_sample_set_mode", [c_int])(int(mode))
 
 

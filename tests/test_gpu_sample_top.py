@@ -1,0 +1,44 @@
+"""The sampling kernel's three ways to a token (the threads' maxima for the first k, bins, radix descent) give the same one, over row
+lengths around the loads' groups and the clusters' slices, equal logits, masks and what is no number."""
+import pytest
+import torch
+
+DEV = "cuda:0"
+
+
+def _tokens(logits, k, p, t, u):
+    from paged_batch_engine_b200.csrc import ops
+    n = logits.shape[0]
+    full = lambda x, dt: torch.full((n,), x, dtype=dt, device=DEV)
+    out = []
+    for mode in (0, 2, 1):
+        ops.sample_set_mode(mode)
+        try:
+            out.append(ops.sample(logits, full(t, torch.float32), full(k, torch.int32), full(p, torch.float32), u).tolist())
+        finally:
+            ops.sample_set_mode(0)
+    return out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,rows,stride", [(5, 3, 5), (1000, 4, 1000), (1027, 3, 1028), (8191, 5, 8191), (8192, 20, 8192), (9001, 40, 9003),
+                                           (32000, 64, 32000), (40001, 100, 40001), (152064, 64, 152064), (151936, 150, 151936)])
+@pytest.mark.parametrize("kind", ["normal", "coarse", "equal", "masked"])
+def test_three_ways(V, rows, stride, kind):
+    g = torch.Generator(device=DEV).manual_seed(V + rows)
+    x = torch.empty(rows, stride, device=DEV).normal_(0, 2.5, generator=g)
+    if kind == "coarse":
+        x = (x * 2).round() / 2
+    elif kind == "equal":
+        x = x.sign()
+    elif kind == "masked":
+        x[:, ::3] = float("-inf")
+        x[:, 1::7] = float("nan")
+        x[0] = float("-inf")
+        x[-1, V // 2] = 1e9
+    x = x[:, :V]
+    u = torch.rand(rows, device=DEV, generator=g)
+    for k in {1, 2, 50, 511, 512, 513, V - 1, 0} - ({0} if V > 100000 and kind == "equal" else set()):
+        for p, t in ((1.0, 0.8), (0.9, 0.8), (0.0, 1.5), (0.5, 1e-7)):
+            top, bins, radix = _tokens(x, k, p, t, u)
+            assert top == bins == radix, (k, p, t)
