@@ -5,6 +5,7 @@
 // swiglu_kernel.cu:6-25.  The residual stream is float32 in every run mode; statistics,
 // the sum and the products are float32 and each result is rounded once on store.
 #include "common.cuh"
+#include "status.cuh"
 #include "pdl.cuh"
 
 using namespace pbe;
@@ -620,23 +621,8 @@ PBE_EXPORT int pbe_glu_act(const void* in, const float* bias, void* out, int dty
   return launch_status();
 }
 
-// ------------------------------------------------------------------ kernel status word
-// Kernels with bounded waits (tcgen05 attention and GEMM, the mbarrier tile rings of the
-// mma.sync attention) record a wait that ran out in a flag of their own.  This kernel folds up
-// to 32 such flags into one word (bit i: flag i was set) and clears the flags it found set, so
-// the host learns of an invalid launch with the same copy that brings the sampled ids back.
-__global__ void collect_status_kernel(const unsigned long long* __restrict__ flag_addresses, int n,
-                                      int* __restrict__ out) {
-  unsigned word = 0;
-  for (int i = 0; i < n && i < 32; ++i) {
-    int* flag = reinterpret_cast<int*>(flag_addresses[i]);
-    if (flag != nullptr && atomicExch(flag, 0) != 0) word |= 1u << i;
-  }
-  *out = (int)word;
-}
-
 PBE_EXPORT int pbe_collect_status(const unsigned long long* flag_addresses, int n, int* out,
                                   cudaStream_t stream) {
-  collect_status_kernel<<<1, 1, 0, stream>>>(flag_addresses, n, out);
+  pbe::collect_status_kernel<<<1, 1, 0, stream>>>(flag_addresses, n, out);
   return pbe::launch_status();
 }

@@ -21,6 +21,7 @@
 
 #include "common.cuh"
 #include "pdl.cuh"
+#include "status.cuh"
 
 using namespace pbe;
 
@@ -980,6 +981,24 @@ PBE_EXPORT int pbe_sample(const float* logits, long long ld, int num_rows, int v
   else PBE_SAMPLE_LAUNCH(1);
 #undef PBE_SAMPLE_LAUNCH
   return launch_status();
+}
+
+// A whole step of sampling in one call: the rows' parameters from pinned memory ([6, num_rows]: temperature, top_p, uniform, top_k, and two
+// rows that are not read here), the tokens, the kernels' status word behind them, and both to pinned memory.  out, out_host: num_rows + 1.
+PBE_EXPORT int pbe_sample_step(const float* logits, long long ld, int num_rows, int vocab, const int32_t* params_host, int32_t* params,
+                               int32_t* out, int32_t* out_host, const unsigned long long* flag_addresses, int num_flags,
+                               cudaStream_t stream) {
+  if (num_rows <= 0) return (int)cudaErrorInvalidValue;
+  const size_t n = (size_t)num_rows;
+  cudaError_t e = cudaMemcpyAsync(params, params_host, 6 * n * sizeof(int32_t), cudaMemcpyHostToDevice, stream);
+  if (e != cudaSuccess) return (int)e;
+  const float* f = reinterpret_cast<const float*>(params);
+  const int rc = pbe_sample(logits, ld, num_rows, vocab, f, params + 3 * n, f + n, f + 2 * n, out, stream);
+  if (rc != 0) return rc;
+  collect_status_kernel<<<1, 1, 0, stream>>>(flag_addresses, num_flags, out + n);
+  if (const int status = launch_status()) return status;
+  e = cudaMemcpyAsync(out_host, out, (n + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, stream);
+  return (int)e;
 }
 
 // 0: the quick ways with the radix descent behind them; 1: the radix descent only; 2: bins, with the radix descent behind them

@@ -1282,8 +1282,14 @@ def collect_status(out: torch.Tensor) -> torch.Tensor:
     A flag is set by a kernel whose bounded wait ran out: the results of that launch are not
     valid.  Costs one launch of one thread; nothing waits."""
     _need_cuda(out)
-    device = out.device
-    # the flags' addresses are looked up again only when a new flag has come into being
+    flags, n = _status_flags(out.device)
+    fn = _fn("elementwise", "pbe_collect_status", [c_void_p, c_int, c_void_p, c_void_p])
+    _check(fn(flags, n, _ptr(out), _stream()), "collect_status")
+    return out
+
+
+def _status_flags(device):
+    """(address on the device of the flags' addresses, how many): looked up again only when a new flag has come into being."""
     key = (device in _tc5_attn_err, device in _tc5_err, len(_mma_flag_heads))
     st = _status_state.get(device)
     if st is None or st[2] != key:
@@ -1292,9 +1298,7 @@ def collect_status(out: torch.Tensor) -> torch.Tensor:
         addrs = torch.from_numpy(np.array([a for _, a in src] + [0], dtype=np.uint64).view(np.int64)).to(device)
         st = _status_state[device] = (addrs, len(src), key)
         _STATUS_NAMES[device] = [n for n, _ in src]
-    fn = _fn("elementwise", "pbe_collect_status", [c_void_p, c_int, c_void_p, c_void_p])
-    _check(fn(_ptr(st[0]), st[1], _ptr(out), _stream()), "collect_status")
-    return out
+    return st[0].data_ptr(), st[1]
 
 
 def status_message(device, word: int) -> str:
@@ -1355,6 +1359,23 @@ def sample(logits, temperature, top_k, top_p, uniform, out=None) -> torch.Tensor
     _check(fn(_ptr(logits), logits.stride(0), n, V, _ptr(temperature), _ptr(top_k), _ptr(top_p),
               _ptr(uniform), _ptr(out), _stream()), "sample")
     return out
+
+
+def sample_step(logits: torch.Tensor, params_host: torch.Tensor, params: torch.Tensor, out: torch.Tensor, out_host: torch.Tensor) -> None:
+    """``sample`` and ``collect_status`` between the copies of a step, in one call: the rows' parameters go up from pinned
+    memory (int32 [6 * rows] and more: temperature, top_p, uniform as float32 bits, top_k, two rows that are not read), the tokens and the status word
+    behind them come down to ``out_host`` (int32, rows + 1 and more, pinned; ``out`` the same on the device)."""
+    _need_cuda(logits, params, out)
+    if logits.dtype != torch.float32 or logits.stride(1) != 1:
+        raise KernelError("sample takes float32 logits with unit column stride")
+    n, V = logits.shape
+    if min(params_host.numel(), params.numel()) < 6 * n or min(out.numel(), out_host.numel()) < n + 1:
+        raise KernelError("sample_step: a buffer is too small")
+    flags, num_flags = _status_flags(logits.device)
+    fn = _fn("sampling", "pbe_sample_step", [c_void_p, c_ll, c_int, c_int] + [c_void_p] * 5 + [c_int, c_void_p])
+    _check(fn(_ptr(logits), logits.stride(0), n, V, params_host.data_ptr(), _ptr(params), _ptr(out), out_host.data_ptr(), flags, num_flags,
+              _stream()), "sample_step")
+    count_launches(1)
 
 
 def seen_mark(seen: torch.Tensor, tokens: torch.Tensor, slots: Optional[torch.Tensor] = None, slot: int = -1) -> None:

@@ -5,6 +5,8 @@ from __future__ import annotations
 from dataclasses import dataclass, field
 from typing import List
 
+import numpy as np
+
 _MASK64 = (1 << 64) - 1
 
 
@@ -18,6 +20,16 @@ def request_sample_uniform(seed: int, counter: int) -> float:
     z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & _MASK64
     z ^= z >> 31
     return float(z >> 40) * (1.0 / 16777216.0)
+
+
+def request_sample_uniforms(seeds, counters) -> np.ndarray:
+    """``request_sample_uniform`` of many (seed, counter) pairs: the same draws, as float64."""
+    z = np.array([s & _MASK64 for s in seeds], dtype=np.uint64)
+    z += np.array([(c + 1) & _MASK64 for c in counters], dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15)
+    z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
+    z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
+    z ^= z >> np.uint64(31)
+    return (z >> np.uint64(40)).astype(np.float64) * (1.0 / 16777216.0)
 
 
 @dataclass

@@ -1,13 +1,16 @@
 """Turns the step's logits into one token per sampled row, on the device."""
 from __future__ import annotations
 
+from operator import attrgetter
 from typing import List, Sequence
 
 import numpy as np
 import torch
 
 from ..csrc import ops
-from .params import SamplingParams, request_sample_uniform
+from .params import SamplingParams, request_sample_uniform, request_sample_uniforms
+
+_FIELDS = attrgetter("temperature", "top_p", "top_k", "seed", "repetition_penalty")
 
 
 class Sampler:
@@ -83,8 +86,10 @@ class Sampler:
         rows' parameters go up from pinned memory (a copy from pageable memory would first wait
         for the stream, i.e. for the step that is still running).  Buffers rotate over four steps."""
         n = logits.shape[0]
-        if any(p.repetition_penalty != 1.0 and (keys is None or not self.tracked(k))
-               for p, k in zip(params, keys if keys is not None else [None] * n)):
+        temperature, top_p, top_k, seeds, penalties = zip(*map(_FIELDS, params)) if len(params) else ((),) * 5
+        some = penalties.count(1.0) != len(penalties)
+        if some and any(x != 1.0 and (keys is None or not self.tracked(k))
+                        for x, k in zip(penalties, keys if keys is not None else [None] * n)):
             raise ValueError("sample_async: a row with a repetition penalty needs a tracked request")
         slot = self._async_slots[self._async_next % len(self._async_slots)] if self._async_slots else None
         if slot is None or slot[0].numel() < n + 1:
@@ -92,8 +97,8 @@ class Sampler:
             self._async_slots = [(torch.empty(cap, dtype=torch.int32, device=self.device),
                                   torch.empty(cap, dtype=torch.int32, pin_memory=True),
                                   torch.cuda.Event(),
-                                  torch.empty((6, cap), dtype=torch.int32, device=self.device),
-                                  torch.empty((6, cap), dtype=torch.int32, pin_memory=True)) for _ in range(4)]
+                                  torch.empty(6 * cap, dtype=torch.int32, device=self.device),
+                                  torch.empty(6 * cap, dtype=torch.int32, pin_memory=True)) for _ in range(4)]
             slot = self._async_slots[0]
             self._async_next = 0
         self._async_next += 1
@@ -102,26 +107,33 @@ class Sampler:
             ops.argmax(logits, dev[:n])
         else:
             # rows of the parameter block: temperature, top_p, uniform (float32 bits), top_k, the
-            # penalty's slot of seen tokens (-1: none), the penalty (float32 bits)
+            # penalty's slot of seen tokens (-1: none), the penalty (float32 bits); the block's n columns lie
+            # together, so that one copy takes them up
             event.synchronize()              # the copy that last read this pinned block is over (four steps ago)
-            block = phost.numpy()
+            block = phost.numpy()[:6 * n].reshape(6, n)
             fl = block.view(np.float32)
-            fl[0, :n] = [p.temperature for p in params]
-            fl[1, :n] = [p.top_p for p in params]
-            fl[2, :n] = [request_sample_uniform(p.seed, c) for p, c in zip(params, counters)]
-            block[3, :n] = [p.top_k for p in params]
-            slots = [self._slot_of.get(k, -1) if p.repetition_penalty != 1.0 else -1
-                     for p, k in zip(params, keys if keys is not None else [None] * n)]
-            block[4, :n] = slots
-            fl[5, :n] = [p.repetition_penalty for p in params]
-            pdev[:, :n].copy_(phost[:, :n], non_blocking=True)
+            fl[0] = temperature
+            fl[1] = top_p
+            fl[2] = request_sample_uniforms(seeds, counters)
+            block[3] = top_k
+            if not some:
+                ops.sample_step(logits, phost, pdev, dev, host)
+                event.record()
+                return dev[:n], host[:n + 1], event
+            slots = [self._slot_of.get(k, -1) if x != 1.0 else -1
+                     for x, k in zip(penalties, keys if keys is not None else [None] * n)]
+            block[4] = slots
+            fl[5] = penalties
+            pdev = pdev[:6 * n]
+            pdev.copy_(phost[:6 * n], non_blocking=True)
+            pdev = pdev.view(6, n)
             fdev = pdev.view(torch.float32)
             penalised = any(sl >= 0 for sl in slots)
             if penalised:
-                ops.penalty_seen(logits, self._seen, pdev[4, :n], fdev[5, :n])
-            ops.sample(logits, fdev[0, :n], pdev[3, :n], fdev[1, :n], fdev[2, :n], out=dev[:n])
+                ops.penalty_seen(logits, self._seen, pdev[4], fdev[5])
+            ops.sample(logits, fdev[0], pdev[3], fdev[1], fdev[2], out=dev[:n])
             if penalised:
-                ops.seen_mark(self._seen, dev[:n], pdev[4, :n])
+                ops.seen_mark(self._seen, dev[:n], pdev[4])
         ops.collect_status(dev[n:n + 1])
         host[:n + 1].copy_(dev[:n + 1], non_blocking=True)
         event.record()

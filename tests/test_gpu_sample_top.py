@@ -1,7 +1,10 @@
 """The sampling kernel's three ways to a token (the threads' maxima for the first k, bins, radix descent) give the same one, over row
-lengths around the loads' groups and the clusters' slices, equal logits, masks and what is no number."""
+lengths around the loads' groups and the clusters' slices, equal logits, masks and what is no number; and the draws of many rows
+made at once are those made one by one."""
 import pytest
 import torch
+
+from paged_batch_engine_b200.sampling.params import request_sample_uniform, request_sample_uniforms
 
 DEV = "cuda:0"
 
@@ -42,3 +45,9 @@ def test_three_ways(V, rows, stride, kind):
         for p, t in ((1.0, 0.8), (0.9, 0.8), (0.0, 1.5), (0.5, 1e-7)):
             top, bins, radix = _tokens(x, k, p, t, u)
             assert top == bins == radix, (k, p, t)
+
+
+def test_draws_of_many_rows():
+    seeds = [0, 1, 0xC0FFEE, 2 ** 63 + 5, 2 ** 64 - 1, 2 ** 64 + 7, -3]
+    counters = [0, 5, 2 ** 20, 1, 3, 2, 7]
+    assert request_sample_uniforms(seeds, counters).tolist() == [request_sample_uniform(s, c) for s, c in zip(seeds, counters)]
