@@ -50,6 +50,9 @@ struct PmParams {
   int bt_tok_stride, bt_pool_stride;
   int H, G, page_tokens, window, pool;
   float scale_log2;         // scale * log2(e): scores in units of the exponential's base
+  // when not null: tiles are of 128 rows, another kernel's but for those with a flag set ([n, flags_a_tile])
+  const int32_t* flags = nullptr;
+  int flags_a_tile = 0;
 };
 
 // The probabilities' buffer: [head][row][key], rows and heads padded so that eight rows of a head and eight heads of
@@ -82,8 +85,13 @@ __global__ void __launch_bounds__(32 * HEADS, 1) pooled_attention_mma_kernel(PmP
   const int krow = (lane & 7) + (lane >> 4) * 8, kcol = ((lane >> 3) & 1) * 8;     // B operands as they lie
   pdl_launch_dependents();
   pdl_wait();
-  const int32_t* tile = p.tiles + (size_t)blockIdx.x * 3;
-  const int r = tile[0], row0 = tile[1], rows = tile[2];
+  const int32_t* tile = p.tiles + (size_t)(p.flags ? blockIdx.x / 8 : blockIdx.x) * 3;
+  const int r = tile[0], skip = p.flags ? (int)blockIdx.x % 8 * BM : 0, row0 = tile[1] + skip, rows = p.flags ? min(BM, tile[2] - skip) : tile[2];
+  if (p.flags) {
+    int set = 0;
+    for (int i = threadIdx.x; i < p.flags_a_tile; i += blockDim.x) set |= p.flags[(size_t)(blockIdx.x / 8) * p.flags_a_tile + i];
+    if (!__syncthreads_or(set) || rows <= 0) return;
+  }
   const int pos0 = p.seq_len[r] - p.q_len[r] + (row0 - p.q_start[r]);     // position of the tile's first row
   const int pos_last = pos0 + rows - 1;
   const int W = p.window, PL = p.pool;

@@ -627,6 +627,50 @@ def pooled_attention_mma(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, num_tiles
     return out
 
 
+POOLED_TC5_ROWS = 128       # rows of a tile of the tcgen05 form
+POOLED_TC5_SCRATCH = 128 << 20      # bytes its heads' products take at most (a row of sixteen heads over four: 32 KB)
+
+
+def pooled_tc5_kv(dtype: torch.dtype, heads: int, kv_heads: int, key_dim: int, value_dim: int, page_tokens: int) -> int:
+    """Key/value heads a block of the tcgen05 form takes (0: not built for these sizes)."""
+    if dtype != torch.bfloat16 or key_dim != 128 or value_dim != 128 or heads > 16:
+        return 0
+    return _fn("pooled_attention_tc5", "pbe_pooled_attention_tc5_kv", [c_int] * 3)(int(heads), int(kv_heads), int(page_tokens))
+
+
+def pooled_attention_tc5(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, num_tiles: int, tile_starts, q_start, q_len, seq_len, bt_tok,
+                         bt_pool, heads: int, kv_heads: int, scale: float, window: int, pool: int, page_tokens: int) -> torch.Tensor:
+    """``pooled_attention`` with mixed heads on tcgen05, over row tiles of ``POOLED_TC5_ROWS`` (sizes for which ``pooled_tc5_kv`` is not
+    zero).  ``tile_starts``: int32 [num_tiles + 1] on the host, the tiles' first rows and the step's rows."""
+    _need_cuda(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, q_start, q_len, seq_len, bt_tok, bt_pool)
+    _need_contiguous(q, k_tok, v_tok, k_pool, v_pool, talk, tiles, q_start, q_len, seq_len, bt_tok, bt_pool)
+    T = q.shape[0]
+    D, E = k_tok.shape[3], v_tok.shape[3]
+    nkv = pooled_tc5_kv(q.dtype, heads, kv_heads, D, E, page_tokens)
+    if nkv == 0 or q.shape[1] != heads * D or k_tok.shape[1] != kv_heads or any(
+            x is not None and x.dtype != torch.bfloat16 for x in (k_tok, v_tok, k_pool, v_pool)):
+        raise KernelError("pooled_attention_tc5: shapes or dtypes do not agree")
+    if talk is None or talk.dtype != torch.float32 or tuple(talk.shape) != (heads, heads):
+        raise KernelError("pooled_attention_tc5: the mixing matrix is float32 [heads, heads]")
+    if pool and (k_pool is None or bt_pool is None):
+        raise KernelError("pooled_attention_tc5: pooled blocks need their pages and block table")
+    if len(tile_starts) != num_tiles + 1 or int(tile_starts[-1]) != T:
+        raise KernelError("pooled_attention_tc5: the tiles' first rows and the step's rows")
+    out = torch.empty((T, heads * E), dtype=q.dtype, device=q.device)
+    row_bytes = heads * kv_heads * E * 4
+    rows = max(POOLED_TC5_ROWS, min(T, POOLED_TC5_SCRATCH // row_bytes))
+    products = torch.empty(rows * row_bytes // 4, dtype=torch.float32, device=q.device)
+    flags = torch.empty(num_tiles * heads * (kv_heads // nkv), dtype=torch.int32, device=q.device)
+    fn = _fn("pooled_attention_tc5", "pbe_pooled_attention_tc5",
+             [c_void_p] * 8 + [c_int] + [c_void_p] * 5 + [c_int, c_void_p] + [c_int] * 8 + [c_float, c_void_p, c_int] + [c_void_p] * 3)
+    _check(fn(_ptr(q), _ptr(k_tok), _ptr(v_tok), _ptr(k_pool), _ptr(v_pool), _ptr(out), _ptr(talk), _ptr(tiles), num_tiles,
+              tile_starts.ctypes.data, _ptr(q_start), _ptr(q_len), _ptr(seq_len), _ptr(bt_tok), bt_tok.shape[1], _ptr(bt_pool),
+              bt_pool.shape[1] if bt_pool is not None else 0, heads, kv_heads, page_tokens, int(k_tok.shape[0]),
+              int(k_pool.shape[0]) if pool else 0, int(window), int(pool or 0), float(scale), _ptr(products), rows, _ptr(flags),
+              _ptr(tc5_attention_error_buffer(q.device)), _stream()), "pooled_attention_tc5")
+    return out
+
+
 # ------------------------------------------------------------------ rope + cache write
 def rope_kv_write(qkv: torch.Tensor, bias: Optional[torch.Tensor], q_out: torch.Tensor,
                   k_cache: Optional[torch.Tensor], v_cache: Optional[torch.Tensor],
@@ -1140,7 +1184,7 @@ DECODE_BLOCK_ITEMS_PER_SM = 3
 _sm_counts = {}
 
 
-def decode_block_max_items(device) -> int:
+def multiprocessors(device) -> int:
     sms = _sm_counts.get(device)
     if sms is None:
         try:
@@ -1148,7 +1192,11 @@ def decode_block_max_items(device) -> int:
         except (RuntimeError, AssertionError):
             sms = 148
         _sm_counts[device] = sms
-    return DECODE_BLOCK_ITEMS_PER_SM * sms
+    return sms
+
+
+def decode_block_max_items(device) -> int:
+    return DECODE_BLOCK_ITEMS_PER_SM * multiprocessors(device)
 
 
 class AttnFusedParams(ctypes.Structure):

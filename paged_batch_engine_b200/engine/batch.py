@@ -409,6 +409,15 @@ class StepContext:
             got = self._row_tiles[tile_rows] = (host.to(self.device, non_blocking=True), len(tiles), host)
         return got[0], got[1]
 
+    def row_tile_starts(self, tile_rows: int) -> np.ndarray:
+        """The first rows of ``row_tiles(tile_rows)`` and the step's rows, int32 on the host."""
+        kept = self.__dict__.setdefault("_row_tile_starts", {})
+        got = kept.get(tile_rows)
+        if got is None:
+            starts = [np.arange(int(qs), int(qs + n), tile_rows) for qs, n in zip(self.q_start_host, self.q_len_host)]
+            got = kept[tile_rows] = np.concatenate(starts + [[self.num_tokens]]).astype(np.int32)
+        return got
+
     def attention_work_of(self, group: int, group_size: int, tile_rows: int, window, some) -> AttentionWork:
         """The work list of the requests in ``some`` (a bool per request) only, made on first use; the other requests' rows
         are in no tile."""

@@ -64,6 +64,7 @@ class PooledWindowAttention(Mixer):
         self.w_qkv = self.w_o = self.q_gain = self.k_gain = self.talk = None
         self._tile_rows = None
         self._mma = False         # whether prompt portions take the tensor-core form (known once the kernels are loaded)
+        self._tc5 = False         # and its tcgen05 form
 
     # ---- what it keeps
     def cache_need(self):
@@ -79,6 +80,8 @@ class PooledWindowAttention(Mixer):
     def kernel_libraries(self, dtype):
         mma = [("pooled_attention_mma", ops._pm_defines(self.key_dim, self.value_dim))] \
             if ops.pooled_mma_applies(dtype, self.num_heads, self.key_dim, self.value_dim) else []
+        if mma and self.talking_heads and self.key_dim == 128 and self.value_dim == 128:
+            mma.append(("pooled_attention_tc5", None))
         return [("pooled_attention", {"PBE_PA_F32": 1 if dtype == torch.float32 else 0})] + mma + ops.gemm_libraries(dtype)
 
     # ---- tensors
@@ -108,6 +111,33 @@ class PooledWindowAttention(Mixer):
             self.talk = tensors.pop(prefix + n["talk"]).to(torch.float32).contiguous()
 
     # ---- compute
+    def _takes_tc5(self, ctx, seen: int) -> bool:
+        """Whether a step's portions take the tcgen05 form, kept on the step.  Its blocks (128 rows, one head, one or two key/value
+        heads) run one a multiprocessor, 8 us and 2.3 us a tile of 64 keys; the mixture and the look for odd values take 25 us
+        behind.  The mma.sync form's blocks (16 rows, all heads) take 25 us and 0.21 us a key.  Steps of fewer keys wait for the
+        host, where the tcgen05 form has 18 us more to do.  Layers of sixteen heads over four, mma.sync or split form -> tcgen05: 2,048 rows,
+        window 1,024 352 -> 233 us, window 256 and blocks of 16 182 / 193 (stays); 300 rows 133 -> 119, 256 rows 106 / 116
+        (stays); 16 rows behind 1,057 151 -> 121, behind 300 109 / 125 (stays); 64 rows beside 30 decoded tokens 311 / 358 (stays)."""
+        H, G = self.num_heads, self.num_kv_heads
+        kept = ctx.__dict__.setdefault("_pooled_tc5", {})
+        key = (H, G, self.window, self.pool)
+        if key not in kept:
+            rows, far = ops.POOLED_TC5_ROWS, self.window + ops.POOLED_TC5_ROWS - 1
+            work = longest = 0.0
+            blocks_16 = 0
+            for n, end in zip(ctx.q_len_host.tolist(), ctx.seq_len_host.tolist()):
+                a, b = min(end, end - n + rows), end                  # the keys that its first and its last row tile reach over
+                mean = (a + b) / 2 if b <= far else far if a >= far else ((far - a) * (a + far) / 2 + (b - far) * far) / (b - a)
+                older = max(0, end - self.window) / (64 * self.pool) if self.pool else 0.0
+                work += -(-n // rows) * (8 + 2.3 * (mean / 64 + 1 + older / 2))
+                longest = max(longest, 8 + 2.3 * (min(far, end) / 64 + 1 + older))
+                blocks_16 += -(-n // ops.POOLED_MMA_ROWS)
+            sms = ops.multiprocessors(self.device)
+            here = max(longest, work * H * (G // (2 if G % 2 == 0 else 1)) / sms) + 25
+            there = -(-blocks_16 // sms) * (25 + 0.21 * seen)
+            kept[key] = there > 95 and here < 0.97 * there
+        return kept[key]
+
     def forward(self, x, ctx, cache):
         H, G, D, E = self.num_heads, self.num_kv_heads, self.key_dim, self.value_dim
         proj = ops.linear(x, self.w_qkv, None, out_dtype=self.dtype, kind=1)
@@ -128,6 +158,7 @@ class PooledWindowAttention(Mixer):
         if self._tile_rows is None:
             self._tile_rows = ops.pooled_attention_tile_rows(H, E, 16, self.dtype)
             self._mma = ops.pooled_mma_applies(self.dtype, H, D, E) and ops.pooled_mma_fits(H, G, D, E)
+            self._tc5 = self._mma and self.talk is not None and self.scale > 0 and ops.pooled_tc5_kv(self.dtype, H, G, D, E, ctx.page_tokens) > 0
         # decoded tokens only (always so in a captured step): a row a tile
         single = getattr(ctx, "captured", False) or int(ctx.q_len_host.max(initial=1)) == 1
         # Prompt portions take the tensor-core form, whose blocks walk all keys of sixteen rows (30 us and 0.25 us a
@@ -136,6 +167,12 @@ class PooledWindowAttention(Mixer):
         # 188; 394 keys: 48 rows 126 / 132; 335 keys: 16 rows 115 / 101).
         longest = int(ctx.seq_len_host.max(initial=1))
         seen = min(longest, self.window + ops.POOLED_MMA_ROWS) + (longest // self.pool if self.pool else 0)
+        if self._tc5 and not single and self._takes_tc5(ctx, seen):
+            tiles, n_tiles = ctx.row_tiles(ops.POOLED_TC5_ROWS)
+            out = ops.pooled_attention_tc5(q, tok.k, tok.v, k_pool, v_pool, self.talk, tiles, n_tiles,
+                                           ctx.row_tile_starts(ops.POOLED_TC5_ROWS), ctx.q_start, ctx.q_len, ctx.seq_len,
+                                           gt.block_table, bt_pool, H, G, self.scale, self.window, self.pool, ctx.page_tokens)
+            return ops.linear(out, self.w_o, None, out_dtype=self.dtype, kind=2)
         if self._mma and not single and (ctx.num_tokens >= (80 if seen > 700 else 64) or seen <= 350):
             tiles, n_tiles = ctx.row_tiles(ops.POOLED_MMA_ROWS)
             out = ops.pooled_attention_mma(q, tok.k, tok.v, k_pool, v_pool, self.talk, tiles, n_tiles, ctx.q_start,
