@@ -4,14 +4,17 @@
 // The tensor cores cut off what does not fit a sum instead of rounding it, so the state is not left to them: what a chunk
 // writes is summed from zero and added to the state with one rounding.
 //
-// A block takes 64 columns of a head's state: warps 0-3 compute, sixteen columns each, whose [16, D] piece of S^T stays in
-// float32 accumulators and turns into an operand in registers; warps 4-7 fetch the next chunk's record and values,
-// split them and lay them down in the other of two buffers, one barrier a chunk.  Per chunk a computing warp has
-//   [W | QG]: S^T (as it lies) times the records' vectors, two tiles of eight tokens each;
+// A block takes 64 columns of a head's state (32 or 16 where two or four warps share sixteen columns, see launch): warps 0-3
+// compute, sixteen columns each, whose [16, D] piece of S^T (or their share of its key channels) stays in float32
+// accumulators and turns into an operand in registers; the other warps fetch the next chunk's record and values, split
+// them and lay them down in the other of two buffers, one barrier a chunk.  Per chunk a computing warp has
+//   [W | QG]: S^T (as it lies) times the records' vectors, two tiles of eight tokens each (warps that share columns add
+//   their parts through shared memory);
 //   u = U - S^T W;   o = S^T QG + u MQ;   S^T <- decays S^T + u KD.
 // What binds the scan of chunk_scan.cuh is the shared-memory pipe (every half warp reads the whole record for its
 // two or four columns); here sixteen columns share each fragment, and the 300 products of a chunk and computing warp bind.
-// Delta rule, 1,100 + 37 + 911 tokens, 16 heads of 128 x 128: 264 -> 157 us (the longest request's 69 chunks, 2.3 us each);
+// Delta rule, 1,100 + 37 + 911 tokens, 16 heads of 128 x 128: 264 -> 157 us (the longest request's 69 chunks, 2.3 us each), with
+// two warps to sixteen columns 112;
 // time mixing, 2,048 tokens in segments, both passes: 118 -> 95 us.  Two terms a factor took 91 and 77, but read-outs and
 // state were 5e-6 off 64 bits on given inputs; the multiply-adds are 0.5e-7 to 5e-7 off and this 0.6 to 1.4 times that.
 #pragma once
@@ -23,9 +26,12 @@ namespace scan_mma {
 
 using namespace mma_sync;
 
-constexpr int COLS = 64;                 // columns of a block
-constexpr int USTR = COLS + 4;           // floats a row of U: four rows apart start in different banks
+constexpr int USTR = 64 + 4;             // floats a row of U: four rows apart start in different banks
 constexpr int MSTR = CH + 8;             // elements a row of MQ
+template <int DS>
+__host__ __device__ constexpr int block_cols() { return 64 / DS; }
+template <int DS>
+__host__ __device__ constexpr int fetch_threads() { return DS > 1 ? 256 : 128; }
 
 template <int DP>
 __host__ __device__ constexpr int row_elems() { return DP + 8; }
@@ -63,16 +69,22 @@ __device__ __forceinline__ void products(float (&big)[2][4], float (&small)[2][4
   }
 }
 
-template <int DP, bool CORRECT, bool OWN, typename TU>
-__global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(ChunkScanParams<TU> p) {
+// DS: computing warps that share sixteen columns, DP / DS of their key channels each
+template <int DP, bool CORRECT, bool OWN, typename TU, int DS>
+__global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) scan_chunks_mma_kernel(ChunkScanParams<TU> p) {
+  static_assert(DS == 1 || ((DS == 2 || DS == 4) && !OWN), "warps of sixteen columns");
+  constexpr int COLS = block_cols<DS>();
+  constexpr int DW = DP / DS;                            // key channels of a warp
   constexpr int STR = row_elems<DP>();
   constexpr int MATS = CORRECT ? 3 : 2;                  // QG, KD, W
   constexpr int REC = record_floats(DP, CORRECT);
   constexpr int BYTES = buffer_bytes<DP, CORRECT>();
-  constexpr int PER = (REC / 4 + 127) / 128;             // float4s of a record a fetching thread takes
-  constexpr int UPER = CH * COLS / 128;
+  constexpr int FT = fetch_threads<DS>();
+  constexpr int PER = (REC / 4 + FT - 1) / FT;           // float4s of a record a fetching thread takes
+  constexpr int UPER = CH * COLS / FT;
   constexpr bool U_EXACT = sizeof(TU) == 2 && !CORRECT;  // u is a bfloat16 number: its other terms are zero
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ float shares[DS > 1 ? 4 : 1][16][33];       // of the products with the state, by warp
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y;
@@ -109,17 +121,17 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
       const float4* from = reinterpret_cast<const float4*>(rec0 + (size_t)c * H * REC);
 #pragma unroll
       for (int i = 0; i < PER; ++i)
-        raw[i] = ft + i * 128 < REC / 4 ? from[ft + i * 128] : make_float4(0.f, 0.f, 0.f, 0.f);
+        raw[i] = ft + i * FT < REC / 4 ? from[ft + i * FT] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < UPER; ++i) {
-        const int x = ft + i * 128, t = c * CH + x / COLS, e = e0 + x % COLS;
+        const int x = ft + i * FT, t = c * CH + x / COLS, e = e0 + x % COLS;
         u[i] = t < n && e < E ? to_float(p.u[(size_t)(t0 + t) * p.ld_u + h * E + e]) : 0.f;
       }
     };
     auto lay_down = [&](int buf) {
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        const int x = (ft + i * 128) * 4;
+        const int x = (ft + i * FT) * 4;
         if (x >= REC) break;
         unsigned t0[TERMS], t1[TERMS];
         split3(raw[i].x, raw[i].y, t0);
@@ -139,7 +151,7 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
       }
 #pragma unroll
       for (int i = 0; i < UPER; ++i) {
-        const int x = ft + i * 128;
+        const int x = ft + i * FT;
         values(buf)[(x / COLS) * USTR + x % COLS] = u[i];
       }
     };
@@ -160,20 +172,21 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
   const int g8 = lane >> 2, q2 = (lane & 3) * 2;
   const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lcol = (lane >> 4) * 8;
   const int krow = (lane & 7) + (lane >> 4) * 8, kcol = ((lane >> 3) & 1) * 8;
-  const int col = e0 + warp * 16 + g8;                   // this thread's columns: col and col + 8
+  const int group = warp / DS, d0 = warp % DS * DW;      // of sixteen columns; this warp's first key channel
+  const int col = e0 + group * 16 + g8;                  // this thread's columns: col and col + 8
   auto place = [&](int v) -> float* {
     if (v == -1) return nullptr;
     return (v >= 0 ? p.state + ((size_t)v * H + h) * E * D : p.scratch + ((size_t)(-(v + 2)) * H + h) * E * D);
   };
   const float* st_in = place(src);
-  float S[DP / 8][4];                                    // S^T: columns g8 (+ 8), key channels 8 j + q2 (+ 1)
+  float S[DW / 8][4];                                    // S^T: columns g8 (+ 8), key channels d0 + 8 j + q2 (+ 1)
 #pragma unroll
-  for (int j = 0; j < DP / 8; ++j)
+  for (int j = 0; j < DW / 8; ++j)
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
       float2 x = make_float2(0.f, 0.f);
-      if (st_in && col + hh * 8 < E && j * 8 + q2 < D)
-        x = *reinterpret_cast<const float2*>(st_in + (size_t)(col + hh * 8) * D + j * 8 + q2);
+      if (st_in && col + hh * 8 < E && d0 + j * 8 + q2 < D)
+        x = *reinterpret_cast<const float2*>(st_in + (size_t)(col + hh * 8) * D + d0 + j * 8 + q2);
       S[j][2 * hh] = x.x;
       S[j][2 * hh + 1] = x.y;
     }
@@ -192,16 +205,32 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
       for (int k = 0; k < 4; ++k) w[t][k] = q[t][k] = wc[t][k] = qc[t][k] = 0.f;
     if (CORRECT || !OWN) {
 #pragma unroll
-      for (int kk = 0; kk < DP / 16; ++kk) {
+      for (int kk = 0; kk < DW / 16; ++kk) {
         unsigned a[TERMS][4];
         as_operand(S[2 * kk], S[2 * kk + 1], a);
-        const int at = krow * STR + kk * 16 + kcol;
+        const int at = krow * STR + d0 + kk * 16 + kcol;
         if (CORRECT) products<false>(w, wc, a, matrix(buf, 2, 0) + at, CH * STR);
         if (!OWN) products<false>(q, qc, a, matrix(buf, 0, 0) + at, CH * STR);
       }
     }
+    if constexpr (DS > 1) {                              // of all its warps, added in their order (the block's barrier parts two chunks' uses)
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        shares[warp][k][lane] = w[k >> 2][k & 3] + wc[k >> 2][k & 3];
+        shares[warp][8 + k][lane] = q[k >> 2][k & 3] + qc[k >> 2][k & 3];
+        w[k >> 2][k & 3] = q[k >> 2][k & 3] = wc[k >> 2][k & 3] = qc[k >> 2][k & 3] = 0.f;
+      }
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * DS) : "memory");
+#pragma unroll
+      for (int i = 0; i < DS; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          w[k >> 2][k & 3] += shares[group * DS + i][k][lane];
+          q[k >> 2][k & 3] += shares[group * DS + i][8 + k][lane];
+        }
+    }
     // u: token 8 t + q2 (+ 1) of columns g8 (+ 8)
-    const float* U = values(buf) + warp * 16 + g8;
+    const float* U = values(buf) + group * 16 + g8;
     float u[2][4];
 #pragma unroll
     for (int t = 0; t < 2; ++t)
@@ -209,12 +238,12 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
       for (int k = 0; k < 4; ++k) u[t][k] = U[(t * 8 + q2 + (k & 1)) * USTR + (k >> 1) * 8] - (w[t][k] + wc[t][k]);
     unsigned ua[TERMS][4];
     as_operand(u[0], u[1], ua);
-    if (!OWN) products<true, U_EXACT>(q, qc, ua, mixed(buf, 0) + lrow * MSTR + lcol, CH * MSTR);
-    const float* decay = decays(buf) + q2;
+    if (!OWN && (DS == 1 || d0 == 0)) products<true, U_EXACT>(q, qc, ua, mixed(buf, 0) + lrow * MSTR + lcol, CH * MSTR);
+    const float* decay = decays(buf) + d0 + q2;
 #pragma unroll
-    for (int j = 0; j < DP / 16; ++j) {
+    for (int j = 0; j < DW / 16; ++j) {
       float y[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}}, yc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-      products<true, U_EXACT>(y, yc, ua, matrix(buf, 1, 0) + lrow * STR + j * 16 + lcol, CH * STR);
+      products<true, U_EXACT>(y, yc, ua, matrix(buf, 1, 0) + lrow * STR + d0 + j * 16 + lcol, CH * STR);
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const float2 f = *reinterpret_cast<const float2*>(decay + (2 * j + t) * 8);
@@ -226,7 +255,7 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
         for (int k = 0; k < 4; ++k) S[2 * j + t][k] = fmaf(k & 1 ? f.y : f.x, S[2 * j + t][k], y[t][k] + yc[t][k]);
       }
     }
-    if (!OWN) {
+    if (!OWN && (DS == 1 || d0 == 0)) {
 #pragma unroll
       for (int t = 0; t < 2; ++t)
 #pragma unroll
@@ -246,26 +275,47 @@ __global__ void __launch_bounds__(256, CORRECT ? 1 : 2) scan_chunks_mma_kernel(C
   }
   if (!st_out || (dst >= 0 && !p.write_state)) return;
 #pragma unroll
-  for (int j = 0; j < DP / 8; ++j)
+  for (int j = 0; j < DW / 8; ++j)
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh)
-      if (col + hh * 8 < E && j * 8 + q2 < D)
-        *reinterpret_cast<float2*>(st_out + (size_t)(col + hh * 8) * D + j * 8 + q2) = make_float2(S[j][2 * hh], S[j][2 * hh + 1]);
+      if (col + hh * 8 < E && d0 + j * 8 + q2 < D)
+        *reinterpret_cast<float2*>(st_out + (size_t)(col + hh * 8) * D + d0 + j * 8 + q2) = make_float2(S[j][2 * hh], S[j][2 * hh + 1]);
 }
 
-// Heads of an even number of key channels in records of DP of them (64 or 128).
-template <int DP, bool CORRECT, bool OWN, typename TU>
-int launch(const ChunkScanParams<TU>& p, int items, cudaStream_t stream) {
-  constexpr int smem = 2 * buffer_bytes<DP, CORRECT>();
-  auto kernel = scan_chunks_mma_kernel<DP, CORRECT, OWN, TU>;
+template <int DP, bool CORRECT, bool OWN, typename TU, int DS>
+int launch_of(const ChunkScanParams<TU>& p, int items, cudaStream_t stream) {
+  // warps that share columns: one block a multiprocessor, so that blocks behind the first wave find the ones that short requests leave
+  constexpr int smem = 2 * buffer_bytes<DP, CORRECT>() > 120 * 1024 || DS == 1 ? 2 * buffer_bytes<DP, CORRECT>() : 120 * 1024;
+  auto kernel = scan_chunks_mma_kernel<DP, CORRECT, OWN, TU, DS>;
   static bool opted = false;
   if (!opted) {
     const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;
     opted = true;
   }
-  launch_spread(kernel, dim3(items, p.H, (p.E + COLS - 1) / COLS), 256, smem, stream, p);
+  launch_spread(kernel, dim3(items, p.H, (p.E + block_cols<DS>() - 1) / block_cols<DS>()), 128 + fetch_threads<DS>(), smem, stream, p);
   return launch_status();
+}
+
+// Heads of an even number of key channels in records of DP of them (64 or 128).
+template <int DP, bool CORRECT, bool OWN, typename TU>
+int launch(const ChunkScanParams<TU>& p, int items, cudaStream_t stream, int busy = 0) {
+  // Corrected writes walk a request's chunks one after the other: two or four warps share sixteen columns where the blocks, as many
+  // times more then, still find a multiprocessor each (`busy` requests of about the longest one's rows; 0: not known).
+  // A layer of 16 heads of 128, one warp -> two: 1,100 + 37 + 911 tokens 359 -> 312 us; with blocks for more than every
+  // multiprocessor 359 -> 397.  2,048 tokens, one -> two -> four: 488 -> 391 -> 361.
+  if constexpr (CORRECT && !OWN) {
+    static int sms = 0;
+    if (sms == 0) {
+      int dev = 0, got = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&got, cudaDevAttrMultiProcessorCount, dev);
+      sms = got > 0 ? got : 148;
+    }
+    if (busy > 0 && (long long)busy * p.H * ((p.E + 15) / 16) <= sms) return launch_of<DP, CORRECT, OWN, TU, 4>(p, items, stream);
+    if (busy > 0 && (long long)busy * p.H * ((p.E + 31) / 32) <= sms) return launch_of<DP, CORRECT, OWN, TU, 2>(p, items, stream);
+  }
+  return launch_of<DP, CORRECT, OWN, TU, 1>(p, items, stream);
 }
 }  // namespace scan_mma
 }  // namespace pbe

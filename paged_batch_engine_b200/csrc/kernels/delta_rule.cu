@@ -677,7 +677,7 @@ __global__ void __launch_bounds__(128, 4) delta_chunks_kernel(ChunkParams p) {
 }
 
 template <int RPT, int CPT, int WARPS>
-int launch_chunks(const ChunkParams& g, const ChunkScanParams<float>& p, int records, bool chan, bool matrix,
+int launch_chunks(const ChunkParams& g, const ChunkScanParams<float>& p, int records, bool chan, bool matrix, int busy,
                   cudaStream_t stream) {
   constexpr int DP = 16 * RPT, COLS = 2 * WARPS * CPT;
   constexpr size_t smem_g = sizeof(float) * 3 * CH * DP, smem_p = sizeof(float) * 2 * record_floats(DP, true);
@@ -696,7 +696,7 @@ int launch_chunks(const ChunkParams& g, const ChunkScanParams<float>& p, int rec
   const int err = launch_status();
   if (err != 0) return err;
   if constexpr (DP <= 128) {
-    if (matrix && g.D % 2 == 0) return scan_mma::launch<DP, true, false, float>(p, g.R, stream);
+    if (matrix && g.D % 2 == 0) return scan_mma::launch<DP, true, false, float>(p, g.R, stream, busy);
   }
   launch_spread(scan_chunks_kernel<RPT, CPT, WARPS, true, false, float>, dim3(g.R, g.H, (g.E + COLS - 1) / COLS), 32 * WARPS, smem_p,
                 stream, p);
@@ -785,12 +785,12 @@ PBE_EXPORT int pbe_delta_record_floats(int D) {
 PBE_EXPORT int pbe_delta_chunk_tokens() { return CH; }
 
 // The same for steps with prompt portions, sixteen tokens of a request at a time: two launches.  v is
-// overwritten.  matrix: the scan's products on the tensor cores, every float32 factor as two bfloat16 terms (bfloat16
-// runs).  records: [T / 16 + R][H][pbe_delta_record_floats(D)] floats of scratch memory.
+// overwritten.  matrix: the scan's products on the tensor cores, every float32 factor as three bfloat16 terms (bfloat16
+// runs); longest: the most rows of a request (0: not known), by which their blocks are cut.  records: [T / 16 + R][H][pbe_delta_record_floats(D)] floats of scratch memory.
 PBE_EXPORT int pbe_delta_scan_chunks(const float* qk, float* v, const float* beta, const float* decay, int per_channel,
                                      float* out, float* state, float* records, const int32_t* q_start,
                                      const int32_t* q_len, const int32_t* slots, int T, int R, int G, int H, int D,
-                                     int E, int write_state, int matrix, cudaStream_t stream) {
+                                     int E, int write_state, int matrix, int longest, cudaStream_t stream) {
   if (R <= 0 || T <= 0) return 0;
   if (D < 1 || D > 256 || E < 1 || G < 1 || H % G != 0 || records == nullptr) return (int)cudaErrorInvalidValue;
   if ((((uintptr_t)state | (uintptr_t)records) & 15) != 0) return (int)cudaErrorMisalignedAddress;
@@ -800,7 +800,8 @@ PBE_EXPORT int pbe_delta_scan_chunks(const float* qk, float* v, const float* bet
   const ChunkScanParams<float> p{records, v, H * E, out, state, q_start, q_len, slots, H, D, E, write_state};
   const int n = T / CH + R;
   const bool chan = per_channel != 0;
-  if (D <= 64) return launch_chunks<4, 2, 4>(g, p, n, chan, matrix != 0, stream);
-  if (D <= 128) return launch_chunks<8, 2, 4>(g, p, n, chan, matrix != 0, stream);
-  return launch_chunks<16, 2, 4>(g, p, n, chan, matrix != 0, stream);
+  const int busy = longest > 0 ? (T + longest - 1) / longest : 0;
+  if (D <= 64) return launch_chunks<4, 2, 4>(g, p, n, chan, matrix != 0, busy, stream);
+  if (D <= 128) return launch_chunks<8, 2, 4>(g, p, n, chan, matrix != 0, busy, stream);
+  return launch_chunks<16, 2, 4>(g, p, n, chan, matrix != 0, busy, stream);
 }

@@ -2553,13 +2553,14 @@ DELTA_CHUNK_MAX_DIM = 256     # wider key heads always run token by token
 def delta_scan(qk: torch.Tensor, kq: torch.Tensor, v: torch.Tensor, beta: torch.Tensor, decay: torch.Tensor,
                state: torch.Tensor, q_start: torch.Tensor, q_len: torch.Tensor, slots: torch.Tensor, num_requests: int,
                update_state: bool = True, zero_out: bool = False,
-               chunked: bool = False, matrix: bool = False) -> torch.Tensor:
+               chunked: bool = False, matrix: bool = False, longest: int = 0) -> torch.Tensor:
     """The gated delta rule request by request over the rows each brings: S <- g S,
     u = beta (v - S^T k), S <- S + k u^T, o = S^T q, with the inputs of ``delta_inputs`` and ``state``
     float32 [slots, H, E, D] (S transposed: a value column's key channels side by side), read at
     ``slots[r]`` and left updated.  ``chunked``: sixteen tokens at a time
     (prompt portions: two launches, v is overwritten), else one by one.  ``matrix``: the chunks' scan on the tensor
-    cores, every float32 factor as two bfloat16 terms (bfloat16 runs).  Returns o, float32 [T, H * E]."""
+    cores, every float32 factor as three bfloat16 terms (bfloat16 runs); ``longest``: the most rows a request brings, which
+    tells how its blocks are cut (0: not known).  Returns o, float32 [T, H * E]."""
     _need_cuda(qk, kq, v, beta, decay, state, q_start, q_len, slots)
     _need_contiguous(qk, kq, v, beta, decay, state)
     T, G, _, D = qk.shape
@@ -2580,11 +2581,11 @@ def delta_scan(qk: torch.Tensor, kq: torch.Tensor, v: torch.Tensor, beta: torch.
         size = _fn("delta_rule", "pbe_delta_record_floats", [c_int])(D)
         ct = _fn("delta_rule", "pbe_delta_chunk_tokens", [])()
         records = torch.empty((T // ct + int(num_requests), H, size), dtype=torch.float32, device=v.device)
-        fn = _fn("delta_rule", "pbe_delta_scan_chunks", [c_void_p] * 4 + [c_int] + [c_void_p] * 6 + [c_int] * 8 + [c_void_p])
+        fn = _fn("delta_rule", "pbe_delta_scan_chunks", [c_void_p] * 4 + [c_int] + [c_void_p] * 6 + [c_int] * 9 + [c_void_p])
         global _launches
         _check(fn(_ptr(qk), _ptr(v), _ptr(beta), _ptr(decay), 1 if per_channel else 0, _ptr(out), _ptr(state),
                   _ptr(records), _ptr(q_start), _ptr(q_len), _ptr(slots), T, int(num_requests), G, H, D, E,
-                  1 if update_state else 0, 1 if matrix else 0, _stream()), "delta_scan_chunks")
+                  1 if update_state else 0, 1 if matrix else 0, int(longest), _stream()), "delta_scan_chunks")
         _launches += 1
         return out
     fn = _fn("delta_rule", "pbe_delta_scan", [c_void_p] * 5 + [c_int] + [c_void_p] * 5 + [c_int] * 6 + [c_void_p])

@@ -161,7 +161,8 @@ class GatedDeltaRule(Mixer):
             single_tokens=single)
         o = ops.delta_scan(qk, kq, v, beta, decay, cache.sub["delta"].state, ctx.q_start, ctx.q_len, ctx.state_slots,
                            ctx.num_requests, update_state=cache.writes, zero_out=captured,
-                           chunked=not single, matrix=self.dtype == torch.bfloat16)
+                           chunked=not single, matrix=self.dtype == torch.bfloat16,
+                           longest=0 if single else int(ctx.q_len_host.max()))
         y = ops.gated_rms(o, gate, self.gain, H, self.eps, True, self.gate, self.dtype)
         return ops.linear(y, self.w_o, None, out_dtype=self.dtype, kind=2)
 
