@@ -594,36 +594,47 @@ __global__ void __launch_bounds__(128, 4) delta_chunks_kernel(ChunkParams p) {
   float* out = p.records + ((size_t)rec * H + h) * record_floats(DP, true);
   float* mq = out + rec_mq(DP);
   {
-    // eight lanes share a token i, DP / 8 channels each; x runs over k_i times the decays after i
-    constexpr int MPT = DP / 8;
-    const int i = tid >> 3, slice = tid & 7;
-    float x[MPT];
+    // Sixteen lanes share the tokens i = pair and CH - 1 - pair, one after the other (together as many later tokens for every
+    // pair), DP / 16 channels each; x runs over k_i times the decays after i.  The products with the later tokens are summed
+    // over the lanes at the end, all at once.  Eight lanes a token, single channels and a sum a product took 71 us
+    // for 2,048 tokens and 16 heads of 128, this 60, and 46 with the loops behind it kept from loading all of Lk and Tb ahead
+    // (128 registers and spills; more blocks a multiprocessor with fewer registers: 47 to 52).
+    constexpr int F = DP / 64;
+    const int part = tid & 15;
+#pragma unroll 1
+    for (int t = 0; t < 2; ++t) {
+      const int i = t == 0 ? tid >> 4 : CH - 1 - (tid >> 4);
+      float4 x[F];
+      float ck[CH], cq[CH];
 #pragma unroll
-    for (int m = 0; m < MPT; ++m) x[m] = K[i * DP + slice + 8 * m];
-    for (int j = 0; j < CH; ++j) {
-      float ck = 0.f, cq = 0.f;
-      if (j >= i) {
+      for (int f = 0; f < F; ++f) x[f] = *reinterpret_cast<const float4*>(K + i * DP + part * 4 + f * 64);
 #pragma unroll
-        for (int m = 0; m < MPT; ++m) {
-          const int d = j * DP + slice + 8 * m;
-          if (j > i) x[m] *= W[d];
-          ck = fmaf(x[m], K[d], ck);
-          cq = fmaf(x[m], Q[d], cq);
+      for (int j = 0; j < CH; ++j) {
+        float a = 0.f, b = 0.f;
+        if (j >= i) {
+#pragma unroll
+          for (int f = 0; f < F; ++f) {
+            const int at = j * DP + part * 4 + f * 64;
+            const float4 k = *reinterpret_cast<const float4*>(K + at), q = *reinterpret_cast<const float4*>(Q + at);
+            if (j > i) {
+              const float4 w = *reinterpret_cast<const float4*>(W + at);
+              x[f].x *= w.x; x[f].y *= w.y;
+              x[f].z *= w.z; x[f].w *= w.w;
+            }
+            a = fmaf(x[f].x, k.x, fmaf(x[f].y, k.y, fmaf(x[f].z, k.z, fmaf(x[f].w, k.w, a))));
+            b = fmaf(x[f].x, q.x, fmaf(x[f].y, q.y, fmaf(x[f].z, q.z, fmaf(x[f].w, q.w, b))));
+          }
         }
+        ck[j] = a;
+        cq[j] = b;
       }
+      __syncwarp();
+      const float a = scatter_sum(ck, part), b = scatter_sum(cq, part);      // lane `part`: those of token `part`, zeros before i
+      Lk[part][i] = part > i ? beta[part] * a : 0.f;
+      mq[i * CH + part] = b;
 #pragma unroll
-      for (int m = 1; m < 8; m <<= 1) {
-        ck += __shfl_xor_sync(0xffffffffu, ck, m);
-        cq += __shfl_xor_sync(0xffffffffu, cq, m);
-      }
-      if (slice == 0) {
-        Lk[j][i] = j > i ? beta[j] * ck : 0.f;
-        mq[i * CH + j] = j >= i ? cq : 0.f;
-      }
+      for (int f = 0; f < F; ++f) *reinterpret_cast<float4*>(out + rec_kd(DP) + i * DP + part * 4 + f * 64) = x[f];
     }
-    float* kd = out + rec_kd(DP) + i * DP;
-#pragma unroll
-    for (int m = 0; m < MPT; ++m) kd[slice + 8 * m] = x[m];
   }
   __syncthreads();
   if (tid < CH) {                          // a thread a column of the inverse, by substitution
@@ -635,6 +646,7 @@ __global__ void __launch_bounds__(128, 4) delta_chunks_kernel(ChunkParams p) {
       for (int i = 0; i < j; ++i) s = fmaf(-Lk[j][i], t[i], s);      // t[i] is 0 above the diagonal
       t[j] = s;
       Tb[j][tid] = s * beta[tid];
+      asm volatile("" ::: "memory");     // a row of Lk ahead, not all of it in registers
     }
   }
   __syncthreads();
@@ -652,6 +664,7 @@ __global__ void __launch_bounds__(128, 4) delta_chunks_kernel(ChunkParams p) {
         if (i + 3 <= j) s = fmaf(t4.w, y[i + 3], s);
       }
       put(j, s);
+      if (j % 4 == 3) asm volatile("" ::: "memory");
     }
   };
   for (int d = tid; d < DP; d += 128) {
