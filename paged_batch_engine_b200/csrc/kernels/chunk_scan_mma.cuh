@@ -80,7 +80,9 @@ __global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) sc
   constexpr int REC = record_floats(DP, CORRECT);
   constexpr int BYTES = buffer_bytes<DP, CORRECT>();
   constexpr int FT = fetch_threads<DS>();
-  constexpr int PER = (REC / 4 + FT - 1) / FT;           // float4s of a record a fetching thread takes
+  // what is fetched of a record: all of it, or KD and the decays behind it where nothing is read out
+  constexpr int FROM = OWN ? rec_kd(DP) : 0, TO = OWN ? rec_mq(DP) : REC;
+  constexpr int PER = ((TO - FROM) / 4 + FT - 1) / FT;   // float4s of a record a fetching thread takes
   constexpr int UPER = CH * COLS / FT;
   constexpr bool U_EXACT = sizeof(TU) == 2 && !CORRECT;  // u is a bfloat16 number: its other terms are zero
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -121,7 +123,7 @@ __global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) sc
       const float4* from = reinterpret_cast<const float4*>(rec0 + (size_t)c * H * REC);
 #pragma unroll
       for (int i = 0; i < PER; ++i)
-        raw[i] = ft + i * FT < REC / 4 ? from[ft + i * FT] : make_float4(0.f, 0.f, 0.f, 0.f);
+        raw[i] = ft + i * FT < (TO - FROM) / 4 ? from[FROM / 4 + ft + i * FT] : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
       for (int i = 0; i < UPER; ++i) {
         const int x = ft + i * FT, t = c * CH + x / COLS, e = e0 + x % COLS;
@@ -131,8 +133,8 @@ __global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) sc
     auto lay_down = [&](int buf) {
 #pragma unroll
       for (int i = 0; i < PER; ++i) {
-        const int x = (ft + i * FT) * 4;
-        if (x >= REC) break;
+        const int x = FROM + (ft + i * FT) * 4;
+        if (x >= TO) break;
         unsigned t0[TERMS], t1[TERMS];
         split3(raw[i].x, raw[i].y, t0);
         split3(raw[i].z, raw[i].w, t1);
