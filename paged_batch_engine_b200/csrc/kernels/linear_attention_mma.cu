@@ -319,6 +319,7 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
         }
       }
     }
+    if (c0 + L >= n && dst == -1) break;               // nothing is passed on: an item in the middle of a portion, its outputs made
     // the chunk's writes: k times its weight in the new state, split in registers, times v
 #pragma unroll
     for (int m = 0; m < MT; ++m) {
