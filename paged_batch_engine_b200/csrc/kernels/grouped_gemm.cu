@@ -240,46 +240,62 @@ __global__ void __launch_bounds__(128) grouped_gemm_kernel(GroupGemmParams p) {
   }
 }
 
-// The tile list of rows sorted by group, every group's run padded to whole tiles of `tile_rows`: from the groups'
-// row counts.  start[g]: first row of group g's run; tiles[i] = (group, first row, rows), idle
-// entries (group -1) up to max_tiles.  One block: a thread a group, a scan over the groups' tile counts
-// instead of one thread walking over all of them.
+// The tile list of rows sorted by group, from the groups' row counts: tiles[i] = (group, first row, rows), idle
+// entries (group -1) up to max_tiles; start[g]: first row of group g's run.  One block: a thread a group, a scan over
+// the groups' tile (and row) counts instead of one thread walking over all of them.
+//   PADDED: every group's run is padded to whole tiles of `tile_rows`.
+//   otherwise the runs lie one behind the other, and a run's tiles share its rows evenly (a multiple of sixteen each,
+//   `tile_rows`, a multiple of sixteen, at most): 264 rows are tiles of 144 and 120, not of 256 and 8.
 constexpr int TILES_THREADS = 256;
 
+template <bool PADDED>
 __global__ void __launch_bounds__(TILES_THREADS) run_tiles_kernel(const int32_t* counts, int groups,
                                                                   int max_tiles, int tile_rows,
                                                                   int32_t* start,
                                                                   int32_t* tiles) {
-  __shared__ int warp_tot[TILES_THREADS / 32];
+  __shared__ int warp_tot[TILES_THREADS / 32], warp_rows[TILES_THREADS / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   pdl_launch_dependents();
   pdl_wait();
-  int base = 0;                         // tiles of the groups before this round's
+  int base = 0, base_row = 0;           // tiles and rows of the groups before this round's
   for (int g0 = 0; g0 < groups; g0 += TILES_THREADS) {
     const int g = g0 + threadIdx.x;
     const int rows = g < groups ? counts[g] : 0;
     const int own = (rows + tile_rows - 1) / tile_rows;
-    int upto = own;
+    int upto = own, upto_row = rows;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int n = __shfl_up_sync(0xffffffffu, upto, o);
-      if (lane >= o) upto += n;
+      const int m = PADDED ? 0 : __shfl_up_sync(0xffffffffu, upto_row, o);
+      if (lane >= o) {
+        upto += n;
+        upto_row += m;
+      }
     }
-    if (lane == 31) warp_tot[warp] = upto;
+    if (lane == 31) {
+      warp_tot[warp] = upto;
+      if (!PADDED) warp_rows[warp] = upto_row;
+    }
     __syncthreads();
-    int first = base + upto - own;
+    int first = base + upto - own, row = base_row + upto_row - rows;
 #pragma unroll
     for (int w = 0; w < TILES_THREADS / 32; ++w) {
       if (w < warp) first += warp_tot[w];
       base += warp_tot[w];
+      if (!PADDED) {
+        if (w < warp) row += warp_rows[w];
+        base_row += warp_rows[w];
+      }
     }
     // a list that is too short cuts the runs off where it ends
-    if (g < groups) start[g] = min(first, max_tiles) * tile_rows;
+    if (PADDED) row = min(first, max_tiles) * tile_rows;
+    if (g < groups) start[g] = row;
+    const int height = PADDED || own == 0 ? tile_rows : (rows + 16 * own - 1) / (16 * own) * 16;
     for (int j = 0; j < own && first + j < max_tiles; ++j) {
       int32_t* tile = tiles + 3 * (first + j);
       tile[0] = g;
-      tile[1] = (first + j) * tile_rows;
-      tile[2] = min(tile_rows, rows - j * tile_rows);
+      tile[1] = row + j * height;
+      tile[2] = min(height, rows - j * height);
     }
     __syncthreads();                    // warp_tot is written again
   }
@@ -312,10 +328,11 @@ PBE_EXPORT int pbe_grouped_gemm(const void* a, int a_dtype, int lda, long long a
   return launch_status();
 }
 
-PBE_EXPORT int pbe_run_tiles(const int32_t* counts, int groups, int max_tiles, int tile_rows, int32_t* start,
+PBE_EXPORT int pbe_run_tiles(const int32_t* counts, int groups, int max_tiles, int tile_rows, int padded, int32_t* start,
                              int32_t* tiles, cudaStream_t stream) {
   if (groups <= 0 || max_tiles <= 0) return 0;
-  if (tile_rows <= 0) return (int)cudaErrorInvalidValue;
-  launch_k(run_tiles_kernel, 1, TILES_THREADS, 0, stream, counts, groups, max_tiles, tile_rows, start, tiles);
+  if (tile_rows <= 0 || (!padded && (tile_rows & 15))) return (int)cudaErrorInvalidValue;
+  launch_k(padded ? run_tiles_kernel<true> : run_tiles_kernel<false>, 1, TILES_THREADS, 0, stream, counts, groups, max_tiles,
+           tile_rows, start, tiles);
   return launch_status();
 }

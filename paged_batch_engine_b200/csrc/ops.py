@@ -2236,16 +2236,17 @@ def most_run_tiles(rows: int, groups: int, tile_rows: int) -> int:
     return some + (rows - some) // tile_rows
 
 
-def run_tiles(counts: torch.Tensor, max_tiles: int, tile_rows: int = GROUP_TILE_ROWS):
+def run_tiles(counts: torch.Tensor, max_tiles: int, tile_rows: int = GROUP_TILE_ROWS, padded: bool = True):
     """(start int32 [G], tiles int32 [max_tiles, 3]) for rows sorted by group with every group's run
     padded to whole tiles of ``tile_rows``: a group's first row, and per tile (group, first
-    row, rows), idle tiles with group -1 behind all others."""
+    row, rows), idle tiles with group -1 behind all others.  ``padded`` False: the runs lie one behind the other, and a
+    run's tiles share its rows evenly, sixteen at a time (``tile_rows`` a multiple of sixteen)."""
     _need_cuda(counts)
     G = counts.numel()
     start = torch.empty(G, dtype=torch.int32, device=counts.device)
     tiles = torch.empty((max_tiles, 3), dtype=torch.int32, device=counts.device)
-    fn = _fn("grouped_gemm", "pbe_run_tiles", [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p])
-    _check(fn(_ptr(counts), G, int(max_tiles), int(tile_rows), _ptr(start), _ptr(tiles), _stream()), "run_tiles")
+    fn = _fn("grouped_gemm", "pbe_run_tiles", [c_void_p, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p])
+    _check(fn(_ptr(counts), G, int(max_tiles), int(tile_rows), 1 if padded else 0, _ptr(start), _ptr(tiles), _stream()), "run_tiles")
     return start, tiles
 
 
@@ -2262,7 +2263,7 @@ def grouped_runs(a: torch.Tensor, w: torch.Tensor, tiles: torch.Tensor, out_dtyp
     return _grouped(a, K, 0, w, N * K, 1, K, out, N, 0, rows, K, N, G, tiles, tiles.shape[0], activation=activation)
 
 
-GROUPED_TC5_ROWS = 128       # rows of a tile of the tcgen05 form
+GROUPED_TC5_ROWS = 256       # most rows of a tile of the tcgen05 form
 GROUPED_TC5_EPILOGUES = {None: 0, "relu2": 1, "silu": 2, "capped_swish": 3}
 
 
@@ -2275,7 +2276,7 @@ def grouped_tc5_applies(x: torch.Tensor, *weights: torch.Tensor) -> bool:
 
 def grouped_runs_tc5(a: torch.Tensor, w: torch.Tensor, tiles: Optional[torch.Tensor], activation: Optional[str] = None,
                      limit: float = 0.0, alpha: float = 1.0) -> torch.Tensor:
-    """``grouped_runs`` on tcgen05 (``tiles`` of ``GROUPED_TC5_ROWS`` rows, bfloat16 result), with the activation as
+    """``grouped_runs`` on tcgen05 (``tiles`` of up to ``GROUPED_TC5_ROWS`` rows, bfloat16 result), with the activation as
     the epilogue: "relu2" squares the relu; "silu" and "capped_swish" take ``w`` [G, 2 * I, K] as gate rows followed
     by up rows and give [rows, I] as ``gated_activation`` does.  ``tiles`` None: all rows belong to one group."""
     _need_cuda(a, w, tiles)

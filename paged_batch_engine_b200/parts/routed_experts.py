@@ -149,16 +149,18 @@ class RoutedExperts(FeedForward):
         return rows, (None if on_input else weights)
 
     def _tiled(self, x, chosen, weights, shared):
-        """bfloat16: rows sorted by expert, every expert's run padded to whole row tiles, and one
-        launch per projection that multiplies every tile with its expert's matrix on the tensor
-        cores.  Nothing is read on the host."""
+        """bfloat16: rows sorted by expert, and one launch per projection that multiplies every row
+        tile with its expert's matrix on the tensor cores.  The tcgen05 form takes runs that lie one
+        behind the other, in tiles of any height; for the other form every expert's run is padded to
+        whole tiles.  Nothing is read on the host."""
         T = x.shape[0]
         tc5 = ops.grouped_tc5_applies(x, self.w_gate_up, self.w_down)
         tile_rows = ops.GROUPED_TC5_ROWS if tc5 else ops.GROUP_TILE_ROWS
         counts, place = ops.expert_places(chosen, self.num_experts)
         max_tiles = ops.most_run_tiles(T * self.top, self.num_experts, tile_rows)
-        start, tiles = ops.run_tiles(counts, max_tiles, tile_rows)
-        rows, weights = self._gathered(x, chosen, place, start, weights, total_rows=max_tiles * tile_rows)
+        start, tiles = ops.run_tiles(counts, max_tiles, tile_rows, padded=not tc5)
+        rows, weights = self._gathered(x, chosen, place, start, weights,
+                                       total_rows=T * self.top if tc5 else max_tiles * tile_rows)
         if tc5:
             hidden = ops.grouped_runs_tc5(rows, self.w_gate_up, tiles, self.activation, self.limit, self.alpha)
             out = ops.grouped_runs_tc5(hidden, self.w_down, tiles)
