@@ -13,16 +13,18 @@
 //   - the order: all column blocks of eight row tiles before the next eight, so that these rows stay in L2 while the
 //     matrices stream past; with the column blocks of all experts one after another the rows were fetched again and
 //     again (525 MB for 402).  The matrices give their place in L2 up first.
-// A persistent pair of blocks walks over the tiles.  Warp 0 is the TMA producer (six stages), warp 1 of the leader issues
-// the MMAs, warps 2-5 are the epilogue; two accumulators alternate, so a tile's epilogue overlaps the next tile's
-// products.  Results leave through shared memory: stores of two bytes along the accumulator's lanes took ten
+// A persistent pair of blocks walks over the tiles.  Warp 0 is the TMA producer, warp 1 of the leader issues the MMAs,
+// warps 2-5 are the epilogue; two accumulators alternate, so a tile's epilogue overlaps the next tile's products.  Three
+// stages of 128 k: between two stages the issuer waits, fences and commits while the tensor pipe runs dry, some 200
+// clocks whatever the tile's height, so stages of 64 k (six) cost a tenth (matrices in L2, 256-row tiles: 77.8 -> 69.0 us,
+// 1.21 -> 1.37 PFLOP/s).  Results leave through shared memory: stores of two bytes along the accumulator's lanes took ten
 // microseconds a tile.
 //
 // Epilogues: none, relu squared, and gates (W_g = [gate rows; up rows]: a block takes 64 of each, and the threads of an
 // output's gate and up sums swap halves of their rows, so the activation costs no pass over memory and sees float32 sums).
 //
-// 2,048 rows, 4 of 32 experts, 2,048 -> 2 x 1,408 -> 2,048 (matrices from DRAM): 130 + 73 -> 118 + 66 us; 4,096 rows
-// 204 + 106 -> 173 + 92, 16 rows 83 + 46 -> 70 + 38 (one block a tile of 128 rows x 256 columns before; the mma.sync
+// 2,048 rows, 4 of 32 experts, 2,048 -> 2 x 1,408 -> 2,048 (matrices from DRAM): 130 + 73 -> 111 + 63 us; 4,096 rows
+// 204 + 106 -> 162 + 90, 16 rows 83 + 46 -> 68 + 36 (one block a tile of 128 rows x 256 columns before; the mma.sync
 // products of grouped_gemm.cu and the activation's own pass took 826 + 95 at 2,048 rows).
 //
 // Every wait on an mbarrier is bounded; one that runs out sets *err and the block goes on to its end.
@@ -38,8 +40,9 @@ using namespace pbe::tc5;
 namespace {
 typedef __nv_bfloat16 bf16;
 constexpr int BAND = 8;                  // row tiles that all column blocks are made for before the next ones
-constexpr int BM = 128, MAX_ROWS = 256, BK = 64, UMMA_K = 16, STAGES = 6;
-constexpr int A_BYTES = BM * BK * 2, B_BYTES = MAX_ROWS / 2 * BK * 2, STAGE_BYTES = A_BYTES + B_BYTES;
+constexpr int BM = 128, MAX_ROWS = 256, BK = 64, UMMA_K = 16, STAGES = 3, IN_STAGE = 2;
+constexpr int A_BYTES = BM * BK * 2, B_BYTES = MAX_ROWS / 2 * BK * 2, BLOCK_BYTES = A_BYTES + B_BYTES;
+constexpr int STAGE_BYTES = IN_STAGE * BLOCK_BYTES;        // a stage is two blocks of 64 k
 constexpr int BOUNCE_BYTES = 2 * 32 * (128 + 8) * 2;         // results of 32 rows on their way out, twice (gated ones
 static_assert(BOUNCE_BYTES >= 2 * 32 * (64 + 8) * 2 + 16 * 128 * 4, "");      // are half, and the swap beside them)
 constexpr int NTHREADS = 192, TMEM_COLS = 512;
@@ -171,16 +174,19 @@ grouped_tc5_kernel(const __grid_constant__ Maps maps, GroupedParams p) {
                           : tile.group * p.N + tile.n0 + rank * 128;
       const int to = for_x ? A_BYTES + before * BK * 2 : lane * 64 * BK * 2;
       const uint32_t bytes = 2 * (A_BYTES + half * BK * 2);                  // both blocks' copies
-      for (int kb = 0; kb < kblocks; ++kb, ++it) {
-        const int s = it % STAGES;
+      for (int kb = 0; kb < kblocks; kb += IN_STAGE, ++it) {
+        const int s = it % STAGES, blocks = min(IN_STAGE, kblocks - kb);
         ok = mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, p.err);
         ok = __all_sync(0xffffffffu, ok);
         if (!ok) break;
-        if (leader && lane == 0) mbar_expect_tx(&full_bar[s], bytes);
+        if (leader && lane == 0) mbar_expect_tx(&full_bar[s], blocks * bytes);
         __syncwarp();
         unsigned char* dst = stages + (size_t)s * STAGE_BYTES + to;
-        if (for_w) tma_load_2d_pair_once(dst, map, kb * BK, y, map_to_rank(&full_bar[s], 0));
-        else if (for_x) tma_load_2d_pair(dst, map, kb * BK, y, map_to_rank(&full_bar[s], 0));
+        const uint32_t bar = map_to_rank(&full_bar[s], 0);
+        for (int h = 0; h < blocks; ++h) {
+          if (for_w) tma_load_2d_pair_once(dst + h * BLOCK_BYTES, map, (kb + h) * BK, y, bar);
+          else if (for_x) tma_load_2d_pair(dst + h * BLOCK_BYTES, map, (kb + h) * BK, y, bar);
+        }
       }
     }
     // The commits that release the last stages arrive on both blocks' barriers: neither leaves before they have.
@@ -197,16 +203,19 @@ grouped_tc5_kernel(const __grid_constant__ Maps maps, GroupedParams p) {
         ok = mbar_wait(&acc_empty[buf], ((j >> 1) & 1) ^ 1, p.err);   // the epilogues have drained this accumulator
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t tmem_d = tmem_base + buf * MAX_ROWS;
-        for (int kb = 0; kb < kblocks && ok; ++kb, ++it) {
+        for (int kb = 0; kb < kblocks && ok; kb += IN_STAGE, ++it) {
           const int s = it % STAGES;
           ok = mbar_wait(&full_bar[s], (it / STAGES) & 1, p.err);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t a_addr = smem_u32(stages + (size_t)s * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
+          const int blocks = min(IN_STAGE, kblocks - kb);
+          for (int h = 0; h < blocks; ++h) {
+            const uint32_t a_addr = smem_u32(stages + (size_t)s * STAGE_BYTES + h * BLOCK_BYTES);
+            const uint32_t b_addr = a_addr + A_BYTES;
 #pragma unroll
-          for (int k = 0; k < BK / UMMA_K; ++k)
-            umma_pair(tmem_d, make_desc(a_addr + k * UMMA_K * 2), make_desc(b_addr + k * UMMA_K * 2), idesc,
-                      (kb > 0 || k > 0) ? 1u : 0u);
+            for (int k = 0; k < BK / UMMA_K; ++k)
+              umma_pair(tmem_d, make_desc(a_addr + k * UMMA_K * 2), make_desc(b_addr + k * UMMA_K * 2), idesc,
+                        (kb > 0 || h > 0 || k > 0) ? 1u : 0u);
+          }
           umma_commit_pair(&empty_bar[s]);   // the stage is free in both blocks once these MMAs have read it
         }
         umma_commit_pair(&acc_full[buf]);    // the accumulator is complete in both blocks
