@@ -15,7 +15,7 @@
 // two or four columns); here sixteen columns share each fragment, and the 300 products of a chunk and computing warp bind.
 // Delta rule, 1,100 + 37 + 911 tokens, 16 heads of 128 x 128: 264 -> 157 us (the longest request's 69 chunks, 2.3 us each), with
 // two warps to sixteen columns 112;
-// time mixing, 2,048 tokens in segments, both passes: 118 -> 95 us.  Two terms a factor took 91 and 77, but read-outs and
+// time mixing, 2,048 tokens in segments, both passes: 118 -> 91 us.  Two terms a factor took 91 and 77, but read-outs and
 // state were 5e-6 off 64 bits on given inputs; the multiply-adds are 0.5e-7 to 5e-7 off and this 0.6 to 1.4 times that.
 #pragma once
 #include "chunk_scan.cuh"

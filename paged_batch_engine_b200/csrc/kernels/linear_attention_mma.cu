@@ -18,7 +18,7 @@
 // state in registers; o's weights pass from score accumulators to operands in registers.  Two blocks a multiprocessor
 // (99 KB at 128 x 64) fill each other's barriers and copies.  Work items cut long portions as in
 // linear_attention.cu: a pass without outputs leaves each item's own contribution and decay product.
-// 2,048 tokens, 64 heads of 128 x 64 over 8 groups (both passes): 148 us against 823 of the recurrence token by token.  Two
+// 2,048 tokens, 64 heads of 128 x 64 over 8 groups (both passes): 144 us against 823 of the recurrence token by token.  Two
 // terms a factor, the weighted v in shared memory, took 104, but outputs and state were 10 to 30 times further off 64 bits
 // than the recurrence's (1 to 3e-7); now they are 0.6 to 1.2 times.
 #include "common.cuh"
