@@ -1086,17 +1086,24 @@ def _mma_available() -> bool:
 
 
 F32_TILE_ROWS = 128     # packed rows per block of the float32 tensor-core kernel, which takes the steps
-F32_SMALL_ROWS = 64     # that have a request of more packed rows than this
+F32_SMALL_ROWS = 64     # that have a request of more packed rows than this, which see
+F32_FEW_KEYS = 32       # more keys than this (twice as many in a step of few rows)
 
 
 def attention_f32_tiles(q_len, seq_len, group_size: int, window, split_keys: int) -> int:
     """Blocks a key/value head that ``attention_f32_tc5.cu`` takes a step in (the requests' lengths as numpy arrays): the row
-    tiles of requests of many rows and the key splits of the others; 0 where it does not take the step."""
+    tiles of requests of many rows and the key splits of the others; 0 where it does not take the step.
+
+    Few keys are the multiply-adds': one request of 30 rows 13 us against 17 there, of 40 19 against 17 (12 heads of 128
+    over 2; 28 over 4 the same, 14 of 64 over 2 9 against 12 and 14 against 12), four of 60 22 against 17.  Steps of 64
+    rows and less wait for the host, which this form costs 3 us a layer more (60 rows: the layer 680 -> 700 us)."""
     packed = q_len * group_size
     wide = packed > F32_SMALL_ROWS
     if not wide.any():
         return 0
     low = (seq_len - q_len - window + 1).clip(0) if window else 0 * seq_len
+    if int((seq_len - low)[wide].max()) <= F32_FEW_KEYS * (1 if int(q_len.sum()) > 64 else 2):
+        return 0
     splits = (seq_len + split_keys - 1) // split_keys - low // split_keys
     tiles = (packed + F32_TILE_ROWS - 1) // F32_TILE_ROWS
     return int(tiles[wide].sum() + splits[~wide & (packed > 0)].sum())

@@ -90,4 +90,6 @@ def test_blocks_are_those_of_the_work_list():
         wide = q_len * G > o.F32_SMALL_ROWS
         want = sum(-(-int(n) * G // o.F32_TILE_ROWS) if w else int(work[work[:, 0] == r][0, 3])
                    for r, (n, w) in enumerate(zip(q_len, wide)))
-        assert o.attention_f32_tiles(q_len, seq_len, G, window, split) == (want if wide.any() else 0)
+        seen = np.minimum(seq_len, q_len + window - 1) if window else seq_len
+        takes = wide.any() and seen[wide].max() > o.F32_FEW_KEYS * (1 if q_len.sum() > 64 else 2)
+        assert o.attention_f32_tiles(q_len, seq_len, G, window, split) == (want if takes else 0)
