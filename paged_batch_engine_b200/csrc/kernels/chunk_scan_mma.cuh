@@ -8,13 +8,14 @@
 // compute, sixteen columns each, whose [16, D] piece of S^T (or their share of its key channels) stays in float32
 // accumulators and turns into an operand in registers; the other warps fetch the next chunk's record and values, split
 // them and lay them down in the other of two buffers, one barrier a chunk.  Per chunk a computing warp has
-//   [W | QG]: S^T (as it lies) times the records' vectors, two tiles of eight tokens each (warps that share columns add
-//   their parts through shared memory);
+//   [W | QG]: S^T (as it lies) times the records' vectors, two tiles of eight tokens each; with corrected writes a quarter of the
+//   key channels at a time, summed from zero, the quarters q added as (q0 + q1) + (q2 + q3) by one warp or, through shared
+//   memory, by those that share columns: a request has the same bits whatever its neighbours let the blocks be cut into;
 //   u = U - S^T W;   o = S^T QG + u MQ;   S^T <- decays S^T + u KD.
 // What binds the scan of chunk_scan.cuh is the shared-memory pipe (every half warp reads the whole record for its
 // two or four columns); here sixteen columns share each fragment, and the 300 products of a chunk and computing warp bind.
 // Delta rule, 1,100 + 37 + 911 tokens, 16 heads of 128 x 128: 264 -> 157 us (the longest request's 69 chunks, 2.3 us each), with
-// two warps to sixteen columns 112;
+// two warps to sixteen columns 114;
 // time mixing, 2,048 tokens in segments, both passes: 118 -> 91 us.  Two terms a factor took 91 and 77, but read-outs and
 // state were 5e-6 off 64 bits on given inputs; the multiply-adds are 0.5e-7 to 5e-7 off and this 0.6 to 1.4 times that.
 #pragma once
@@ -72,7 +73,8 @@ __device__ __forceinline__ void products(float (&big)[2][4], float (&small)[2][4
 // DS: computing warps that share sixteen columns, DP / DS of their key channels each
 template <int DP, bool CORRECT, bool OWN, typename TU, int DS>
 __global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) scan_chunks_mma_kernel(ChunkScanParams<TU> p) {
-  static_assert(DS == 1 || ((DS == 2 || DS == 4) && !OWN), "warps of sixteen columns");
+  static_assert(DS == 1 || ((DS == 2 || DS == 4) && CORRECT), "warps of sixteen columns");
+  static_assert(!(CORRECT && OWN), "what a segment adds of its own is made of given rows: it fetches no W");
   constexpr int COLS = block_cols<DS>();
   constexpr int DW = DP / DS;                            // key channels of a warp
   constexpr int STR = row_elems<DP>();
@@ -86,7 +88,8 @@ __global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) sc
   constexpr int UPER = CH * COLS / FT;
   constexpr bool U_EXACT = sizeof(TU) == 2 && !CORRECT;  // u is a bfloat16 number: its other terms are zero
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  __shared__ float shares[DS > 1 ? 4 : 1][16][33];       // of the products with the state, by warp
+  constexpr int QUARTERS = CORRECT ? 4 / DS : 1;         // a warp's parts of the products with the state (one: left to the tensor cores)
+  __shared__ float shares[DS > 1 ? 4 : 1][16][33];       // their sums, by warp
   pdl_launch_dependents();
   pdl_wait();
   const int h = blockIdx.y;
@@ -200,36 +203,48 @@ __global__ void __launch_bounds__(128 + fetch_threads<DS>(), CORRECT ? 1 : 2) sc
   for (int c = 0; c < nc; ++c) {
     const int buf = c & 1;
     // S^T times the records' vectors
-    float w[2][4], q[2][4], wc[2][4], qc[2][4];
+    float w[2][4], q[2][4], wc[2][4], qc[2][4], sums[16], pair[16];
 #pragma unroll
-    for (int t = 0; t < 2; ++t)
+    for (int part = 0; part < QUARTERS; ++part) {
 #pragma unroll
-      for (int k = 0; k < 4; ++k) w[t][k] = q[t][k] = wc[t][k] = qc[t][k] = 0.f;
-    if (CORRECT || !OWN) {
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
-      for (int kk = 0; kk < DW / 16; ++kk) {
-        unsigned a[TERMS][4];
-        as_operand(S[2 * kk], S[2 * kk + 1], a);
-        const int at = krow * STR + d0 + kk * 16 + kcol;
-        if (CORRECT) products<false>(w, wc, a, matrix(buf, 2, 0) + at, CH * STR);
-        if (!OWN) products<false>(q, qc, a, matrix(buf, 0, 0) + at, CH * STR);
+        for (int k = 0; k < 4; ++k) w[t][k] = q[t][k] = wc[t][k] = qc[t][k] = 0.f;
+      if (CORRECT || !OWN) {
+#pragma unroll
+        for (int kk = part * (DW / 16 / QUARTERS); kk < (part + 1) * (DW / 16 / QUARTERS); ++kk) {
+          unsigned a[TERMS][4];
+          as_operand(S[2 * kk], S[2 * kk + 1], a);
+          const int at = krow * STR + d0 + kk * 16 + kcol;
+          if (CORRECT) products<false>(w, wc, a, matrix(buf, 2, 0) + at, CH * STR);
+          if (!OWN) products<false>(q, qc, a, matrix(buf, 0, 0) + at, CH * STR);
+        }
+      }
+      if constexpr (CORRECT) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float of = k < 8 ? w[k >> 2][k & 3] + wc[k >> 2][k & 3] : q[k / 4 - 2][k & 3] + qc[k / 4 - 2][k & 3];
+          pair[k] = part & 1 ? pair[k] + of : of;
+          if (part & 1 || QUARTERS == 1) sums[k] = part > 1 ? sums[k] + pair[k] : pair[k];
+        }
       }
     }
-    if constexpr (DS > 1) {                              // of all its warps, added in their order (the block's barrier parts two chunks' uses)
+    if constexpr (DS > 1) {                              // (the block's barrier parts two chunks' uses)
+#pragma unroll
+      for (int k = 0; k < 16; ++k) shares[warp][k][lane] = sums[k];
+      asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * DS) : "memory");
+      const auto of = &shares[group * DS];
+#pragma unroll
+      for (int k = 0; k < 16; ++k)
+        sums[k] = DS == 2 ? of[0][k][lane] + of[1][k][lane] : (of[0][k][lane] + of[1][k][lane]) + (of[DS - 2][k][lane] + of[DS - 1][k][lane]);
+    }
+    if constexpr (CORRECT) {
 #pragma unroll
       for (int k = 0; k < 8; ++k) {
-        shares[warp][k][lane] = w[k >> 2][k & 3] + wc[k >> 2][k & 3];
-        shares[warp][8 + k][lane] = q[k >> 2][k & 3] + qc[k >> 2][k & 3];
-        w[k >> 2][k & 3] = q[k >> 2][k & 3] = wc[k >> 2][k & 3] = qc[k >> 2][k & 3] = 0.f;
+        w[k >> 2][k & 3] = sums[k];
+        q[k >> 2][k & 3] = sums[8 + k];
+        wc[k >> 2][k & 3] = qc[k >> 2][k & 3] = 0.f;
       }
-      asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "n"(32 * DS) : "memory");
-#pragma unroll
-      for (int i = 0; i < DS; ++i)
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          w[k >> 2][k & 3] += shares[group * DS + i][k][lane];
-          q[k >> 2][k & 3] += shares[group * DS + i][8 + k][lane];
-        }
     }
     // u: token 8 t + q2 (+ 1) of columns g8 (+ 8)
     const float* U = values(buf) + group * 16 + g8;

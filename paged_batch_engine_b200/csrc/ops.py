@@ -2568,7 +2568,7 @@ def delta_scan(qk: torch.Tensor, kq: torch.Tensor, v: torch.Tensor, beta: torch.
     ``slots[r]`` and left updated.  ``chunked``: sixteen tokens at a time
     (prompt portions: two launches, v is overwritten), else one by one.  ``matrix``: the chunks' scan on the tensor
     cores, every float32 factor as three bfloat16 terms (bfloat16 runs); ``longest``: the most rows a request brings, which
-    tells how its blocks are cut (0: not known).  Returns o, float32 [T, H * E]."""
+    tells how its blocks are cut (0: not known; the result's bits do not hang on it).  Returns o, float32 [T, H * E]."""
     _need_cuda(qk, kq, v, beta, decay, state, q_start, q_len, slots)
     _need_contiguous(qk, kq, v, beta, decay, state)
     T, G, _, D = qk.shape

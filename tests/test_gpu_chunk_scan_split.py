@@ -65,3 +65,19 @@ def test_as_close_to_64_bits(H, E):
     split, one, fma = off(_run(case, lens, 400)), off(_run(case, lens, 0)), off(_run(case, lens, 0, matrix=False))
     assert all(a <= 1.4 * max(b, c) for a, b, c in zip(split, one, fma)), (split, one, fma)
     print(split, one, fma)
+
+
+@pytest.mark.parametrize("D,E,H,lens", [(128, 128, 16, [144, 90, 130, 17]), (128, 128, 16, [33, 144]), (64, 64, 32, [95, 96, 80, 2, 90]),
+                                        (100, 72, 16, [70, 64, 66])])
+def test_a_request_alone_and_beside_others(D, E, H, lens):
+    """One, two or four warps to sixteen columns, as its neighbours in the step let the blocks be cut: a request has the same bits."""
+    qk, kq, v, beta, decay, start = case = _case(D, E, H, lens, seed=2)
+    together, t0 = _run(case, lens, max(lens)), 0
+    for i, n in enumerate(lens):
+        slot, rows = len(lens) - 1 - i, slice(t0, t0 + n)
+        own = (qk[rows].contiguous(), kq[rows].contiguous(), v[rows].contiguous(), beta[rows].contiguous(), decay[rows].contiguous(),
+               start[slot:slot + 1].contiguous())
+        alone = _run(own, [n], n)
+        assert torch.equal(alone[0], together[0][rows])
+        assert torch.equal(alone[1][0], together[1][slot])
+        t0 += n
