@@ -377,7 +377,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_f32_tc5_kernel(AttnPara
     bool ok = true;
     // in the order in which the buffers come free: K0 V0 K1 | K2 V1 | K3 V2 | ...
     const int items = 2 * n_tiles;
-    for (int it = 0; it < items && ok; ++it) {
+    for (int it = 0; it < items; ++it) {                   // to its end also where a wait has run out: the four warps meet in it
       auto tile_of = [&](int i, bool& keys) {              // the last is a value tile
         keys = i == 0 || i == 2 || (i > 2 && (i & 1) && i != items - 1);
         return i < 2 ? 0 : i == items - 1 ? n_tiles - 1 : keys ? (i + 1) / 2 : i / 2 - 1;

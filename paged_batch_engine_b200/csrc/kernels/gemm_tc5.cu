@@ -380,7 +380,7 @@ gemm_tc5_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_con
       const int tile_m = t % tiles_m, tile_n = t / tiles_m;
       const int buf = j & 1;
       const int row = tile_m * 256 + (int)rank * 128 + quarter * 32 + lane;
-      if (!mbar_wait(&acc_full[buf], (j >> 1) & 1, p.err)) break;      // flagged; the roles run to their end
+      if (!mbar_wait_warp(&acc_full[buf], (j >> 1) & 1, p.err)) break;      // flagged; the roles run to their end
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint32_t lane_addr = tmem_base + ((uint32_t)(quarter * 32) << 16) + buf * BN;
       if (p.swiglu) {

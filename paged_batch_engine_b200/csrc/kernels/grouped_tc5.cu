@@ -176,8 +176,7 @@ grouped_tc5_kernel(const __grid_constant__ Maps maps, GroupedParams p) {
       const uint32_t bytes = 2 * (A_BYTES + half * BK * 2);                  // both blocks' copies
       for (int kb = 0; kb < kblocks; kb += IN_STAGE, ++it) {
         const int s = it % STAGES, blocks = min(IN_STAGE, kblocks - kb);
-        ok = mbar_wait(&empty_bar[s], ((it / STAGES) & 1) ^ 1, p.err);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = mbar_wait_warp(&empty_bar[s], ((it / STAGES) & 1) ^ 1, p.err);
         if (!ok) break;
         if (leader && lane == 0) mbar_expect_tx(&full_bar[s], blocks * bytes);
         __syncwarp();

@@ -217,7 +217,7 @@ sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
     for (int t = blockIdx.x; t < items && ok; t += gridDim.x)
       for (int kb = first_block(t); kb < last_block(t); ++kb, ++b) {
         const int st = b % W_STAGES;
-        ok = mbar_wait(&bar.w_full[st], (b / W_STAGES) & 1, p.err);
+        ok = mbar_wait_warp(&bar.w_full[st], (b / W_STAGES) & 1, p.err);
         if (!ok) break;
         uint32_t w[TERMS][BK / 2];
 #pragma unroll
@@ -238,7 +238,7 @@ sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         if (lane == 0) mbar_arrive(&bar.w_empty[st]);
         const int h = slot_h(b);
         // the term h of two blocks before is given back with that block's accumulator
-        ok = mbar_wait(&bar.l_empty, (b & 1) ^ 1, p.err) && mbar_wait(&bar.acc_full[b & 1], ((b >> 1) & 1) ^ 1, p.err);
+        ok = mbar_wait_warp(&bar.l_empty, (b & 1) ^ 1, p.err) && mbar_wait_warp(&bar.acc_full[b & 1], ((b >> 1) & 1) ^ 1, p.err);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem_st32_nowait(a_addr + slot_l() * (BK / 2), w[2]);
@@ -247,7 +247,7 @@ sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
         if (lane == 0) mbar_arrive(&bar.a_lh_full);
-        ok = mbar_wait(&bar.m_empty, (b & 1) ^ 1, p.err);
+        ok = mbar_wait_warp(&bar.m_empty, (b & 1) ^ 1, p.err);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem_st32_nowait(a_addr + slot_m() * (BK / 2), w[1]);
@@ -280,7 +280,7 @@ sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constan
         const int k1 = min(k0 + slice, end);
         for (int kb = k0; kb < k1; ++kb, ++it) {
           const int buf = it & 1;
-          ok = mbar_wait(&bar.acc_full[buf], (it >> 1) & 1, p.err);
+          ok = mbar_wait_warp(&bar.acc_full[buf], (it >> 1) & 1, p.err);
           if (!ok) break;                             // flagged; the roles run to their end
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll

@@ -44,6 +44,12 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   if (err) atomicExch(err, 1);
   return false;
 }
+// The same by a whole warp, whose lanes agree: a role that leaves its loop when a wait runs out, with something in the loop that all
+// lanes take part in, waits so.  (Each lane has its own limit, and the barrier may complete between two lanes'.)  Nothing that
+// several warps take part in may stand in a loop that is left so.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err)) != 0;
+}
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"

@@ -50,3 +50,35 @@ def test_loads_stay_behind_the_wait_for_the_kernel_before():
             broken += [f"{file}: {name}: ld.global.nc" for _ in re.findall(r"ld\.global\.nc", body)]
     assert waiting > 50                      # the sources were found and understood
     assert not broken, broken
+
+
+def _loops(text):
+    """(line, head, body) of every for and while loop; the body of a loop without braces is its statement."""
+    for found in re.finditer(r"\b(?:for|while)\s*\(", text):
+        closed = _closing(text, found.end() - 1)
+        at = closed + 1 + len(text[closed + 1:]) - len(text[closed + 1:].lstrip())
+        end = _closing(text, at, "{}") if text[at] == "{" else text.index(";", at)
+        yield text.count("\n", 0, found.start()) + 1, text[found.start():closed + 1], text[at:end + 1]
+
+
+def test_no_warp_waits_for_one_that_gave_up():
+    """A bounded wait that runs out in one thread may be completed in the next: a loop that is left after such a wait has nothing in it
+    that several warps take part in, and what a warp's lanes take part in only where the lanes agree on the wait."""
+    found, broken = 0, []
+    for file in sorted(os.listdir(KERNELS)):
+        if not file.endswith((".cu", ".cuh")):
+            continue
+        with open(os.path.join(KERNELS, file)) as f:
+            text = re.sub(r"//[^\n]*", "", f.read())
+        for line, head, body in _loops(text):
+            waits = re.findall(r"\bmbar_wait\w*", body)
+            left = re.search(r"\bok\b", head) or re.search(r"if \(!(?:ok|mbar_wait\w*\([^;]*)\)\s*(?:break|return)", body)
+            if not waits or not left:
+                continue
+            found += 1
+            if re.search(r"bar\.sync|__syncthreads|cluster_sync|barrier\.cluster", body):
+                broken.append(f"{file}:{line}: a barrier of several warps")
+            if re.search(r"__syncwarp|\w+_sync\(|\btmem_(?:ld|st)", body) and "mbar_wait" in waits:
+                broken.append(f"{file}:{line}: lanes that do not agree")
+    assert found > 10
+    assert not broken, broken
