@@ -10,13 +10,17 @@
 // candidates; everything else goes through the host with the whole logits matrix.
 //
 // Weights are summed as 64-bit fixed point (2^-40 units), so sums are exact,
-// order-independent and the result is the same whatever else is in the batch.  Every "first
-// element of the ordered list whose cumulative weight reaches a target" is found in two steps:
-// one pass over the row sums count and weight of 1,024 bins by distance from the maximum, a
-// prefix sum names the element's bin, and that bin's elements are gathered, sorted and scanned
-// (select_quick).  Rows whose bin is too crowded for that (thousands of equal logits) take a
-// radix descent over the order-preserving integer image of the logit, four bits a pass, with
-// per-thread histograms in registers (select_by_weight); both give the same element.
+// order-independent and the result is the same whatever else is in the batch.  There are three ways
+// to the token, and all give the same one:
+//  * top_k up to TOP_MAX: the k-th largest of the threads' own maxima bounds the first k elements from
+//    below; what is above it is gathered, sorted and scanned (list_top, sample_top);
+//  * else every "first element of the ordered list whose cumulative weight reaches a target" is found
+//    in two steps: one pass over the row sums weight (and count, where top_k asks for it) of 1,024 bins
+//    by distance from the maximum, a prefix sum names the element's bin, and that bin's elements are
+//    gathered, sorted and scanned (select_quick);
+//  * rows with too many elements for either list (thousands of equal logits) take a radix descent over
+//    the order-preserving integer image of the logit, four bits a pass, with per-thread histograms in
+//    registers (select_by_weight).
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -478,9 +482,10 @@ __device__ void fill_bins(const float* slice, int n, float mx, float temp, float
   sync_row<CL>();
 }
 
-// An element into the list of the row's block 0; every block learns if that is full.
+// An element into the list of the row's block 0; every block learns if that is full, and pushes nothing more.
 template <int CL>
 __device__ __forceinline__ void push(Quick& q, uint32_t key, int token) {
+  if (*(volatile int*)&q.overflow) return;
   Quick* q0 = of_block<CL>(&q, 0);
   const int pos = atomicAdd(&q0->n_list, 1);
   if (pos < LIST_CAP) {
@@ -529,13 +534,17 @@ __device__ void sort_list(Quick& q, int n, int n2) {
 // The row's first k elements without bins (k up to TOP_MAX): the k largest of a block's threads' own maxima are k elements, so no
 // element below the smallest of these is among the first k, and only the threads whose maximum is not below it have to be looked
 // through again.  The bound is found to TOP_BITS of the key, by halving, and what is not below it goes to block 0's list.
+// Elements 28 temperatures and more below the maximum weigh nothing (exp(-28) < 2^-40) and are never the token: the bound stays above
+// them, or the masked ones of a row with fewer than k others in k threads would all go to the list, one after the other, and it would
+// run over (64 rows of 152,064, all but 20 logits masked, k = 50: 1,866 us without this, as by the radix descent; all but 200
+// neighbours masked 133 us).
 // What is left is one pass over the row, which memory bounds; bins take four shared-memory atomics a logit, and their elements a pass
 // for each of the three choices.  k = 50, top_p 0.9, launch and all: 64 rows of 152,064 90 -> 27 us, of 32,000 43 -> 19; one row
 // of 152,064 52 -> 25.  The line: with k = 128 86 -> 31 and 43 -> 41 us (64 rows of 152,064, one of 32,000), with 512 one row of 32,000
 // was slower, 35 -> 49 (top_p 1).
 constexpr int TOP_MAX = 128, TOP_BITS = 20;
 template <int CL>
-__device__ void list_top(const float* slice, int lo, int n_slice, int k, float own, Quick& q) {
+__device__ void list_top(const float* slice, int lo, int n_slice, int k, float own, float mx, float temp, Quick& q) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t key = order_key(own);
   uint32_t bound = 0;
@@ -544,6 +553,8 @@ __device__ void list_top(const float* slice, int lo, int n_slice, int k, float o
     const uint32_t higher = bound | (1u << bit);
     if (__syncthreads_count(key >= higher) >= k) bound = higher;
   }
+  const float floor = mx - 28.f * temp;                  // no number where both are infinite: nothing is left out then
+  if (floor == floor) bound = max(bound, order_key(clean(floor)));
   if (key >= bound) q.found[atomicAdd(&q.n_found, 1)] = tid;
   __syncthreads();
   const int n = q.n_found;
@@ -578,7 +589,7 @@ __device__ int sample_top(int k, int amax, float mx, float temp, float p_in, flo
   for (int i = n + tid; i < n2; i += THREADS) q.list[i] = 0;     // below every real key
   __syncthreads();
   sort_list(q, n, n2);
-  const u64 w = tid < k ? weight_of(key_value((uint32_t)(q.list[tid] >> 32)), mx, temp, false) : 0;
+  const u64 w = tid < min(k, n) ? weight_of(key_value((uint32_t)(q.list[tid] >> 32)), mx, temp, false) : 0;
   u64 kept;
   const u64 upto = block_exclusive_scan(w, q, &kept) + w;
   if (kept == 0) return amax;
@@ -608,11 +619,11 @@ __device__ int sample_top(int k, int amax, float mx, float temp, float p_in, flo
 // inclusive cumulative weight (count in count mode) reaches `target`; the domain's last element
 // if there is none: what select_by_weight returns.  In count mode *weight_cum gets the cumulative
 // weight at that element.  false (the same in every block of the row): the element's bin is too
-// crowded for the list.  Every block gathers from its slice (first token `lo`) into block 0's
+// crowded for the list (`counts`: fill_bins made counts, which tell at once).  Every block gathers from its slice (first token `lo`) into block 0's
 // list; block 0 sorts, scans and hands the result to all.
 template <int CL>
 __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, float temp, float scale,
-                             bool count_mode, u64 target, const Limit& lim, Quick& q, Cut* out, int* out_bin,
+                             bool counts, bool count_mode, u64 target, const Limit& lim, Quick& q, Cut* out, int* out_bin,
                              u64* weight_cum) {
   const int tid = threadIdx.x;
   const int rank = block_rank<CL>();
@@ -630,6 +641,7 @@ __device__ bool select_quick(const float* slice, int lo, int n_slice, float mx, 
   }
   __syncthreads();
   const int bin = q.chosen;
+  if (counts && q.cnt[bin] > (unsigned)LIST_CAP) return false;           // where they were not made, the list tells
   // the bin's elements inside the domain (block 0's counter is zero: it is reset after every use,
   // a row barrier before the next)
   for_each_logit(slice, n_slice, [&](float x, int i) {
@@ -778,7 +790,7 @@ sample_kernel(const float* logits, size_t ld, int V,
   const float temp = fmaxf(t_in, 1e-6f);
   const float u = fminf(fmaxf(uniform[r], 0.f), 0.99999994f);
   if (top) {
-    list_top<CL>(slice, lo, n_slice, k_in, own, q);
+    list_top<CL>(slice, lo, n_slice, k_in, own, mx, temp, q);
     sync_row<CL>();
     if (!q.overflow) {             // else thousands of equal logits
       if (rank != 0) return;
@@ -804,7 +816,7 @@ sample_kernel(const float* logits, size_t ld, int V,
     int bin = 0;
     if (counts) {
       u64 wc = 0;
-      ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, true, (u64)k_in, lim, q, &c, &bin, &wc);
+      ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, true, true, (u64)k_in, lim, q, &c, &bin, &wc);
       if (ok) {
         lim.on = true; lim.key = c.key; lim.token = c.token; lim.bin = bin;
         kept = wc;
@@ -817,7 +829,7 @@ sample_kernel(const float* logits, size_t ld, int V,
     if (ok && p_in < 1.f) {
       u64 tp = (u64)((double)p_in * (double)kept);
       if ((double)tp < (double)p_in * (double)kept) ++tp;   // ceil: cumulative >= top_p * total
-      ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, false, tp, lim, q, &c, &bin, nullptr);
+      ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, counts, false, tp, lim, q, &c, &bin, nullptr);
       if (ok) {
         lim.on = true; lim.key = c.key; lim.token = c.token; lim.bin = bin;
         kept = c.cum;
@@ -826,7 +838,7 @@ sample_kernel(const float* logits, size_t ld, int V,
     if (ok) {
       u64 draw = (u64)((double)u * (double)kept);
       if ((double)draw < (double)u * (double)kept) ++draw;
-      ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, false, draw, lim, q, &c, &bin, nullptr);
+      ok = select_quick<CL>(slice, lo, n_slice, mx, temp, scale, counts, false, draw, lim, q, &c, &bin, nullptr);
       if (ok) {
         if (writer) out[r] = c.token >= 0 ? c.token : amax;
         return;

@@ -24,7 +24,7 @@ def _tokens(logits, k, p, t, u):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("V,rows,stride", [(5, 3, 5), (1000, 4, 1000), (1027, 3, 1028), (8191, 5, 8191), (8192, 20, 8192), (9001, 40, 9003),
+@pytest.mark.parametrize("V,rows,stride", [(5, 3, 5), (200, 3, 203), (1000, 4, 1000), (1027, 3, 1028), (8191, 5, 8191), (8192, 20, 8192), (9001, 40, 9003),
                                            (32000, 64, 32000), (40001, 100, 40001), (152064, 64, 152064), (151936, 150, 151936)])
 @pytest.mark.parametrize("kind", ["normal", "coarse", "equal", "masked"])
 def test_three_ways(V, rows, stride, kind):
@@ -41,10 +41,57 @@ def test_three_ways(V, rows, stride, kind):
         x[-1, V // 2] = 1e9
     x = x[:, :V]
     u = torch.rand(rows, device=DEV, generator=g)
-    for k in {1, 2, 50, 511, 512, 513, V - 1, 0} - ({0} if V > 100000 and kind == "equal" else set()):
+    for k in {1, 2, 50, 127, 128, 129, 511, 512, 513, V - 1, 0} - ({0} if V > 100000 and kind == "equal" else set()):
         for p, t in ((1.0, 0.8), (0.9, 0.8), (0.0, 1.5), (0.5, 1e-7)):
             top, bins, radix = _tokens(x, k, p, t, u)
             assert top == bins == radix, (k, p, t)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,rows", [(200, 3), (9001, 5), (32000, 2), (152064, 64)])
+@pytest.mark.parametrize("low", [float("-inf"), -1e9, torch.finfo(torch.float32).min])
+@pytest.mark.parametrize("finite,neighbours", [(1, False), (20, False), (127, False), (128, True), (150, True)])
+def test_rows_with_few_logits(V, rows, low, finite, neighbours):
+    """All but a few logits masked, by an infinity, a large number or the type's lowest."""
+    g = torch.Generator(device=DEV).manual_seed(V + finite)
+    x = torch.full((rows, V), low, device=DEV)
+    at = torch.arange(finite, device=DEV)
+    at = at + (V - finite) // 3 if neighbours else at * (V // finite)
+    x[:, at] = torch.empty(rows, finite, device=DEV).normal_(0, 2.5, generator=g)
+    u = torch.rand(rows, device=DEV, generator=g)
+    for k in {1, 50, 128, V - 1}:
+        for p, t in ((1.0, 0.8), (0.9, 0.8), (1.0, 100.0)):
+            top, bins, radix = _tokens(x, k, p, t, u)
+            assert top == bins == radix, (k, p, t)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,rows", [(32000, 1), (152064, 1), (152064, 64)])
+@pytest.mark.parametrize("finite,neighbours", [(20, False), (200, True)])
+def test_masked_rows_take_no_longer(V, rows, finite, neighbours):
+    """17 to 19 us either way; with the masked logits in the list it was 100 to 1,900, hence a bound of three times."""
+    from paged_batch_engine_b200.csrc import ops
+    full = lambda x, dt: torch.full((rows,), x, dtype=dt, device=DEV)
+    args = full(0.8, torch.float32), full(50, torch.int32), full(0.9, torch.float32), full(0.5, torch.float32)
+
+    def time(x):
+        best = float("inf")
+        for _ in range(5):
+            start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            start.record()
+            for _ in range(10):
+                ops.sample(x, *args)
+            end.record()
+            end.synchronize()
+            best = min(best, start.elapsed_time(end))
+        return best
+    x = torch.randn(rows, V, device=DEV)
+    whole = time(x)
+    keep = torch.arange(finite, device=DEV)
+    keep = keep + V // 3 if neighbours else keep * (V // finite)
+    masked = torch.full_like(x, float("-inf"))
+    masked[:, keep] = x[:, keep]
+    assert time(masked) <= 3 * whole
 
 
 def test_draws_of_many_rows():
