@@ -98,3 +98,21 @@ def test_draws_of_many_rows():
     seeds = [0, 1, 0xC0FFEE, 2 ** 63 + 5, 2 ** 64 - 1, 2 ** 64 + 7, -3]
     counters = [0, 5, 2 ** 20, 1, 3, 2, 7]
     assert request_sample_uniforms(seeds, counters).tolist() == [request_sample_uniform(s, c) for s, c in zip(seeds, counters)]
+    # pairs as zip makes them: what is left over on either side is not looked at
+    want = [request_sample_uniform(s, c) for s, c in zip(seeds, counters)]
+    assert request_sample_uniforms(seeds, counters + [9, 10]).tolist() == want
+    assert request_sample_uniforms(seeds[:3], iter(counters)).tolist() == want[:3]
+    assert request_sample_uniforms(seeds, counters[:1]).tolist() == want[:1]
+    assert request_sample_uniforms([], counters).tolist() == []
+
+
+@pytest.mark.gpu
+def test_more_counters_than_rows():
+    from paged_batch_engine_b200.sampling import Sampler, SamplingParams
+    params = [SamplingParams(temperature=0.8, top_k=20, seed=i) for i in range(3)]
+    logits, tokens = torch.randn(3, 1000, device=DEV), []
+    for counters in ([4, 5, 6], [4, 5, 6, 7, 8]):
+        _, host, event = Sampler(torch.device(DEV)).sample_async(logits, params, counters)
+        event.synchronize()
+        tokens.append(host[:3].tolist())
+    assert tokens[0] == tokens[1]
