@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 
 #include "attention_simple.cu"
+#include "opt_in.cuh"
 #include "tcgen05.cuh"
 
 using namespace pbe::tc5;
@@ -475,12 +476,8 @@ PBE_EXPORT int pbe_attn_f32(const AttnParams* params, int num_work, int num_tile
   // rows that do not start on a 16-byte boundary are the multiply-adds' too
   if (((uintptr_t)p.q | (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (uintptr_t)p.out | (uintptr_t)p.part_o) & 15)
     return launch_simple(params, num_work, PBE_F32, Rest{nullptr}, stream);
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(attention_f32_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(SMEM_BYTES, attention_f32_tc5_kernel)) return (int)e;
   launch_k(attention_f32_tc5_kernel, num_tiles * p.num_kv_heads, NTHREADS, SMEM_BYTES, stream, p, F32Extra{num_tiles, R, flags}, err);
   const int rc = launch_status();
   return rc != 0 ? rc : launch_simple(params, num_work, PBE_F32, Rest{flags}, stream);

@@ -26,6 +26,7 @@
 #include <cstring>
 
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "kv_tensor_map.cuh"
 #include "pdl.cuh"
@@ -1286,11 +1287,8 @@ PBE_EXPORT int pbe_attn_mma(const AttnParams* params, int num_work, int dtype, c
       p.split_keys % BN_KEYS != 0)
     return (int)cudaErrorInvalidValue;
   const size_t smem_rows = sizeof(bf16) * (size_t)(BM + 4 * BN_ROWS) * LDS;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(attn_mma_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_rows);
-    opted = true;
-  }
+  static OptIn opt_in;
+  opt_in(smem_rows, attn_mma_kernel<0>);
   dim3 grid(num_work, p.num_kv_heads);
   p.kinds &= ~16;            // the launcher's own bit
   const int kinds = (p.kinds & 3) == 0 ? (p.kinds | 3) : p.kinds;
@@ -1313,20 +1311,18 @@ PBE_EXPORT int pbe_attn_mma(const AttnParams* params, int num_work, int dtype, c
   if ((kinds & 1) && (kinds & 4)) {
     // few requests: four warps share every key tile
     const size_t smem_keys = sizeof(bf16) * (size_t)(16 + 4 * BN_KEYS) * LDS;
-    static bool opted_keys = false;
-    if (!opted_keys) {
-      cudaFuncSetAttribute(attn_mma_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_keys);
-      opted_keys = true;
-    }
+    static OptIn opt_in_keys;
+    opt_in_keys(smem_keys, attn_mma_kernel<1>);
     CUtensorMap map_k = {}, map_v = {};
     AttnParams pk = p;
     tiles_by_page(pk, &map_k, &map_v);
     launch_k(attn_mma_kernel<1>, grid, NTHREADS, smem_keys, stream, pk, AttnFusedParams{}, map_k, map_v);
   } else if (kinds & 1) {
     const size_t smem_dec = sizeof(bf16) * (size_t)DEC_WARPS * DEC_STAGES * 2 * DEC_KEYS * LDS;
+    static OptIn opt_in_decode;
+    opt_in_decode(smem_dec, attn_decode_kernel);
     static int dec_blocks = 0;
     if (dec_blocks == 0) {
-      cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dec);
       dec_blocks = sm_count * (HD <= 128 ? 2 : 1);
     }
     const int items = num_work * p.num_kv_heads;
@@ -1355,11 +1351,8 @@ void launch_fused(const AttnParams& p, const AttnFusedParams& f, const CUtensorM
   static_assert(HD % 64 != 0 || (16 + 2 * 2 * BN_KEYS) * LDS * 2 >= 16 * LDS * 2 + 1024 + 2 * 2 * BN_KEYS * HD * 2,
                 "the swizzled tiles must fit into the padded layout's shared memory");
   const size_t smem = (p.kinds & 16) ? smem_pages : smem_padded;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(attn_mma_kernel<2, NST, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_padded);
-    opted = true;
-  }
+  static OptIn opt_in;
+  opt_in(smem_padded, attn_mma_kernel<2, NST, CS>);
   launch_k_cluster(attn_mma_kernel<2, NST, CS>, dim3(CS, f.num_requests, p.num_kv_heads), NTHREADS, smem, stream, CS,
                    p, f, map_k, map_v);
 }

@@ -18,6 +18,7 @@
 //
 // Compile with -DPBE_HEAD_DIM=<multiple of 16>.
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "pdl.cuh"
 
@@ -313,18 +314,12 @@ int launch_simple(const AttnParams* params, int num_work, int dtype, Rest rest, 
   dim3 grid(num_work, p.num_kv_heads);
   // the shared-memory opt-in is set once per process and kernel, outside any stream capture
   // that a later launch may be part of
-  static bool opted[2] = {false, false};
+  static OptIn opt_in[2];
   if (dtype == PBE_F32) {
-    if (!opted[0]) {
-      cudaFuncSetAttribute(attn_simple_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      opted[0] = true;
-    }
+    if (const cudaError_t e = opt_in[0](smem, attn_simple_kernel<float>)) return (int)e;
     launch_k(attn_simple_kernel<float>, grid, NWARPS * 32, smem, stream, p, rest);
   } else {
-    if (!opted[1]) {
-      cudaFuncSetAttribute(attn_simple_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      opted[1] = true;
-    }
+    if (const cudaError_t e = opt_in[1](smem, attn_simple_kernel<__nv_bfloat16>)) return (int)e;
     launch_k(attn_simple_kernel<__nv_bfloat16>, grid, NWARPS * 32, smem, stream, p, rest);
   }
   return launch_status();

@@ -34,6 +34,7 @@
 #include <cuda_bf16.h>
 
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "kv_tensor_map.cuh"
 #include "pdl.cuh"
@@ -620,11 +621,8 @@ PBE_EXPORT int pbe_attn_tc5(const AttnParams* params, int num_work, int num_page
   rc = make_kv_tensor_map(&map_v, p.v_cache, rows, HD, box_rows);
   if (rc != 0) return rc;
   const size_t smem = (size_t)Q_BYTES + (NK + NV) * KV_BYTES + 1024;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(attn_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, attn_tc5_kernel)) return (int)e;
   if ((long long)num_work * p.num_kv_heads > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   dim3 grid((unsigned)(num_work * p.num_kv_heads));          // work-major: heavy tiles of every head first
   launch_k(attn_tc5_kernel, grid, NTHREADS, smem, stream, map_k, map_v, p, err);

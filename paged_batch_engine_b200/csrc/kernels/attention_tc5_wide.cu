@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "masked_attention.cuh"
 #include "pdl.cuh"
@@ -617,12 +618,8 @@ int map_rows(CUtensorMap* map, const void* at, long long rows, int columns, long
 int launch_wide(const CUtensorMap& a, const CUtensorMap& b, const AttnParams& p, const MaskedExtra& x, const LatentExtra& y,
                 long long blocks, int* err, cudaStream_t stream) {
   if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(attention_tc5_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(SMEM_BYTES, attention_tc5_wide_kernel)) return (int)e;
   launch_k(attention_tc5_wide_kernel, (int)blocks, NTHREADS, SMEM_BYTES, stream, a, b, p, x, y, err);
   return launch_status();
 }

@@ -20,6 +20,7 @@
 // state were 5e-6 off 64 bits on given inputs; the multiply-adds are 0.5e-7 to 5e-7 off and this 0.6 to 1.4 times that.
 #pragma once
 #include "chunk_scan.cuh"
+#include "opt_in.cuh"
 #include "mma_sync.cuh"
 
 namespace pbe {
@@ -304,12 +305,8 @@ int launch_of(const ChunkScanParams<TU>& p, int items, cudaStream_t stream) {
   // warps that share columns: one block a multiprocessor, so that blocks behind the first wave find the ones that short requests leave
   constexpr int smem = 2 * buffer_bytes<DP, CORRECT>() > 120 * 1024 || DS == 1 ? 2 * buffer_bytes<DP, CORRECT>() : 120 * 1024;
   auto kernel = scan_chunks_mma_kernel<DP, CORRECT, OWN, TU, DS>;
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, kernel)) return (int)e;
   launch_spread(kernel, dim3(items, p.H, (p.E + block_cols<DS>() - 1) / block_cols<DS>()), 128 + fetch_threads<DS>(), smem, stream, p);
   return launch_status();
 }

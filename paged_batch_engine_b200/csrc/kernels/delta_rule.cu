@@ -33,6 +33,7 @@
 //   overflow; the inverse's entries are bounded by one because every step of the rule is a contraction
 //   for keys of at most unit length.  Everything is float32.
 #include "chunk_scan.cuh"
+#include "opt_in.cuh"
 #include "chunk_scan_mma.cuh"
 #include "common.cuh"
 #include "pdl.cuh"
@@ -694,15 +695,9 @@ int launch_chunks(const ChunkParams& g, const ChunkScanParams<float>& p, int rec
                   cudaStream_t stream) {
   constexpr int DP = 16 * RPT, COLS = 2 * WARPS * CPT;
   constexpr size_t smem_g = sizeof(float) * 3 * CH * DP, smem_p = sizeof(float) * 2 * record_floats(DP, true);
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(delta_chunks_kernel<DP, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g);
-    cudaFuncSetAttribute(delta_chunks_kernel<DP, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g);
-    const cudaError_t e = cudaFuncSetAttribute(scan_chunks_kernel<RPT, CPT, WARPS, true, false, float>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in, opt_in_scan;
+  if (const cudaError_t e = opt_in(smem_g, delta_chunks_kernel<DP, true>, delta_chunks_kernel<DP, false>)) return (int)e;
+  if (const cudaError_t e = opt_in_scan(smem_p, scan_chunks_kernel<RPT, CPT, WARPS, true, false, float>)) return (int)e;
   const dim3 grid(records, g.H);
   if (chan) launch_k(delta_chunks_kernel<DP, true>, grid, 128, smem_g, stream, g);
   else launch_k(delta_chunks_kernel<DP, false>, grid, 128, smem_g, stream, g);

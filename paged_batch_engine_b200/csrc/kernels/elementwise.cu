@@ -5,6 +5,7 @@
 // swiglu_kernel.cu:6-25.  The residual stream is float32 in every run mode; statistics,
 // the sum and the products are float32 and each result is rounded once on store.
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "status.cuh"
 #include "pdl.cuh"
 
@@ -149,12 +150,8 @@ PBE_EXPORT int pbe_add_rmsnorm(float* residual, const void* delta, int delta_dty
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
 #define LAUNCH(TD, TO)                                                                          \
   do {                                                                                          \
-    static size_t opted = 48 * 1024;                                                            \
-    if (smem > opted) {                                                                         \
-      cudaFuncSetAttribute(add_rmsnorm_kernel<TD, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                           200 * 1024);                                                         \
-      opted = 200 * 1024;                                                                       \
-    }                                                                                           \
+    static OptIn opt_in;                                                                        \
+    if (smem > 48 * 1024) opt_in(200 * 1024, add_rmsnorm_kernel<TD, TO>);                       \
     launch_k(add_rmsnorm_kernel<TD, TO>, num_rows, threads, smem, stream, residual,             \
              (const TD*)delta, gain, (TO*)out, row_index, d, eps);                              \
   } while (0)
@@ -215,12 +212,8 @@ PBE_EXPORT int pbe_add2_rmsnorm2(float* residual, const void* delta_a, const voi
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
 #define LAUNCH2(TD, TO)                                                                            \
   do {                                                                                             \
-    static size_t opted = 48 * 1024;                                                               \
-    if (smem > opted) {                                                                            \
-      cudaFuncSetAttribute(add2_rmsnorm2_kernel<TD, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                           200 * 1024);                                                            \
-      opted = 200 * 1024;                                                                          \
-    }                                                                                              \
+    static OptIn opt_in;                                                                           \
+    if (smem > 48 * 1024) opt_in(200 * 1024, add2_rmsnorm2_kernel<TD, TO>);                        \
     launch_k(add2_rmsnorm2_kernel<TD, TO>, num_rows, threads, smem, stream, residual,              \
              (const TD*)delta_a, (const TD*)delta_b, gain1, gain2, (TO*)out1, (TO*)out2, row_index, d, eps, \
              delta_scale);                                                                         \

@@ -22,6 +22,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 
 using namespace pbe;
@@ -279,12 +280,8 @@ gemm_skinny_kernel(SkinnyParams p) {
 template <int NT, int WN, int WK, int CL, bool SWIGLU, typename TY, bool SHORT = false, bool GROUPS = false>
 int launch_cfg(const SkinnyParams& p, int row_blocks, cudaStream_t stream) {
   constexpr size_t smem = sizeof(uint4) * WN * WK * Stages<NT, WN * WK, SHORT>::value * (2 + NT) * 32;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(gemm_skinny_kernel<NT, WN, WK, CL, SWIGLU, TY, SHORT, GROUPS>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, gemm_skinny_kernel<NT, WN, WK, CL, SWIGLU, TY, SHORT, GROUPS>)) return (int)e;
   launch_k_cluster(gemm_skinny_kernel<NT, WN, WK, CL, SWIGLU, TY, SHORT, GROUPS>, dim3(row_blocks * CL, p.groups), WN * WK * 32,
                    smem, stream, CL, p);
   return launch_status();

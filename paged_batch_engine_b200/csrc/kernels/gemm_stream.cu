@@ -28,6 +28,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
 
@@ -354,11 +355,8 @@ void plan(int N_out, int K, int* tiles_n, int* splits, int* kb_per_split) {
 template <bool SWIGLU>
 int launch(const CUtensorMap& map_x, const CUtensorMap& map_w, const StreamParams& p, cudaStream_t stream) {
   constexpr size_t smem = (size_t)Ring<SWIGLU>::stages * Ring<SWIGLU>::stage_bytes + 1024;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(gemm_stream_kernel<SWIGLU>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, gemm_stream_kernel<SWIGLU>)) return (int)e;
   const long long items = (long long)p.tiles_n * p.splits;
   const int blocks = (int)(items < sm_count() ? items : sm_count());
   launch_k(gemm_stream_kernel<SWIGLU>, blocks, NTHREADS, smem, stream, map_x, map_w, p);

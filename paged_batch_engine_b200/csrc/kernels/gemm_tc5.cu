@@ -30,6 +30,7 @@
 #include <stdlib.h>
 
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
 
@@ -457,11 +458,8 @@ PBE_EXPORT int pbe_gemm_tc5(const void* X, const void* W, void* Y, int y_dtype, 
   p.y_float = y_dtype == PBE_F32;
   p.err = err;
   const size_t smem = (size_t)STAGES * STAGE_BYTES + 1024;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(gemm_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, gemm_tc5_kernel)) return (int)e;
   static int num_sms = 0;
   if (num_sms == 0) {
     int dev = 0;
@@ -474,11 +472,8 @@ PBE_EXPORT int pbe_gemm_tc5(const void* X, const void* W, void* Y, int y_dtype, 
     p.tiles_n = mode == 1 ? (p.N_out + 127) / 128 : (N + BN - 1) / BN;
     p.tiles_m = (M + 255) / 256;
     const size_t smem2 = (size_t)STAGES2 * STAGE2_BYTES + 1024;
-    static bool opted2 = false;
-    if (!opted2) {
-      cudaFuncSetAttribute(gemm_tc5_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
-      opted2 = true;
-    }
+    static OptIn opt_in_pair;
+    if (const cudaError_t e = opt_in_pair(smem2, gemm_tc5_pair_kernel)) return (int)e;
     const long long total2 = (long long)p.tiles_m * p.tiles_n;
     const int pairs = (int)(total2 < num_sms / 2 ? total2 : num_sms / 2);
     launch_k_cluster(gemm_tc5_pair_kernel, 2 * pairs, NTHREADS, smem2, stream, 2, map_x, map_w, p);

@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 #include "tcgen05.cuh"
 
@@ -305,11 +306,12 @@ grouped_tc5_kernel(const __grid_constant__ Maps maps, GroupedParams p) {
 }
 
 template <int EPI>
-void launch_grouped(const Maps& maps, const GroupedParams& p, cudaStream_t stream) {
+int launch_grouped(const Maps& maps, const GroupedParams& p, cudaStream_t stream) {
   const size_t smem = (size_t)STAGES * STAGE_BYTES + BOUNCE_BYTES + 1024;
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, grouped_tc5_kernel<EPI>)) return (int)e;
   static int num_sms = 0;
   if (num_sms == 0) {
-    cudaFuncSetAttribute(grouped_tc5_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int dev = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
@@ -319,6 +321,7 @@ void launch_grouped(const Maps& maps, const GroupedParams& p, cudaStream_t strea
   const long long most = (long long)p.max_tiles * ((p.N_out + cols - 1) / cols);
   const int pairs = (int)(most < num_sms / 2 ? most : num_sms / 2);
   launch_k_cluster(grouped_tc5_kernel<EPI>, 2 * pairs, NTHREADS, smem, stream, 2, maps, p);
+  return launch_status();
 }
 }  // namespace
 
@@ -340,10 +343,9 @@ PBE_EXPORT int pbe_grouped_tc5(const void* a, const void* w, void* out, int rows
   if (rc != 0) return rc;
   GroupedParams p{(bf16*)out, N, glu ? N / 2 : N, K, tiles, rows, tiles ? max_tiles : (rows + MAX_ROWS - 1) / MAX_ROWS, limit, alpha, err};
   switch (epilogue) {
-    case RELU2: launch_grouped<RELU2>(maps, p, stream); break;
-    case SILU_GLU: launch_grouped<SILU_GLU>(maps, p, stream); break;
-    case CAPPED_GLU: launch_grouped<CAPPED_GLU>(maps, p, stream); break;
-    default: launch_grouped<PLAIN>(maps, p, stream); break;
+    case RELU2: return launch_grouped<RELU2>(maps, p, stream);
+    case SILU_GLU: return launch_grouped<SILU_GLU>(maps, p, stream);
+    case CAPPED_GLU: return launch_grouped<CAPPED_GLU>(maps, p, stream);
+    default: return launch_grouped<PLAIN>(maps, p, stream);
   }
-  return launch_status();
 }

@@ -18,6 +18,7 @@
 //                    packing and key splits as the engine's other paged attention kernels)
 //   latent_merge     the key splits' partial results and the sink into one result
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "pdl.cuh"
 
@@ -661,11 +662,8 @@ int launch_latent_mma(const LatentAttnParams& lp, int num_work, cudaStream_t str
   const int wide = lp.dk > 32 * NT ? lp.dk : 32 * NT;
   const size_t smem = 2 * ((size_t)ROWS * (lp.dk + 8) + 2 * (size_t)LM_BN * (wide + 8)) + sizeof(float) * ROWS * (LM_BN + 1);
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  static size_t opted = 48 * 1024;
-  if (smem > opted) {
-    cudaFuncSetAttribute(latent_attention_mma_kernel<NT, RG>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    opted = 200 * 1024;
-  }
+  static OptIn opt_in;
+  if (smem > 48 * 1024) opt_in(200 * 1024, latent_attention_mma_kernel<NT, RG>);
   dim3 grid(num_work, (lp.a.tile_rows + ROWS - 1) / ROWS, lp.sub);
   launch_k(latent_attention_mma_kernel<NT, RG>, grid, LM_WARPS * 32 * RG, smem, stream, lp);
   return launch_status();
@@ -743,11 +741,8 @@ template <typename T, int DPL>
 int launch_latent(const LatentAttnParams& lp, int num_work, cudaStream_t stream) {
   const size_t smem = sizeof(float) * ((size_t)LA_BM * lp.dk + (size_t)LA_BN * (lp.dk | 1));
   if (smem > 200 * 1024) return (int)cudaErrorInvalidValue;
-  static size_t opted = 48 * 1024;
-  if (smem > opted) {
-    cudaFuncSetAttribute(latent_attention_kernel<T, DPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    opted = 200 * 1024;
-  }
+  static OptIn opt_in;
+  if (smem > 48 * 1024) opt_in(200 * 1024, latent_attention_kernel<T, DPL>);
   dim3 grid(num_work, lp.a.tile_rows / LA_BM);
   launch_k(latent_attention_kernel<T, DPL>, grid, LA_WARPS * 32, smem, stream, lp);
   return launch_status();

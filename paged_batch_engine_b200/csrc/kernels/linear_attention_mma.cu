@@ -22,6 +22,7 @@
 // terms a factor, the weighted v in shared memory, took 104, but outputs and state were 10 to 30 times further off 64 bits
 // than the recurrence's (1 to 3e-7); now they are 0.6 to 1.2 times.
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "mma_sync.cuh"
 #include "pdl.cuh"
 
@@ -376,12 +377,8 @@ __global__ void __launch_bounds__(THREADS, 2) linear_attention_mma_kernel(SsdPar
 template <int D, int E>
 int launch_ssd(const SsdParams& p, int R, cudaStream_t stream) {
   const int smem = (int)ssd_smem<D, E>();
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(linear_attention_mma_kernel<D, E>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, linear_attention_mma_kernel<D, E>)) return (int)e;
   // without the programmatic dependency: few long-running blocks, which would else be placed several to a
   // multiprocessor while the kernel before still fills the others
   linear_attention_mma_kernel<D, E><<<dim3(R, p.H), THREADS, smem, stream>>>(p);

@@ -30,6 +30,7 @@
 //   what the cache holds.
 // masked_merge: the key splits of a row put together, with the sink and the gate.
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "masked_attention.cuh"
 #include "pdl.cuh"
@@ -740,11 +741,8 @@ size_t ma_smem(int D, int E) {
 template <typename T, int EPL>
 int launch_ma(const AttnParams& p, const MaskedExtra& x, int num_work, cudaStream_t stream) {
   const size_t smem = ma_smem(x.D, x.E);
-  static size_t opted = 48 * 1024;
-  if (smem > opted) {
-    cudaFuncSetAttribute(masked_attention_kernel<T, EPL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    opted = 200 * 1024;
-  }
+  static OptIn opt_in;
+  if (smem > 48 * 1024) opt_in(200 * 1024, masked_attention_kernel<T, EPL>);
   launch_k(masked_attention_kernel<T, EPL>, dim3(num_work, p.num_kv_heads), NWARPS * 32, smem, stream, p, x);
   return launch_status();
 }

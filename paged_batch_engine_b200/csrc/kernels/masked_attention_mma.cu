@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 
 #include "attention_params.cuh"
+#include "opt_in.cuh"
 #include "common.cuh"
 #include "masked_attention.cuh"
 #include "pdl.cuh"
@@ -502,13 +503,8 @@ PBE_EXPORT int pbe_masked_attention_mma(const AttnParams* params, const float* b
   if ((((uintptr_t)p.q | (uintptr_t)turn | (uintptr_t)p.k_cache | (uintptr_t)p.v_cache | (uintptr_t)p.part_o) & 15) != 0 ||
       ((uintptr_t)p.out & 3) != 0)
     return (int)cudaErrorMisalignedAddress;
-  static bool opted = false;
-  if (!opted && SMEM_BYTES > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(masked_attention_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(SMEM_BYTES, masked_attention_mma_kernel)) return (int)e;
   MaskedExtra x{bias, bias_rows, mask_kind, has_sink, sink, softcap, turn, gate, ldg, D, E};
   x.gate_pairs = gate != nullptr && ((uintptr_t)gate & 3) == 0 && (ldg & 1) == 0;
   launch_k(masked_attention_mma_kernel, dim3(num_work, p.num_kv_heads), NT, SMEM_BYTES, stream, p, x);

@@ -21,6 +21,7 @@
 //
 // Compile with -DPBE_PA_F32=1 for float32 tensors, 0 for bfloat16: a library holds one of them.
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 #include "vec.cuh"
 
@@ -625,11 +626,8 @@ __global__ void pa_sum_kernel(const float* part_o, void* out, const int32_t* til
 
 template <typename T, int BM>
 int launch_pa(PoolAttnParams p, int mode, int n_tiles, size_t smem, cudaStream_t stream) {
-  static size_t opted = 0;
-  if (smem > 48 * 1024 && opted < smem) {
-    cudaFuncSetAttribute(pooled_attention_kernel<T, BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    opted = smem;
-  }
+  static OptIn opt_in;
+  if (smem > 48 * 1024) opt_in(smem, pooled_attention_kernel<T, BM>);
   p.mode = mode;
   dim3 grid(n_tiles, mode == 0 ? 1 : p.splits);
   launch_k(pooled_attention_kernel<T, BM>, grid, PA_THREADS, smem, stream, p);

@@ -29,6 +29,7 @@
 #define PBE_PM_D 128
 #define PBE_PM_E 128
 #include "pooled_attention_mma.cu"
+#include "opt_in.cuh"
 #include "tcgen05.cuh"
 
 using namespace pbe::tc5;
@@ -446,12 +447,8 @@ int map_pages(CUtensorMap* map, const void* at, long long rows, int page_tokens)
 
 template <int NKV>
 int launch_tc5(const CUtensorMap (&maps)[4], const TcParams& x, cudaStream_t stream) {
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(pooled_attention_tc5_kernel<NKV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes<NKV>());
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem_bytes<NKV>(), pooled_attention_tc5_kernel<NKV>)) return (int)e;
   launch_k(pooled_attention_tc5_kernel<NKV>, x.num_tiles * x.m.H * (x.m.G / NKV), NTHREADS, smem_bytes<NKV>(), stream, maps[0], maps[1],
            maps[2], maps[3], x);
   return launch_status();

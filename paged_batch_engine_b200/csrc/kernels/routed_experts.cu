@@ -24,6 +24,7 @@
 // For many rows the host side sorts the rows by expert (pair_rows / scatter below) and runs one
 // matrix product per expert over its rows.
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 
 using namespace pbe;
@@ -514,12 +515,8 @@ PBE_EXPORT int pbe_expert_rows(const void* x, const void* w_gate, const void* w_
   dim3 grid1(T * top, (F + ER_UNITS - 1) / ER_UNITS), grid2(T * top, (W + ER_UNITS - 1) / ER_UNITS);
 #define PBE_ER(TT)                                                                                             \
   do {                                                                                                         \
-    static size_t opted = 48 * 1024;                                                                           \
-    if (smem1 > opted || smem2 > opted) {                                                                      \
-      cudaFuncSetAttribute(expert_hidden_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024); \
-      cudaFuncSetAttribute(expert_down_kernel<TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);   \
-      opted = 200 * 1024;                                                                                      \
-    }                                                                                                          \
+    static OptIn opt_in;                                                                                       \
+    if (smem1 > 48 * 1024 || smem2 > 48 * 1024) opt_in(200 * 1024, expert_hidden_kernel<TT>, expert_down_kernel<TT>);\
     launch_k(expert_hidden_kernel<TT>, grid1, ER_WARPS * 32, smem1, stream, p);                                \
     launch_k(expert_down_kernel<TT>, grid2, ER_WARPS * 32, smem2, stream, p);                                  \
   } while (0)

@@ -24,6 +24,7 @@
 #include <cooperative_groups.h>
 
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 #include "status.cuh"
 
@@ -963,14 +964,9 @@ PBE_EXPORT int pbe_sample(const float* logits, long long ld, int num_rows, int v
                           const float* temperature, const int32_t* top_k, const float* top_p,
                           const float* uniform, int32_t* out, cudaStream_t stream) {
   if (num_rows <= 0) return 0;
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(sample_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Quick));
-    cudaFuncSetAttribute(sample_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Quick));
-    cudaFuncSetAttribute(sample_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Quick));
-    cudaFuncSetAttribute(sample_kernel<SAMPLE_CLUSTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Quick));
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(sizeof(Quick), sample_kernel<1>, sample_kernel<2>, sample_kernel<4>, sample_kernel<SAMPLE_CLUSTER>))
+    return (int)e;
   static int sm_count = 0;
   if (sm_count == 0) {
     int dev = 0;

@@ -29,6 +29,7 @@
 //    49 TFLOP/s).  With few output tiles the slices become blocks of their own (grid z) and
 //    the last block of a tile adds them in order.
 #include "common.cuh"
+#include "opt_in.cuh"
 
 using namespace pbe;
 
@@ -491,12 +492,8 @@ int launch_skinny(const TX* X, const float* W, const float* bias, float* part, T
   const long long tasks = (long long)num_slices * num_ntiles;
   const size_t smem = (size_t)SK_WARPS * skinny_warp_floats<MT, NPER>() * sizeof(float);
   auto kern = sgemm_skinny_kernel<MT, NPER, VEC, TX, TY>;
-  static bool attr_set = false;          // per instantiation
-  if (!attr_set) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static OptIn opt_in;          // per instantiation
+  if (const cudaError_t e = opt_in(smem, kern)) return (int)e;
   const long long blocks = (tasks + SK_WARPS - 1) / SK_WARPS;
   if (blocks > 0x7fffffffLL) return (int)cudaErrorInvalidValue;
   const int x_vec = (sizeof(TX) == 4 && ldx % 4 == 0 && ((uintptr_t)X % 16) == 0) ? 1 : 0;
@@ -559,12 +556,8 @@ int launch_tiled(const TX* X, const float* W, const float* bias, TY* Y, float* p
                  int ldx, int ldy, int vec_x, int vec_w, cudaStream_t stream, const int* only_if = nullptr) {
   auto kern = sgemm_tiled_kernel<BM, SPLIT, TX, TY>;
   const int smem = SPLIT ? 0 : tiled_dyn_smem<BM>();
-  static bool attr_set = false;
-  if (!attr_set && smem > 0) {
-    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(smem, kern)) return (int)e;
   dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, SPLIT ? (K + SLICE - 1) / SLICE : 1);
   if (grid.y > 65535 || grid.z > 65535) return (int)cudaErrorInvalidValue;
   kern<<<grid, 256, smem, stream>>>(X, W, bias, Y, part, tickets, M, N, K, ldx, ldy, vec_x, vec_w,

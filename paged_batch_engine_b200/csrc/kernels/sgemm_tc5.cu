@@ -39,6 +39,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "tcgen05.cuh"
 
 using namespace pbe;
@@ -449,12 +450,8 @@ int make_map_f32(CUtensorMap* map, const float* base, int rows, int K, int ld) {
 }
 
 int launch_product(const CUtensorMap& map_w, const CUtensorMap& map_x, const ProductParams& p, cudaStream_t stream) {
-  static bool opted = false;
-  if (!opted) {
-    const cudaError_t e = cudaFuncSetAttribute(sgemm_tc5_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PRODUCT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in;
+  if (const cudaError_t e = opt_in(PRODUCT_SMEM, sgemm_tc5_kernel)) return (int)e;
   const long long tiles = (long long)((p.M + p.bn - 1) / p.bn) * ((p.N + BM - 1) / BM) * p.parts;
   const int blocks = (int)(tiles < multiprocessors() ? tiles : multiprocessors());
   sgemm_tc5_kernel<<<blocks, NTHREADS, PRODUCT_SMEM, stream>>>(map_w, map_x, p);

@@ -16,6 +16,7 @@
 // gain, times sigmoid(g) or silu(g) of a gate that lies in a wider matrix; or, gate first, the
 // gated values o * act(g) divided by their own root mean square, times the gain.
 #include "common.cuh"
+#include "opt_in.cuh"
 #include "pdl.cuh"
 
 using namespace pbe;
@@ -291,11 +292,8 @@ PBE_EXPORT int pbe_stream_norm(float* streams, const void* y, int y_dtype, const
   cudaError_t e;
 #define PBE_SN(TY, TO)                                                                                  \
   do {                                                                                                  \
-    static int opted = 0;                                                                               \
-    if (smem > 48 * 1024 && opted < (int)smem) {                                                        \
-      cudaFuncSetAttribute(stream_norm_kernel<TY, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-      opted = (int)smem;                                                                                \
-    }                                                                                                   \
+    static OptIn opt_in;                                                                                \
+    if (smem > 48 * 1024) opt_in(smem, stream_norm_kernel<TY, TO>);                                     \
     e = launch_k(stream_norm_kernel<TY, TO>, n, threads, smem, stream, p);                              \
   } while (0)
   const bool yb = y != nullptr && y_dtype == PBE_BF16;

@@ -18,6 +18,7 @@
 //   formed, so nothing can overflow.
 // The state is laid out [head][column][key channel]: the lanes of a column move consecutive 16-byte pieces.
 #include "chunk_scan.cuh"
+#include "opt_in.cuh"
 #include "chunk_scan_mma.cuh"
 #include "common.cuh"
 #include "pdl.cuh"
@@ -364,16 +365,11 @@ template <typename T, int RPT, int CPT, int WARPS>
 int launch_chunks(const WkvParams& g, float* records, int count, const Segments& s, cudaStream_t stream) {
   constexpr int DP = 16 * RPT, COLS = 2 * WARPS * CPT;
   constexpr size_t smem_g = sizeof(float) * 3 * CH * DP, smem_p = sizeof(float) * 2 * record_floats(DP, false);
-  static bool opted = false;
-  if (!opted) {
-    cudaFuncSetAttribute(wkv_chunks_kernel<T, DP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g);
-    cudaFuncSetAttribute(scan_chunks_kernel<RPT, CPT, WARPS, false, true, T>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p);
-    const cudaError_t e = cudaFuncSetAttribute(scan_chunks_kernel<RPT, CPT, WARPS, false, false, T>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_p);
-    if (e != cudaSuccess) return (int)e;
-    opted = true;
-  }
+  static OptIn opt_in, opt_in_scans;
+  if (const cudaError_t e = opt_in(smem_g, wkv_chunks_kernel<T, DP>)) return (int)e;
+  if (const cudaError_t e = opt_in_scans(smem_p, scan_chunks_kernel<RPT, CPT, WARPS, false, true, T>,
+                                         scan_chunks_kernel<RPT, CPT, WARPS, false, false, T>))
+    return (int)e;
   launch_k(wkv_chunks_kernel<T, DP>, dim3(count, g.H), 128, smem_g, stream, g, records);
   int err = launch_status();
   if (err != 0) return err;
