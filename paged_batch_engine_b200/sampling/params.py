@@ -25,9 +25,9 @@ def request_sample_uniform(seed: int, counter: int) -> float:
 
 def request_sample_uniforms(seeds, counters) -> np.ndarray:
     """``request_sample_uniform`` of many (seed, counter) pairs, as ``zip`` makes them of the two: the same draws, as float64."""
-    counters = list(islice(counters, len(seeds)))
-    z = np.array([s & _MASK64 for s in seeds[:len(counters)]], dtype=np.uint64)
-    z += np.array([(c + 1) & _MASK64 for c in counters], dtype=np.uint64) * np.uint64(0x9E3779B97F4A7C15)
+    steps = np.array([(c + 1) & _MASK64 for c in islice(counters, len(seeds))], dtype=np.uint64)
+    z = np.array([s & _MASK64 for s in seeds], dtype=np.uint64)[:len(steps)]
+    z += steps * np.uint64(0x9E3779B97F4A7C15)
     z = (z ^ (z >> np.uint64(30))) * np.uint64(0xBF58476D1CE4E5B9)
     z = (z ^ (z >> np.uint64(27))) * np.uint64(0x94D049BB133111EB)
     z ^= z >> np.uint64(31)
