@@ -31,6 +31,7 @@
 #include <cuda_bf16.h>
 
 #include "attention_simple.cu"
+#include "float_terms.cuh"
 #include "opt_in.cuh"
 #include "tcgen05.cuh"
 
@@ -51,7 +52,6 @@ constexpr int NTHREADS = 32 * (MMA_WARP + 1);
 constexpr int Q_BYTES = BM * HD * 2, KV_BYTES = BN * HD * 2;          // a term
 constexpr int S_COL = 0, P_COL = 2 * BN, O_COL = 256, TMEM_COLS = 512;
 static_assert(P_COL + TERMS * BN / 2 <= O_COL && O_COL + 2 * HD <= TMEM_COLS, "tensor memory");
-constexpr float SMALLEST = 0x1p-102f, LARGEST = 0x1p47f;
 
 struct Barriers {
   uint64_t q_full, k_full, k_empty, v_full, v_empty, s_full[2], p_full, o_ready[2];
@@ -69,50 +69,10 @@ struct F32Extra {
   int32_t* flags;                               // [places, max_splits, KV]: 1 where a block hands its rows back
 };
 
-// Are numbers zero, or of a size from SMALLEST to LARGEST?  Without a branch a number: the largest size and the smallest that is
-// not zero, as integers (zero less one is the largest integer; infinities and what is no number are above LARGEST).
-struct Sizes {
-  uint32_t largest = 0, smallest = 0xffffffffu;
-  __device__ __forceinline__ void add(float x) {
-    const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
-    largest = max(largest, u);
-    smallest = min(smallest, u - 1u);
-  }
-  __device__ __forceinline__ bool whole() const {
-    return largest <= __float_as_uint(LARGEST) && smallest >= __float_as_uint(SMALLEST) - 1u;
-  }
-};
-__device__ __forceinline__ uint32_t pack2(float x, float y) {
-  const __nv_bfloat162 h = __floats2bfloat162_rn(x, y);
-  return *reinterpret_cast<const uint32_t*>(&h);
-}
-// two numbers' next terms; what is left of them stays in x and y (exact: it has fewer bits than they had)
-__device__ __forceinline__ uint32_t next_term(float& x, float& y) {
-  const uint32_t w = pack2(x, y);
-  x -= __uint_as_float(w << 16);
-  y -= __uint_as_float(w & 0xffff0000u);
-  return w;
-}
 // byte offset of element (row, col) in a [64-wide blocks][rows] bf16 tile with 128-byte swizzle
 __device__ __forceinline__ uint32_t swz(int row, int col, int rows) {
   const int blk = col >> 6, cc = col & 63;
   return (uint32_t)(blk * rows * 128 + row * 128 + ((((cc >> 3) ^ (row & 7)) << 4) | ((cc & 7) << 1)));
-}
-// the values as they lie: MN-major, [64 keys][64 columns] blocks
-__device__ __forceinline__ uint64_t desc_mn_major(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((BN * 128) >> 4) << 16;       // the next 64 columns
-  d |= (uint64_t)(1024 >> 4) << 32;             // eight keys further
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 __device__ __forceinline__ void tmem_st16_nowait(uint32_t taddr, const uint32_t* v) {
   asm volatile(
@@ -445,7 +405,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) attention_f32_tc5_kernel(AttnPara
 #pragma unroll
           for (int ks = 0; ks < BN / 16; ++ks)
             umma_ts(tmem_base + O_COL + (j & 1) * HD, tmem_base + P_COL + t * (BN / 2) + ks * 8,
-                    desc_mn_major(v_addr + (sum - t) * KV_BYTES + ks * 16 * 128), idesc_o,
+                    desc_mn_major(v_addr + (sum - t) * KV_BYTES + ks * 16 * 128, BN), idesc_o,
                     (sum < TERMS - 1 || t > 0 || ks > 0) ? 1u : 0u);
       umma_commit(&bar.v_empty);
       umma_commit(&bar.o_ready[j & 1]);

@@ -74,22 +74,6 @@ struct LatentExtra {
   int ldg, gate_each;        // a value per output column, or one per head
 };
 
-__device__ __forceinline__ uint64_t desc_mn_major(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((BN * 128) >> 4) << 16;       // the next 64 columns: one [64 keys][64] block further
-  d |= (uint64_t)(1024 >> 4) << 32;             // eight keys further
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// A from tensor memory (128 lanes x 8 columns of two bfloat16 per k-step), B from shared memory
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
 __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, float* v) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
@@ -99,16 +83,6 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, float* v) {
         "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
         "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
       : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st32_nowait(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
 }
 __device__ __forceinline__ float ex2(float x) {
   float y;
@@ -389,7 +363,7 @@ attention_tc5_wide_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         for (int term = 0; term < 2; ++term)
 #pragma unroll
           for (int ks = 0; ks < BN / 16; ++ks)
-            umma_ts(tmem_base + O_COL, tmem_base + S_COL + st * BN + term * 32 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128),
+            umma_ts(tmem_base + O_COL, tmem_base + S_COL + st * BN + term * 32 + ks * 8, desc_mn_major(v_addr + ks * 16 * 128, BN),
                     idesc_o, (j > 0 || term > 0 || ks > 0) ? 1u : 0u);
         umma_commit(&bar.v_empty);
         umma_commit(&bar.o_ready);

@@ -29,6 +29,7 @@
 #define PBE_PM_D 128
 #define PBE_PM_E 128
 #include "pooled_attention_mma.cu"
+#include "float_terms.cuh"
 #include "opt_in.cuh"
 #include "tcgen05.cuh"
 
@@ -61,32 +62,6 @@ struct TcParams {
   int* err;
 };
 
-__device__ __forceinline__ uint64_t desc_mn_major(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((BN * 128) >> 4) << 16;       // the next 64 columns: one [64 keys][64] block further
-  d |= (uint64_t)(1024 >> 4) << 32;             // eight keys further
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
 __device__ __forceinline__ void tmem_st8_nowait(uint32_t taddr, const uint32_t (&v)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
                ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]) : "memory");
@@ -251,7 +226,7 @@ pooled_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_kt, const __
           for (int t = TERMS - 1; t >= 0; --t)             // the small terms first
 #pragma unroll
             for (int ks = 0; ks < BN / 16; ++ks)
-              umma_ts(tmem_base + O_COL + kv * WIDTH, tmem_base + P_COL + (j & 1) * P_COLS + t * (BN / 2) + ks * 8, desc_mn_major(v_addr + ks * 16 * 128),
+              umma_ts(tmem_base + O_COL + kv * WIDTH, tmem_base + P_COL + (j & 1) * P_COLS + t * (BN / 2) + ks * 8, desc_mn_major(v_addr + ks * 16 * 128, BN),
                       idesc_o, t < TERMS - 1 || ks > 0 ? 1u : 0u);
         }
         umma_commit(&bar.v_empty[j % NV]);
@@ -340,12 +315,7 @@ pooled_attention_tc5_kernel(const __grid_constant__ CUtensorMap map_kt, const __
       for (int k = 0; k < TERMS; ++k) {
         uint32_t w[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const __nv_bfloat162 h = __floats2bfloat162_rn(s[2 * i], s[2 * i + 1]);
-          w[i] = *reinterpret_cast<const uint32_t*>(&h);
-          s[2 * i] -= __uint_as_float(w[i] << 16);
-          s[2 * i + 1] -= __uint_as_float(w[i] & 0xffff0000u);
-        }
+        for (int i = 0; i < 8; ++i) w[i] = next_term(s[2 * i], s[2 * i + 1]);
         tmem_st8_nowait(lane_addr + P_COL + (j & 1) * P_COLS + k * (BN / 2) + part * 8, w);
       }
       if (j > 0) {

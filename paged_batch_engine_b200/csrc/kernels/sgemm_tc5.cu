@@ -39,6 +39,7 @@
 #include <cuda_bf16.h>
 
 #include "common.cuh"
+#include "float_terms.cuh"
 #include "opt_in.cuh"
 #include "tcgen05.cuh"
 
@@ -51,24 +52,8 @@ constexpr int BM = 128, BK = 64, UMMA_K = 16, TERMS = 3;
 constexpr int SLICE = 28;                         // K blocks whose sums are added in one chain, at most
 constexpr int MAX_BN = 192;                       // rows of X a tile has at most
 constexpr int SPLIT_WARPS = 4, EPI_WARPS = 8, X_WARP = 12, MMA_WARP = 13, W_WARP = 14, NTHREADS = 32 * 15;
-constexpr float SMALLEST = 0x1p-102f;              // its last bit, 2^-125, is a bfloat16 number
-constexpr float LARGEST = 0x1p47f;                 // a sum of 2^31 products of two such numbers stays below 2^127
 
 // ------------------------------------------------------------------ the terms
-// Are numbers zero, or of a size from SMALLEST to LARGEST?  Without a branch a number: the largest size and the smallest that is
-// not zero, as integers (zero less one is the largest integer; infinities and what is no number are above LARGEST).
-struct Sizes {
-  uint32_t largest = 0, smallest = 0xffffffffu;
-  __device__ __forceinline__ void add(float x) {
-    const uint32_t u = __float_as_uint(x) & 0x7fffffffu;
-    largest = max(largest, u);
-    smallest = min(smallest, u - 1u);
-  }
-  __device__ __forceinline__ bool whole() const {
-    return largest <= __float_as_uint(LARGEST) && smallest >= __float_as_uint(SMALLEST) - 1u;
-  }
-};
-
 // planes [TERMS][rows][Kp]; a thread takes eight k of a row
 __global__ void __launch_bounds__(256) split3_kernel(const float* x, bf16* planes, int rows, int K, int Kp, int vec, int* flag) {
   const int pieces = Kp / 8;
@@ -130,43 +115,6 @@ struct ProductBarriers {
   uint64_t w_full[W_STAGES], w_empty[W_STAGES], a_lh_full, a_m_full, l_empty, m_empty, x_full[2], acc_full[2], acc_empty[2];
   uint32_t tmem_base;
 };
-
-// A from tensor memory (128 lanes x 8 columns of two bfloat16 per k-step), B from shared memory
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void tmem_st32_nowait(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-// two numbers' next terms; what is left of them stays in x and y (exact: it has fewer bits than they had)
-__device__ __forceinline__ uint32_t next_term(float& x, float& y) {
-  const __nv_bfloat162 p = __floats2bfloat162_rn(x, y);
-  const uint32_t w = *reinterpret_cast<const uint32_t*>(&p);
-  x -= __uint_as_float(w << 16);
-  y -= __uint_as_float(w & 0xffff0000u);
-  return w;
-}
 
 __global__ void __launch_bounds__(NTHREADS, 1)
 sgemm_tc5_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, ProductParams p) {
