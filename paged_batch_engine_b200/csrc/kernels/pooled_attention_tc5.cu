@@ -20,7 +20,7 @@
 // What bounds the first is the softmax warps' chain, 4,500 clocks a key tile, of which reads of tensor memory, 350 clocks each
 // beside the products, are 1,900 (the products are 2,048); 96 registers a thread leave room for sixteen columns at a time.
 // 2,048 tokens, sixteen heads over four key/value heads, window 1,024, blocks of 64: 291 us on mma.sync, 151 here and
-// some 20 for the mixture (a layer 352 -> 233); over two key/value heads a layer 330 -> 166, 8,192 tokens over four 1,378 -> 965.
+// some 20 for the mixture (a layer 352 -> 229); over two key/value heads a layer 330 -> 166, 8,192 tokens over four 1,378 -> 965.
 //
 // A value that is not finite reaches, as a product with a weight of zero, rows of its tile that do not see it.  Blocks that find one in
 // a tile which not all of their rows see whole set a flag; the rows of flagged tiles are made by pooled_attention_mma.cu, launched behind.

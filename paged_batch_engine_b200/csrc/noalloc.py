@@ -30,7 +30,8 @@ def scratch_floats(head_dim: int) -> int:
 
 def paged_attention_noalloc(q, k_cache, v_cache, out, meta, num_heads, num_kv_heads, head_dim, scale,
                             window, page_tokens) -> torch.Tensor:
-    """Same result as ``ops.paged_attention(..., kind="simple")``; ``meta.part_o`` and
+    """Same result as ``ops.paged_attention(..., kind="simple")``, bit for bit but for float32 steps that
+    run on the tensor cores there (``meta.wide_tiles``): both are float32 sums, in another order.  ``meta.part_o`` and
     ``meta.part_ml`` are not used.  Raises when the partial results would not fit the
     built-in scratch."""
     lib = library(head_dim)

@@ -114,9 +114,9 @@ class PooledWindowAttention(Mixer):
     def _takes_tc5(self, ctx, seen: int) -> bool:
         """Whether a step's portions take the tcgen05 form, kept on the step.  Its blocks (128 rows, one head, one or two key/value
         heads) run one a multiprocessor, 8 us and 2.3 us a tile of 64 keys; the mixture and the look for odd values take 25 us
-        behind.  The mma.sync form's blocks (16 rows, all heads) take 25 us and 0.21 us a key.  Steps of fewer keys wait for the
-        host, where the tcgen05 form has 18 us more to do.  Layers of sixteen heads over four, mma.sync or split form -> tcgen05: 2,048 rows,
-        window 1,024 352 -> 233 us, window 256 and blocks of 16 182 / 193 (stays); 300 rows 133 -> 119, 256 rows 106 / 116
+        behind.  The mma.sync form's blocks (16 rows, all heads) are counted as 25 us and 0.21 us a key, less than they take alone (see
+        ``forward``): so counted the line lies where the layers' times cross.  Steps of fewer keys wait for the host, where the tcgen05 form has 18 us more to do.  Layers of sixteen heads over four, mma.sync or split form -> tcgen05: 2,048 rows,
+        window 1,024 352 -> 229 us, window 256 and blocks of 16 182 / 193 (stays); 300 rows 133 -> 119, 256 rows 106 / 116
         (stays); 16 rows behind 1,057 151 -> 121, behind 300 109 / 125 (stays); 64 rows beside 30 decoded tokens 311 / 358 (stays)."""
         H, G = self.num_heads, self.num_kv_heads
         kept = ctx.__dict__.setdefault("_pooled_tc5", {})
@@ -162,7 +162,7 @@ class PooledWindowAttention(Mixer):
         # decoded tokens only (always so in a captured step): a row a tile
         single = getattr(ctx, "captured", False) or int(ctx.q_len_host.max(initial=1)) == 1
         # Prompt portions take the tensor-core form, whose blocks walk all keys of sixteen rows (30 us and 0.25 us a
-        # key).  A short portion behind a long context leaves most of the GPU idle that way: there the split form is
+        # key: 277 keys 92 us, 526 159, 1,072 294).  A short portion behind a long context leaves most of the GPU idle that way: there the split form is
         # ahead (1,073 keys: 64 rows 225 against 303 us, 80 rows 319 / 303; 648 keys: 48 rows 117 / 187, 64 rows 198 /
         # 188; 394 keys: 48 rows 126 / 132; 335 keys: 16 rows 115 / 101).
         longest = int(ctx.seq_len_host.max(initial=1))
