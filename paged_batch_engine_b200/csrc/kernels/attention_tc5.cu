@@ -38,8 +38,10 @@
 #include "common.cuh"
 #include "kv_tensor_map.cuh"
 #include "pdl.cuh"
+#include "tcgen05.cuh"
 
 using namespace pbe;
+using namespace pbe::tc5;
 
 #ifndef PBE_HEAD_DIM
 #error "PBE_HEAD_DIM must be defined"
@@ -58,124 +60,7 @@ constexpr int NTHREADS = 224;
 constexpr int NK = 2, NV = 2;           // key tiles and value tiles in flight
 constexpr int TMEM_COLS = 256;
 constexpr int S_COL = 0, O_COL = 128;   // S buffers at columns 0 and 64 (P in their first 32 columns), O at 128
-constexpr long long WAIT_CLOCKS = 2000LL * 1000 * 1000;   // about a second
 
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err) {
-  const uint32_t addr = smem_u32(bar);
-  uint32_t done;
-  // the common case, the phase is already complete: one probe, no clock read
-  asm volatile(
-      "{\n.reg .pred p;\n"
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-      "selp.u32 %0, 1, 0, p;\n}\n"
-      : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-  if (done) return true;
-  const long long t0 = clock64();
-  for (;;) {
-    asm volatile(
-        "{\n.reg .pred p;\n"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-        "selp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(done) : "r"(addr), "r"(parity) : "memory");
-    if (done) return true;
-    if (clock64() - t0 > WAIT_CLOCKS) break;
-  }
-  if (err) atomicExch(err, 1);
-  return false;
-}
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(smem_u32(smem_dst)), "l"(map), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
-}
-// K-major operand, 128-byte swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
-__device__ __forceinline__ uint64_t desc_k_major(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-// MN-major operand, 128-byte swizzle (V as it lies in the pages: [key][head_dim]): a row of 64
-// head-dim elements is 128 bytes, rows of consecutive keys are 128 bytes apart, groups of 8
-// keys 1024 bytes apart (stride byte offset), the next 64 head-dim elements one whole
-// [128 keys][64] block further (leading byte offset).
-__device__ __forceinline__ uint64_t desc_mn_major(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
-  d |= (uint64_t)((BN * 128) >> 4) << 16;
-  d |= (uint64_t)(1024 >> 4) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
-  return d;
-}
-__device__ __forceinline__ uint32_t make_idesc(int m, int n, bool b_mn_major) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((b_mn_major ? 1u : 0u) << 16) | ((uint32_t)(n >> 3) << 17) |
-         ((uint32_t)(m >> 4) << 24);
-}
-__device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-// A from tensor memory (128 lanes x 8 columns of two bfloat16 per k-step), B from shared memory
-__device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                        uint32_t accumulate) {
-  asm volatile(
-      "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}\n"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32]) {
-  uint32_t r[32];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
-        "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
-        "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-      : "r"(taddr) : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
-}
-__device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, float* v) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
-        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
-        "=f"(v[16]), "=f"(v[17]), "=f"(v[18]), "=f"(v[19]), "=f"(v[20]), "=f"(v[21]), "=f"(v[22]), "=f"(v[23]),
-        "=f"(v[24]), "=f"(v[25]), "=f"(v[26]), "=f"(v[27]), "=f"(v[28]), "=f"(v[29]), "=f"(v[30]), "=f"(v[31])
-      : "r"(taddr) : "memory");
-}
-__device__ __forceinline__ void tmem_st32_nowait(uint32_t taddr, const uint32_t* v) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-      "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]),
-        "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]),
-        "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]),
-        "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
-}
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -346,8 +231,8 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
   } else if (warp == 1) {
     if (lane == 0 && n_tiles > 0) {
       // ------------------------------------------------------------ MMA issuer
-      const uint32_t idesc_s = make_idesc(BM, BN, false);
-      const uint32_t idesc_o = make_idesc(BM, HD, true);
+      const uint32_t idesc_s = make_idesc(BM, BN);
+      const uint32_t idesc_o = make_idesc(BM, HD) | (1u << 16);      // B as it lies: MN-major
       const uint32_t q_addr = smem_u32(Qs);
       bool ok = true;
       auto issue_qk = [&](int j) {
@@ -359,7 +244,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
         for (int ks = 0; ks < HD / 16; ++ks) {
           const uint32_t q_off = (ks >> 2) * (BM * 128) + (ks & 3) * 32;
           const uint32_t k_off = (ks >> 2) * (BN * 128) + (ks & 3) * 32;
-          umma(tmem_base + S_COL + st * BN, desc_k_major(q_addr + q_off), desc_k_major(k_addr + k_off), idesc_s,
+          umma(tmem_base + S_COL + st * BN, make_desc(q_addr + q_off), make_desc(k_addr + k_off), idesc_s,
                ks > 0 ? 1u : 0u);
         }
         umma_commit(&k_empty[kst]);                           // the key tile is free once its scores exist
@@ -379,7 +264,7 @@ attn_tc5_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant
 #pragma unroll
         for (int ks = 0; ks < BN / 16; ++ks) {
           const uint32_t b_off = ks * 16 * 128;                            // V: 16 keys further down
-          umma_ts(tmem_base + O_COL, tmem_base + S_COL + st * BN + ks * 8, desc_mn_major(v_addr + b_off), idesc_o,
+          umma_ts(tmem_base + O_COL, tmem_base + S_COL + st * BN + ks * 8, desc_mn_major(v_addr + b_off, BN), idesc_o,
                   (j > 0 || ks > 0) ? 1u : 0u);
         }
         umma_commit(&v_empty[vst]);
