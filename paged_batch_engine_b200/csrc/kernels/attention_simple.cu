@@ -12,10 +12,10 @@
 // sums taken in another order.
 //
 // It takes the float32 path's decode steps, its other steps with heads of neither 64 nor 128 or with
-// few keys, and the row tiles that attention_f32_tc5.cu, which takes the rest, hands back; and it is
-// the checker for the tensor-core kernels.  It stands where the reference runs paged_mha_kernel.cu:363-550 (decode) and
-// paged_mha_prefill_kernel.cu:120-237,368-520 (prompt portions): s_j = (q.k_j) * scale,
-// online softmax with running maximum and sum, o = acc / l.
+// few keys, and the row tiles that attention_f32_tc5.cu, which takes the rest, hands back; the
+// tensor-core kernels are tested against it.  It stands where the reference runs
+// paged_mha_kernel.cu:363-550 (decode) and paged_mha_prefill_kernel.cu:120-237,368-520 (prompt
+// portions): s_j = (q.k_j) * scale, online softmax with running maximum and sum, o = acc / l.
 //
 // Compile with -DPBE_HEAD_DIM=<multiple of 16>.
 #include "attention_params.cuh"
